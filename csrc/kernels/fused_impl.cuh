@@ -79,7 +79,7 @@ struct FusedComm {
     int phases;              // Phase bits
     unsigned long long timeout_ns;
     int* status;             // int[4] local
-    int* ctrl;               // int[C_WORDS] local, zero at launch
+    int* ctrl;               // int[C_WORDS] local, zero between launches
     int* pad;                // my signal pad, int[F_KINDS][MAX_RANKS], indexed by source rank
     int* const* peer_pad;    // [world] every rank's pad as mapped into this process
     const int* read_from;    // ranks whose memory I read
@@ -106,7 +106,7 @@ __device__ __forceinline__ int warp_ticket(int* ctr, int lane, int n = 1) {
 
 // Work per ticket: large enough to keep the counter quiet, small enough that the last tickets (the tail of
 // the kernel, when other warps already idle) are short: about 1/32 of a warp's share, at most MAX.
-constexpr int SDDMM_UNITS_PER_TICKET_MAX = 8;
+constexpr int SDDMM_WINDOWS_PER_TICKET_MAX = 8;
 constexpr int SPMM_ITEMS_PER_TICKET_MAX = 4;
 
 
@@ -393,6 +393,12 @@ struct PullGate {
     }
 };
 
+// The control words are zero between launches: the last warp to be done with a launch clears them (a memset before
+// every launch cost 1 us of stream time and a second launch).
+__device__ __forceinline__ void clear_ctrl(const FusedComm& c, int lane) {
+    for (int i = lane; i < C_WORDS; i += 32) c.ctrl[i] = 0;
+}
+
 // Every warp calls this after its MAIN work; the last one to arrive publishes
 // DONE and PART for this rank.
 __device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane, int nwarps) {
@@ -413,6 +419,7 @@ __device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane, int 
         for (int i = lane; i < c.n_read; i += 32) signal(c, F_DONE, c.read_from[i]);
         for (int i = lane; i < c.n_push; i += 32) signal(c, F_PART, c.push_to[i]);
         if (lane == 0) stamp(c, T_MAIN);
+        if (!(c.phases & PH_FINISH)) clear_ctrl(c, lane);
     }
 }
 
@@ -423,9 +430,13 @@ __device__ __forceinline__ void finish_epilogue(const FusedComm& c, int lane, in
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_FIN_DONE, 1);
     old = __shfl_sync(0xffffffffu, old, 0);
-    if (old == nwarps - 1 && lane == 0) {
-        wait_all(c, F_DONE, c.readers, c.n_readers, W_DONE);
-        stamp(c, T_FINISH);
+    if (old == nwarps - 1) {
+        if (lane == 0) {
+            wait_all(c, F_DONE, c.readers, c.n_readers, W_DONE);
+            stamp(c, T_FINISH);
+        }
+        __syncwarp();
+        clear_ctrl(c, lane);
     }
 }
 
@@ -529,9 +540,9 @@ struct StorePartial {
     int direct, Z, my_z, parity;
     unsigned zbase, zrem;
     long long zwidth;
-    __device__ __forceinline__ void operator()(long long i, real dot) const {
+    __device__ __forceinline__ real scale(long long i) const { return __ldg(sval + i); }
+    __device__ __forceinline__ void put(long long i, real v) const {
         const unsigned ii = orig ? (unsigned)__ldg(orig + i) : (unsigned)i;
-        const real v = dot * __ldg(sval + i);
         if (!direct) { dst[ii] = v; return; }
         // direct mode (wide rows: a lane group stores >= 32 contiguous bytes): straight into the owner's buffer
         const unsigned split = zrem * (zbase + 1);
@@ -547,7 +558,7 @@ __device__ __forceinline__ long long slice_off(int z, unsigned zbase, unsigned z
     return (long long)z * zbase + ((unsigned)z < zrem ? z : (int)zrem);
 }
 
-template <int G, int R, int U>
+template <int G, int R>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(const FusedSddmmArgs a) {
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
@@ -569,9 +580,10 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
         // pull tickets: tiles of needed A rows first (when A rows are staged), then tiles of needed B rows
         const int n_pull_a = (a.n_recv_a + PULL_ROWS - 1) / PULL_ROWS;
         const int n_pull = n_pull_a + (a.n_recv_b + PULL_ROWS - 1) / PULL_ROWS;
-        const long long per_unit = (long long)SLOTS * SDDMM_PER_SLOT;
+        const int per_unit = window_nnz(a.nnz, nwarps, SLOTS);   // nonzeros of a work unit
         const long long n_units = (a.nnz + per_unit - 1) / per_unit;
-        const RowsByPeerRef<real> arows{a.a_refs, a_bases, (unsigned long long)a.nvec * 16ull, c.me << PEER_REF_SHIFT};
+        const bool aligned = ((unsigned long long)a.rowidx | (unsigned long long)a.colidx) % 16 == 0;
+        const RowsByPeerRef arows{a.a_refs, a_bases, (unsigned)a.nvec * 16u, c.me << PEER_REF_SHIFT};
         const int direct = a.Z > 1 && a.direct_push == 1;
         const bool self_push = a.Z > 1 && a.direct_push == 2 && a.orig == nullptr;
         const bool in_switch = a.Z > 1 && a.direct_push == 3;
@@ -610,16 +622,16 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
         // The pullers serve pull tickets until none are left while the others start on the units that need no
         // pulled row.
         if (is_puller && ok) gate.pull_all(lane);
-        const int SDDMM_UNITS_PER_TICKET = per_ticket(n_units, nwarps, SDDMM_UNITS_PER_TICKET_MAX);
+        const int UNITS_PER_TICKET = per_ticket(n_units, nwarps, SDDMM_WINDOWS_PER_TICKET_MAX);
         while (ok) {
-            const long long u0 = (long long)warp_ticket(c.ctrl + C_TICKET_WORK, lane, SDDMM_UNITS_PER_TICKET);
+            const long long u0 = (long long)warp_ticket(c.ctrl + C_TICKET_WORK, lane, UNITS_PER_TICKET);
             if (u0 >= n_units) break;
-            const long long u1 = u0 + SDDMM_UNITS_PER_TICKET < n_units ? u0 + SDDMM_UNITS_PER_TICKET : n_units;
+            const long long u1 = u0 + UNITS_PER_TICKET < n_units ? u0 + UNITS_PER_TICKET : n_units;
             ok = gate.ensure(u1, lane);
             if (!ok) break;
-            for (long long u = u0; u < u1; ++u)
-                sddmm_warp_unit<real, G, R, U, RowsByPeerRef<real>, StorePartial, false>(
-                    u, a.nnz, a.rowidx, a.colidx, arows, Bv, ldb_v, a.nvec, store, lane);
+            sddmm_windows<real, 16, G, R, sddmm_unroll(R), false, false>(
+                u0, 1, u1, per_unit, a.nnz, a.rowidx, a.colidx, arows, reinterpret_cast<const char*>(Bv),
+                (unsigned)ldb_v * 16u, a.nvec, aligned, store, lane);
             if (self_push) {
                 // the values [i0, i1) of `part` were written by this warp just now (still in L2): send the pieces
                 // that belong to other fiber ranks as contiguous remote stores while other warps compute
@@ -736,6 +748,7 @@ struct FusedSpmmArgs {
     FusedComm comm;
     int nitems;
     const int4* items;
+    int n_rows;                   // rows of the local block (rowptr has one more)
     const long long* rowptr;
     const int* colidx;
     const real* val;
@@ -777,6 +790,15 @@ struct FusedSpmmArgs {
     const int* pull_order;
 };
 
+__device__ __forceinline__ vec as_vec(const Row<real, 16>& r) {
+#if SP3_FUSED_IS_F32
+    const float2 a = unpack2(r.x[0]), b = unpack2(r.x[1]);
+    return make_float4(a.x, a.y, b.x, b.y);
+#else
+    return make_double2(r.x[0], r.x[1]);
+#endif
+}
+
 // Rows I own go straight into the result (Y = beta*Y + my partial; the owners' FINISH phase then adds what
 // the peers pushed); rows I do not own are pushed into their slot at the owner.
 struct EmitOwnedOrPush {
@@ -786,7 +808,8 @@ struct EmitOwnedOrPush {
     int n_owned;
     vec* const* y_dst;
     long long parity_off_v;
-    __device__ __forceinline__ void operator()(int row, int v, const vec& acc) const {
+    __device__ __forceinline__ void operator()(int row, int v, const Row<real, 16>& sum) const {
+        const vec acc = as_vec(sum);
         if (row < n_owned) {
             vec* y = Yv + (long long)row * ldy_v + v;
             if (beta != (real)0) { vec o = vscale(beta, *y); vadd(o, acc); *y = o; }
@@ -804,7 +827,8 @@ struct EmitOwnedOrAdd {
     vec* const* y_dst;
     const unsigned char* crow_flag;
     int red_v4;
-    __device__ __forceinline__ void operator()(int row, int v, const vec& acc) const {
+    __device__ __forceinline__ void operator()(int row, int v, const Row<real, 16>& sum) const {
+        const vec acc = as_vec(sum);
         if (row < n_owned) {
             vec* y = Yv + (long long)row * ldy_v + v;
             if (__ldg(crow_flag + row)) vatomic_add(y, acc, true);  // beta was applied in the START phase
@@ -817,20 +841,21 @@ struct EmitOwnedOrAdd {
     }
 };
 
-// Four resident blocks per SM (64 registers per thread) as long as a lane holds at most two vectors of a row:
-// left to itself the compiler takes 128 registers for the wave bookkeeping and halves the occupancy, which costs
-// the gather-bound inner loop far more than the few spills do.
+// Resident blocks per SM as in the local kernel: left to itself the compiler takes 128 registers for the wave
+// bookkeeping and halves the occupancy, which costs the gather-bound inner loop far more than the few spills do.
 // GATED: the items follow the pull waves (wave_items given).  The other form pulls everything first and carries
 // no wave state: its inner loop keeps all 64 registers of a thread, which is worth 10-15 % on blocks that pull
 // nothing or little (meshes 1 x Y x Z).
-template <int G, int R, int U, bool ATOMIC, bool GATED>
-__global__ void __launch_bounds__(256, (R <= 2 ? 4 : 2)) fused_spmm_kernel(const FusedSpmmArgs a) {
+template <int G, int R, bool ATOMIC, bool GATED>
+__global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(const FusedSpmmArgs a) {
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
     const int parity = c.epoch & 1;
     extern __shared__ __align__(128) unsigned char dyn_smem[];   // bulk mode: the pullers' rings, else nothing
     __shared__ long long wave_limit[MAX_WAVES + 1];
+    __shared__ int row_ends[256 / 32][SPMM_ENDS];
+    int* ends = row_ends[threadIdx.x >> 5];
     const bool bulk = a.pull.pullers > 0;
     const int PULL_ROWS = a.pull.tile_rows;
     BulkRing br = bulk_ring_init(dyn_smem, a.pull, threadIdx.x >> 5, lane);
@@ -862,6 +887,7 @@ __global__ void __launch_bounds__(256, (R <= 2 ? 4 : 2)) fused_spmm_kernel(const
             __threadfence_system();
             for (int i = lane; i < c.n_readers; i += 32) signal(c, F_READY, c.readers[i]);
             for (int i = lane; i < c.n_contrib; i += 32) signal(c, F_READY, c.contrib[i]);
+            if (!(c.phases & (PH_MAIN | PH_FINISH))) clear_ctrl(c, lane);
         }
     }
     if (c.phases & PH_MAIN) {
@@ -874,6 +900,10 @@ __global__ void __launch_bounds__(256, (R <= 2 ? 4 : 2)) fused_spmm_kernel(const
         const int n_pull = (a.n_recv_x + PULL_ROWS - 1) / PULL_ROWS;
         vec* Xv = reinterpret_cast<vec*>(a.X_loc);
         const long long ldx_v = a.ldx / VN;
+        const char* Xb = reinterpret_cast<const char*>(Xv);
+        const unsigned ldx_bytes = (unsigned)ldx_v * 16u;
+        const bool aligned = ((unsigned long long)a.colidx | (unsigned long long)a.val) % 16 == 0;
+        const long long nnz = __ldg(a.rowptr + a.n_rows);
         const EmitOwnedOrPush emit{reinterpret_cast<vec*>(a.Y), a.ldy / VN, (real)a.beta, a.n_owned_y, a.y_dst,
                                    parity ? a.parity_off_v : 0};
         if constexpr (!GATED) {
@@ -905,12 +935,12 @@ __global__ void __launch_bounds__(256, (R <= 2 ? 4 : 2)) fused_spmm_kernel(const
                     const EmitOwnedOrAdd add{reinterpret_cast<vec*>(a.Y), a.ldy / VN, (real)a.beta, a.n_owned_y, a.y_dst,
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, G, R, U, EmitOwnedOrAdd, false>(__ldg(a.items + it), a.rowptr, a.colidx, a.val,
-                                                                              Xv, ldx_v, a.nvec, add, a.lg, lane);
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, G, R, U, EmitOwnedOrPush, false>(__ldg(a.items + it), a.rowptr, a.colidx, a.val,
-                                                                               Xv, ldx_v, a.nvec, emit, a.lg, lane);
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
                 }
             }
         } else {
@@ -952,12 +982,12 @@ __global__ void __launch_bounds__(256, (R <= 2 ? 4 : 2)) fused_spmm_kernel(const
                     const EmitOwnedOrAdd add{reinterpret_cast<vec*>(a.Y), a.ldy / VN, (real)a.beta, a.n_owned_y, a.y_dst,
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, G, R, U, EmitOwnedOrAdd, false>(__ldg(a.items + it), a.rowptr, a.colidx, a.val,
-                                                                              Xv, ldx_v, a.nvec, add, a.lg, lane);
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, G, R, U, EmitOwnedOrPush, false>(__ldg(a.items + it), a.rowptr, a.colidx, a.val,
-                                                                               Xv, ldx_v, a.nvec, emit, a.lg, lane);
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
                 }
             }
             if (ok) gate.pull_all(lane);  // no item left but tiles remain (tiny blocks)
@@ -1035,9 +1065,10 @@ SP3_API int sp3_fused_struct_sizes(int* sddmm_bytes, int* spmm_bytes, int* comm_
 // The kernels synchronise their own warps through grid-wide counters, so every block of the grid has to be
 // resident at once.  A cooperative launch gives that guarantee: the grid is sized from the occupancy query and
 // the launch fails with an error (instead of a kernel that waits for blocks that never start) if the device
-// cannot hold it.
+// cannot hold it.  `needed`: blocks that find work; a phase launched alone, or a small block of the matrix, needs
+// fewer than fit.
 template <typename K, typename A>
-static int launch_resident(K kernel, const A& args, cudaStream_t st) {
+static int launch_resident(K kernel, ResidentCache& cache, const A& args, long long needed, cudaStream_t st) {
     A copy = args;
     void* params[] = {&copy};
     if (args.pull.pullers < 0 || args.pull.pullers > BULK_MAX_PULLERS || args.pull.tile_rows < 1 ||
@@ -1048,8 +1079,18 @@ static int launch_resident(K kernel, const A& args, cudaStream_t st) {
         cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    const unsigned blocks = persistent_blocks(kernel, 0, 256, smem);
+    const unsigned blocks = resident_blocks(kernel, cache, needed, 256, smem);
     return (int)cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(256), params, smem, st);
+}
+
+// Blocks with work for the phases of a launch, from the number of independent pieces (one per warp) of MAIN, FINISH
+// and START.
+static long long blocks_needed(int phases, long long main_pieces, long long finish_pieces, long long start_pieces) {
+    long long n = 1;
+    if ((phases & PH_START) && start_pieces > n) n = start_pieces;
+    if ((phases & PH_MAIN) && main_pieces > n) n = main_pieces;
+    if ((phases & PH_FINISH) && finish_pieces > n) n = finish_pieces;
+    return (n + 7) / 8;
 }
 
 #define SP3_FUSED_CAT2(a, b) a##b
@@ -1062,12 +1103,15 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_sddmm_, SP3_FUSED_SUFFIX)(const void* args, 
 #if !SP3_FUSED_IS_F32
     if (a.direct_push == 3) return (int)cudaErrorInvalidValue;   // the in-switch reduction is built for fp32 only
 #endif
-    cudaError_t e = cudaMemsetAsync(a.comm.ctrl, 0, C_WORDS * sizeof(int), st);
-    if (e != cudaSuccess) return (int)e;
     int G, R, rc = 0;
     pick_shape(a.nvec, &G, &R, false);
-#define SP3_FSDDMM(GG, RR) rc = launch_resident(fused_sddmm_kernel<GG, RR, (RR >= 8 ? 2 : 4)>, a, st)
-    SP3_DISPATCH_GR(SP3_FSDDMM)
+    const long long slice = a.zbase + (a.zrem ? 1 : 0);
+    const long long fin = a.Z > 1 ? (slice + REDUCE_ELEMS - 1) / REDUCE_ELEMS : 1;
+    const long long units = (a.nnz + 4 * (32 / G) - 1) / (4 * (32 / G));
+    const long long pulls = ((long long)a.n_recv_a + a.n_recv_b + a.pull.tile_rows - 1) / a.pull.tile_rows + 1;
+    const long long needed = blocks_needed(a.comm.phases, units > pulls ? units : pulls, fin, 1);
+#define SP3_FSDDMM(GG, RR) { static ResidentCache cache; rc = launch_resident(fused_sddmm_kernel<GG, RR>, cache, a, needed, st); }
+    SP3_SDDMM_SHAPES(SP3_FSDDMM)
 #undef SP3_FSDDMM
     return rc ? rc : (int)cudaGetLastError();
 }
@@ -1076,18 +1120,20 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_spmm_, SP3_FUSED_SUFFIX)(const void* args, v
     FusedSpmmArgs a = *reinterpret_cast<const FusedSpmmArgs*>(args);
     cudaStream_t st = (cudaStream_t)stream;
     if (a.n_waves > MAX_WAVES) return (int)cudaErrorInvalidValue;
-    cudaError_t e = cudaMemsetAsync(a.comm.ctrl, 0, C_WORDS * sizeof(int), st);
-    if (e != cudaSuccess) return (int)e;
     int G, R, rc = 0;
     pick_shape(a.nvec, &G, &R, true);
     const bool gated = a.wave_items != nullptr && a.n_waves > 0 && a.n_recv_x > 0;
-#define SP3_FSPMM(GG, RR)                                                                        \
-    rc = a.atomic ? (gated ? launch_resident(fused_spmm_kernel<GG, RR, (RR >= 8 ? 2 : 4), true, true>, a, st)     \
-                           : launch_resident(fused_spmm_kernel<GG, RR, (RR >= 8 ? 2 : 4), true, false>, a, st))   \
-                  : (gated ? launch_resident(fused_spmm_kernel<GG, RR, (RR >= 8 ? 2 : 4), false, true>, a, st)    \
-                           : launch_resident(fused_spmm_kernel<GG, RR, (RR >= 8 ? 2 : 4), false, false>, a, st))
-    SP3_DISPATCH_GR(SP3_FSPMM)
+    const long long rows = ((long long)a.n_crows + REDUCE_ROWS - 1) / REDUCE_ROWS;
+    const long long pulls = ((long long)a.n_recv_x + a.pull.tile_rows - 1) / a.pull.tile_rows + 1;
+    const long long needed = blocks_needed(a.comm.phases, a.nitems > pulls ? a.nitems : pulls, a.atomic ? 1 : rows,
+                                           a.atomic ? rows : 1);
+#define SP3_FSPMM_ONE(GG, RR, AT, GA) { static ResidentCache cache; rc = launch_resident(fused_spmm_kernel<GG, RR, AT, GA>, cache, a, needed, st); }
+#define SP3_FSPMM(GG, RR)                                                                          \
+    if (a.atomic) { if (gated) SP3_FSPMM_ONE(GG, RR, true, true) else SP3_FSPMM_ONE(GG, RR, true, false) }      \
+    else { if (gated) SP3_FSPMM_ONE(GG, RR, false, true) else SP3_FSPMM_ONE(GG, RR, false, false) }
+    SP3_SPMM_SHAPES(SP3_FSPMM)
 #undef SP3_FSPMM
+#undef SP3_FSPMM_ONE
     return rc ? rc : (int)cudaGetLastError();
 }
 

@@ -7,12 +7,8 @@
 // ReMapIndices src/SparseMatrix.hpp:100-106, checksum
 // miniapp/bench_spmm.cpp:117.
 //
-// Layout of the math: a dense row of k elements is spread over a group of G
-// lanes (G = power of two <= 32), each lane holding R 16-byte vectors, so one
-// warp works on 32/G nonzeros (SDDMM) or rows (SpMM) at a time and every
-// global access is a full-width vector load of a contiguous row segment.
-// Both kernels are bound by the gathers of dense rows from HBM/L2; the
-// unroll factor U keeps U independent row loads in flight per lane.
+// The inner loops are in sp3_kernels.cuh.  Both kernels are bound by the gathers
+// of dense rows from HBM/L2.
 #include "sp3_kernels.cuh"
 
 #include <cstdlib>
@@ -21,26 +17,20 @@ namespace sp3 {
 
 // ---------------------------------------------------------------------------
 // SDDMM: out[i] = sval[i] * <A[rowidx[i]], B[colidx[i]]>; persistent grid,
-// warps stride over work units (see sddmm_warp_unit).
+// warps stride over windows of nonzeros (see sddmm_windows).
 // ---------------------------------------------------------------------------
-template <typename T, int G, int R, int U>
+template <typename T, int NB, int G, int R, bool EXACT, typename Store>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R))
-sddmm_vec_kernel(long long nnz, const int* __restrict__ rowidx, const int* __restrict__ colidx,
-                 const T* __restrict__ sval, const T* __restrict__ A, long long lda,
-                 const T* __restrict__ B, long long ldb, int nvec, T* __restrict__ out, const int* __restrict__ orig) {
-    using V = typename Vec<T>::type;
-    constexpr int SLOTS = 32 / G;
+sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
+                 const RowsByStride arows, const char* __restrict__ B, unsigned ldb_bytes, int nvec, bool aligned,
+                 const Store store) {
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const RowsByStride<T> arows{reinterpret_cast<const V*>(A), lda / Vec<T>::N};
-    const StoreLocal<T> store{out, sval, orig};
-    for (long long unit = warp0; unit * SLOTS * (long long)SDDMM_PER_SLOT < nnz; unit += nwarps)
-        sddmm_warp_unit<T, G, R, U>(unit, nnz, rowidx, colidx, arows, reinterpret_cast<const V*>(B),
-                                    ldb / Vec<T>::N, nvec, store, lane);
+    sddmm_windows<T, NB, G, R, sddmm_unroll(R), EXACT, true>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
+                                                      arows, B, ldb_bytes, nvec, aligned, store, threadIdx.x & 31);
 }
 
-// Any k, any leading dimension: one warp per nonzero slot, scalar loads.
+// Rows of more than 256 vectors: one warp per nonzero, scalar loads.
 template <typename T>
 __global__ void __launch_bounds__(256)
 sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __restrict__ colidx,
@@ -65,42 +55,42 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // Rows without nonzeros are covered by rows items, so beta is applied to
 // every row exactly once.
 // ---------------------------------------------------------------------------
-#ifndef SP3_SPMM_ITEMS_PER_STEP
-#define SP3_SPMM_ITEMS_PER_STEP 4
-#endif
-constexpr int SPMM_ITEMS_PER_STEP = SP3_SPMM_ITEMS_PER_STEP;
-
-template <typename T, int G, int R, int U>
-__global__ void __launch_bounds__(256)
-spmm_items_kernel(int nitems, const int4* __restrict__ items, const long long* __restrict__ rowptr,
-                  const int* __restrict__ colidx, const T* __restrict__ val, const T* __restrict__ X,
-                  long long ldx, int nvec, T beta, T* __restrict__ Y, long long ldy, SpmmLong lg) {
-    using V = typename Vec<T>::type;
+template <typename T, int NB, int G, int R, bool EXACT>
+__global__ void __launch_bounds__(256, spmm_min_blocks(R))
+spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
+                  const int* __restrict__ colidx, const T* __restrict__ val, const char* __restrict__ X,
+                  unsigned ldx_bytes, int nvec, bool aligned, const EmitLocal<T, NB> emit, const SpmmLong lg) {
+    __shared__ int row_ends[256 / 32][SPMM_ENDS];
+    int* ends = row_ends[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
     const int warp0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    const EmitLocal<T> emit{reinterpret_cast<V*>(Y), ldy / Vec<T>::N, beta};
-    if (lg.ticket) {
-        // dynamic hand-out, SPMM_ITEMS_PER_STEP items per ticket: rows of a power-law matrix differ too much in
-        // cost for a fixed assignment to balance
-        const int step = per_ticket(nitems, nwarps, SPMM_ITEMS_PER_STEP);
+    const long long nnz = __ldg(rowptr + nrows);
+    auto run = [&](int it) {
+        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT, true>(__ldg(items + it), rowptr, nnz, colidx, val, X, ldx_bytes,
+                                                                 nvec, aligned, emit, lg, ends, lane);
+    };
+    if (lg.ticket && nitems > nwarps) {
+        // dynamic hand-out: items differ too much in cost (cached or not, hub or not) for a fixed assignment to balance
         for (;;) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(lg.ticket, step);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= nitems) break;
-            for (int it = base; it < base + step && it < nitems; ++it)
-                spmm_warp_item<T, G, R, U>(__ldg(items + it), rowptr, colidx, val, reinterpret_cast<const V*>(X),
-                                           ldx / Vec<T>::N, nvec, emit, lg, lane);
+            int it = 0;
+            if (lane == 0) it = atomicAdd(lg.ticket, 1);
+            it = __shfl_sync(0xffffffffu, it, 0);
+            if (it >= nitems) break;
+            run(it);
+        }
+        // the last block to finish leaves the counters at zero for the next launch (no memset per launch)
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(lg.ticket + 1, 1) == (int)gridDim.x - 1) {
+            lg.ticket[0] = 0;
+            lg.ticket[1] = 0;
         }
         return;
     }
-    for (int it = warp0; it < nitems; it += nwarps)
-        spmm_warp_item<T, G, R, U>(__ldg(items + it), rowptr, colidx, val, reinterpret_cast<const V*>(X),
-                                   ldx / Vec<T>::N, nvec, emit, lg, lane);
+    for (int it = warp0; it < nitems; it += nwarps) run(it);
 }
 
-// Any k / leading dimension: one warp per row, scalar loads, no schedule.
+// Rows of more than 256 vectors, or no work items: one warp per row, scalar loads.
 template <typename T>
 __global__ void __launch_bounds__(256)
 spmm_scalar_kernel(int nrows, const long long* __restrict__ rowptr, const int* __restrict__ colidx,
@@ -250,30 +240,86 @@ __global__ void check_range_kernel(long long n, const int* __restrict__ idx, int
 }
 
 // ---- dispatch ---------------------------------------------------------------
+// Widest vector, in bytes, that rows of `bytes` bytes can be cut into when all of `bits` (addresses and strides
+// or-ed together) have to be multiples of it.  Rows of fewer than four 16-byte vectors take narrower ones as long
+// as that fills more of the four lanes of the smallest group.
+template <typename T> int vector_bytes(unsigned long long bytes, unsigned long long bits) {
+    int nb = 16;
+    while (nb > (int)sizeof(T) && ((bytes | bits) % nb != 0 || bytes / nb <= 2)) nb >>= 1;
+    return nb;
+}
+
+template <typename T, int NB, typename Store>
+int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, long long lda_bytes, const char* B,
+                    long long ldb_bytes, int nvec, const Store& store, cudaStream_t st) {
+    const bool aligned = ((uintptr_t)ri | (uintptr_t)ci) % 16 == 0;
+    const RowsByStride arows{A, (unsigned)lda_bytes};
+    int G, R;
+    pick_shape(nvec, &G, &R, false);
+    const bool exact = NB == 16 && nvec == G * R;
+#define SP3_SDDMM(GG, RR)                                                                                     \
+    {                                                                                                         \
+        static ResidentCache caches[2];                                                                       \
+        ResidentCache& cache = caches[exact];                                                                 \
+        auto kernel = exact ? sddmm_vec_kernel<T, NB, GG, RR, NB == 16, Store>                                \
+                            : sddmm_vec_kernel<T, NB, GG, RR, false, Store>;                                  \
+        const unsigned all = resident_blocks(kernel, cache, 0);                                               \
+        const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
+        const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
+        kernel<<<needed < all ? (unsigned)needed : all, 256, 0, st>>>(nnz, wn, ri, ci, arows, B,              \
+                                                                      (unsigned)ldb_bytes, nvec, aligned, store); \
+    }
+    SP3_SDDMM_SHAPES(SP3_SDDMM)
+#undef SP3_SDDMM
+    return (int)cudaGetLastError();
+}
+
 template <typename T>
 int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const T* A, long long lda, const T* B,
                  long long ldb, int k, T* out, cudaStream_t st, const int* orig = nullptr) {
     if (nnz == 0) return 0;
-    constexpr int VN = Vec<T>::N;
-    const bool vec_ok = k % VN == 0 && lda % VN == 0 && ldb % VN == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)B % 16 == 0;
-    const int nvec = k / VN;
-    if (!vec_ok || nvec > 256) {
+    const long long lda_b = lda * (long long)sizeof(T), ldb_b = ldb * (long long)sizeof(T);
+    const unsigned long long bytes = (unsigned long long)k * sizeof(T);
+    const int nb = vector_bytes<T>(bytes, lda_b | ldb_b | (uintptr_t)A | (uintptr_t)B);
+    const unsigned long long nvec = bytes / nb;
+    if (nvec > 256 || nvec == 0 || lda_b >= 1ll << 32 || ldb_b >= 1ll << 32) {
         if (orig) return -1;  // the scatter form exists for the vector kernel only
         long long warps = nnz < (1ll << 22) ? nnz : (1ll << 22);
         sddmm_scalar_kernel<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(nnz, ri, ci, sv, A, lda, B, ldb, k, out);
         return (int)cudaGetLastError();
     }
+    const StoreLocal<T> store{out, sv};
+    const char *a = reinterpret_cast<const char*>(A), *b = reinterpret_cast<const char*>(B);
+    if (orig) {
+        if (nb != 16) return -1;
+        return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, StoreScattered<T>{out, sv, orig}, st);
+    }
+    if (nb == 16) return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
+    if (nb == 8) return launch_sddmm_nb<T, 8>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
+    if constexpr (sizeof(T) == 4) return launch_sddmm_nb<T, 4>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
+    return -1;
+}
+
+template <typename T, int NB>
+int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
+                   const char* X, long long ldx_bytes, int nvec, T beta, char* Y, long long ldy_bytes,
+                   const SpmmLong& lg, cudaStream_t st) {
+    const bool aligned = ((uintptr_t)ci | (uintptr_t)val) % 16 == 0;
+    const EmitLocal<T, NB> emit{Y, ldy_bytes, beta};
     int G, R;
-    pick_shape(nvec, &G, &R, false);
-    const long long slots = (nnz + SDDMM_PER_SLOT - 1) / SDDMM_PER_SLOT;
-    const long long warps = (slots + (32 / G) - 1) / (32 / G);
-    const long long needed = (warps + 7) / 8;
-#define SP3_SDDMM(GG, RR)                                                                                      \
-    sddmm_vec_kernel<T, GG, RR, (RR >= 8 ? 2 : 4)>                                                             \
-        <<<persistent_blocks(sddmm_vec_kernel<T, GG, RR, (RR >= 8 ? 2 : 4)>, needed), 256, 0, st>>>(           \
-            nnz, ri, ci, sv, A, lda, B, ldb, nvec, out, orig)
-    SP3_DISPATCH_GR(SP3_SDDMM)
-#undef SP3_SDDMM
+    pick_shape(nvec, &G, &R, true);
+    const bool exact = NB == 16 && nvec == G * R;
+    const long long needed = ((long long)nitems + 7) / 8;
+#define SP3_SPMM(GG, RR)                                                                                      \
+    {                                                                                                         \
+        static ResidentCache caches[2];                                                                       \
+        ResidentCache& cache = caches[exact];                                                                 \
+        auto kernel = exact ? spmm_items_kernel<T, NB, GG, RR, NB == 16> : spmm_items_kernel<T, NB, GG, RR, false>; \
+        kernel<<<resident_blocks(kernel, cache, needed), 256, 0, st>>>(nitems, items, nrows, rowptr, ci, val, X, \
+                                                                       (unsigned)ldx_bytes, nvec, aligned, emit, lg); \
+    }
+    SP3_SPMM_SHAPES(SP3_SPMM)
+#undef SP3_SPMM
     return (int)cudaGetLastError();
 }
 
@@ -281,28 +327,22 @@ template <typename T>
 int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
                 const T* X, long long ldx, int k, T beta, T* Y, long long ldy, SpmmLong lg, cudaStream_t st) {
     if (nrows == 0) return 0;
-    constexpr int VN = Vec<T>::N;
-    const bool vec_ok = k % VN == 0 && ldx % VN == 0 && ldy % VN == 0 && (uintptr_t)X % 16 == 0 &&
-                        (uintptr_t)Y % 16 == 0 && items != nullptr && (lg.ldc % VN == 0);
-    const int nvec = k / VN;
-    if (!vec_ok || nvec > 256) {
+    const long long ldx_b = ldx * (long long)sizeof(T), ldy_b = ldy * (long long)sizeof(T);
+    unsigned long long bits = ldx_b | ldy_b | (uintptr_t)X | (uintptr_t)Y;
+    if (lg.carry) bits |= (uintptr_t)lg.carry | (unsigned long long)lg.ldc * sizeof(T);
+    const unsigned long long bytes = (unsigned long long)k * sizeof(T);
+    const int nb = vector_bytes<T>(bytes, bits);
+    const unsigned long long nvec = bytes / nb;
+    if (items == nullptr || nvec > 256 || nvec == 0 || ldx_b >= 1ll << 32) {
         spmm_scalar_kernel<T><<<(unsigned)(((long long)nrows * 32 + 255) / 256), 256, 0, st>>>(nrows, rowptr, ci, val, X, ldx, k, beta, Y, ldy);
         return (int)cudaGetLastError();
     }
-    int G, R;
-    pick_shape(nvec, &G, &R, true);
-    if (lg.ticket) {
-        cudaError_t e = cudaMemsetAsync(lg.ticket, 0, sizeof(int), st);
-        if (e != cudaSuccess) return (int)e;
-    }
-    const long long needed = ((long long)nitems + 7) / 8;
-#define SP3_SPMM(GG, RR)                                                                                       \
-    spmm_items_kernel<T, GG, RR, (RR >= 8 ? 2 : 4)>                                                            \
-        <<<persistent_blocks(spmm_items_kernel<T, GG, RR, (RR >= 8 ? 2 : 4)>, needed), 256, 0, st>>>(          \
-            nitems, items, rowptr, ci, val, X, ldx, nvec, beta, Y, ldy, lg)
-    SP3_DISPATCH_GR(SP3_SPMM)
-#undef SP3_SPMM
-    return (int)cudaGetLastError();
+    const char* x = reinterpret_cast<const char*>(X);
+    char* y = reinterpret_cast<char*>(Y);
+    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
+    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
+    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
+    return -1;
 }
 
 template <typename T>

@@ -9,184 +9,328 @@
 //   SpMM    emit:    EmitLocal (Y = beta*Y + acc) | the fused kernel's
 //                    owned-or-push emit
 //
+// Layout of the math: a dense row is cut into vectors of NB bytes (16, 8 or 4:
+// the widest that the width and the alignment of the operands allow); a group
+// of G lanes holds R vectors per lane, and the 32/G groups of a warp work on
+// different nonzeros.  Column indices and values are taken four at a time.
+//
 // Reference loops: src/core_ops.cpp:5-35.
 #pragma once
 #include "sp3_cuda.cuh"
 
+#include <atomic>
+#include <cstdlib>
+
 namespace sp3 {
-
-constexpr int SDDMM_PER_SLOT = 32;  // nonzeros per lane group; multiple of every G
-
-// Tuning knobs (compile time): resident 256-thread blocks per SM the SDDMM
-// kernels are compiled for, and whether the loop over the sub-batches of an
-// index batch is unrolled (more loads in flight per warp, more registers).
-#ifndef SP3_SDDMM_MINB
-#define SP3_SDDMM_MINB 4
-#endif
-// With more than two vectors per lane the row registers alone need the larger budget of two blocks per SM.
-constexpr int sddmm_min_blocks(int R) { return R <= 2 ? SP3_SDDMM_MINB : 2; }
-#ifndef SP3_SDDMM_UNROLL_BATCH
-#define SP3_SDDMM_UNROLL_BATCH 1
-#endif
 
 template <int G> __device__ __forceinline__ unsigned group_mask(int slot) {
     return G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (slot * G));
 }
 
-// Sums N values per lane across a group of G lanes with a halving butterfly:
-// at each step a lane keeps one half of its values and hands the other half
-// to its partner, so the whole reduction costs N-1 + log2(G/N) shuffles instead
-// of N*log2(G).  N <= G, both powers of two.  On return v[0] of lane gl holds
-// the group total of value number gl / (G/N).
-template <typename T, int G, int N>
-__device__ __forceinline__ void group_transpose_reduce(T (&v)[N], unsigned gmask, int gl) {
-    int n = N;
-#pragma unroll
-    for (int m = G / 2; m > 0; m >>= 1) {
-        if (n > 1) {
-            const int half = n >> 1;
-            const bool upper = (gl & m) != 0;
-#pragma unroll
-            for (int t = 0; t < N / 2; ++t) {
-                if (t < half) {
-                    const T send = upper ? v[t] : v[t + half];
-                    const T keep = upper ? v[t + half] : v[t];
-                    v[t] = keep + __shfl_xor_sync(gmask, send, m, G);
-                }
-            }
-            n = half;
-        } else {
-            v[0] += __shfl_xor_sync(gmask, v[0], m, G);
-        }
-    }
-}
+// ---- a lane's vector of a dense row ------------------------------------------
+// fp32 vectors of 8 and 16 bytes keep their values as pairs in 64-bit registers and use the packed
+// multiply-add of sm_100 (`fma.rn.f32x2`: two fp32 products per instruction, each rounded like `fmaf`).
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pack2(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 unpack2(u64 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 
-// ---- dense-row loads ----------------------------------------------------------
+template <typename T, int NB> struct Row;
+template <> struct Row<float, 16> { using E = u64; static constexpr int N = 2; E x[2]; };
+template <> struct Row<float, 8> { using E = u64; static constexpr int N = 1; E x[1]; };
+template <> struct Row<float, 4> { using E = float; static constexpr int N = 1; E x[1]; };
+template <> struct Row<double, 16> { using E = double; static constexpr int N = 2; E x[2]; };
+template <> struct Row<double, 8> { using E = double; static constexpr int N = 1; E x[1]; };
+
 // NC = true: the non-coherent read-only path (ld.global.nc), for operands that no thread writes while the
 // kernel runs (the local kernels).  NC = false: an ordinary load.  The fused kernels use it for every dense
 // row, because rows of the pulled part of a block are written by other warps of the same launch; ordinary
 // loads are ordered after the acquire that tells a warp the rows are there, the read-only path is not.
-template <bool NC, typename V> __device__ __forceinline__ V ld_row(const V* p) {
-    if constexpr (NC) return __ldg(p);
-    else return *p;
+template <bool NC, typename T, int NB> __device__ __forceinline__ void row_load(Row<T, NB>& v, const char* p) {
+    using E = typename Row<T, NB>::E;
+    if constexpr (NB == 16 && sizeof(T) == 4) {
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
+        const ulonglong2 t = NC ? __ldg(q) : *q;
+        v.x[0] = t.x; v.x[1] = t.y;
+    } else if constexpr (NB == 16) {
+        const double2* q = reinterpret_cast<const double2*>(p);
+        const double2 t = NC ? __ldg(q) : *q;
+        v.x[0] = t.x; v.x[1] = t.y;
+    } else {
+        const E* q = reinterpret_cast<const E*>(p);
+        v.x[0] = NC ? __ldg(q) : *q;
+    }
+}
+template <typename T, int NB> __device__ __forceinline__ void row_store(char* p, const Row<T, NB>& v) {
+    using E = typename Row<T, NB>::E;
+    if constexpr (NB == 16 && sizeof(T) == 4) *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.x[0], v.x[1]);
+    else if constexpr (NB == 16) *reinterpret_cast<double2*>(p) = make_double2(v.x[0], v.x[1]);
+    else *reinterpret_cast<E*>(p) = v.x[0];
+}
+// past the L1: rows that other warps of the same launch wrote
+template <typename T, int NB> __device__ __forceinline__ void row_load_cg(Row<T, NB>& v, const char* p) {
+    using E = typename Row<T, NB>::E;
+#pragma unroll
+    for (int h = 0; h < Row<T, NB>::N; ++h) v.x[h] = __ldcg(reinterpret_cast<const E*>(p) + h);
+}
+template <typename T, int NB> __device__ __forceinline__ void row_zero(Row<T, NB>& v) {
+#pragma unroll
+    for (int h = 0; h < Row<T, NB>::N; ++h) v.x[h] = 0;
+}
+// elementwise sums and products of the register elements (a pair of fp32 values or one value)
+__device__ __forceinline__ u64 e_fma(u64 a, u64 b, u64 c) { return fma2(a, b, c); }
+__device__ __forceinline__ float e_fma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double e_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ u64 e_add(u64 a, u64 b) { return add2(a, b); }
+__device__ __forceinline__ float e_add(float a, float b) { return a + b; }
+__device__ __forceinline__ double e_add(double a, double b) { return a + b; }
+template <typename E, typename T> __device__ __forceinline__ E e_splat(T s) {
+    if constexpr (sizeof(E) == 8 && sizeof(T) == 4) return pack2(s, s);
+    else return s;
+}
+template <typename T, int NB> __device__ __forceinline__ void row_fma(Row<T, NB>& acc, T s, const Row<T, NB>& x) {
+    using E = typename Row<T, NB>::E;
+    const E w = e_splat<E>(s);
+#pragma unroll
+    for (int h = 0; h < Row<T, NB>::N; ++h) acc.x[h] = e_fma(w, x.x[h], acc.x[h]);
+}
+template <typename T, int NB> __device__ __forceinline__ void row_add(Row<T, NB>& acc, const Row<T, NB>& x) {
+#pragma unroll
+    for (int h = 0; h < Row<T, NB>::N; ++h) acc.x[h] = e_add(acc.x[h], x.x[h]);
+}
+// this lane's part of a dot product over R vectors; vectors q with on[q] false do not count
+template <bool ALL, typename T, int NB, int R>
+__device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> (&b)[R], const bool (&on)[R]) {
+    using E = typename Row<T, NB>::E;
+    E s = 0;
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (ALL || on[q])
+#pragma unroll
+            for (int h = 0; h < Row<T, NB>::N; ++h) s = e_fma(a[q].x[h], b[q].x[h], s);
+    if constexpr (sizeof(E) == 8 && sizeof(T) == 4) {
+        const float2 f = unpack2(s);
+        return f.x + f.y;
+    } else {
+        return s;
+    }
+}
+
+// Four consecutive values base[i .. i+3] of a read-only array, i a multiple of 4 counted from a 16-byte
+// boundary when `aligned`; positions at or past `end` repeat the last value before it.
+template <typename I> struct Quad { I v[4]; };
+__device__ __forceinline__ Quad<int> quad_load_vec(const int* p) {
+    const int4 t = __ldg(reinterpret_cast<const int4*>(p));
+    return {{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ Quad<float> quad_load_vec(const float* p) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    return {{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ Quad<double> quad_load_vec(const double* p) {
+    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+    return {{a.x, a.y, b.x, b.y}};
+}
+template <typename I> __device__ __forceinline__ Quad<I> quad_load(const I* base, int i, int end, bool aligned) {
+    if (aligned && i + 4 <= end) return quad_load_vec(base + i);
+    Quad<I> q;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q.v[j] = __ldg(base + (i + j < end ? i + j : end - 1));
+    return q;
 }
 
 // ---- row access policies ---------------------------------------------------
 // A policy turns the local row index of a nonzero into a 31-bit *reference*
-// (`ref`, evaluated by every lane for its own nonzero when a batch of indices
+// (`ref`, evaluated by every lane for its own nonzeros when a window of indices
 // is read, so a table lookup is off the critical path) and a reference into
 // the address of the dense row (`resolve`, pure arithmetic).  The reference is
 // what the lane group passes round by shuffle and compares to detect a row
 // change.
-template <typename T> struct RowsByStride {
-    using V = typename Vec<T>::type;
-    const V* base;
-    long long ld_v;
+struct RowsByStride {
+    const char* base;
+    unsigned ld_bytes;
     __device__ __forceinline__ int ref(int row) const { return row; }
-    __device__ __forceinline__ const V* resolve(int r) const { return base + (long long)r * ld_v; }
+    __device__ __forceinline__ const char* resolve(int r) const { return base + (u64)(unsigned)r * ld_bytes; }
 };
 // Rows that live in the owners' heaps: reference = owner rank (6 bits) and row
 // number inside the owner's block (25 bits); `bases` (shared memory) holds the
 // block address of every rank as mapped into this process.
 constexpr int PEER_REF_SHIFT = 25;
-template <typename T> struct RowsByPeerRef {
-    using V = typename Vec<T>::type;
+struct RowsByPeerRef {
     const int* table;                  // [local rows] references; null: every row is in this rank's own block
     const unsigned long long* bases;   // [ranks] block base addresses
-    unsigned long long row_bytes;
+    unsigned row_bytes;
     int self_bits;                     // this rank << PEER_REF_SHIFT (used when table is null)
     __device__ __forceinline__ int ref(int row) const { return table ? __ldg(table + row) : (self_bits | row); }
-    __device__ __forceinline__ const V* resolve(int r) const {
-        return reinterpret_cast<const V*>(bases[r >> PEER_REF_SHIFT] +
-                                          (unsigned long long)(r & ((1 << PEER_REF_SHIFT) - 1)) * row_bytes);
+    __device__ __forceinline__ const char* resolve(int r) const {
+        return reinterpret_cast<const char*>(bases[r >> PEER_REF_SHIFT] +
+                                             (u64)(unsigned)(r & ((1 << PEER_REF_SHIFT) - 1)) * row_bytes);
     }
 };
 
+// Where values go: `scale(i)` is read together with the dense rows, `put(i, v)` stores dot * scale.
 template <typename T> struct StoreLocal {
     T* out;
+    const T* sval;    // null: no scaling
+    __device__ __forceinline__ T scale(long long i) const { return sval ? __ldg(sval + i) : (T)1; }
+    __device__ __forceinline__ void put(long long i, T v) const { out[i] = v; }
+};
+template <typename T> struct StoreScattered {
+    T* out;
     const T* sval;
-    const int* orig;  // optional: result position of nonzero i (null: i)
-    __device__ __forceinline__ void operator()(long long i, T dot) const {
-        const T v = sval ? dot * __ldg(sval + i) : dot;
-        if (orig) out[__ldg(orig + i)] = v;
-        else out[i] = v;
-    }
+    const int* orig;  // result position of nonzero i
+    __device__ __forceinline__ T scale(long long i) const { return sval ? __ldg(sval + i) : (T)1; }
+    __device__ __forceinline__ void put(long long i, T v) const { out[__ldg(orig + i)] = v; }
 };
 
+// Sums four values per lane over a group of G lanes (4 <= G) with a halving butterfly: log2(G) + 1 shuffles
+// instead of 4 log2(G).  On return lane gl holds the total of value number gl / (G / 4).
+template <typename T, int G> __device__ __forceinline__ T group_sum4(T (&v)[4], int gl) {
+    {
+        constexpr int m = G / 2;
+        const bool up = (gl & m) != 0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const T send = up ? v[t] : v[t + 2], keep = up ? v[t + 2] : v[t];
+            v[t] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    }
+    {
+        constexpr int m = G / 4;
+        const bool up = (gl & m) != 0;
+        const T send = up ? v[0] : v[1], keep = up ? v[1] : v[0];
+        v[0] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
+#pragma unroll
+    for (int m = G / 8; m > 0; m >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], m);
+    return v[0];
+}
+
 // ---------------------------------------------------------------------------
-// SDDMM work unit of one warp: 32/G lane groups x SDDMM_PER_SLOT consecutive
-// nonzeros each, starting at nonzero `unit * (32/G) * SDDMM_PER_SLOT`.
-// A group reads its (row, col) pairs G at a time with one coalesced load per
-// array and hands them round with in-group shuffles; each lane holds R
-// 16-byte vectors of a dense row, so a dot product costs R vector loads and 4R
-// FMAs per lane, and U dot products are reduced together with the butterfly
-// above.  The list is sorted by row, so the A row stays in registers until
-// the row changes.  Results leave as one coalesced store per G nonzeros.
+// SDDMM over windows first, first + step, ... < end of `wn` consecutive nonzeros each (wn a multiple of 4, at
+// most 128), one warp per window.  Lane l holds the indices of nonzeros 4l .. 4l+3 (one 16-byte load per array,
+// requested a whole window ahead); every group of G lanes works through an equal share of these quads: four
+// column indices by shuffle, four dense B rows in flight, four dot products reduced together, the A row kept in
+// registers until the row changes (the list is sorted by row).
+//
+// Bound by the row gathers out of L2 and by the issue of what surrounds them, so the split keeps the lanes per
+// row few (each shuffle then serves 32/G nonzeros) and fetches the A row of a quad's last nonzero together with
+// its B rows.
 // ---------------------------------------------------------------------------
-template <typename T, int G, int R, int U, typename ARows, typename Store, bool NC = true>
-__device__ __forceinline__ void sddmm_warp_unit(long long unit, long long nnz, const int* __restrict__ rowidx,
-                                                const int* __restrict__ colidx, const ARows& arows,
-                                                const typename Vec<T>::type* __restrict__ Bv, long long ldb_v,
-                                                int nvec, const Store& store, int lane) {
-    using V = typename Vec<T>::type;
+constexpr int WINDOW_MAX = 128;
+
+// Nonzeros per window: 128, less when that would leave warps without work.
+__host__ __device__ inline int window_nnz(long long nnz, long long nwarps, int groups_per_warp) {
+    const int quantum = 4 * groups_per_warp;
+    const long long share = (nnz + nwarps - 1) / nwarps;
+    const long long w = (share + quantum - 1) / quantum * quantum;
+    return (int)(w < quantum ? quantum : (w > WINDOW_MAX ? WINDOW_MAX : w));
+}
+
+template <typename T, int NB, int G, int R, int U, bool EXACT, bool NC, typename ARows, typename Store>
+__device__ __forceinline__ void sddmm_windows(long long first, long long step, long long end, int wn, long long nnz,
+                                              const int* __restrict__ rowidx, const int* __restrict__ colidx,
+                                              const ARows& arows, const char* __restrict__ B, unsigned ldb_bytes,
+                                              int nvec, bool aligned, const Store& store, int lane) {
+    static_assert(G >= 4, "a group reduces four values");
+    constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;
-    constexpr int UU = U < G ? U : G;
     const int slot = lane / G, gl = lane % G;
-    const unsigned gmask = group_mask<G>(slot);
-    const long long begin = (unit * SLOTS + slot) * (long long)SDDMM_PER_SLOT;
-    int cur_row = -1;
-    V a[R];
+    unsigned off[R];
+    bool on[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = vzero((V*)nullptr);
-    for (int base = 0; base < SDDMM_PER_SLOT; base += G) {
-        const long long i = begin + base + gl;
-        const bool ok = i < nnz;
-        const int my_r = ok ? arows.ref(__ldg(rowidx + i)) : -1;
-        const int my_c = ok ? __ldg(colidx + i) : -1;
-        T my_out = 0;
-#if SP3_SDDMM_UNROLL_BATCH
+    for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and do not count
+        const int v = gl + q * G;
+        on[q] = EXACT || v < nvec;
+        off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
+    }
+    auto length = [&](long long w) { return (int)(nnz - w * wn < wn ? nnz - w * wn : (long long)wn); };
+    auto load = [&](long long w, Quad<int>& c, Quad<int>& r) {
+        const int n = length(w), i = 4 * lane < n ? 4 * lane : (n - 1) & ~3;
+        c = quad_load(colidx + w * wn, i, n, aligned);
+        r = quad_load(rowidx + w * wn, i, n, aligned);
 #pragma unroll
-#else
-#pragma unroll 1
-#endif
-        for (int j = 0; j < G; j += UU) {
-            int rr[UU], cc[UU];
-            V b[UU][R];
-            T acc[UU];
+        for (int j = 0; j < 4; ++j) r.v[j] = arows.ref(r.v[j]);
+    };
+    auto fetch = [&](Row<T, NB> (&a)[R], const char* p) {
 #pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                rr[u] = __shfl_sync(gmask, my_r, j + u, G);
-                cc[u] = __shfl_sync(gmask, my_c, j + u, G);
-            }
+        for (int q = 0; q < R; ++q) row_load<NC>(a[q], p + (off[q] - off[0]));
+    };
+    if (first >= end) return;
+    B += off[0];
+    const int mine = gl / (G / 4);              // which of the four results ends up in this lane
+    const bool writer = gl % (G / 4) == 0;
+    Quad<int> c4, r4;
+    load(first, c4, r4);
+    int cur = -1;
+    Row<T, NB> a[R];
 #pragma unroll
-            for (int u = 0; u < UU; ++u)
+    for (int q = 0; q < R; ++q) row_zero(a[q]);
+    for (long long w = first; w < end; w += step) {
+        Quad<int> cn = c4, rn = r4;
+        if (w + step < end) load(w + step, cn, rn);
+        const int n = length(w);
+        const long long w0 = w * wn;
+        const int nq = (((n + 3) >> 2) + SLOTS - 1) / SLOTS;   // quads per group
+        // lanes whose quad is not all one row (a list sorted by row class by class may leave and re-enter a row)
+        const unsigned mixed = __ballot_sync(FULL, r4.v[0] != r4.v[3] || r4.v[1] != r4.v[3] || r4.v[2] != r4.v[3]);
+        for (int i = 0; i < nq; ++i) {
+            const int src = slot * nq + i;                     // lane that holds this group's quad
+            int c[4];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int v = gl + r * G;
-                    b[u][r] = (cc[u] >= 0 && v < nvec) ? ld_row<NC>(Bv + (long long)cc[u] * ldb_v + v) : vzero((V*)nullptr);
+            for (int u = 0; u < 4; ++u) c[u] = __shfl_sync(FULL, c4.v[u], src);
+            const int last = __shfl_sync(FULL, r4.v[3], src);
+            Row<T, NB> b[U][R];
+#pragma unroll
+            for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[u] * ldb_bytes);
+            const int pos = 4 * src + mine;
+            const bool st = writer && pos < n;
+            const T s = store.scale(w0 + (pos < n ? pos : n - 1));
+            T d[4];
+            if (__all_sync(FULL, last == cur && !(mixed >> src & 1))) {
+#pragma unroll
+                for (int h = 0; h < 4; h += U) {
+                    if (h > 0)
+#pragma unroll
+                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
                 }
+            } else {
+                int r[4];
 #pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                if (rr[u] >= 0 && rr[u] != cur_row) {
-                    cur_row = rr[u];
-                    const V* ap = arows.resolve(cur_row);
+                for (int u = 0; u < 3; ++u) r[u] = __shfl_sync(FULL, r4.v[u], src);
+                r[3] = last;
+                Row<T, NB> a2[R];
+                const bool staged = last != cur;
+                fetch(a2, arows.resolve(last) + off[0]);   // (unconditional: a load under a condition costs more)
 #pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const int v = gl + r * G;
-                        a[r] = v < nvec ? ld_row<NC>(ap + v) : vzero((V*)nullptr);
+                for (int h = 0; h < 4; h += U) {
+                    if (h > 0)
+#pragma unroll
+                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (r[h + u] != cur) {
+                            cur = r[h + u];
+                            if (staged && cur == last) {
+#pragma unroll
+                                for (int q = 0; q < R; ++q) a[q] = a2[q];
+                            } else {
+                                fetch(a, arows.resolve(cur) + off[0]);
+                            }
+                        }
+                        d[h + u] = row_dot<EXACT>(a, b[u], on);
                     }
                 }
-                T d = 0;
-#pragma unroll
-                for (int r = 0; r < R; ++r) d += vdot(a[r], b[u][r]);
-                acc[u] = d;
             }
-            // UU dot products reduced together; value u ends up in lanes [u*G/UU, (u+1)*G/UU)
-            group_transpose_reduce<T, G, UU>(acc, gmask, gl);
-            const T mine = __shfl_sync(gmask, acc[0], (gl % UU) * (G / UU), G);
-            if (gl / UU == j / UU) my_out = mine;  // lane gl keeps nonzero gl of the batch
+            const T total = group_sum4<T, G>(d, gl);
+            if (st) store.put(w0 + pos, total * s);
         }
-        if (ok) store(i, my_out);
+        c4 = cn;
+        r4 = rn;
     }
 }
 
@@ -194,6 +338,8 @@ __device__ __forceinline__ void sddmm_warp_unit(long long unit, long long nnz, c
 // SpMM
 // ---------------------------------------------------------------------------
 constexpr int SPMM_PIECE_SHIFT = 20;   // at most 2^20 split rows, 2^11 pieces per row
+constexpr int SPMM_ITEM_ROWS = 32;     // most rows of a rows item: a lane holds the end of one row
+constexpr int SPMM_ENDS = SPMM_ITEM_ROWS + 1;   // ints of shared memory per warp for the row ends
 
 struct SpmmLong {
     const int* first_piece;  // [nlong] first carry slot of each long row
@@ -202,200 +348,225 @@ struct SpmmLong {
     void* carry;             // [total pieces, ldc] scratch
     long long ldc;           // elements per carry row
     int piece_len;           // largest number of nonzeros of a piece
-    int* ticket;             // optional work counter (zero at launch): items are then handed out dynamically
+    int* ticket;             // optional work counters {next item, blocks done}, zero between launches: items are
+                             // then handed out dynamically
 };
 
-template <typename T> struct EmitLocal {
-    using V = typename Vec<T>::type;
-    V* Yv;
-    long long ldy_v;
+template <typename T, int NB> struct EmitLocal {
+    char* Y;
+    long long ldy_bytes;
     T beta;
     // writes vector v of row `row`
-    __device__ __forceinline__ void operator()(int row, int v, const V& acc) const {
-        V* y = Yv + (long long)row * ldy_v + v;
-        if (beta != (T)0) { V o = vscale(beta, *y); vadd(o, acc); *y = o; }
-        else *y = acc;
+    __device__ __forceinline__ void operator()(int row, int v, Row<T, NB> acc) const {
+        char* y = Y + row * ldy_bytes + (long long)v * NB;
+        if (beta != (T)0) {
+            Row<T, NB> old;
+            row_load<false>(old, y);
+            row_fma(acc, beta, old);
+        }
+        row_store(y, acc);
     }
 };
 
-// Adds val[q] * X[colidx[q]] for q in [p0, p1) taken in batches of G (one
-// coalesced index/value load per batch, broadcast inside the lane group);
-// consecutive batches of this group are `batch_stride` apart.
-template <typename T, int G, int R, int U, bool NC = true>
-__device__ __forceinline__ void spmm_accumulate(typename Vec<T>::type (&acc)[R], long long p0, long long p1,
-                                                int batch_stride, unsigned gmask,
-                                                const int* __restrict__ colidx, const T* __restrict__ val,
-                                                const typename Vec<T>::type* __restrict__ Xv, long long ldx_v,
-                                                int gl, int nvec) {
-    using V = typename Vec<T>::type;
-    constexpr int UU = U < G ? U : G;
-    for (long long base = p0; base < p1; base += batch_stride) {
-        const long long q = base + gl;
-        const bool ok = q < p1;
-        const int my_c = ok ? __ldg(colidx + q) : -1;
-        const T my_v = ok ? __ldg(val + q) : (T)0;
-        const int n = (p1 - base) < G ? (int)(p1 - base) : G;
-        for (int j = 0; j < n; j += UU) {
-            int cc[UU];
-            T vv[UU];
-#pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                cc[u] = __shfl_sync(gmask, my_c, j + u, G);
-                vv[u] = __shfl_sync(gmask, my_v, j + u, G);
-            }
-            V x[UU][R];
-#pragma unroll
-            for (int u = 0; u < UU; ++u)
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int v = gl + r * G;
-                    x[u][r] = (cc[u] >= 0 && v < nvec) ? ld_row<NC>(Xv + (long long)cc[u] * ldx_v + v) : vzero((V*)nullptr);
-                }
-#pragma unroll
-            for (int u = 0; u < UU; ++u)
-#pragma unroll
-                for (int r = 0; r < R; ++r) vfma(acc[r], vv[u], x[u][r]);
-        }
-    }
-}
-
-// Rows [r0, r1) of the CSR matrix as one flat stream of nonzeros: entries are
-// fetched G at a time (the next batch is requested before the current one is
-// consumed), U dense rows are in flight per lane, and the accumulator is
-// emitted whenever the stream crosses into the next row.  Rows without
-// nonzeros are emitted too (as zeros).  One lane group runs this alone, so no
-// atomics are involved and the result is reproducible.
-template <typename T, int G, int R, int U, typename Emit, bool NC = true>
-__device__ __forceinline__ void spmm_rows_stream(int r0, int r1, const long long* __restrict__ rowptr,
-                                                 const int* __restrict__ colidx, const T* __restrict__ val,
-                                                 const typename Vec<T>::type* __restrict__ Xv, long long ldx_v,
-                                                 const Emit& emit, unsigned gmask, int gl, int nvec) {
-    using V = typename Vec<T>::type;
-    constexpr int UU = U < G ? U : G;
-    if (r0 >= r1) return;
-    // positions are kept as 32-bit offsets from the first nonzero of the range (an item holds far fewer
-    // than 2^31 nonzeros); the dense-row stride is a 32-bit factor so that a row address costs one wide multiply
-    const long long q0 = rowptr[r0];
-    const int* __restrict__ cix = colidx + q0;
-    const T* __restrict__ vls = val + q0;
-    const int qend = (int)(rowptr[r1] - q0);
-    const int ld = (int)ldx_v;
-    int base = 0;
-    int row = r0;
-    int row_end = (int)(rowptr[r0 + 1] - q0);
-    V acc[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = vzero((V*)nullptr);
-    auto flush = [&](int rw) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int v = gl + r * G;
-            if (v < nvec) emit(rw, v, acc[r]);
-            acc[r] = vzero((V*)nullptr);
-        }
-    };
-    int nxt_c = (gl < qend) ? __ldg(cix + gl) : -1;
-    T nxt_v = (gl < qend) ? __ldg(vls + gl) : (T)0;
-    while (base < qend) {
-        const int my_c = nxt_c;
-        const T my_v = nxt_v;
-        const int nb = base + G;
-        nxt_c = (nb + gl < qend) ? __ldg(cix + nb + gl) : -1;
-        nxt_v = (nb + gl < qend) ? __ldg(vls + nb + gl) : (T)0;
-        const int n = (qend - base) < G ? (qend - base) : G;
-        for (int j = 0; j < n; j += UU) {
-            int cc[UU];
-            T vv[UU];
-#pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                cc[u] = __shfl_sync(gmask, my_c, j + u, G);  // -1 past the end of the range
-                vv[u] = __shfl_sync(gmask, my_v, j + u, G);
-            }
-            V x[UU][R];
-#pragma unroll
-            for (int u = 0; u < UU; ++u)
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int v = gl + r * G;
-                    x[u][r] = (cc[u] >= 0 && v < nvec) ? ld_row<NC>(Xv + (long long)cc[u] * ld + v) : vzero((V*)nullptr);
-                }
-#pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                if (cc[u] >= 0) {
-                    const int q = base + j + u;
-                    while (q >= row_end) {
-                        flush(row);
-                        ++row;
-                        row_end = (int)(rowptr[row + 1] - q0);
-                    }
-#pragma unroll
-                    for (int r = 0; r < R; ++r) vfma(acc[r], vv[u], x[u][r]);
-                }
-            }
-        }
-        base = nb;
-    }
-    while (row < r1) {
-        flush(row);
-        ++row;
-    }
-}
-
-template <typename T, int G, int R, int U, typename Emit, bool NC = true>
-__device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* __restrict__ rowptr,
+// One item, one warp (see build_spmm_items in ops/cuda_ops.py):
+//   rows item   (first row, end row, first nonzero, -1 - nonzeros): at most SPMM_ITEM_ROWS whole rows
+//   piece item  (row, first nonzero, end nonzero, long-row slot | piece number << SPMM_PIECE_SHIFT)
+//
+// The nonzeros of an item are dealt to the lane groups in equal shares of whole quads, wherever the rows end: a
+// group emits the rows that lie inside its share, and the sums of rows that go on in the next group travel along
+// the groups by shuffle, in order, at the end.  (Dealing whole rows to the groups left most lanes idle behind the
+// longest one: R-MAT scale 20, k = 32, 0.44 ms against 0.26 ms.)  Row ends are kept in shared memory (`ends`,
+// SPMM_ENDS ints per warp), indices and values come as quads that all lanes of a group read, requested one
+// quad ahead; U x R dense vectors are in flight per lane.  No atomics on values: bitwise reproducible.
+template <typename T, int NB, int G, int R, int U, bool EXACT, bool NC, typename Emit>
+__device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* __restrict__ rowptr, long long nnz,
                                                const int* __restrict__ colidx, const T* __restrict__ val,
-                                               const typename Vec<T>::type* __restrict__ Xv, long long ldx_v,
-                                               int nvec, const Emit& emit, const SpmmLong& lg, int lane) {
-    using V = typename Vec<T>::type;
+                                               const char* __restrict__ X, unsigned ldx_bytes, int nvec, bool aligned,
+                                               const Emit& emit, const SpmmLong& lg, int* ends, int lane) {
+    constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;
     const int slot = lane / G, gl = lane % G;
-    const unsigned gmask = group_mask<G>(slot);
-    if (item.w < 0) {
-        const int nr = item.y - item.x;
-        const int r0 = item.x + (int)(((long long)nr * slot) / SLOTS);
-        const int r1 = item.x + (int)(((long long)nr * (slot + 1)) / SLOTS);
-        spmm_rows_stream<T, G, R, U, Emit, NC>(r0, r1, rowptr, colidx, val, Xv, ldx_v, emit, gmask, gl, nvec);
+    unsigned off[R];
+    bool on[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and emit nothing
+        const int v = gl + q * G;
+        on[q] = EXACT || v < nvec;
+        off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
+    }
+    X += off[0];
+    auto clear = [&](Row<T, NB> (&v)[R]) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) row_zero(v[q]);
+    };
+    auto flush = [&](int row, const Row<T, NB> (&v)[R]) {
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+            if (on[q]) emit(row, gl + q * G, v[q]);
+    };
+    const bool is_rows = item.w < 0;
+    const int nr = is_rows ? item.y - item.x : 0;
+    const long long p0 = is_rows ? item.z : item.y;
+    const int n = is_rows ? -1 - item.w : item.z - item.y;
+    // positions count from the 16-byte boundary at or before the first nonzero
+    const int lead = (int)(p0 & 3), stop = lead + n;
+    const int share = ((stop + 4 * SLOTS - 1) / (4 * SLOTS)) * 4;
+    const int begin = slot * share, end = begin + share < stop ? begin + share : stop;
+    int row_end_lane = stop;                 // lane l: end of row l of the item
+    if (lane < nr) row_end_lane = lead + (int)(__ldg(rowptr + item.x + lane + 1) - p0);
+    const int* cp = colidx + (p0 - lead);
+    const T* vp = val + (p0 - lead);
+    const int avail = (int)(nnz - (p0 - lead) < 0x7fffffff ? nnz - (p0 - lead) : 0x7fffffff);
+    Quad<int> c4;
+    Quad<T> v4;
+    if (begin < end) {
+        c4 = quad_load(cp, begin, avail, aligned);
+        v4 = quad_load(vp, begin, avail, aligned);
+    }
+    int r = 0;                               // row of the item this group is in
+    if (is_rows) {
+        ends[lane] = row_end_lane;
+#pragma unroll
+        for (int g = 1; g < SLOTS; ++g) {
+            const unsigned done = __ballot_sync(FULL, lane < nr && row_end_lane <= g * share);
+            if (slot == g) r = __popc(done);
+        }
+        __syncwarp();
+    }
+    int row_end = r < nr ? ends[r] : stop;
+    const bool open = is_rows && slot > 0 && begin < end && (r == 0 ? lead : ends[r - 1]) < begin;   // began in an earlier group
+    bool in_head = open;
+    Row<T, NB> acc[R], first[R];             // first: this group's part of a row that began in an earlier group
+    clear(acc);
+    if (SLOTS > 1) clear(first);
+    auto close = [&]() {                     // the current row ends here
+        if (SLOTS > 1 && in_head) {
+#pragma unroll
+            for (int q = 0; q < R; ++q) first[q] = acc[q];
+            in_head = false;
+        } else {
+            flush(item.x + r, acc);
+        }
+        clear(acc);
+        ++r;
+        row_end = ends[r];
+    };
+    for (int i = begin; i < end; i += 4) {
+        int c[4];
+        T v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { c[u] = c4.v[u]; v[u] = v4.v[u]; }
+        const bool whole = i >= lead && i + 4 <= end;      // no position of this quad lies outside the item
+#pragma unroll
+        for (int h = 0; h < 4; h += U) {
+            Row<T, NB> x[U][R];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                // Positions outside the item are read too (their columns are those of the neighbouring items) and
+                // left out below: with the loads under a condition the kernel took 0.71 ms instead of 0.65 ms
+                // (R-MAT scale 20, k = 128).
+                const char* row = X + (u64)(unsigned)c[h + u] * ldx_bytes;
+#pragma unroll
+                for (int q = 0; q < R; ++q) row_load<NC>(x[u][q], row + (off[q] - off[0]));
+            }
+            // the next quad is requested behind the rows of this one: loads come back in order, and the indices may
+            // have to come from device memory (requested ahead of the rows: 0.84 ms instead of 0.66 ms at R-MAT
+            // scale 20, k = 128)
+            if (h == 0 && i + 4 < end) {
+                c4 = quad_load(cp, i + 4, avail, aligned);
+                v4 = quad_load(vp, i + 4, avail, aligned);
+            }
+            if (whole && i + h + U <= row_end) {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int q = 0; q < R; ++q) row_fma(acc[q], v[h + u], x[u][q]);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int p = i + h + u;
+                    if (p >= lead && p < end) {
+                        while (p >= row_end) close();
+#pragma unroll
+                        for (int q = 0; q < R; ++q) row_fma(acc[q], v[h + u], x[u][q]);
+                    }
+                }
+            }
+        }
+    }
+    if (is_rows) {
+        // rows that end with this share, and the empty rows after them
+        if (begin < end || (slot == 0 && n == 0))
+            while (r < nr && ends[r] <= end) close();
+        if (SLOTS > 1) {
+            // A row that goes on: its sum so far (acc) moves to the next group.  in_head still set: the whole share
+            // lies inside one row that began earlier and goes on.
+            if (__any_sync(FULL, open)) {
+                Row<T, NB> carry[R];
+                clear(carry);
+#pragma unroll
+                for (int g = 1; g < SLOTS; ++g)
+#pragma unroll
+                    for (int q = 0; q < R; ++q)
+#pragma unroll
+                        for (int h = 0; h < Row<T, NB>::N; ++h) {
+                            const auto sum = in_head ? e_add(carry[q].x[h], acc[q].x[h]) : acc[q].x[h];
+                            const auto up = __shfl_up_sync(FULL, sum, G);
+                            if (slot == g) carry[q].x[h] = up;
+                        }
+                if (open && !in_head) {
+#pragma unroll
+                    for (int q = 0; q < R; ++q) row_add(carry[q], first[q]);
+                    int h = 0;           // the row in which this share begins
+                    while (ends[h] <= begin) ++h;
+                    flush(item.x + h, carry);
+                }
+            }
+        }
+        __syncwarp();
         return;
     }
-    // piece of a long row: the warp reads 32 consecutive entries per step, each
-    // group takes its G of them; groups are combined afterwards
-    V acc[R];
+    // piece of a long row: add up the groups, leave the sum in the carry; the last piece to arrive adds the carries
+    // in order
+    auto add_groups = [&]() {
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = vzero((V*)nullptr);
-    spmm_accumulate<T, G, R, U, NC>(acc, (long long)item.y + slot * G, item.z, 32, gmask, colidx, val, Xv, ldx_v, gl, nvec);
+        for (int m = G; m < 32; m <<= 1)
 #pragma unroll
-    for (int m = G; m < 32; m <<= 1)
+            for (int q = 0; q < R; ++q)
 #pragma unroll
-        for (int r = 0; r < R; ++r) vadd(acc[r], shfl_xor_vec(acc[r], m));
-    // item.w = long-row slot | number of this piece inside its row << SPMM_PIECE_SHIFT
-    const int lr = item.w & ((1 << SPMM_PIECE_SHIFT) - 1), row = item.x;
-    const int first = __ldg(lg.first_piece + lr), np = __ldg(lg.npieces + lr);
-    const int piece = first + (item.w >> SPMM_PIECE_SHIFT);
-    V* carry = reinterpret_cast<V*>(lg.carry);
-    const long long ldc_v = lg.ldc / Vec<T>::N;
+                for (int h = 0; h < Row<T, NB>::N; ++h) acc[q].x[h] = e_add(acc[q].x[h], __shfl_xor_sync(FULL, acc[q].x[h], m));
+    };
+    add_groups();
+    const int lr = item.w & ((1 << SPMM_PIECE_SHIFT) - 1);
+    const int first_piece = __ldg(lg.first_piece + lr), np = __ldg(lg.npieces + lr);
+    char* carry = static_cast<char*>(lg.carry);
+    const long long ldc_bytes = lg.ldc * (long long)sizeof(T);
     if (slot == 0)
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int v = gl + r * G;
-            if (v < nvec) __stcg(carry + (long long)piece * ldc_v + v, acc[r]);
-        }
+        for (int q = 0; q < R; ++q)
+            if (on[q]) row_store(carry + (first_piece + (item.w >> SPMM_PIECE_SHIFT)) * ldc_bytes + (gl + q * G) * NB, acc[q]);
     __threadfence();
     __syncwarp();
     int old = 0;
     if (lane == 0) old = atomicAdd(lg.counters + lr, 1);
-    old = __shfl_sync(0xffffffffu, old, 0);
+    old = __shfl_sync(FULL, old, 0);
     if (old != np - 1) return;
     __threadfence();
-    if (slot == 0) {
+    // group g adds every SLOTS-th carry, then the groups are added up (more loads in flight here would take registers
+    // from the loop above: the kernel is compiled for a fixed number of warps)
+    clear(acc);
+    carry += first_piece * ldc_bytes + off[0];
+#pragma unroll 2
+    for (int j = slot; j < np; j += SLOTS) {
+        Row<T, NB> x[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int v = gl + r * G;
-            if (v >= nvec) continue;
-            V s = vzero((V*)nullptr);
-            for (int j = 0; j < np; ++j) vadd(s, __ldcg(carry + (long long)(first + j) * ldc_v + v));
-            emit(row, v, s);
+        for (int q = 0; q < R; ++q) {
+            row_load_cg(x[q], carry + j * ldc_bytes + (off[q] - off[0]));
+            row_add(acc[q], x[q]);
         }
     }
+    add_groups();
+    if (slot == 0) flush(item.x, acc);
     if (lane == 0) lg.counters[lr] = 0;
 }
 
@@ -411,46 +582,65 @@ inline int env_int(const char* name, int dflt) {
     return e ? atoi(e) : dflt;
 }
 
-// Resident blocks of `threads` threads for a persistent launch of `kernel`.
+constexpr int MAX_DEVICES = 64;
+
+// Blocks of `threads` threads of a persistent launch of `kernel`: all that fit at once, at most `needed` (0: no
+// limit).  `cache` belongs to this kernel and keeps the answer for the dynamic shared memory asked for last: the
+// occupancy query costs more than a launch.
+struct ResidentCache { std::atomic<unsigned long long> last[MAX_DEVICES] = {}; };   // smem << 32 | blocks
 template <typename K>
-unsigned persistent_blocks(K kernel, long long needed, int threads = 256, size_t smem = 0) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    static const int mult = env_int("SP3_PERSIST", 1);
-    long long b = mult > 0 ? (long long)sms * (per_sm > 0 ? per_sm : 1) * mult : needed;
-    if (needed > 0 && b > needed) b = needed;
-    return (unsigned)(b > 0 ? b : 1);
-}
-
-// Lane-group shape for a row of `nvec` 16-byte vectors.  SDDMM (spmm ==
-// false) runs best with about 16 lanes per row and 2-4 vectors per lane; SpMM
-// with as many lanes per row as the row has vectors (measured on B200, R-MAT
-// scale 20, k = 32..256).  SP3_VEC_PER_LANE overrides R for tuning.
-inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
-    static const int forced_sddmm = env_int("SP3_VEC_PER_LANE", 0);
-    static const int forced_spmm = env_int("SP3_SPMM_VEC_PER_LANE", 0);
-    const int forced = spmm ? forced_spmm : forced_sddmm;
-    int r = 1;
-    if (!spmm) { r = 2; while (nvec > 16 * r && r < 8) r <<= 1; }
-    if (forced > 0) r = forced;
-    while (r > 1 && r > nvec) r >>= 1;
-    int g = pick_group((nvec + r - 1) / r);
-    while (g * r < nvec) r <<= 1;  // nvec > 32 * r
-    *G = g; *R = r;
-}
-
-#define SP3_DISPATCH_GR(MACRO)                                                          \
-    switch (R) {                                                                        \
-        case 1: switch (G) { case 1: MACRO(1, 1); break; case 2: MACRO(2, 1); break; case 4: MACRO(4, 1); break; \
-                             case 8: MACRO(8, 1); break; case 16: MACRO(16, 1); break; default: MACRO(32, 1); } break; \
-        case 2: switch (G) { case 1: MACRO(1, 2); break; case 2: MACRO(2, 2); break; case 4: MACRO(4, 2); break; \
-                             case 8: MACRO(8, 2); break; case 16: MACRO(16, 2); break; default: MACRO(32, 2); } break; \
-        case 4: switch (G) { case 1: MACRO(1, 4); break; case 2: MACRO(2, 4); break; case 4: MACRO(4, 4); break; \
-                             case 8: MACRO(8, 4); break; case 16: MACRO(16, 4); break; default: MACRO(32, 4); } break; \
-        default: switch (G) { case 1: MACRO(1, 8); break; case 2: MACRO(2, 8); break; case 4: MACRO(4, 8); break; \
-                              case 8: MACRO(8, 8); break; case 16: MACRO(16, 8); break; default: MACRO(32, 8); } break; \
+unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int threads = 256, size_t smem = 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    unsigned long long v = dev < MAX_DEVICES ? cache.last[dev].load(std::memory_order_relaxed) : 0;
+    if (v == 0 || v >> 32 != smem) {
+        int sms = 0, per_sm = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+        const int b = sms * (per_sm > 0 ? per_sm : 1);
+        v = (unsigned long long)smem << 32 | (unsigned)(b > 0 ? b : 1);
+        if (dev < MAX_DEVICES) cache.last[dev].store(v, std::memory_order_relaxed);
     }
+    const long long b = (long long)(v & 0xffffffffu);
+    return (unsigned)(needed > 0 && needed < b ? needed : b);
+}
+
+// Lanes per row (G) and vectors per lane (R) for a row of `nvec` vectors, at most 256.
+//   SDDMM  few lanes with several vectors each: every index shuffle and every step of the reduction then serves
+//          32 / G nonzeros (R-MAT scale 20, fp32: k = 64 0.35 ms as 8 x 2, 0.38 as 16 x 1; k = 128 0.60 ms as
+//          8 x 4, 0.71 as 32 x 1).
+//   SpMM   as many lanes as the row has vectors: an accumulator costs R vectors of registers, and nothing is
+//          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).
+inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
+    int g = 4;
+    const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
+    while (g < top && g < nvec) g <<= 1;
+    int r = (nvec + g - 1) / g;
+    r = r <= 4 ? r : 8;
+    *G = g;
+    *R = r;
+}
+
+#define SP3_SDDMM_SHAPES(MACRO)                                                                           \
+    switch (G * 16 + R) {                                                                                 \
+        case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
+        case 8 * 16 + 2: MACRO(8, 2); break;   case 8 * 16 + 3: MACRO(8, 3); break;                       \
+        case 8 * 16 + 4: MACRO(8, 4); break;   case 16 * 16 + 3: MACRO(16, 3); break;                     \
+        case 16 * 16 + 4: MACRO(16, 4); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \
+        case 32 * 16 + 4: MACRO(32, 4); break; default: MACRO(32, 8); break;                              \
+    }
+#define SP3_SPMM_SHAPES(MACRO)                                                                            \
+    switch (G * 16 + R) {                                                                                 \
+        case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
+        case 16 * 16 + 1: MACRO(16, 1); break; case 32 * 16 + 1: MACRO(32, 1); break;                     \
+        case 32 * 16 + 2: MACRO(32, 2); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \
+        case 32 * 16 + 4: MACRO(32, 4); break; default: MACRO(32, 8); break;                              \
+    }
+// Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
+// half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.
+__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? (R <= 2 ? 4 : 2) : 1; }
+__host__ __device__ constexpr int sddmm_unroll(int R) { return R <= 4 ? 4 : 2; }
+__host__ __device__ constexpr int sddmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : (R <= 4 ? 2 : 1)); }
+__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R <= 3 ? 3 : 2); }
 
 }  // namespace sp3

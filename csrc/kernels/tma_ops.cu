@@ -25,6 +25,50 @@
 namespace sp3 {
 
 constexpr int TMA_MAX_STAGES = 8;
+constexpr int SDDMM_PER_SLOT = 32;      // nonzeros per lane group of a work unit; multiple of every G
+
+// Sums N values per lane across a group of G lanes with a halving butterfly (N <= G, both powers of two).  On
+// return v[0] of lane gl holds the group total of value number gl / (G / N).
+template <typename T, int G, int N>
+__device__ __forceinline__ void group_transpose_reduce(T (&v)[N], unsigned gmask, int gl) {
+    int n = N;
+#pragma unroll
+    for (int m = G / 2; m > 0; m >>= 1) {
+        if (n > 1) {
+            const int half = n >> 1;
+            const bool upper = (gl & m) != 0;
+#pragma unroll
+            for (int t = 0; t < N / 2; ++t) {
+                if (t < half) {
+                    const T send = upper ? v[t] : v[t + half];
+                    const T keep = upper ? v[t + half] : v[t];
+                    v[t] = keep + __shfl_xor_sync(gmask, send, m, G);
+                }
+            }
+            n = half;
+        } else {
+            v[0] += __shfl_xor_sync(gmask, v[0], m, G);
+        }
+    }
+}
+
+// Resident blocks of a persistent launch, at most `needed` (the shared memory differs from call to call).
+template <typename K> unsigned tma_blocks(K kernel, long long needed, int threads, size_t smem) {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+    const long long b = (long long)sms * (per_sm > 0 ? per_sm : 1);
+    return (unsigned)(needed < b ? (needed > 0 ? needed : 1) : b);
+}
+
+// Two or four vectors per lane, as few lanes as that takes (rows of at most 64 vectors).
+inline void tma_shape(int nvec, int* G, int* R) {
+    int r = nvec > 32 ? 4 : 2;
+    while (r > 1 && r > nvec) r >>= 1;
+    *G = pick_group((nvec + r - 1) / r);
+    *R = r;
+}
 constexpr int TMA_ROWS = 32;            // B rows per batch and warp (one per lane)
 __device__ __forceinline__ void tma_gather4(unsigned dst, const CUtensorMap* map, unsigned bar, int col, int r0,
                                             int r1, int r2, int r3) {
@@ -311,7 +355,7 @@ SP3_API int sp3_cuda_sddmm_tma_f32(long long nnz, const int* ri, const int* ci, 
     if (stages < 2) return -1;
     const size_t smem = stage_bytes * stages * warps + (size_t)warps * stages * 8;
     int G, R;
-    pick_shape(nvec, &G, &R, false);
+    tma_shape(nvec, &G, &R);
     cudaStream_t st = (cudaStream_t)stream;
     const long long per_unit = (long long)(32 / G) * SDDMM_PER_SLOT;
     const long long units = (nnz + per_unit - 1) / per_unit;
@@ -321,8 +365,8 @@ SP3_API int sp3_cuda_sddmm_tma_f32(long long nnz, const int* ri, const int* ci, 
         cudaError_t e = cudaFuncSetAttribute(sddmm_tma_kernel<GG, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                              (int)smem);                                                         \
         if (e != cudaSuccess) return (int)e;                                                                     \
-        sddmm_tma_kernel<GG, RR><<<persistent_blocks(sddmm_tma_kernel<GG, RR>, needed, 32 * warps, smem),         \
-                                   32 * warps, smem, st>>>(map, nnz, ri, ci, sv, A, lda, nvec, out, status, stages); \
+        sddmm_tma_kernel<GG, RR><<<tma_blocks(sddmm_tma_kernel<GG, RR>, needed, 32 * warps, smem), 32 * warps, smem,  \
+                                   st>>>(map, nnz, ri, ci, sv, A, lda, nvec, out, status, stages); \
     }
     if (R == 2) {
         switch (G) { case 1: SP3_TMA(1, 2) break; case 2: SP3_TMA(2, 2) break; case 4: SP3_TMA(4, 2) break;
@@ -369,7 +413,7 @@ SP3_API int sp3_cuda_spmm_tma_f32(long long nnz, const int* ri, const int* ci, c
     const long long per_unit = (long long)SPMM_TMA_NB * TMA_ROWS;
     const long long units = (nnz + per_unit - 1) / per_unit;
     const long long needed = (units + warps - 1) / warps;
-    spmm_tma_kernel<<<persistent_blocks(spmm_tma_kernel, needed, 32 * warps, smem), 32 * warps, smem, st>>>(
+    spmm_tma_kernel<<<tma_blocks(spmm_tma_kernel, needed, 32 * warps, smem), 32 * warps, smem, st>>>(
         map, nnz, ri, ci, sv, nvec, Y, ldy, status, stages);
     return (int)cudaGetLastError();
 }

@@ -16,10 +16,19 @@ _F = {torch.float32: "f32", torch.float64: "f64"}
 
 # SpMM schedule parameters: rows with more than LONG_ROW nonzeros are cut into
 # pieces of LONG_ROW; other rows are grouped into items of about ITEM_NNZ
-# nonzeros and at most ITEM_ROWS rows.
-LONG_ROW = int(os.environ.get("SP3_LONG_ROW", 512))
-ITEM_NNZ = int(os.environ.get("SP3_ITEM_NNZ", 128))
-ITEM_ROWS = int(os.environ.get("SP3_ITEM_ROWS", 64))
+# nonzeros and at most ITEM_ROWS rows (SPMM_ITEM_ROWS of csrc/kernels/sp3_kernels.cuh).
+LONG_ROW, ITEM_NNZ, ITEM_ROWS = 512, 128, 32
+_TARGET_ITEMS = 148 * 32   # warps that a B200 runs at once
+
+
+def item_sizes(nnz: int):
+    """(long_row, item_nnz) of a block of `nnz` nonzeros: LONG_ROW and ITEM_NNZ once there is enough work for every
+    warp, smaller powers of two (down to 16 nonzeros) below that, because the time of a small SpMM is that of its
+    longest item: each group of four nonzeros costs one trip to memory.  SP3_LONG_ROW / SP3_ITEM_NNZ override."""
+    item = ITEM_NNZ
+    while item > 16 and nnz < item * _TARGET_ITEMS:
+        item //= 2
+    return (int(os.environ.get("SP3_LONG_ROW", item * (LONG_ROW // ITEM_NNZ))), int(os.environ.get("SP3_ITEM_NNZ", item)))
 
 
 PIECE_SHIFT = 20   # SPMM_PIECE_SHIFT of csrc/kernels/sp3_kernels.cuh
@@ -72,19 +81,28 @@ def sddmm(rowidx, colidx, svals, A, B, out):
     return out
 
 
+def _long_row(nnz: int, deg: np.ndarray) -> int:
+    """Default piece length: as `item_sizes`, longer where the longest row would have too many pieces to number."""
+    n = item_sizes(nnz)[0]
+    while deg.size and int(deg.max()) > n * ((1 << (31 - PIECE_SHIFT)) - 64):
+        n *= 2
+    return n
+
+
 def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: int | None = None,
                      item_rows: int | None = None):
     """Work items of the SpMM kernel from a CSR row pointer (host, vectorised).
 
     Returns (items int32[n,4], first_piece int32[nlong], npieces int32[nlong]).
-    rows item  = (row_begin, row_end, 0, -1)
+    rows item  = (row_begin, row_end, first nonzero, -1 - number of nonzeros)
     piece item = (row, nnz_begin, nnz_end, long_row_slot | piece_number_in_row << PIECE_SHIFT)
     """
-    long_row = LONG_ROW if long_row is None else long_row
-    item_nnz = ITEM_NNZ if item_nnz is None else item_nnz
-    item_rows = ITEM_ROWS if item_rows is None else item_rows
     nrows = rowptr.shape[0] - 1
     deg = np.diff(rowptr)
+    nnz = int(rowptr[-1])
+    long_row = _long_row(nnz, deg) if long_row is None else long_row
+    item_nnz = item_sizes(nnz)[1] if item_nnz is None else item_nnz
+    item_rows = ITEM_ROWS if item_rows is None else min(item_rows, ITEM_ROWS)
     is_long = deg > long_row
     key = rowptr[:-1] // item_nnz
     bnd = np.ones(nrows, bool)
@@ -93,8 +111,8 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
     starts = np.flatnonzero(bnd)
     ends = np.append(starts[1:], nrows)
     short = ~is_long[starts]
-    rows_items = np.stack([starts[short], ends[short], np.zeros(short.sum(), np.int64),
-                           -np.ones(short.sum(), np.int64)], axis=1)
+    first_nnz = rowptr[starts[short]]
+    rows_items = np.stack([starts[short], ends[short], first_nnz, first_nnz - rowptr[ends[short]] - 1], axis=1)
     long_rows = np.flatnonzero(is_long)
     npieces = (deg[long_rows] + long_row - 1) // long_row
     first = np.concatenate([[0], np.cumsum(npieces)[:-1]]) if long_rows.size else np.zeros(0, np.int64)
@@ -127,9 +145,9 @@ def build_spmm_wave_items(rowptr: np.ndarray, cls: np.ndarray, n_classes: int, l
 
     Returns (perm int64[nnz]: source position of every nonzero of the re-ordered CSR arrays, items, first_piece,
     npieces, class_items int32[n_classes]: number of items of classes 0..c)."""
-    long_row = LONG_ROW if long_row is None else long_row
     nnz = int(rowptr[-1])
     deg = np.diff(rowptr)
+    long_row = _long_row(nnz, deg) if long_row is None else long_row
     std_items, _, _ = build_spmm_items(rowptr, long_row, item_nnz, item_rows)
     rows_items = std_items[std_items[:, 3] < 0].astype(np.int64)
     perm = np.arange(nnz, dtype=np.int64)
@@ -198,12 +216,12 @@ class SpmmSchedule:
         else:   # (items, first_piece, npieces) built elsewhere, e.g. by build_spmm_wave_items
             items, first, npieces = arrays
         dev = rowptr.device
-        self.piece_len = kw.get("long_row", LONG_ROW)
+        self.piece_len = kw.get("long_row") or item_sizes(int(rp[-1]) if arrays is None else int(rowptr[-1]))[0]
         self.items = torch.from_numpy(items).to(dev).contiguous()
         self.first = torch.from_numpy(first).to(dev)
         self.npieces = torch.from_numpy(npieces).to(dev)
         self.counters = torch.zeros(max(1, first.shape[0]), dtype=torch.int32, device=dev)
-        self.ticket = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.ticket = torch.zeros(2, dtype=torch.int32, device=dev)   # next item, blocks done: zero between launches
         self.total_pieces = int(npieces.sum())
         self.carry = None
         self.nlong = int(first.shape[0])

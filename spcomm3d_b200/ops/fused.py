@@ -61,7 +61,7 @@ class _SpmmLong(C.Structure):
 
 
 class _SpmmArgs(C.Structure):
-    _fields_ = [("comm", _Comm), ("nitems", C.c_int), ("items", P), ("rowptr", P), ("colidx", P), ("val", P),
+    _fields_ = [("comm", _Comm), ("nitems", C.c_int), ("items", P), ("n_rows", C.c_int), ("rowptr", P), ("colidx", P), ("val", P),
                 ("X_loc", P), ("ldx", C.c_longlong), ("n_owned_x", C.c_int), ("n_recv_x", C.c_int),
                 ("x_src", P), ("nvec", C.c_int), ("lg", _SpmmLong), ("n_owned_y", C.c_int), ("n_crows", C.c_int),
                 ("crows", P), ("y_dst", P), ("parity_off_v", C.c_longlong), ("Y", P),
@@ -564,6 +564,7 @@ class FusedSpMM(_FusedBase):
         contrib = [row_r[q] for q in range(rp.npeers) if rp.send_counts[q] > 0]
         self._fill_comm(a.comm, read_from, readers, push_to, contrib)
         a.nitems, a.items = self.sched.items.shape[0], self.sched.items.data_ptr()
+        a.n_rows = rp.n_local
         a.rowptr, a.colidx, a.val = op.rowptr.data_ptr(), self._colidx.data_ptr(), self._vals.data_ptr()
         a.X_loc, a.ldx = self._X_full.data_ptr(), kp
         a.n_owned_x, a.n_recv_x = p.col.n_owned, p.col.n_recv

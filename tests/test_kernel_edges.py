@@ -1,0 +1,141 @@
+"""SDDMM and SpMM at the sizes where their split of the work changes: widths that take 16-, 8- and 4-byte vectors and
+every lanes-per-row shape, lists that end inside a window or a quad, rows that cross the lane groups of an item, empty
+rows, rows cut into pieces, index arrays that do not start on a 16-byte boundary.
+
+Reference: fp64 sums of the same (already rounded) inputs.  A sum of n products in precision u, in any order, is off
+by at most gamma(n) = n u / (1 - n u) times the sum of the products' magnitudes (Higham, "Accuracy and Stability of
+Numerical Algorithms", section 3.1); two more roundings cover the scaling and the previous result."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+U = {torch.float32: 2.0 ** -24, torch.float64: 2.0 ** -53}
+
+
+def _gamma(n, dtype):
+    return n * U[dtype] / (1 - n * U[dtype])
+
+
+def _strided(rows, k, ld, dtype, g):
+    return torch.randn(rows, ld, generator=g, dtype=torch.float64).to(dtype)[:, :k]
+
+
+def _on_gpu(t, shift):
+    """Copy on the GPU whose first element sits `shift` elements behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + shift, dtype=t.dtype, device="cuda")
+    buf[shift:].copy_(t)
+    return buf[shift:]
+
+
+WIDTHS = [1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 33, 48, 50, 66, 96, 98, 100, 129, 130, 192, 200, 258, 260, 400, 512, 1024]
+
+
+def _check_sddmm(rows, cols, k, dtype, shift=0, ld=None, nrows=40, ncols=50, seed=0):
+    from spcomm3d_b200.ops import local
+    g = torch.Generator().manual_seed(seed)
+    ld = ld or k
+    A, B = _strided(nrows, k, ld, dtype, g), _strided(ncols, k, ld, dtype, g)
+    s = torch.rand(len(rows), generator=g, dtype=torch.float64).to(dtype)
+    r, c = torch.as_tensor(rows, dtype=torch.int32), torch.as_tensor(cols, dtype=torch.int32)
+    a, b = A.double()[r.long()], B.double()[c.long()]
+    ref, mag = (a * b).sum(1) * s.double(), (a * b).abs().sum(1) * s.double()
+    out = torch.full((len(rows),), float("nan"), dtype=dtype, device="cuda")
+    Ad = torch.empty(nrows, ld, dtype=dtype, device="cuda")[:, :k]
+    Bd = torch.empty(ncols, ld, dtype=dtype, device="cuda")[:, :k]
+    Ad.copy_(A), Bd.copy_(B)
+    local.sddmm(_on_gpu(r, shift), _on_gpu(c, shift), s.cuda(), Ad, Bd, out)
+    err = (out.cpu().double() - ref).abs()
+    assert bool((err <= _gamma(k + 2, dtype) * mag).all()), float((err / mag.clamp_min(1e-300)).max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", WIDTHS)
+def test_sddmm_widths(dtype, k):
+    rng = np.random.default_rng(k)
+    rows = np.sort(rng.integers(0, 40, 301))
+    _check_sddmm(rows, rng.integers(0, 50, 301), k, dtype)
+    _check_sddmm(rows, rng.integers(0, 50, 301), k, dtype, shift=1, ld=k + 3)
+
+
+@pytest.mark.parametrize("k", [8, 33, 64, 128])
+@pytest.mark.parametrize("nnz", [1, 2, 3, 4, 5, 15, 16, 17, 31, 33, 63, 65, 127, 128, 129, 511, 513])
+def test_sddmm_list_ends(k, nnz):
+    rng = np.random.default_rng(nnz)
+    _check_sddmm(np.sort(rng.integers(0, 40, nnz)), rng.integers(0, 50, nnz), k, torch.float32)
+
+
+@pytest.mark.parametrize("k", [32, 64, 128])
+@pytest.mark.parametrize("nnz", [200, 700_000])   # 700,000: full windows of 128 nonzeros
+def test_sddmm_row_changes(k, nnz):
+    """Runs of 1, 2, 3, 4, 5 and 300 nonzeros per row; and a list that leaves a row and comes back to it."""
+    rng = np.random.default_rng(7)
+    runs = rng.choice([1, 1, 2, 3, 4, 5, 300], nnz)
+    rows = np.repeat(np.arange(runs.size), runs)[:nnz] % 40
+    _check_sddmm(rows, rng.integers(0, 50, nnz), k, torch.float32)
+    again = rng.choice([3, 7], nnz)
+    _check_sddmm(again, rng.integers(0, 50, nnz), k, torch.float32)
+
+
+def _check_spmm(deg, k, dtype, beta, shift=0, ld=None, ncols=60, seed=0):
+    from spcomm3d_b200.ops import cuda_ops, local
+    g = torch.Generator().manual_seed(seed)
+    deg = np.asarray(deg, np.int64)
+    nrows, ld = deg.size, ld or k
+    rowptr = torch.zeros(nrows + 1, dtype=torch.int64)
+    rowptr[1:] = torch.from_numpy(np.cumsum(deg))
+    nnz = int(rowptr[-1])
+    ri = torch.from_numpy(np.repeat(np.arange(nrows), deg)).int()
+    ci = torch.randint(0, ncols, (nnz,), generator=g).int()
+    v = torch.rand(nnz, generator=g, dtype=torch.float64).to(dtype)
+    X, Y0 = _strided(ncols, k, ld, dtype, g), _strided(nrows, k, ld, dtype, g)
+    ref, mag = beta * Y0.double(), abs(beta) * Y0.double().abs()
+    prod = X.double()[ci.long()] * v.double()[:, None]
+    ref.index_add_(0, ri.long(), prod)
+    mag.index_add_(0, ri.long(), prod.abs())
+    Xd = torch.empty(ncols, ld, dtype=dtype, device="cuda")[:, :k]
+    Xd.copy_(X)
+    args = (rowptr.cuda(), ri.cuda(), _on_gpu(ci, shift), _on_gpu(v, shift), Xd)
+    sched = cuda_ops.SpmmSchedule(args[0])
+    bound = torch.from_numpy(_gamma(deg + 3.0, dtype))[:, None] * mag
+    got = []
+    for _ in range(2):
+        wide = torch.full((nrows, ld), 7.0, dtype=dtype, device="cuda")
+        Yd = wide[:, :k]
+        Yd.copy_(Y0) if beta else Yd.fill_(float("nan"))
+        local.spmm(*args, Yd, beta, sched)
+        assert bool(((Yd.cpu().double() - ref).abs() <= bound).all())
+        assert bool((wide[:, k:] == 7.0).all())
+        got.append(Yd)
+    assert torch.equal(got[0], got[1])          # reproducible, the counters are back at zero
+    assert int(sched.counters.abs().sum()) == 0 and int(sched.ticket.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", WIDTHS)
+def test_spmm_widths(dtype, k):
+    deg = np.random.default_rng(k).poisson(6, 90)
+    deg[[0, 40, 41, 89]] = 0
+    deg[50] = 333                                # cut into pieces
+    _check_spmm(deg, k, dtype, 0.0)
+    _check_spmm(deg, k, dtype, 0.5, shift=1, ld=k + 3)
+
+
+@pytest.mark.parametrize("k", [8, 32, 64, 128, 33])
+@pytest.mark.parametrize("deg", [[0], [1], [3], [4], [5], [0, 0, 0], [0] * 70, [64], [65], [63, 1], [1] * 33, [1] * 64,
+                                 [15, 1], [16, 16], [17, 15], [0, 16, 0, 0, 16, 0], [2, 60, 2], [5000], [64, 65, 0, 64],
+                                 [130_000, 3]])
+def test_spmm_items(k, deg):
+    """Rows that fill, straddle and span the shares of the lane groups; rows of one item and of many pieces."""
+    _check_spmm(deg, k, torch.float32, 0.0)
+    _check_spmm(deg, k, torch.float32, 1.0, shift=3)
+
+
+@pytest.mark.parametrize("k", [32, 128])
+def test_spmm_many_items(k):
+    """More items than warps: handed out dynamically, full-size items and pieces of 512."""
+    rng = np.random.default_rng(3)
+    deg = np.minimum(rng.zipf(1.9, 30_000), 3000)
+    deg = np.concatenate([deg, np.full(8000, 90), [5000, 513, 512]])
+    _check_spmm(deg, k, torch.float32, 0.5)
