@@ -398,6 +398,58 @@ SP3_API int sp3_cuda_spmm_f64(int nrows, int nitems, const void* items, const lo
     return launch_spmm<double>(nrows, nitems, (const int4*)items, rowptr, ci, val, X, ldx, k, beta, Y, ldy, lg,
                                (cudaStream_t)stream);
 }
+// The same two calls with their arguments in a record that the caller keeps between launches (field order:
+// ops/cuda_ops.py): converting some twenty arguments costs the Python front end more than a small kernel runs.
+struct SddmmCall {
+    long long nnz;
+    const int *ri, *ci;
+    const void *sv, *A;
+    long long lda;
+    const void* B;
+    long long ldb;
+    void* out;
+    int k, f64;
+};
+struct SpmmCall {
+    int nrows, nitems;
+    const void* items;
+    const long long* rowptr;
+    const int* ci;
+    const void *val, *X;
+    long long ldx;
+    void* Y;
+    long long ldy;
+    const int *first_piece, *npieces;
+    int* counters;
+    void* carry;
+    long long ldc;
+    int* ticket;
+    double beta;
+    int k, f64, piece_len;
+};
+SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
+    *sddmm_bytes = (int)sizeof(SddmmCall);
+    *spmm_bytes = (int)sizeof(SpmmCall);
+    return 0;
+}
+SP3_API int sp3_cuda_sddmm_call(const void* record, void* stream) {
+    const SddmmCall& c = *static_cast<const SddmmCall*>(record);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (c.f64) return launch_sddmm<double>(c.nnz, c.ri, c.ci, (const double*)c.sv, (const double*)c.A, c.lda,
+                                           (const double*)c.B, c.ldb, c.k, (double*)c.out, st);
+    return launch_sddmm<float>(c.nnz, c.ri, c.ci, (const float*)c.sv, (const float*)c.A, c.lda, (const float*)c.B,
+                               c.ldb, c.k, (float*)c.out, st);
+}
+SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
+    const SpmmCall& c = *static_cast<const SpmmCall*>(record);
+    cudaStream_t st = (cudaStream_t)stream;
+    const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.piece_len, c.ticket};
+    if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
+                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st);
+    return launch_spmm<float>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const float*)c.val,
+                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st);
+}
+
 SP3_API int sp3_cuda_rows_f32(int mode, long long n, const long long* idx, const float* src, long long lds,
                               float* dst, long long ldd, int k, void* stream) {
     return launch_rows<float>(mode, n, idx, src, lds, dst, ldd, k, (cudaStream_t)stream);

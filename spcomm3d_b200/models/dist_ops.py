@@ -129,6 +129,11 @@ class _Dist3DOp:
         for buf, side in self._local_buffers():
             buf[side.n_owned:].fill_(float("nan"))
 
+    def _single_rank(self) -> bool:
+        """One rank, one GPU, plain kernels: a run is a single launch, which can be bound to its tensors."""
+        return (self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
+                and self._panels is None)
+
     def _finish(self):
         if not self.timer.enabled:
             return None
@@ -221,6 +226,19 @@ class DistSDDMM(_Dist3DOp):
             self._panels = PanelSDDMM(p.rowidx, p.colidx, p.vals, p.row.n_local, p.col.n_local, self.device,
                                       **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
         self.owned_off, self.owned_len = p.owned_nnz_slice()
+        self._bound = None
+        self._single = self._single_rank() and p.nnz > 0
+
+    def _run_bound(self) -> torch.Tensor:
+        """The run of a single rank without phase timers: one launch."""
+        t = (self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial)
+        b = self._bound
+        if b is None or not b.bound_to(*t):
+            from ..ops import cuda_ops
+            b = self._bound = cuda_ops.bind_sddmm(*t)
+            self._slice = self.partial[self.owned_off:self.owned_off + self.owned_len]
+        b.launch()
+        return self._slice
 
     def _local_buffers(self):
         return [(self.A_loc, self.plan.row), (self.B_loc, self.plan.col)]
@@ -228,6 +246,8 @@ class DistSDDMM(_Dist3DOp):
     def run(self) -> torch.Tensor:
         """One distributed SDDMM; returns my slice of C's values."""
         t = self.timer
+        if not t.enabled and self._single and not local.opt_in_kernels("sddmm"):
+            return self._run_bound()
         if self.variant == "fused":
             with t.span("comp"):
                 c = self._fused.run()
@@ -359,6 +379,20 @@ class DistSpMM(_Dist3DOp):
             self._panels = PanelSpMM(p.rowidx, p.colidx, p.vals, p.row.n_local, p.col.n_local, self.device,
                                      **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
 
+        self._bound = None
+        self._single = self._single_rank() and p.row.n_local > 0 and p.nnz > 0
+
+    def _run_bound(self, beta: float) -> torch.Tensor:
+        """The run of a single rank without phase timers: one launch."""
+        t = (self.rowptr, self.colidx, self.vals, self.X_loc, self.Y_loc)
+        b = self._bound
+        if b is None or not b.bound_to(*t):
+            from ..ops import cuda_ops
+            b = self._bound = cuda_ops.bind_spmm(*t, self.sched)
+        b._record.beta = beta
+        b.launch()
+        return self.Y_owned
+
     def _local_buffers(self):
         return [(self.X_loc, self.plan.col)]
 
@@ -372,6 +406,8 @@ class DistSpMM(_Dist3DOp):
     def run(self, beta: float = 0.0) -> torch.Tensor:
         """One distributed SpMM: Y_owned = beta*Y_owned + (S X)[owned rows]."""
         t, p = self.timer, self.plan
+        if not t.enabled and self._single and not local.opt_in_kernels("spmm"):
+            return self._run_bound(beta)
         if self.variant == "fused":
             with t.span("comp"):
                 self._fused.run(self.Y_owned, beta)
@@ -389,14 +425,17 @@ class DistSpMM(_Dist3DOp):
                     self._dense_row.reduce_scatter(self._Yslab, self.Y_owned)
                     self.Y_owned += prev
         else:
-            prev = self.Y_owned * beta if beta != 0.0 else None
+            # with nobody to add to my rows (or to send partial rows to) the kernel applies beta itself
+            alone = self.exY.trivial
+            prev = self.Y_owned * beta if beta != 0.0 and not alone else None
+            b = beta if alone else 0.0
             with t.span("comm1"):
                 self.exX.expand(self.X_loc)
             with t.span("comp"):
                 if self._panels is not None:
-                    self._panels.run(self.X_loc, self.Y_loc, 0.0)
+                    self._panels.run(self.X_loc, self.Y_loc, b)
                 else:
-                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self.X_loc, self.Y_loc, 0.0,
+                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self.X_loc, self.Y_loc, b,
                                self.sched)
             with t.span("comm2"):
                 self.exY.reduce(self.Y_loc)  # adds the peers' partial rows into the owned head = Y_owned

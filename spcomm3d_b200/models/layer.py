@@ -186,6 +186,9 @@ class GatLayer:
         dev = torch.device(device)
         self._mine = torch.zeros(self.width, dtype=dtype, device=dev)
         self._all = torch.zeros(Z, self.width, dtype=dtype, device=dev)
+        if Z == 1 and self.sddmm.variant in ("sparse", "sparseNRB"):
+            # one layer holds all of k: the SDDMM writes its scores where the SpMM reads its values
+            self.sddmm.partial = self.spmm.vals
         # the SpMM wants its values in CSR order; a fused SDDMM stores them in its own order
         order = self.sddmm.value_order
         self._pos = None if order is None else torch.from_numpy(np.ascontiguousarray(order)).to(dev)
@@ -195,7 +198,8 @@ class GatLayer:
         Z = self.plan.mesh.Z
         if Z == 1:
             if self._pos is None:
-                self.spmm.vals.copy_(c)
+                if c.data_ptr() != self.spmm.vals.data_ptr():
+                    self.spmm.vals.copy_(c)
             else:
                 self.spmm.vals.index_copy_(0, self._pos, c)
         else:

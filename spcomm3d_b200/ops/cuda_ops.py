@@ -5,6 +5,7 @@ pointers; nothing here falls back to a torch implementation.
 """
 from __future__ import annotations
 
+import ctypes as C
 import os
 
 import numpy as np
@@ -36,6 +37,14 @@ PIECE_SHIFT = 20   # SPMM_PIECE_SHIFT of csrc/kernels/sp3_kernels.cuh
 
 def _stream():
     return torch.cuda.current_stream().cuda_stream
+
+
+if hasattr(torch._C, "_cuda_getCurrentRawStream"):
+    def _raw_stream():
+        """`_stream` without the Stream object (0.4 us instead of 2)."""
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+else:
+    _raw_stream = _stream
 
 
 LAUNCHES = 0  # kernels launched through this module (bench.py reports the count)
@@ -266,6 +275,75 @@ def spmm(rowptr, rowidx, colidx, vals, X, Y, beta, sched: SpmmSchedule | None):
            _ld(Y), native.ptr(sched.first), native.ptr(sched.npieces), native.ptr(sched.counters),
            native.ptr(carry), ldc, sched.piece_len, native.ptr(sched.ticket), _stream()), "spmm")
     return Y
+
+
+# ---- bound calls -------------------------------------------------------------
+class _SddmmCall(C.Structure):
+    _fields_ = [("nnz", C.c_longlong), ("ri", C.c_void_p), ("ci", C.c_void_p), ("sv", C.c_void_p), ("A", C.c_void_p),
+                ("lda", C.c_longlong), ("B", C.c_void_p), ("ldb", C.c_longlong), ("out", C.c_void_p), ("k", C.c_int),
+                ("f64", C.c_int)]
+
+
+class _SpmmCall(C.Structure):
+    _fields_ = [("nrows", C.c_int), ("nitems", C.c_int), ("items", C.c_void_p), ("rowptr", C.c_void_p),
+                ("ci", C.c_void_p), ("val", C.c_void_p), ("X", C.c_void_p), ("ldx", C.c_longlong), ("Y", C.c_void_p),
+                ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
+                ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
+                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int)]
+
+
+_checked_calls = False
+
+
+class _BoundCall:
+    """One operation with its tensors, its arguments converted once: a launch then costs a few microseconds of host
+    time (the plain calls above convert every pointer each time, 15-25 us).  `bound_to` says whether the tensors
+    are still the ones given; an operator that had its tensors replaced binds again."""
+
+    def __init__(self, name, record, tensors, keep=()):
+        global _checked_calls
+        lib = native.cuda()
+        if not _checked_calls:
+            a, b = C.c_int(), C.c_int()
+            lib.sp3_cuda_call_sizes(C.byref(a), C.byref(b))
+            if (a.value, b.value) != (C.sizeof(_SddmmCall), C.sizeof(_SpmmCall)):
+                raise RuntimeError("call record layout differs between Python and the kernel library")
+            _checked_calls = True
+        self._name, self._record, self._tensors, self._keep = name, record, tensors, keep
+        self._addr = C.addressof(record)
+        self._fn = getattr(lib, f"sp3_cuda_{name}_call")
+        self._ptrs = [t.data_ptr() for t in tensors]
+
+    def bound_to(self, *tensors):
+        for t, own, ptr in zip(tensors, self._tensors, self._ptrs):
+            if t is not own or t.data_ptr() != ptr:
+                return False
+        return True
+
+    def launch(self):
+        global LAUNCHES
+        LAUNCHES += 1
+        rc = self._fn(self._addr, _raw_stream())
+        if rc != 0:
+            raise RuntimeError(f"{self._name}: CUDA launch error {rc}")
+
+
+def bind_sddmm(rowidx, colidx, svals, A, B, out):
+    """`sddmm` bound to its tensors (all given)."""
+    p = native.ptr
+    rec = _SddmmCall(rowidx.shape[0], p(rowidx), p(colidx), p(svals), p(A), _ld(A), p(B), _ld(B), p(out), A.shape[1],
+                     int(A.dtype == torch.float64))
+    return _BoundCall("sddmm", rec, (rowidx, colidx, svals, A, B, out))
+
+
+def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule):
+    """`spmm` bound to its tensors; `launch(beta)`."""
+    p = native.ptr
+    carry, ldc = sched.carry_for(X.shape[1], X.dtype, X.device)
+    rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(X),
+                    _ld(X), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
+                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len)
+    return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry))
 
 
 def rows(mode, idx, src, dst):

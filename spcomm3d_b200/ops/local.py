@@ -32,6 +32,12 @@ def _row_major(t: torch.Tensor):
     return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
 
 
+def opt_in_kernels(kernel: str) -> bool:
+    """Whether an opt-in kernel (the TMA gather twins) takes the place of the default one on a GPU."""
+    from . import cuda_ops
+    return cuda_ops.USE_TMA if kernel == "sddmm" else cuda_ops.USE_SPMM_TMA
+
+
 def sddmm(rowidx, colidx, svals, A, B, out=None):
     """out[i] = svals[i] * dot(A[rowidx[i]], B[colidx[i]]); svals may be None."""
     nnz = rowidx.shape[0]
