@@ -12,6 +12,7 @@
 #include "sp3_kernels.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace sp3 {
 
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R))
 sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
                  const RowsByStride arows, const char* __restrict__ B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
+    after_previous_kernel();
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     sddmm_windows<T, NB, G, R, sddmm_unroll(R), EXACT, true>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
@@ -55,11 +57,12 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // Rows without nonzeros are covered by rows items, so beta is applied to
 // every row exactly once.
 // ---------------------------------------------------------------------------
-template <typename T, int NB, int G, int R, bool EXACT>
+template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
 __global__ void __launch_bounds__(256, spmm_min_blocks(R))
 spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
                   const int* __restrict__ colidx, const T* __restrict__ val, const char* __restrict__ X,
-                  unsigned ldx_bytes, int nvec, bool aligned, const EmitLocal<T, NB> emit, const SpmmLong lg) {
+                  unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
+    after_previous_kernel();
     __shared__ int row_ends[256 / 32][SPMM_ENDS];
     int* ends = row_ends[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -266,8 +269,8 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
         const unsigned all = resident_blocks(kernel, cache, 0);                                               \
         const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
-        kernel<<<needed < all ? (unsigned)needed : all, 256, 0, st>>>(nnz, wn, ri, ci, arows, B,              \
-                                                                      (unsigned)ldb_bytes, nvec, aligned, store); \
+        launch_early(kernel, needed < all ? (unsigned)needed : all, 0, st, nnz, wn, ri, ci, arows, B,               \
+                     (unsigned)ldb_bytes, nvec, aligned, store);                                              \
     }
     SP3_SDDMM_SHAPES(SP3_SDDMM)
 #undef SP3_SDDMM
@@ -300,23 +303,23 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
     return -1;
 }
 
-template <typename T, int NB>
+template <typename T, int NB, typename Emit>
 int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
-                   const char* X, long long ldx_bytes, int nvec, T beta, char* Y, long long ldy_bytes,
-                   const SpmmLong& lg, cudaStream_t st) {
+                   const char* X, long long ldx_bytes, int nvec, const Emit& emit, const SpmmLong& lg, cudaStream_t st) {
     const bool aligned = ((uintptr_t)ci | (uintptr_t)val) % 16 == 0;
-    const EmitLocal<T, NB> emit{Y, ldy_bytes, beta};
+    constexpr bool VECTORS = std::is_same<Emit, EmitLocal<T, NB>>::value;
     int G, R;
     pick_shape(nvec, &G, &R, true);
-    const bool exact = NB == 16 && nvec == G * R;
+    const bool exact = VECTORS && NB == 16 && nvec == G * R;
     const long long needed = ((long long)nitems + 7) / 8;
 #define SP3_SPMM(GG, RR)                                                                                      \
     {                                                                                                         \
         static ResidentCache caches[2];                                                                       \
         ResidentCache& cache = caches[exact];                                                                 \
-        auto kernel = exact ? spmm_items_kernel<T, NB, GG, RR, NB == 16> : spmm_items_kernel<T, NB, GG, RR, false>; \
-        kernel<<<resident_blocks(kernel, cache, needed), 256, 0, st>>>(nitems, items, nrows, rowptr, ci, val, X, \
-                                                                       (unsigned)ldx_bytes, nvec, aligned, emit, lg); \
+        auto kernel = exact ? spmm_items_kernel<T, NB, GG, RR, VECTORS && NB == 16, Emit>                     \
+                            : spmm_items_kernel<T, NB, GG, RR, false, Emit>;                                  \
+        launch_early(kernel, resident_blocks(kernel, cache, needed), 0, st, nitems, items, nrows, rowptr, ci, val, X, \
+                     (unsigned)ldx_bytes, nvec, aligned, emit, lg);                                           \
     }
     SP3_SPMM_SHAPES(SP3_SPMM)
 #undef SP3_SPMM
@@ -325,23 +328,30 @@ int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* ro
 
 template <typename T>
 int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
-                const T* X, long long ldx, int k, T beta, T* Y, long long ldy, SpmmLong lg, cudaStream_t st) {
+                const T* X, long long ldx, int k, T beta, T* Y, long long ldy, SpmmLong lg, cudaStream_t st,
+                int k_out = 0) {
     if (nrows == 0) return 0;
     const long long ldx_b = ldx * (long long)sizeof(T), ldy_b = ldy * (long long)sizeof(T);
-    unsigned long long bits = ldx_b | ldy_b | (uintptr_t)X | (uintptr_t)Y;
+    unsigned long long bits = ldx_b | (uintptr_t)X;
+    const bool padded = k_out > 0 && k_out < k;   // Y takes the first k_out columns, value by value
+    if (!padded) bits |= ldy_b | (uintptr_t)Y;
     if (lg.carry) bits |= (uintptr_t)lg.carry | (unsigned long long)lg.ldc * sizeof(T);
     const unsigned long long bytes = (unsigned long long)k * sizeof(T);
     const int nb = vector_bytes<T>(bytes, bits);
     const unsigned long long nvec = bytes / nb;
-    if (items == nullptr || nvec > 256 || nvec == 0 || ldx_b >= 1ll << 32) {
+    if (padded && (bytes | bits) % 16 == 0 && items != nullptr && bytes <= 256 * 16 && ldx_b < 1ll << 32)
+        return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, reinterpret_cast<const char*>(X), ldx_b,
+                                     (int)(bytes / 16), EmitPacked<T>{Y, ldy, k_out, beta}, lg, st);
+    if (padded) k = k_out;
+    if (padded || items == nullptr || nvec > 256 || nvec == 0 || ldx_b >= 1ll << 32) {
         spmm_scalar_kernel<T><<<(unsigned)(((long long)nrows * 32 + 255) / 256), 256, 0, st>>>(nrows, rowptr, ci, val, X, ldx, k, beta, Y, ldy);
         return (int)cudaGetLastError();
     }
     const char* x = reinterpret_cast<const char*>(X);
     char* y = reinterpret_cast<char*>(Y);
-    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
-    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
-    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, beta, y, ldy_b, lg, st);
+    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 16>{y, ldy_b, beta}, lg, st);
+    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 8>{y, ldy_b, beta}, lg, st);
+    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 4>{y, ldy_b, beta}, lg, st);
     return -1;
 }
 
@@ -426,6 +436,7 @@ struct SpmmCall {
     int* ticket;
     double beta;
     int k, f64, piece_len;
+    int k_out;              // columns of Y (k of X counts the padding of its rows)
 };
 SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *sddmm_bytes = (int)sizeof(SddmmCall);
@@ -445,9 +456,9 @@ SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.piece_len, c.ticket};
     if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
-                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st);
+                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out);
     return launch_spmm<float>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const float*)c.val,
-                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st);
+                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st, c.k_out);
 }
 
 SP3_API int sp3_cuda_rows_f32(int mode, long long n, const long long* idx, const float* src, long long lds,

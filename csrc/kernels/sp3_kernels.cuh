@@ -107,7 +107,7 @@ __device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> 
     E s = 0;
 #pragma unroll
     for (int q = 0; q < R; ++q)
-        if (ALL || on[q])
+        if (ALL || (q < R - 1 && R <= 4) || on[q])   // (pick_shape: only the last vector of a lane can be past the row)
 #pragma unroll
             for (int h = 0; h < Row<T, NB>::N; ++h) s = e_fma(a[q].x[h], b[q].x[h], s);
     if constexpr (sizeof(E) == 8 && sizeof(T) == 4) {
@@ -368,6 +368,28 @@ template <typename T, int NB> struct EmitLocal {
     }
 };
 
+// Rows of k values without padding, written value by value (X rows are padded, result rows are not).
+template <typename T> struct EmitPacked {
+    T* Y;
+    long long ldy;
+    int k;
+    T beta;
+    __device__ __forceinline__ void operator()(int row, int v, const Row<T, 16>& acc) const {
+        constexpr int N = 16 / (int)sizeof(T);
+        T x[N];
+        if constexpr (sizeof(T) == 4) {
+            const float2 a = unpack2(acc.x[0]), b = unpack2(acc.x[1]);
+            x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+        } else {
+            x[0] = acc.x[0]; x[1] = acc.x[1];
+        }
+        T* y = Y + row * ldy + v * N;
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (v * N + j < k) y[j] = beta != (T)0 ? beta * y[j] + x[j] : x[j];
+    }
+};
+
 // One item, one warp (see build_spmm_items in ops/cuda_ops.py):
 //   rows item   (first row, end row, first nonzero, -1 - nonzeros): at most SPMM_ITEM_ROWS whole rows
 //   piece item  (row, first nonzero, end nonzero, long-row slot | piece number << SPMM_PIECE_SHIFT)
@@ -402,7 +424,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     auto flush = [&](int row, const Row<T, NB> (&v)[R]) {
 #pragma unroll
         for (int q = 0; q < R; ++q)
-            if (on[q]) emit(row, gl + q * G, v[q]);
+            if ((q < R - 1 && R <= 4) || on[q]) emit(row, gl + q * G, v[q]);
     };
     const bool is_rows = item.w < 0;
     const int nr = is_rows ? item.y - item.x : 0;
@@ -582,6 +604,28 @@ inline int env_int(const char* name, int dflt) {
     return e ? atoi(e) : dflt;
 }
 
+// Launch that may begin while the previous kernel of the stream drains (programmatic dependent launch): the kernel
+// has to call `after_previous_kernel` before it touches memory.
+template <typename... P, typename... A>
+inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+__device__ __forceinline__ void after_previous_kernel() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __threadfence();   // nothing of an earlier kernel's lines may be left in the L1
+}
+
 constexpr int MAX_DEVICES = 64;
 
 // Blocks of `threads` threads of a persistent launch of `kernel`: all that fit at once, at most `needed` (0: no
@@ -608,13 +652,15 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
 // Lanes per row (G) and vectors per lane (R) for a row of `nvec` vectors, at most 256.
 //   SDDMM  few lanes with several vectors each: every index shuffle and every step of the reduction then serves
 //          32 / G nonzeros (R-MAT scale 20, fp32: k = 64 0.35 ms as 8 x 2, 0.38 as 16 x 1; k = 128 0.60 ms as
-//          8 x 4, 0.71 as 32 x 1).
+//          8 x 4, 0.71 as 32 x 1).  9 to 12 vectors go as 4 x 3 (R-MAT scale 17, k = 40: 39 us, 47 as 8 x 2, where a
+//          third of the lanes idles); 13 to 16 do not fit 4 x 4 as well (k = 64, scale 20: 0.375 ms).
 //   SpMM   as many lanes as the row has vectors: an accumulator costs R vectors of registers, and nothing is
 //          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).
 inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
     int g = 4;
     const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
     while (g < top && g < nvec) g <<= 1;
+    if (!spmm && nvec > 8 && nvec <= 12) g = 4;
     int r = (nvec + g - 1) / g;
     r = r <= 4 ? r : 8;
     *G = g;
@@ -624,6 +670,7 @@ inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
 #define SP3_SDDMM_SHAPES(MACRO)                                                                           \
     switch (G * 16 + R) {                                                                                 \
         case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
+        case 4 * 16 + 3: MACRO(4, 3); break;                                                              \
         case 8 * 16 + 2: MACRO(8, 2); break;   case 8 * 16 + 3: MACRO(8, 3); break;                       \
         case 8 * 16 + 4: MACRO(8, 4); break;   case 16 * 16 + 3: MACRO(16, 3); break;                     \
         case 16 * 16 + 4: MACRO(16, 4); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \

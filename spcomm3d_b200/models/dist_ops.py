@@ -109,7 +109,16 @@ class _Dist3DOp:
 
     # ---- helpers ---------------------------------------------------------
     def _alloc_local(self, side):
-        return torch.zeros(side.n_local, self.k_loc, dtype=self.dtype, device=self.device)
+        """A local dense block as (padded storage, block).  On a single GPU nothing is exchanged, so the rows of an
+        operand can lie a whole number of 16-byte vectors apart whatever k is; the padding columns are zero and stay
+        zero, and the kernels read full vectors across them.  Elsewhere the block is contiguous (the collectives
+        move whole rows)."""
+        ld = self.k_loc
+        if self.mesh.size == 1 and self.device.type == "cuda" and self.variant in ("sparse", "sparseNRB"):
+            per = 16 // torch.empty((), dtype=self.dtype).element_size()
+            ld = (ld + per - 1) // per * per
+        full = torch.zeros(side.n_local, ld, dtype=self.dtype, device=self.device)
+        return full, full[:, :self.k_loc]
 
     def _exchange(self, side, group):
         mode = "buffered" if self.variant == "sparse" else "nrb"
@@ -204,7 +213,7 @@ class DistSDDMM(_Dist3DOp):
                 "heap", "fabric", "timeout_s", "overlap", "direct_push", "stage_a", "zreduce", "bulk_pull")})
             self.A_loc, self.B_loc = self._fused.A_loc, self._fused.B_loc
         else:
-            self.A_loc, self.B_loc = self._alloc_local(p.row), self._alloc_local(p.col)
+            (self._A_full, self.A_loc), (self._B_full, self.B_loc) = self._alloc_local(p.row), self._alloc_local(p.col)
         self.A_owned, self.B_owned = self.A_loc[:p.row.n_owned], self.B_loc[:p.col.n_owned]
         self.partial = torch.zeros(p.nnz, dtype=dtype, device=self.device)
         self.exAB = None
@@ -231,7 +240,7 @@ class DistSDDMM(_Dist3DOp):
 
     def _run_bound(self) -> torch.Tensor:
         """The run of a single rank without phase timers: one launch."""
-        t = (self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial)
+        t = (self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, self.partial)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
@@ -270,7 +279,7 @@ class DistSDDMM(_Dist3DOp):
                 if self._panels is not None:
                     self._panels.run(self.A_loc, self.B_loc, self.partial)
                 else:
-                    local.sddmm(self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, out=self.partial)
+                    local.sddmm(self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, out=self.partial)
             with t.span("comm2"):
                 c = self.fiber(self.partial)
         if self.mesh.Z == 1:
@@ -334,7 +343,8 @@ class DistSpMM(_Dist3DOp):
                                                        "overlap")})
             self.X_loc, self.Y_loc = self._fused.X_loc, self._fused.Y_loc
         else:
-            self.X_loc, self.Y_loc = self._alloc_local(p.col), self._alloc_local(p.row)
+            self._X_full, self.X_loc = self._alloc_local(p.col)
+            self.Y_loc = torch.zeros(p.row.n_local, self.k_loc, dtype=dtype, device=self.device)
         self.X_owned = self.X_loc[:p.col.n_owned]
         # sparse variants: the result is the owned head of the local Y block (no copy); fused and dense write
         # into a buffer of their own
@@ -384,13 +394,12 @@ class DistSpMM(_Dist3DOp):
 
     def _run_bound(self, beta: float) -> torch.Tensor:
         """The run of a single rank without phase timers: one launch."""
-        t = (self.rowptr, self.colidx, self.vals, self.X_loc, self.Y_loc)
+        t = (self.rowptr, self.colidx, self.vals, self._X_full, self.Y_loc)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
             b = self._bound = cuda_ops.bind_spmm(*t, self.sched)
-        b._record.beta = beta
-        b.launch()
+        b.launch(beta)
         return self.Y_owned
 
     def _local_buffers(self):
@@ -435,7 +444,7 @@ class DistSpMM(_Dist3DOp):
                 if self._panels is not None:
                     self._panels.run(self.X_loc, self.Y_loc, b)
                 else:
-                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self.X_loc, self.Y_loc, b,
+                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self._X_full, self.Y_loc, b,
                                self.sched)
             with t.span("comm2"):
                 self.exY.reduce(self.Y_loc)  # adds the peers' partial rows into the owned head = Y_owned

@@ -56,15 +56,23 @@ class SddmmSpmmStep:
     def make_host_operands(self):
         sd = self.sddmm
         pin = self.device.type == "cuda"
-        self.host = {"A": sd.A_owned.cpu(), "B": sd.B_owned.cpu()}
+        # whole storages travel (rows of an operand may be padded, see `_alloc_local`): one contiguous copy each
+        self._dev_full = {"A": self._owned_storage(sd.A_owned), "B": self._owned_storage(sd.B_owned)}
+        self._host_full = {n: t.cpu() for n, t in self._dev_full.items()}
         if pin:
-            self.host = {n: t.pin_memory() for n, t in self.host.items()}
+            self._host_full = {n: t.pin_memory() for n, t in self._host_full.items()}
+        self.host = {n: t[:, :sd.k_loc] for n, t in self._host_full.items()}
         self._sums = torch.zeros(2, dtype=torch.float64, device=self.device)
         return self.host
 
+    @staticmethod
+    def _owned_storage(t):
+        """The rows of `t` with their padding columns (contiguous)."""
+        return t.as_strided((t.shape[0], t.stride(0)), (t.stride(0), 1)) if t.shape[0] > 1 else t.contiguous()
+
     @property
     def h2d_bytes(self):
-        h = self.host
+        h = self._host_full
         return int(h["A"].numel() * h["A"].element_size() + h["B"].numel() * h["B"].element_size())
 
     @property
@@ -76,26 +84,26 @@ class SddmmSpmmStep:
         SpMM is B: one device-to-device copy), runs SDDMM and SpMM (the SpMM
         overlaps the copy of A) and reads back the checksums of this rank's
         results (two fp64 scalars)."""
-        sd, sp, h = self.sddmm, self.spmm, self.host
+        sd, sp, h, d = self.sddmm, self.spmm, self._host_full, self._dev_full
         if self.device.type == "cuda":
             # B first; while A follows on a copy stream the SpMM (which needs only X = B) already runs
             main = torch.cuda.current_stream(self.device)
             if getattr(self, "_copy_stream", None) is None:
                 self._copy_stream = torch.cuda.Stream(self.device)
                 self._ev_b, self._ev_a = torch.cuda.Event(), torch.cuda.Event()
-            sd.B_owned.copy_(h["B"], non_blocking=True)
+            d["B"].copy_(h["B"], non_blocking=True)
             self._ev_b.record(main)
             self._copy_stream.wait_event(self._ev_b)   # also orders this copy of A after the previous step's SDDMM
             with torch.cuda.stream(self._copy_stream):
-                sd.A_owned.copy_(h["A"], non_blocking=True)
+                d["A"].copy_(h["A"], non_blocking=True)
                 self._ev_a.record(self._copy_stream)
             sp.X_owned.copy_(sd.B_owned)
             y = sp.run_async()
             main.wait_event(self._ev_a)
             c = sd.run_async()
         else:
-            sd.A_owned.copy_(h["A"], non_blocking=True)
-            sd.B_owned.copy_(h["B"], non_blocking=True)
+            d["A"].copy_(h["A"])
+            d["B"].copy_(h["B"])
             sp.X_owned.copy_(sd.B_owned)
             c = sd.run_async()
             y = sp.run_async()

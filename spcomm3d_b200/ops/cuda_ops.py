@@ -264,11 +264,14 @@ def spmm_tma(rowidx, colidx, vals, X, Y, beta=0.0, status=None):
 
 
 def spmm(rowptr, rowidx, colidx, vals, X, Y, beta, sched: SpmmSchedule | None):
-    if USE_SPMM_TMA and X.dtype == torch.float32 and X.shape[1] % 8 == 0 and 8 <= X.shape[1] <= 256:
+    if USE_SPMM_TMA and X.shape[1] == Y.shape[1] and X.dtype == torch.float32 and X.shape[1] % 8 == 0 and 8 <= X.shape[1] <= 256:
         return spmm_tma(rowidx, colidx, vals, X, Y, beta)
     if sched is None:
         sched = SpmmSchedule(rowptr)
     carry, ldc = sched.carry_for(X.shape[1], X.dtype, X.device)
+    if X.shape[1] != Y.shape[1]:
+        bind_spmm(rowptr, colidx, vals, X, Y, sched).launch(float(beta))
+        return Y
     fn = getattr(native.cuda(), f"sp3_cuda_spmm_{_F[X.dtype]}")
     _ck(fn(rowptr.shape[0] - 1, sched.items.shape[0], native.ptr(sched.items), native.ptr(rowptr),
            native.ptr(colidx), native.ptr(vals), native.ptr(X), _ld(X), X.shape[1], float(beta), native.ptr(Y),
@@ -289,7 +292,7 @@ class _SpmmCall(C.Structure):
                 ("ci", C.c_void_p), ("val", C.c_void_p), ("X", C.c_void_p), ("ldx", C.c_longlong), ("Y", C.c_void_p),
                 ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
                 ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
-                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int)]
+                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int), ("k_out", C.c_int)]
 
 
 _checked_calls = False
@@ -320,8 +323,10 @@ class _BoundCall:
                 return False
         return True
 
-    def launch(self):
+    def launch(self, beta=None):
         global LAUNCHES
+        if beta is not None:
+            self._record.beta = beta
         LAUNCHES += 1
         rc = self._fn(self._addr, _raw_stream())
         if rc != 0:
@@ -337,12 +342,12 @@ def bind_sddmm(rowidx, colidx, svals, A, B, out):
 
 
 def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule):
-    """`spmm` bound to its tensors; `launch(beta)`."""
+    """`spmm` bound to its tensors; `launch(beta)`.  X may be wider than Y, see `local.spmm`."""
     p = native.ptr
     carry, ldc = sched.carry_for(X.shape[1], X.dtype, X.device)
     rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(X),
                     _ld(X), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
-                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len)
+                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1])
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry))
 
 

@@ -56,7 +56,8 @@ def sddmm(rowidx, colidx, svals, A, B, out=None):
 
 
 def spmm(rowptr, rowidx, colidx, vals, X, Y, beta: float = 0.0, sched=None):
-    """Y[r] = beta*Y[r] + sum_p vals[p] * X[colidx[p]] over CSR rows r."""
+    """Y[r] = beta*Y[r] + sum_p vals[p] * X[colidx[p]] over CSR rows r.  On a GPU X may have more columns than Y
+    (the padding of its rows to whole 16-byte vectors); Y takes the first ones."""
     nrows = rowptr.shape[0] - 1
     if nrows == 0:
         return Y
