@@ -64,14 +64,27 @@ constexpr bool IS_F32 = sizeof(real) == 4;
 constexpr int MAX_RANKS = 64;
 enum FlagKind : int { F_READY = 0, F_DONE = 1, F_PART = 2, F_KINDS = 3 };
 constexpr int MAX_WAVES = 32;
-// words [C_WAVE0, C_WAVE0 + MAX_WAVES): pull tiles finished per wave (see FusedSddmmArgs::wave_nnz)
-enum Ctrl : int { C_TICKET_MAIN = 0, C_PULLS_DONE = 1, C_MAIN_DONE = 2, C_TICKET_FIN = 3, C_FIN_DONE = 4, C_ABORT = 5, C_TICKET_WORK = 6, C_WORK_DONE = 7, C_TICKET_PUSH = 8, C_TICKET_START = 9, C_START_DONE = 10, C_WAVE0 = 16, C_WORDS = C_WAVE0 + MAX_WAVES };
+// Control words, each on a 128-byte line of its own (a counter that thousands of warps draw tickets from must not
+// share its line with one that others poll).  Lines from C_WAVE0: pull tiles finished per wave (see
+// FusedSddmmArgs::wave_nnz).
+constexpr int CL = 32;
+enum Ctrl : int { C_TICKET_MAIN = 0 * CL, C_PULLS_DONE = 1 * CL, C_MAIN_DONE = 2 * CL, C_TICKET_FIN = 3 * CL, C_FIN_DONE = 4 * CL, C_ABORT = 5 * CL, C_TICKET_WORK = 6 * CL, C_WORK_DONE = 7 * CL, C_TICKET_PUSH = 8 * CL, C_TICKET_START = 9 * CL, C_START_DONE = 10 * CL, C_WAVE0 = 11 * CL, C_WORDS = C_WAVE0 + MAX_WAVES * CL };
 enum Phase : int { PH_START = 1, PH_MAIN = 2, PH_FINISH = 4 };
 enum WaitSite : int { W_READY = 1, W_PULLS = 2, W_PART = 3, W_DONE = 4, W_WORK = 5 };
 
-constexpr int REDUCE_ELEMS = 2048; // values per SDDMM reduce ticket
+constexpr int REDUCE_ELEMS = 2048; // most values per SDDMM reduce ticket
 constexpr int PUSH_ELEMS = 4096;   // partial values per SDDMM push ticket
-constexpr int REDUCE_ROWS = 32;    // owned rows per SpMM reduce ticket
+constexpr int REDUCE_STEP = 128;   // values that a warp adds up in one step (four per lane)
+constexpr int REDUCE_ROWS = 32;    // most owned rows per SpMM reduce ticket
+
+// Size of a reduce ticket: what one warp adds up in a single step (`step`) as long as there are warps for all of it,
+// at most `most`.  A ticket is a serial chain of steps, each a trip to memory: with fixed tickets of 2048 values
+// (32 rows) the reduction of a small block took 24 us, nearly all of it in 30 to 130 busy warps.
+__device__ __forceinline__ int reduce_ticket(long long n, int nwarps, int step, int most) {
+    const long long p = (n + nwarps - 1) / nwarps;
+    const long long t = (p + step - 1) / step * step;
+    return (int)(t < step ? step : (t > most ? most : t));
+}
 
 struct FusedComm {
     int me;                  // my world rank
@@ -143,8 +156,15 @@ __device__ __forceinline__ bool wait_all(const FusedComm& c, int kind, const int
     for (int i = 0; i < n; ++i) ok = wait_flag(c, kind, list[i], site) && ok;
     return ok;
 }
+// The same for a whole block: thread i waits for flag i, the barrier passes the acquire on.  Every thread calls it.
+__device__ __forceinline__ bool block_wait_all(const FusedComm& c, int kind, const int* list, int n, int site) {
+    bool ok = true;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ok = wait_flag(c, kind, list[i], site) && ok;
+    return __syncthreads_and(ok);
+}
 
-__device__ __forceinline__ bool wait_counter(const FusedComm& c, int which, int want, int site) {
+// Bounded wait of one thread for a counter of this launch.
+__device__ __forceinline__ bool poll_counter(const FusedComm& c, int which, int want, int site) {
     const int* p = c.ctrl + which;
     if (ld_acquire_gpu(p) >= want) return true;
     const unsigned long long t0 = globaltimer_ns();
@@ -155,11 +175,17 @@ __device__ __forceinline__ bool wait_counter(const FusedComm& c, int which, int 
         }
         if (aborted(c)) return false;
         if (globaltimer_ns() - t0 > c.timeout_ns) {
-            report(c.status, ST_WAIT_TIMEOUT, site, which, ld_acquire_gpu(p));
+            report(c.status, ST_WAIT_TIMEOUT, site, which / CL, ld_acquire_gpu(p));
             atomicExch(c.ctrl + C_ABORT, 1);
             return false;
         }
     }
+}
+// The same for a warp: one lane polls (all lanes call it).
+__device__ __forceinline__ bool wait_counter(const FusedComm& c, int which, int want, int site) {
+    int ok = 0;
+    if ((threadIdx.x & 31) == 0) ok = poll_counter(c, which, want, site);
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
 __device__ __forceinline__ void start_phase(const FusedComm& c) {
@@ -205,12 +231,26 @@ constexpr int BULK_STAGES = 3;
 constexpr int BULK_MAX_PULLERS = 4;   // puller warps per block
 
 // Pull set-up of a launch (host side -> kernel): how many warps of every block pull with bulk copies (0: vector
-// loads), the bytes of one ring stage and the dense rows of one pull ticket.
+// loads), the bytes of one ring stage, the dense rows of a tile and the pull tickets that a tile is cut into.  Tiles
+// are what waves are made of, tickets are what a warp pulls at a time: a ticket is a serial chain of stages, so small
+// receive lists are cut finer (52 tiles of 256 rows pulled by 52 of 592 pullers took 39 us, cut into 312 tickets
+// 17 us).
 struct PullConfig {
     int pullers;
     unsigned stage_bytes;
     int tile_rows;
+    int split;
 };
+__host__ __device__ inline int pull_tickets(const PullConfig& pc, int n_rows) {
+    return (n_rows + pc.tile_rows - 1) / pc.tile_rows * pc.split;
+}
+// rows of ticket-sized tile part `part` (tile number * split + part of the tile); none past the end of a short tile
+__device__ __forceinline__ void pull_range(const PullConfig& pc, int part, int n_rows, int& r0, int& r1) {
+    const int tile = part / pc.split, fine = (pc.tile_rows + pc.split - 1) / pc.split;
+    const int end = (tile + 1) * pc.tile_rows < n_rows ? (tile + 1) * pc.tile_rows : n_rows;
+    r0 = tile * pc.tile_rows + (part - tile * pc.split) * fine;
+    r1 = r0 + fine < end ? r0 + fine : end;
+}
 inline size_t bulk_smem_bytes(const PullConfig& pc) {
     return pc.pullers > 0 ? (size_t)pc.pullers * BULK_STAGES * (pc.stage_bytes + 8) + 64 : 0;
 }
@@ -317,13 +357,30 @@ struct PullSide {
     int n_rows;
 };
 
+// What a block knows of the waves.  One warp of a block polls the wave counters, the others look here: with every
+// warp polling, 3,000 of them kept the counter's L2 slice busy and delayed the pulls they waited for.
+struct BlockWaves {
+    int ready;    // leading waves known to be complete
+    int polling;  // 1: a warp of the block is polling
+};
+__device__ __forceinline__ int ld_acquire_cta(const int* p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_cta(int* p, int v) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
+
 struct PullGate {
     FusedComm c;                // a copy: pointing into the kernel's parameters would move all of them to local memory
     PullSide side[2];           // SDDMM: [0] = B rows, [1] = staged A rows; SpMM: [0] = X rows
     const int* order;           // ticket -> side << 30 | tile (null: all tiles of side 1, then side 0)
     const long long* limit;     // shared memory: work runnable once the first w waves are complete, w = 0 .. n_waves
+    BlockWaves* known;          // shared memory: what this block knows of the waves
     long long ld_v;
-    int nvec, tile_rows, n_pull, tiles1, tpw, n_waves;
+    PullConfig pc;
+    int nvec, n_pull, tiles1, tpw, n_waves;
     bool bulk, pulls_left;
     int waves_ready;            // leading waves this warp knows to be complete
     int pending;                // bulk mode: ticket whose stores are issued but not yet published (-1: none)
@@ -334,7 +391,7 @@ struct PullGate {
         __threadfence();
         __syncwarp();
         if (lane == 0) {
-            atomicAdd(c.ctrl + C_WAVE0 + t / tpw, 1);
+            atomicAdd(c.ctrl + C_WAVE0 + t / tpw * CL, 1);
             if (atomicAdd(c.ctrl + C_PULLS_DONE, 1) == n_pull - 1) stamp(c, T_PULLED);
         }
     }
@@ -354,8 +411,9 @@ struct PullGate {
         const int code = order ? __ldg(order + t) : (t < tiles1 ? (t | (1 << 30)) : t - tiles1);
         const int tile = code & ((1 << 30) - 1);
         const PullSide& sd = side[code >> 30];
-        const int r0 = tile * tile_rows;
-        const int r1 = r0 + tile_rows < sd.n_rows ? r0 + tile_rows : sd.n_rows;
+        int r0, r1;
+        pull_range(pc, tile, sd.n_rows, r0, r1);
+        if (r0 >= r1) { publish(t, lane); return true; }
         if (bulk) {
             const bool ok = bulk_pull_tile(br, c, r0, r1, sd.src, sd.dst, nvec, lane, false, [&]() {
                 if (pending >= 0) { publish(pending, lane); pending = -1; }
@@ -379,13 +437,37 @@ struct PullGate {
         while (waves_ready < n_waves && upto > limit[waves_ready]) {
             const int w = waves_ready;
             const int want = (w + 1) * tpw <= n_pull ? tpw : n_pull - w * tpw;
-            if (ld_acquire_gpu(c.ctrl + C_WAVE0 + w) >= want) { ++waves_ready; continue; }
-            if (pulls_left) { pulls_left = pull_one(lane); continue; }
+            if (pulls_left) {
+                if (ld_acquire_gpu(c.ctrl + C_WAVE0 + w * CL) >= want) ++waves_ready;
+                else pulls_left = pull_one(lane);
+                continue;
+            }
             flush(lane);   // never wait while a tile of this warp is unpublished
-            if (!wait_counter(c, C_WAVE0 + w, want, W_PULLS)) return false;
-            ++waves_ready;
+            int now = 0;
+            if (lane == 0) now = await_wave(w, want);
+            waves_ready = __shfl_sync(0xffffffffu, now, 0);
+            if (waves_ready <= w) return false;
         }
         return true;
+    }
+    // One thread: leading waves complete, more than w; w when the wait ran out.  The polling thread's wait has a time
+    // limit and ends by setting `ready` or the abort flag; the others give up after twice that time.
+    __device__ __noinline__ int await_wave(int w, int want) {
+        const unsigned long long t0 = globaltimer_ns();
+        for (int i = 0;; ++i) {
+            const int r = ld_acquire_cta(&known->ready);
+            if (r > w) return r;
+            if (atomicCAS(&known->polling, 0, 1) == 0) {
+                const bool ok = ld_acquire_cta(&known->ready) > w || poll_counter(c, C_WAVE0 + w * CL, want, W_PULLS);
+                if (ok && ld_acquire_cta(&known->ready) <= w) st_release_cta(&known->ready, w + 1);
+                __threadfence_block();
+                atomicExch(&known->polling, 0);
+                if (!ok) return w;
+                continue;
+            }
+            __nanosleep(100);
+            if ((i & 63) == 63 && (aborted(c) || globaltimer_ns() - t0 > 2 * c.timeout_ns)) return w;
+        }
     }
     __device__ __forceinline__ bool ensure(long long upto, int lane) {
         if (waves_ready >= n_waves || upto <= limit[waves_ready]) return true;
@@ -399,22 +481,21 @@ __device__ __forceinline__ void clear_ctrl(const FusedComm& c, int lane) {
     for (int i = lane; i < C_WORDS; i += 32) c.ctrl[i] = 0;
 }
 
-// Every warp calls this after its MAIN work; the last one to arrive publishes
+// Every thread calls this after its MAIN work; the last block to arrive publishes
 // DONE and PART for this rank.
-__device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane, int nwarps) {
+__device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane) {
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
     // remote stores (pushed partial results) must be visible system-wide before PART is signalled; a rank
-    // that pushed nothing only has to order its local writes
-#ifndef SP3_EPILOGUE_GPU_FENCE
+    // that pushed nothing only has to order its local writes.  One fence per block, behind the barrier: it covers
+    // what the other warps of the block wrote.
     if (c.n_push > 0) __threadfence_system();
     else __threadfence();
-#else
-    __threadfence();
-#endif
     __syncwarp();
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_MAIN_DONE, 1);
     old = __shfl_sync(0xffffffffu, old, 0);
-    if (old == nwarps - 1) {
+    if (old == (int)gridDim.x - 1) {
         __threadfence_system();
         for (int i = lane; i < c.n_read; i += 32) signal(c, F_DONE, c.read_from[i]);
         for (int i = lane; i < c.n_push; i += 32) signal(c, F_PART, c.push_to[i]);
@@ -423,14 +504,15 @@ __device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane, int 
     }
 }
 
-// Last warp of the FINISH phase keeps the kernel alive until every reader of
+// Last block of the FINISH phase keeps the kernel alive until every reader of
 // this rank's memory is done with it.
-__device__ __forceinline__ void finish_epilogue(const FusedComm& c, int lane, int nwarps) {
-    __syncwarp();
+__device__ __forceinline__ void finish_epilogue(const FusedComm& c, int lane) {
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_FIN_DONE, 1);
     old = __shfl_sync(0xffffffffu, old, 0);
-    if (old == nwarps - 1) {
+    if (old == (int)gridDim.x - 1) {
         if (lane == 0) {
             wait_all(c, F_DONE, c.readers, c.n_readers, W_DONE);
             stamp(c, T_FINISH);
@@ -489,8 +571,8 @@ struct FusedSddmmArgs {
     long long part_stride;
     // Pull waves.  The pull tickets are served in the order pull_order[t] (bit 30 set: tile of needed A rows,
     // else tile of needed B rows; low bits: tile number; null: A tiles then B tiles) and grouped into n_waves
-    // waves of tiles_per_wave consecutive tickets.  The nonzeros are given sorted by the last wave that brings
-    // one of their two rows (class 0: both rows owned); wave_nnz[c] (c = 0..n_waves) is the number of nonzeros
+    // waves of tiles_per_wave consecutive tickets (parts of tiles, see PullConfig).  The nonzeros are given sorted by
+    // the last wave that brings one of their two rows (class 0: both rows owned); wave_nnz[c] (c = 0..n_waves) is the number of nonzeros
     // that can be computed once the first c waves are complete.  A work unit waits only for the waves its own
     // nonzeros need, so compute follows the pulls wave by wave instead of starting after the last tile.
     const int* pull_order;
@@ -560,26 +642,28 @@ __device__ __forceinline__ long long slice_off(int z, unsigned zbase, unsigned z
 
 template <int G, int R>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(const FusedSddmmArgs a) {
+    after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
     const int parity = c.epoch & 1;
     __shared__ unsigned long long a_bases[MAX_RANKS];
     __shared__ long long wave_limit[MAX_WAVES + 1];
+    __shared__ BlockWaves block_waves;
+    if (threadIdx.x == 0) block_waves = {0, 0};
     extern __shared__ __align__(128) unsigned char dyn_smem[];   // bulk mode: the pullers' rings, else nothing
     if (threadIdx.x < MAX_RANKS) a_bases[threadIdx.x] = threadIdx.x < a.world ? a.a_bases[threadIdx.x] : 0ull;
     const bool bulk = a.pull.pullers > 0;
-    const int PULL_ROWS = a.pull.tile_rows;
     BulkRing br = bulk_ring_init(dyn_smem, a.pull, threadIdx.x >> 5, lane);
     __syncthreads();
     if (c.phases & PH_START) start_phase(c);
     if (c.phases & PH_MAIN) {
         if (!(c.phases & PH_START) && blockIdx.x == 0 && threadIdx.x == 0) stamp(c, T_START);
-        bool ok = wait_all(c, F_READY, c.read_from, c.n_read, W_READY);
+        bool ok = block_wait_all(c, F_READY, c.read_from, c.n_read, W_READY);
         constexpr int SLOTS = 32 / G;
         // pull tickets: tiles of needed A rows first (when A rows are staged), then tiles of needed B rows
-        const int n_pull_a = (a.n_recv_a + PULL_ROWS - 1) / PULL_ROWS;
-        const int n_pull = n_pull_a + (a.n_recv_b + PULL_ROWS - 1) / PULL_ROWS;
+        const int n_pull_a = pull_tickets(a.pull, a.n_recv_a);
+        const int n_pull = n_pull_a + pull_tickets(a.pull, a.n_recv_b);
         const int per_unit = window_nnz(a.nnz, nwarps, SLOTS);   // nonzeros of a work unit
         const long long n_units = (a.nnz + per_unit - 1) / per_unit;
         const bool aligned = ((unsigned long long)a.rowidx | (unsigned long long)a.colidx) % 16 == 0;
@@ -610,8 +694,9 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
         gate.side[1] = {a.a_src, reinterpret_cast<float4*>(a.A_stage), a.n_recv_a};
         gate.order = a.pull_order;
         gate.limit = wave_limit;
+        gate.known = &block_waves;
         gate.ld_v = ldb_v;
-        gate.nvec = a.nvec; gate.tile_rows = PULL_ROWS; gate.n_pull = n_pull; gate.tiles1 = n_pull_a;
+        gate.nvec = a.nvec; gate.pc = a.pull; gate.n_pull = n_pull; gate.tiles1 = n_pull_a;
         gate.tpw = a.n_waves > 0 ? a.tiles_per_wave : (n_pull > 0 ? n_pull : 1);
         gate.n_waves = n_waves;
         gate.bulk = bulk;
@@ -682,15 +767,16 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
                 }
             }
         }
-        main_epilogue(c, lane, nwarps);
+        main_epilogue(c, lane);
     }
     if (c.phases & PH_FINISH) {
         if (a.Z > 1) {
-            bool ok = wait_all(c, F_PART, c.contrib, c.n_contrib, W_PART);
+            bool ok = block_wait_all(c, F_PART, c.contrib, c.n_contrib, W_PART);
             // my own partials come from my own MAIN warps (same launch): wait for all of them
-            if (ok && (c.phases & PH_MAIN)) ok = wait_counter(c, C_MAIN_DONE, nwarps, W_PART);
+            if (ok && (c.phases & PH_MAIN)) ok = wait_counter(c, C_MAIN_DONE, (int)gridDim.x, W_PART);
             const long long my_len = a.zbase + ((unsigned)a.my_z < a.zrem ? 1 : 0);
-            const int n_chunks = (int)((my_len + REDUCE_ELEMS - 1) / REDUCE_ELEMS);
+            const int per = reduce_ticket(my_len, nwarps, REDUCE_STEP, REDUCE_ELEMS);
+            const int n_chunks = (int)((my_len + per - 1) / per);
             const real* mine = a.zbuf[a.my_z] + (long long)parity * a.Z * a.zwidth;
             const real* own = a.part + slice_off(a.my_z, a.zbase, a.zrem);
 #if SP3_FUSED_IS_F32
@@ -701,8 +787,8 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
                 if (t >= n_chunks) break;
                 const long long s0 = slice_off(a.my_z, a.zbase, a.zrem);
                 const real* src = a.mc_part + (long long)parity * a.part_stride;   // 16-byte aligned
-                const long long j0 = s0 + (long long)t * REDUCE_ELEMS;
-                const long long j1 = j0 + REDUCE_ELEMS < s0 + my_len ? j0 + REDUCE_ELEMS : s0 + my_len;
+                const long long j0 = s0 + (long long)t * per;
+                const long long j1 = j0 + per < s0 + my_len ? j0 + per : s0 + my_len;
                 const long long b0 = (j0 + 3) & ~3ll, b1 = j1 & ~3ll;     // aligned body [b0, b1)
                 if (b0 >= b1) {
                     for (long long j = j0 + lane; j < j1; j += 32) a.out[j - s0] = multimem_add_f32(src + j);
@@ -720,8 +806,8 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
             while (ok && a.direct_push != 3) {
                 const int t = warp_ticket(c.ctrl + C_TICKET_FIN, lane);
                 if (t >= n_chunks) break;
-                const long long e0 = (long long)t * REDUCE_ELEMS;
-                const long long e1 = e0 + REDUCE_ELEMS < my_len ? e0 + REDUCE_ELEMS : my_len;
+                const long long e0 = (long long)t * per;
+                const long long e1 = e0 + per < my_len ? e0 + per : my_len;
                 // four values per lane and step, so that 4 * Z independent loads are in flight per lane
                 for (long long j = e0 + lane; j < e1; j += 128) {
                     real s[4] = {(real)0, (real)0, (real)0, (real)0};  // fiber ranks in ascending order; my own partial comes from `part`
@@ -737,7 +823,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
                 }
             }
         }
-        finish_epilogue(c, lane, nwarps);
+        finish_epilogue(c, lane);
     }
 }
 
@@ -848,30 +934,33 @@ struct EmitOwnedOrAdd {
 // nothing or little (meshes 1 x Y x Z).
 template <int G, int R, bool ATOMIC, bool GATED>
 __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(const FusedSpmmArgs a) {
+    after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
     const int parity = c.epoch & 1;
     extern __shared__ __align__(128) unsigned char dyn_smem[];   // bulk mode: the pullers' rings, else nothing
     __shared__ long long wave_limit[MAX_WAVES + 1];
+    __shared__ BlockWaves block_waves;
+    if (threadIdx.x == 0) block_waves = {0, 0};
     __shared__ int row_ends[256 / 32][SPMM_ENDS];
     int* ends = row_ends[threadIdx.x >> 5];
     const bool bulk = a.pull.pullers > 0;
-    const int PULL_ROWS = a.pull.tile_rows;
     BulkRing br = bulk_ring_init(dyn_smem, a.pull, threadIdx.x >> 5, lane);
     __syncthreads();
     if ((c.phases & PH_START) && !ATOMIC) start_phase(c);
     if ((c.phases & PH_START) && ATOMIC) {
         // scale the rows that peers will add to, then tell readers and contributors that this rank is ready
         if (blockIdx.x == 0 && threadIdx.x == 0) stamp(c, T_START);
-        const int n_chunks = (a.n_crows + REDUCE_ROWS - 1) / REDUCE_ROWS;
+        const int per = reduce_ticket(a.n_crows, nwarps, a.nvec < 32 ? 32 / a.nvec : 1, REDUCE_ROWS);
+        const int n_chunks = (a.n_crows + per - 1) / per;
         vec* Yv = reinterpret_cast<vec*>(a.Y);
         const long long ldy_v = a.ldy / VN;
         for (;;) {
             const int t = warp_ticket(c.ctrl + C_TICKET_START, lane);
             if (t >= n_chunks) break;
-            const int r0 = t * REDUCE_ROWS;
-            const int r1 = r0 + REDUCE_ROWS < a.n_crows ? r0 + REDUCE_ROWS : a.n_crows;
+            const int r0 = t * per;
+            const int r1 = r0 + per < a.n_crows ? r0 + per : a.n_crows;
             const int total = (r1 - r0) * a.nvec;
             for (int e = lane; e < total; e += 32) {
                 vec* y = Yv + (long long)__ldg(a.crows + r0 + e / a.nvec) * ldy_v + e % a.nvec;
@@ -892,12 +981,12 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
     }
     if (c.phases & PH_MAIN) {
         if (!(c.phases & PH_START) && blockIdx.x == 0 && threadIdx.x == 0) stamp(c, T_START);
-        bool ok = wait_all(c, F_READY, c.read_from, c.n_read, W_READY);
-        if (ATOMIC) ok = wait_all(c, F_READY, c.push_to, c.n_push, W_READY) && ok;
+        bool ok = block_wait_all(c, F_READY, c.read_from, c.n_read, W_READY);
+        if (ATOMIC) ok = block_wait_all(c, F_READY, c.push_to, c.n_push, W_READY) && ok;
         // atomic mode, START and MAIN in one launch: my own START warps scale (or clear) the rows that receive
         // contributions with plain stores; nobody may add into them, me included, before all of them are done
         if (ATOMIC && (c.phases & PH_START)) ok = wait_counter(c, C_START_DONE, nwarps, W_READY) && ok;
-        const int n_pull = (a.n_recv_x + PULL_ROWS - 1) / PULL_ROWS;
+        const int n_pull = pull_tickets(a.pull, a.n_recv_x);
         vec* Xv = reinterpret_cast<vec*>(a.X_loc);
         const long long ldx_v = a.ldx / VN;
         const char* Xb = reinterpret_cast<const char*>(Xv);
@@ -913,9 +1002,10 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
             while (ok && (!bulk || (int)(threadIdx.x >> 5) < a.pull.pullers) && !aborted(c)) {
                 const int t = warp_ticket(c.ctrl + C_TICKET_MAIN, lane);
                 if (t >= n_pull) break;
-                const int r0 = t * PULL_ROWS;
-                const int r1 = r0 + PULL_ROWS < a.n_recv_x ? r0 + PULL_ROWS : a.n_recv_x;
-                if (bulk) { if (!bulk_pull_tile(br, c, r0, r1, a.x_src, xdst, a.nvec, lane, true, [] {})) break; }
+                int r0, r1;
+                pull_range(a.pull, t, a.n_recv_x, r0, r1);
+                if (r0 >= r1) {}
+                else if (bulk) { if (!bulk_pull_tile(br, c, r0, r1, a.x_src, xdst, a.nvec, lane, true, [] {})) break; }
                 else pull_rows(r0, r1, a.x_src, xdst, ldx_v, a.nvec, lane);
                 __threadfence();
                 __syncwarp();
@@ -961,8 +1051,9 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
             gate.side[1] = {nullptr, nullptr, 0};
             gate.order = a.pull_order;
             gate.limit = wave_limit;
+        gate.known = &block_waves;
             gate.ld_v = ldx_v;
-            gate.nvec = a.nvec; gate.tile_rows = PULL_ROWS; gate.n_pull = n_pull; gate.tiles1 = 0;
+            gate.nvec = a.nvec; gate.pc = a.pull; gate.n_pull = n_pull; gate.tiles1 = 0;
             gate.tpw = a.n_waves > 0 ? a.tiles_per_wave : (n_pull > 0 ? n_pull : 1);
             gate.n_waves = n_waves;
             gate.bulk = bulk;
@@ -992,23 +1083,24 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
             }
             if (ok) gate.pull_all(lane);  // no item left but tiles remain (tiny blocks)
         }
-        main_epilogue(c, lane, nwarps);
+        main_epilogue(c, lane);
     }
     if (c.phases & PH_FINISH) {
-        bool ok = wait_all(c, F_PART, c.contrib, c.n_contrib, W_PART);
+        bool ok = block_wait_all(c, F_PART, c.contrib, c.n_contrib, W_PART);
         // my own partial rows come from my own MAIN warps (same launch): wait for all of them
-        if (ok && (c.phases & PH_MAIN)) ok = wait_counter(c, C_MAIN_DONE, nwarps, W_PART);
+        if (ok && (c.phases & PH_MAIN)) ok = wait_counter(c, C_MAIN_DONE, (int)gridDim.x, W_PART);
         // only rows that receive contributions are touched: crows lists them, cptr/cslot their slot rows in
         // ascending source order
-        const int n_chunks = (a.n_crows + REDUCE_ROWS - 1) / REDUCE_ROWS;
+        const int per = reduce_ticket(a.n_crows, nwarps, a.nvec < 64 ? 64 / a.nvec : 1, REDUCE_ROWS);
+        const int n_chunks = (a.n_crows + per - 1) / per;
         const vec* Sv = reinterpret_cast<const vec*>(a.slots) + (parity ? a.parity_off_v : 0);
         vec* Yv = reinterpret_cast<vec*>(a.Y);
         const long long lds_v = a.lds / VN, ldy_v = a.ldy / VN;
         while (ok && !ATOMIC) {  // atomic mode: the contributions are already in Y
             const int t = warp_ticket(c.ctrl + C_TICKET_FIN, lane);
             if (t >= n_chunks) break;
-            const int r0 = t * REDUCE_ROWS;
-            const int r1 = r0 + REDUCE_ROWS < a.n_crows ? r0 + REDUCE_ROWS : a.n_crows;
+            const int r0 = t * per;
+            const int r1 = r0 + per < a.n_crows ? r0 + per : a.n_crows;
             const int total = (r1 - r0) * a.nvec;
             // two elements per lane and step: their loads (own row, slot rows) are independent and overlap
             for (int e = lane; e < total; e += 64) {
@@ -1041,7 +1133,7 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
                     if (y[q]) *y[q] = s[q];
             }
         }
-        finish_epilogue(c, lane, nwarps);
+        finish_epilogue(c, lane);
     }
 }
 
@@ -1071,7 +1163,7 @@ template <typename K, typename A>
 static int launch_resident(K kernel, ResidentCache& cache, const A& args, long long needed, cudaStream_t st) {
     A copy = args;
     void* params[] = {&copy};
-    if (args.pull.pullers < 0 || args.pull.pullers > BULK_MAX_PULLERS || args.pull.tile_rows < 1 ||
+    if (args.pull.pullers < 0 || args.pull.pullers > BULK_MAX_PULLERS || args.pull.tile_rows < 1 || args.pull.split < 1 ||
         (args.pull.pullers > 0 && (args.pull.stage_bytes < 1024 || args.pull.stage_bytes % 16)))
         return (int)cudaErrorInvalidValue;
     const size_t smem = bulk_smem_bytes(args.pull);
@@ -1080,6 +1172,8 @@ static int launch_resident(K kernel, ResidentCache& cache, const A& args, long l
         if (e != cudaSuccess) return (int)e;
     }
     const unsigned blocks = resident_blocks(kernel, cache, needed, 256, smem);
+    // phases without MAIN wait for nothing that a warp of the same launch still has to do
+    if (!(args.comm.phases & PH_MAIN)) return launch_early(kernel, blocks, smem, st, copy);
     return (int)cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(256), params, smem, st);
 }
 
@@ -1106,9 +1200,9 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_sddmm_, SP3_FUSED_SUFFIX)(const void* args, 
     int G, R, rc = 0;
     pick_shape(a.nvec, &G, &R, false);
     const long long slice = a.zbase + (a.zrem ? 1 : 0);
-    const long long fin = a.Z > 1 ? (slice + REDUCE_ELEMS - 1) / REDUCE_ELEMS : 1;
+    const long long fin = a.Z > 1 ? (slice + REDUCE_STEP - 1) / REDUCE_STEP : 1;
     const long long units = (a.nnz + 4 * (32 / G) - 1) / (4 * (32 / G));
-    const long long pulls = ((long long)a.n_recv_a + a.n_recv_b + a.pull.tile_rows - 1) / a.pull.tile_rows + 1;
+    const long long pulls = (long long)pull_tickets(a.pull, a.n_recv_a) + pull_tickets(a.pull, a.n_recv_b);
     const long long needed = blocks_needed(a.comm.phases, units > pulls ? units : pulls, fin, 1);
 #define SP3_FSDDMM(GG, RR) { static ResidentCache cache; rc = launch_resident(fused_sddmm_kernel<GG, RR>, cache, a, needed, st); }
     SP3_SDDMM_SHAPES(SP3_FSDDMM)
@@ -1123,8 +1217,8 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_spmm_, SP3_FUSED_SUFFIX)(const void* args, v
     int G, R, rc = 0;
     pick_shape(a.nvec, &G, &R, true);
     const bool gated = a.wave_items != nullptr && a.n_waves > 0 && a.n_recv_x > 0;
-    const long long rows = ((long long)a.n_crows + REDUCE_ROWS - 1) / REDUCE_ROWS;
-    const long long pulls = ((long long)a.n_recv_x + a.pull.tile_rows - 1) / a.pull.tile_rows + 1;
+    const long long rows = ((long long)a.n_crows * a.nvec + 31) / 32;
+    const long long pulls = pull_tickets(a.pull, a.n_recv_x);
     const long long needed = blocks_needed(a.comm.phases, a.nitems > pulls ? a.nitems : pulls, a.atomic ? 1 : rows,
                                            a.atomic ? rows : 1);
 #define SP3_FSPMM_ONE(GG, RR, AT, GA) { static ResidentCache cache; rc = launch_resident(fused_spmm_kernel<GG, RR, AT, GA>, cache, a, needed, st); }

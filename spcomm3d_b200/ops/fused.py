@@ -23,6 +23,7 @@ from ..utils import native
 from . import cuda_ops
 
 MAX_RANKS = 64
+PULL_BLOCKS = 148 * 2   # resident blocks that can be counted on
 MAX_WAVES = 32   # pull waves a kernel can track (csrc/kernels/fused_impl.cuh)
 F_KINDS = 3
 PH_START, PH_MAIN, PH_FINISH = 1, 2, 4
@@ -41,7 +42,7 @@ class _Comm(C.Structure):
 
 
 class _PullConfig(C.Structure):
-    _fields_ = [("pullers", C.c_int), ("stage_bytes", C.c_uint), ("tile_rows", C.c_int)]
+    _fields_ = [("pullers", C.c_int), ("stage_bytes", C.c_uint), ("tile_rows", C.c_int), ("split", C.c_int)]
 
 
 class _SddmmArgs(C.Structure):
@@ -170,19 +171,27 @@ class _FusedBase:
     def region_sizes_for(self, plan, k_loc):
         return self.region_sizes(plan, k_loc, dtype=self.dtype)
 
-    def _pull_config(self, cfg: _PullConfig):
-        """Pull set-up of this op: bulk mode = `SP3_FUSED_PULLERS` warps per block (default 1) with ring stages
-        of `SP3_FUSED_STAGE_BYTES` (default 8 KB) and pull tickets of about 64 KB; vector-load mode = tickets
+    def _pull_config(self, cfg: _PullConfig, n_rows: int):
+        """Pull set-up of this op for `n_rows` rows to pull: bulk mode = `SP3_FUSED_PULLERS` warps per block
+        (default 1) with ring stages of `SP3_FUSED_STAGE_BYTES` (default 8 KB) and tiles of about 64 KB, each cut
+        into as many pull tickets of at least 16 rows as it takes to give every puller one; vector-load mode = tiles
         of 64 rows."""
         if self.bulk_pull:
             cfg.pullers = max(1, min(4, int(os.environ.get("SP3_FUSED_PULLERS", "1"))))
             stage = int(os.environ.get("SP3_FUSED_STAGE_BYTES", "8192")) // 16 * 16
             cfg.stage_bytes = max(stage, self.row_bytes, 1024)
             tile_bytes = int(os.environ.get("SP3_FUSED_TILE_BYTES", "65536"))
+            share = -(-n_rows // (PULL_BLOCKS * cfg.pullers))
             cfg.tile_rows = max(16, min(1024, tile_bytes // self.row_bytes))
+            cfg.split = -(-cfg.tile_rows // max(16, min(share, cfg.tile_rows)))
         else:
-            cfg.pullers, cfg.stage_bytes, cfg.tile_rows = 0, 0, 64
-        self.tile_rows = int(cfg.tile_rows)
+            cfg.pullers, cfg.stage_bytes, cfg.tile_rows, cfg.split = 0, 0, 64, 1
+        self.tile_rows, self.split = int(cfg.tile_rows), int(cfg.split)
+
+    def _tickets(self, tiles: np.ndarray) -> np.ndarray:
+        """Pull tickets of a sequence of tile codes (side << 30 | tile): every tile's parts one after another."""
+        side, tile = tiles >> 30 << 30, tiles & ((1 << 30) - 1)
+        return (side[:, None] | (tile[:, None] * self.split + np.arange(self.split))).ravel()
 
     def _fn(self, kernel: str):
         return getattr(native.cuda(), f"sp3_fused_{kernel}_{'f64' if self.dtype == torch.float64 else 'f32'}")
@@ -324,7 +333,7 @@ class FusedSDDMM(_FusedBase):
         a.n_recv_a, a.a_src = n_recv_a, self.a_src.data_ptr()
         a.A_stage = self._A_full.data_ptr() + p.row.n_owned * self.row_bytes
         a.pull_order, a.n_waves, a.tiles_per_wave, a.wave_nnz = None, 0, 0, None
-        self._pull_config(a.pull)
+        self._pull_config(a.pull, n_recv_a + p.col.n_recv)
         self.value_order = None   # None: results are stored in the plan's CSR order
         if overlap and (p.col.n_recv + n_recv_a) > 0 and p.nnz > 0:
             order, wave_nnz = self._plan_waves(p, n_recv_a)
@@ -414,9 +423,9 @@ class FusedSDDMM(_FusedBase):
             np.maximum(cls, ca, out=cls)
         order = np.argsort(cls, kind="stable")
         wave_nnz = np.cumsum(np.bincount(cls, minlength=n_waves + 1)).astype(np.int64)
-        self._pull_order = self._dev_i32(pull_order)
+        self._pull_order = self._dev_i32(self._tickets(pull_order))
         self._wave_nnz = self._dev_i64(wave_nnz)
-        self.args.n_waves, self.args.tiles_per_wave = int(n_waves), int(tpw)
+        self.args.n_waves, self.args.tiles_per_wave = int(n_waves), int(tpw) * self.split
         self.wave_nnz = wave_nnz
         return order, wave_nnz
 
@@ -522,7 +531,7 @@ class FusedSpMM(_FusedBase):
         self.crows = self._dev_i32(crows if crows.size else [0])
         self.cslot = self._dev_i32(order if order.size else [0])
         a = self.args = _SpmmArgs()
-        self._pull_config(a.pull)
+        self._pull_config(a.pull, p.col.n_recv)
         # Work items.  With rows to pull, the items are ordered by the pull wave that completes them and the
         # nonzeros of long rows are sorted so that their owned columns come first: the kernel then works on
         # what is there while the X rows arrive.  The re-ordered column indices and values are private copies
@@ -547,8 +556,8 @@ class FusedSpMM(_FusedBase):
             self._colidx = op.colidx.index_select(0, self._val_perm)
             self._vals = op.vals[self._val_perm]
             self._wave_items = self._dev_i32(class_items)
-            a.n_waves, a.tiles_per_wave, a.wave_items = int(n_waves), int(tpw), self._wave_items.data_ptr()
-            self._pull_order = self._dev_i32(pull_order)
+            a.n_waves, a.tiles_per_wave, a.wave_items = int(n_waves), int(tpw) * self.split, self._wave_items.data_ptr()
+            self._pull_order = self._dev_i32(self._tickets(pull_order))
             a.pull_order = self._pull_order.data_ptr()
         else:
             self.sched = cuda_ops.SpmmSchedule(op.rowptr)
