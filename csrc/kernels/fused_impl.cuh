@@ -933,7 +933,7 @@ struct EmitOwnedOrAdd {
 // no wave state: its inner loop keeps all 64 registers of a thread, which is worth 10-15 % on blocks that pull
 // nothing or little (meshes 1 x Y x Z).
 template <int G, int R, bool ATOMIC, bool GATED>
-__global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(const FusedSpmmArgs a) {
+__global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(const FusedSpmmArgs a) {
     after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
@@ -1215,7 +1215,8 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_spmm_, SP3_FUSED_SUFFIX)(const void* args, v
     cudaStream_t st = (cudaStream_t)stream;
     if (a.n_waves > MAX_WAVES) return (int)cudaErrorInvalidValue;
     int G, R, rc = 0;
-    pick_shape(a.nvec, &G, &R, true);
+    const long long x_rows = (long long)a.n_owned_x + a.n_recv_x;
+    pick_shape(a.nvec, &G, &R, true, x_rows * a.nvec * 16 <= CACHED_BYTES);
     const bool gated = a.wave_items != nullptr && a.n_waves > 0 && a.n_recv_x > 0;
     const long long rows = ((long long)a.n_crows * a.nvec + 31) / 32;
     const long long pulls = pull_tickets(a.pull, a.n_recv_x);

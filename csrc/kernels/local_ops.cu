@@ -58,7 +58,7 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // every row exactly once.
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
-__global__ void __launch_bounds__(256, spmm_min_blocks(R))
+__global__ void __launch_bounds__(256, spmm_min_blocks(G, R))
 spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
                   const int* __restrict__ colidx, const T* __restrict__ val, const char* __restrict__ X,
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
@@ -305,11 +305,12 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
 
 template <typename T, int NB, typename Emit>
 int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
-                   const char* X, long long ldx_bytes, int nvec, const Emit& emit, const SpmmLong& lg, cudaStream_t st) {
+                   const char* X, long long ldx_bytes, int nvec, bool cached, const Emit& emit, const SpmmLong& lg,
+                   cudaStream_t st) {
     const bool aligned = ((uintptr_t)ci | (uintptr_t)val) % 16 == 0;
     constexpr bool VECTORS = std::is_same<Emit, EmitLocal<T, NB>>::value;
     int G, R;
-    pick_shape(nvec, &G, &R, true);
+    pick_shape(nvec, &G, &R, true, cached);
     const bool exact = VECTORS && NB == 16 && nvec == G * R;
     const long long needed = ((long long)nitems + 7) / 8;
 #define SP3_SPMM(GG, RR)                                                                                      \
@@ -329,7 +330,7 @@ int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* ro
 template <typename T>
 int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
                 const T* X, long long ldx, int k, T beta, T* Y, long long ldy, SpmmLong lg, cudaStream_t st,
-                int k_out = 0) {
+                int k_out = 0, long long x_rows = 0) {
     if (nrows == 0) return 0;
     const long long ldx_b = ldx * (long long)sizeof(T), ldy_b = ldy * (long long)sizeof(T);
     unsigned long long bits = ldx_b | (uintptr_t)X;
@@ -337,11 +338,12 @@ int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowpt
     if (!padded) bits |= ldy_b | (uintptr_t)Y;
     if (lg.carry) bits |= (uintptr_t)lg.carry | (unsigned long long)lg.ldc * sizeof(T);
     const unsigned long long bytes = (unsigned long long)k * sizeof(T);
+    const bool cached = x_rows > 0 && x_rows * ldx_b <= CACHED_BYTES;   // (x_rows == 0: not known)
     const int nb = vector_bytes<T>(bytes, bits);
     const unsigned long long nvec = bytes / nb;
     if (padded && (bytes | bits) % 16 == 0 && items != nullptr && bytes <= 256 * 16 && ldx_b < 1ll << 32)
         return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, reinterpret_cast<const char*>(X), ldx_b,
-                                     (int)(bytes / 16), EmitPacked<T>{Y, ldy, k_out, beta}, lg, st);
+                                     (int)(bytes / 16), cached, EmitPacked<T>{Y, ldy, k_out, beta}, lg, st);
     if (padded) k = k_out;
     if (padded || items == nullptr || nvec > 256 || nvec == 0 || ldx_b >= 1ll << 32) {
         spmm_scalar_kernel<T><<<(unsigned)(((long long)nrows * 32 + 255) / 256), 256, 0, st>>>(nrows, rowptr, ci, val, X, ldx, k, beta, Y, ldy);
@@ -349,9 +351,9 @@ int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowpt
     }
     const char* x = reinterpret_cast<const char*>(X);
     char* y = reinterpret_cast<char*>(Y);
-    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 16>{y, ldy_b, beta}, lg, st);
-    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 8>{y, ldy_b, beta}, lg, st);
-    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, EmitLocal<T, 4>{y, ldy_b, beta}, lg, st);
+    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 16>{y, ldy_b, beta}, lg, st);
+    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 8>{y, ldy_b, beta}, lg, st);
+    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 4>{y, ldy_b, beta}, lg, st);
     return -1;
 }
 
@@ -437,6 +439,7 @@ struct SpmmCall {
     double beta;
     int k, f64, piece_len;
     int k_out;              // columns of Y (k of X counts the padding of its rows)
+    int x_rows;             // rows of X
 };
 SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *sddmm_bytes = (int)sizeof(SddmmCall);
@@ -456,9 +459,9 @@ SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.piece_len, c.ticket};
     if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
-                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out);
+                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows);
     return launch_spmm<float>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const float*)c.val,
-                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st, c.k_out);
+                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows);
 }
 
 SP3_API int sp3_cuda_rows_f32(int mode, long long n, const long long* idx, const float* src, long long lds,

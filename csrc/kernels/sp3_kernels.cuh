@@ -655,17 +655,31 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
 //          8 x 4, 0.71 as 32 x 1).  9 to 12 vectors go as 4 x 3 (R-MAT scale 17, k = 40: 39 us, 47 as 8 x 2, where a
 //          third of the lanes idles); 13 to 16 do not fit 4 x 4 as well (k = 64, scale 20: 0.375 ms).
 //   SpMM   as many lanes as the row has vectors: an accumulator costs R vectors of registers, and nothing is
-//          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).
-inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
+//          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).  Where that leaves a quarter
+//          of the lanes idle, three vectors per lane (k = 96, R-MAT scale 17: 67 us as 8 x 3, 100 as 32 x 1;
+//          Erdos-Renyi 1 M rows: 1.81 against 1.96 ms; k = 192: 110 us as 16 x 3, 140 as 32 x 2).  Rows of 25 to 32
+//          vectors that come out of the L2 (`cached`) go as 16 x 2, half the instructions per row (k = 128, scale
+//          17: 86 against 101 us); out of device memory the occupancy counts for more (scale 20: 0.74 against
+//          0.69 ms).
+inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false) {
     int g = 4;
     const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
     while (g < top && g < nvec) g <<= 1;
-    if (!spmm && nvec > 8 && nvec <= 12) g = 4;
+    if (spmm) {
+        if (nvec > 16 && nvec <= 24) g = 8;
+        if (nvec > 24 && nvec <= 32 && cached) g = 16;
+        if (nvec > 32 && nvec <= 48) g = 16;
+    } else if (nvec > 8 && nvec <= 12) {
+        g = 4;
+    }
     int r = (nvec + g - 1) / g;
     r = r <= 4 ? r : 8;
     *G = g;
     *R = r;
 }
+// Dense operands of at most this many bytes are expected to stay in the L2 (126 MB, part of it held twice, once per
+// die, and shared with the results and the sparse matrix).
+constexpr long long CACHED_BYTES = 64ll << 20;
 
 #define SP3_SDDMM_SHAPES(MACRO)                                                                           \
     switch (G * 16 + R) {                                                                                 \
@@ -680,14 +694,16 @@ inline void pick_shape(int nvec, int* G, int* R, bool spmm) {
     switch (G * 16 + R) {                                                                                 \
         case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
         case 16 * 16 + 1: MACRO(16, 1); break; case 32 * 16 + 1: MACRO(32, 1); break;                     \
-        case 32 * 16 + 2: MACRO(32, 2); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \
-        case 32 * 16 + 4: MACRO(32, 4); break; default: MACRO(32, 8); break;                              \
+        case 8 * 16 + 3: MACRO(8, 3); break;   case 16 * 16 + 2: MACRO(16, 2); break;                     \
+        case 16 * 16 + 3: MACRO(16, 3); break; case 32 * 16 + 2: MACRO(32, 2); break;                     \
+        case 32 * 16 + 3: MACRO(32, 3); break; case 32 * 16 + 4: MACRO(32, 4); break;                     \
+        default: MACRO(32, 8); break;                                                                     \
     }
 // Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
 // half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.
-__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? (R <= 2 ? 4 : 2) : 1; }
+__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 3 ? 4 : (R == 4 ? 2 : 1); }
 __host__ __device__ constexpr int sddmm_unroll(int R) { return R <= 4 ? 4 : 2; }
 __host__ __device__ constexpr int sddmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : (R <= 4 ? 2 : 1)); }
-__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R <= 3 ? 3 : 2); }
+__host__ __device__ constexpr int spmm_min_blocks(int G, int R) { return R == 1 ? 4 : (R == 2 && G == 32 ? 3 : 2); }
 
 }  // namespace sp3

@@ -139,9 +139,9 @@ class _Dist3DOp:
             buf[side.n_owned:].fill_(float("nan"))
 
     def _single_rank(self) -> bool:
-        """One rank, one GPU, plain kernels: a run is a single launch, which can be bound to its tensors."""
-        return (self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
-                and self._panels is None)
+        """One rank, one GPU, the default kernels: a run is a single launch, which can be bound to its tensors."""
+        return (not local.opt_in_kernels(self.kernel) and self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
+                and self._panels is None and self.plan.nnz > 0)
 
     def _finish(self):
         if not self.timer.enabled:
@@ -156,6 +156,8 @@ class _Dist3DOp:
     def run_async(self, *a, **kw):
         """`run` without phase timers: no host synchronisation, for callers
         that time a whole loop themselves."""
+        if self._single:
+            return self._run_bound(*a, **kw)
         self.timer.enabled = False
         try:
             return self.run(*a, **kw)
@@ -236,7 +238,7 @@ class DistSDDMM(_Dist3DOp):
                                       **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
         self.owned_off, self.owned_len = p.owned_nnz_slice()
         self._bound = None
-        self._single = self._single_rank() and p.nnz > 0
+        self._single = self._single_rank()
 
     def _run_bound(self) -> torch.Tensor:
         """The run of a single rank without phase timers: one launch."""
@@ -255,7 +257,7 @@ class DistSDDMM(_Dist3DOp):
     def run(self) -> torch.Tensor:
         """One distributed SDDMM; returns my slice of C's values."""
         t = self.timer
-        if not t.enabled and self._single and not local.opt_in_kernels("sddmm"):
+        if not t.enabled and self._single:
             return self._run_bound()
         if self.variant == "fused":
             with t.span("comp"):
@@ -390,9 +392,9 @@ class DistSpMM(_Dist3DOp):
                                      **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
 
         self._bound = None
-        self._single = self._single_rank() and p.row.n_local > 0 and p.nnz > 0
+        self._single = self._single_rank()
 
-    def _run_bound(self, beta: float) -> torch.Tensor:
+    def _run_bound(self, beta: float = 0.0) -> torch.Tensor:
         """The run of a single rank without phase timers: one launch."""
         t = (self.rowptr, self.colidx, self.vals, self._X_full, self.Y_loc)
         b = self._bound
@@ -415,7 +417,7 @@ class DistSpMM(_Dist3DOp):
     def run(self, beta: float = 0.0) -> torch.Tensor:
         """One distributed SpMM: Y_owned = beta*Y_owned + (S X)[owned rows]."""
         t, p = self.timer, self.plan
-        if not t.enabled and self._single and not local.opt_in_kernels("spmm"):
+        if not t.enabled and self._single:
             return self._run_bound(beta)
         if self.variant == "fused":
             with t.span("comp"):

@@ -27,9 +27,13 @@ def item_sizes(nnz: int):
     warp, smaller powers of two (down to 16 nonzeros) below that, because the time of a small SpMM is that of its
     longest item: each group of four nonzeros costs one trip to memory.  SP3_LONG_ROW / SP3_ITEM_NNZ override."""
     item = ITEM_NNZ
-    while item > 16 and nnz < item * _TARGET_ITEMS:
+    while item > 16 and nnz < item * _TARGET_ITEMS * 3 // 4:
         item //= 2
-    return (int(os.environ.get("SP3_LONG_ROW", item * (LONG_ROW // ITEM_NNZ))), int(os.environ.get("SP3_ITEM_NNZ", item)))
+    # a piece costs a partial row and a fence beyond its nonzeros: four items long where that has to be cheap, two
+    # where the longest chain decides (Zipf rows, 357 thousand nonzeros, k = 64: 16.5 us with pieces of 128, 20.2
+    # with 256, 20.1 with 64)
+    long_row = LONG_ROW if item == ITEM_NNZ else 2 * item
+    return int(os.environ.get("SP3_LONG_ROW", long_row)), int(os.environ.get("SP3_ITEM_NNZ", item))
 
 
 PIECE_SHIFT = 20   # SPMM_PIECE_SHIFT of csrc/kernels/sp3_kernels.cuh
@@ -292,7 +296,8 @@ class _SpmmCall(C.Structure):
                 ("ci", C.c_void_p), ("val", C.c_void_p), ("X", C.c_void_p), ("ldx", C.c_longlong), ("Y", C.c_void_p),
                 ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
                 ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
-                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int), ("k_out", C.c_int)]
+                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int), ("k_out", C.c_int),
+                ("x_rows", C.c_int)]
 
 
 _checked_calls = False
@@ -347,7 +352,8 @@ def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule):
     carry, ldc = sched.carry_for(X.shape[1], X.dtype, X.device)
     rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(X),
                     _ld(X), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
-                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1])
+                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1],
+                    X.shape[0])
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry))
 
 
