@@ -384,9 +384,16 @@ template <typename T> struct EmitPacked {
             x[0] = acc.x[0]; x[1] = acc.x[1];
         }
         T* y = Y + row * ldy + v * N;
+        if (beta != (T)0) {
+            T old[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) old[j] = y[v * N + j < k ? j : 0];
+#pragma unroll
+            for (int j = 0; j < N; ++j) x[j] += beta * old[j];
+        }
 #pragma unroll
         for (int j = 0; j < N; ++j)
-            if (v * N + j < k) y[j] = beta != (T)0 ? beta * y[j] + x[j] : x[j];
+            if (v * N + j < k) y[j] = x[j];
     }
 };
 
