@@ -585,7 +585,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     // from the loop above: the kernel is compiled for a fixed number of warps)
     clear(acc);
     carry += first_piece * ldc_bytes + off[0];
-#pragma unroll 2
+#pragma unroll 4
     for (int j = slot; j < np; j += SLOTS) {
         Row<T, NB> x[R];
 #pragma unroll

@@ -240,15 +240,18 @@ class DistSDDMM(_Dist3DOp):
         self._bound = None
         self._single = self._single_rank()
 
-    def _run_bound(self) -> torch.Tensor:
-        """The run of a single rank without phase timers: one launch."""
+    def _bind(self):
         t = (self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, self.partial)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
             b = self._bound = cuda_ops.bind_sddmm(*t)
             self._slice = self.partial[self.owned_off:self.owned_off + self.owned_len]
-        b.launch()
+        return b
+
+    def _run_bound(self) -> torch.Tensor:
+        """The run of a single rank without phase timers: one launch."""
+        self._bind().launch()
         return self._slice
 
     def _local_buffers(self):
@@ -394,14 +397,17 @@ class DistSpMM(_Dist3DOp):
         self._bound = None
         self._single = self._single_rank()
 
-    def _run_bound(self, beta: float = 0.0) -> torch.Tensor:
-        """The run of a single rank without phase timers: one launch."""
+    def _bind(self):
         t = (self.rowptr, self.colidx, self.vals, self._X_full, self.Y_loc)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
             b = self._bound = cuda_ops.bind_spmm(*t, self.sched)
-        b.launch(beta)
+        return b
+
+    def _run_bound(self, beta: float = 0.0) -> torch.Tensor:
+        """The run of a single rank without phase timers: one launch."""
+        self._bind().launch(beta)
         return self.Y_owned
 
     def _local_buffers(self):

@@ -62,6 +62,8 @@ class SddmmSpmmStep:
         if pin:
             self._host_full = {n: t.pin_memory() for n, t in self._host_full.items()}
         self.host = {n: t[:, :sd.k_loc] for n, t in self._host_full.items()}
+        self._host_views = dict(self.host)
+        self._native_step = None
         self._sums = torch.zeros(2, dtype=torch.float64, device=self.device)
         return self.host
 
@@ -79,12 +81,27 @@ class SddmmSpmmStep:
     def d2h_bytes(self):
         return 16
 
+    def _bound_step(self):
+        """The step of a single GPU as one native call (bound again when an operator had a tensor replaced)."""
+        from ..ops import cuda_ops
+        sd, sp, h, d = self.sddmm, self.spmm, self._host_full, self._dev_full
+        bs, bp = sd._bind(), sp._bind()
+        if self._native_step is None or self._native_step[0] is not bs or self._native_step[1] is not bp:
+            x = self._owned_storage(sp.X_owned)
+            self._native_step = (bs, bp, cuda_ops.HostStep(bs, bp, h["A"], h["B"], d["A"], d["B"], x, sp.Y_owned,
+                                                           self.plan.rowptr, self.device))
+        return self._native_step[2]
+
     def run_e2e(self):
         """Copies the step's inputs A and B from pinned host memory (X of the
         SpMM is B: one device-to-device copy), runs SDDMM and SpMM (the SpMM
         overlaps the copy of A) and reads back the checksums of this rank's
         results (two fp64 scalars)."""
         sd, sp, h, d = self.sddmm, self.spmm, self._host_full, self._dev_full
+        if any(self.host[n] is not v for n, v in self._host_views.items()):   # other operands put in their place
+            h, d = self.host, {"A": sd.A_owned, "B": sd.B_owned}
+        elif sd._single and sp._single:
+            return self._bound_step().run()
         if self.device.type == "cuda":
             # B first; while A follows on a copy stream the SpMM (which needs only X = B) already runs
             main = torch.cuda.current_stream(self.device)

@@ -357,6 +357,66 @@ def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule):
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry))
 
 
+STEP_CHUNKS = 8
+STEP_CHUNK_BYTES = 4 << 20   # parts of A of this size: a fraction of the copy, many times the cost of a launch
+
+
+class _StepCall(C.Structure):
+    _fields_ = [("sddmm", _SddmmCall), ("spmm", _SpmmCall), ("host_a", C.c_void_p), ("host_b", C.c_void_p),
+                ("dev_a", C.c_void_p), ("dev_b", C.c_void_p), ("dev_x", C.c_void_p), ("bytes_a", C.c_longlong),
+                ("bytes_b", C.c_longlong), ("y_values", C.c_longlong), ("n_chunks", C.c_int), ("pad", C.c_int),
+                ("chunk_bytes", C.c_longlong * STEP_CHUNKS), ("chunk_nnz", C.c_longlong * STEP_CHUNKS),
+                ("part", C.c_void_p), ("sums", C.c_void_p), ("host_sums", C.c_void_p), ("copy_stream", C.c_void_p),
+                ("ev_b", C.c_void_p), ("ev_a", C.c_void_p * STEP_CHUNKS)]
+
+
+class HostStep:
+    """A step of one GPU from pinned host operands, queued by one native call (`sp3_cuda_step_call`); `run` waits
+    for the two checksums.  `sddmm` and `spmm` are bound calls, `rowptr` the host CSR row pointer."""
+
+    def __init__(self, sddmm: _BoundCall, spmm: _BoundCall, host_a, host_b, dev_a, dev_b, dev_x, Y, rowptr, device):
+        lib = native.cuda()
+        if int(lib.sp3_cuda_step_size()) != C.sizeof(_StepCall):
+            raise RuntimeError("step record layout differs between Python and the kernel library")
+        p = native.ptr
+        self._part = torch.empty(1024, dtype=torch.float64, device=device)
+        self._sums = torch.empty(2, dtype=torch.float64, device=device)
+        self._out = torch.empty(2, dtype=torch.float64).pin_memory()
+        self._result = self._out.numpy()
+        self._copy = torch.cuda.Stream(device)
+        nbytes = host_a.numel() * host_a.element_size()
+        n = max(1, min(STEP_CHUNKS, nbytes // STEP_CHUNK_BYTES))
+        self._events = [torch.cuda.Event() for _ in range(n + 1)]
+        for e in self._events:
+            e.record(self._copy)   # creates the event
+        nrows, nnz = host_a.shape[0], sddmm._record.nnz
+        rows_end = [nrows * (i + 1) // n for i in range(n)]
+        row_bytes = nbytes // max(1, nrows)
+        ends = [int(rowptr[r]) // 4 * 4 for r in rows_end[:-1]] + [nnz]
+        pad = [0] * (STEP_CHUNKS - n)
+        self._rec = _StepCall(
+            sddmm._record, spmm._record, p(host_a), p(host_b), p(dev_a), p(dev_b), p(dev_x), nbytes,
+            host_b.numel() * host_b.element_size(), Y.numel(), n, 0,
+            (C.c_longlong * STEP_CHUNKS)(*([r * row_bytes for r in rows_end] + pad)),
+            (C.c_longlong * STEP_CHUNKS)(*(ends + pad)), p(self._part), p(self._sums), p(self._out),
+            self._copy.cuda_stream, self._events[0].cuda_event,
+            (C.c_void_p * STEP_CHUNKS)(*([e.cuda_event for e in self._events[1:]] + pad)))
+        self._rec.spmm.beta = 0.0
+        self._addr, self._fn = C.addressof(self._rec), lib.sp3_cuda_step_call
+        self._keep = (sddmm, spmm, host_a, host_b, dev_a, dev_b, dev_x, Y)
+        self._launches = 5 + n
+        self._device = device
+
+    def run(self):
+        global LAUNCHES
+        LAUNCHES += self._launches
+        rc = self._fn(self._addr, _raw_stream())
+        if rc != 0:
+            raise RuntimeError(f"step: CUDA error {rc}")
+        torch.cuda.current_stream().synchronize()
+        return self._result.tolist()
+
+
 def rows(mode, idx, src, dst):
     fn = getattr(native.cuda(), f"sp3_cuda_rows_{_F[src.dtype]}")
     _ck(fn(mode, idx.shape[0], native.ptr(idx), native.ptr(src), _ld(src), native.ptr(dst), _ld(dst),

@@ -139,3 +139,32 @@ def test_spmm_many_items(k):
     deg = np.minimum(rng.zipf(1.9, 30_000), 3000)
     deg = np.concatenate([deg, np.full(8000, 90), [5000, 513, 512]])
     _check_spmm(deg, k, torch.float32, 0.5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gen,k", [("uniform:5:7:3", 3), ("er:70001:50000:3", 33), ("zipf:40000:90000:1.8:300", 64)])
+def test_step_from_host_operands(dtype, gen, k):
+    """The step queued by one native call (operands in one part and in several) leaves what the two operators leave
+    when they are run one after the other on the same operands, and returns the sums of it."""
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    from spcomm3d_b200.parallel.mesh import Mesh3D
+    from spcomm3d_b200.parallel.plan import build_my_plan
+    from spcomm3d_b200.utils import generate
+    m = generate.from_spec(gen, seed=4)
+    _, plan = build_my_plan(m, Mesh3D(1, 1, 1), 0, seed=4)
+    step = SddmmSpmmStep(plan, None, k, dtype, "cuda", seed=2)
+    step.fill_device_operands()
+    c, y = (t.clone() for t in step.run_device())
+    step.make_host_operands()
+    for t in (step.sddmm.A_owned, step.sddmm.B_owned, step.spmm.X_owned, step.sddmm.partial, step.spmm.Y_owned):
+        t.fill_(7.0)
+    for _ in range(2):
+        sums = step.run_e2e()
+    assert torch.equal(step.sddmm.run_async(), c) and torch.equal(step.spmm.Y_owned, y)
+    # the checksum adds fp64 values in a fixed shape; torch adds them in another: both within n u of the magnitudes
+    for got, t in zip(sums, (c, y)):
+        t = t.double()
+        assert abs(got - float(t.sum())) <= 2 * t.numel() * 2.0 ** -53 * float(t.abs().sum())
+    step.host = {"A": step.host["A"] * 2, "B": step.host["B"] * 2}      # operands of the user's own
+    twice = step.run_e2e()
+    assert twice[1] == 2 * sums[1] and twice[0] == 4 * sums[0]
