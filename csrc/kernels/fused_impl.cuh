@@ -121,6 +121,7 @@ __device__ __forceinline__ int warp_ticket(int* ctr, int lane, int n = 1) {
 // the kernel, when other warps already idle) are short: about 1/32 of a warp's share, at most MAX.
 constexpr int SDDMM_WINDOWS_PER_TICKET_MAX = 8;
 constexpr int SPMM_ITEMS_PER_TICKET_MAX = 4;
+constexpr int SPMM_FIXED_ITEMS = 8;   // (items per ticket are 1 up to 64 items per warp)
 
 
 __device__ __forceinline__ bool aborted(const FusedComm& c) {
@@ -513,11 +514,9 @@ __device__ __forceinline__ void finish_epilogue(const FusedComm& c, int lane) {
     if (lane == 0) old = atomicAdd(c.ctrl + C_FIN_DONE, 1);
     old = __shfl_sync(0xffffffffu, old, 0);
     if (old == (int)gridDim.x - 1) {
-        if (lane == 0) {
-            wait_all(c, F_DONE, c.readers, c.n_readers, W_DONE);
-            stamp(c, T_FINISH);
-        }
+        for (int i = lane; i < c.n_readers; i += 32) wait_flag(c, F_DONE, c.readers[i], W_DONE);
         __syncwarp();
+        if (lane == 0) stamp(c, T_FINISH);
         clear_ctrl(c, lane);
     }
 }
@@ -708,8 +707,12 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
         // pulled row.
         if (is_puller && ok) gate.pull_all(lane);
         const int UNITS_PER_TICKET = per_ticket(n_units, nwarps, SDDMM_WINDOWS_PER_TICKET_MAX);
+        // a unit for every warp: no counter, on which thousands of warps would queue up
+        const bool fixed = n_units <= nwarps;
+        long long next_unit = gwarp;
         while (ok) {
-            const long long u0 = (long long)warp_ticket(c.ctrl + C_TICKET_WORK, lane, UNITS_PER_TICKET);
+            const long long u0 = fixed ? next_unit : (long long)warp_ticket(c.ctrl + C_TICKET_WORK, lane, UNITS_PER_TICKET);
+            next_unit = n_units;
             if (u0 >= n_units) break;
             const long long u1 = u0 + UNITS_PER_TICKET < n_units ? u0 + UNITS_PER_TICKET : n_units;
             ok = gate.ensure(u1, lane);
@@ -780,10 +783,10 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
             const real* mine = a.zbuf[a.my_z] + (long long)parity * a.Z * a.zwidth;
             const real* own = a.part + slice_off(a.my_z, a.zbase, a.zrem);
 #if SP3_FUSED_IS_F32
-            while (ok && a.direct_push == 3) {
+            // equal portions, dealt out in advance (a counter would serialise the warps)
+            for (int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); ok && a.direct_push == 3; t += nwarps) {
                 // one load per 16 bytes returns the sum over the fiber, added inside the switch; positions of
                 // the multicast buffer that are not 16-byte aligned (slice edges) are read one value at a time
-                const int t = warp_ticket(c.ctrl + C_TICKET_FIN, lane);
                 if (t >= n_chunks) break;
                 const long long s0 = slice_off(a.my_z, a.zbase, a.zrem);
                 const real* src = a.mc_part + (long long)parity * a.part_stride;   // 16-byte aligned
@@ -803,8 +806,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
                 }
             }
 #endif
-            while (ok && a.direct_push != 3) {
-                const int t = warp_ticket(c.ctrl + C_TICKET_FIN, lane);
+            for (int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); ok && a.direct_push != 3; t += nwarps) {
                 if (t >= n_chunks) break;
                 const long long e0 = (long long)t * per;
                 const long long e1 = e0 + per < my_len ? e0 + per : my_len;
@@ -1012,8 +1014,12 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
                 if (lane == 0 && atomicAdd(c.ctrl + C_PULLS_DONE, 1) == n_pull - 1) stamp(c, T_PULLED);
             }
             const int SPMM_ITEMS_PER_TICKET = per_ticket(a.nitems, nwarps, SPMM_ITEMS_PER_TICKET_MAX);
+            // few items, which are then short ones: dealt out in advance, without a counter to queue up on
+            const bool fixed = a.nitems <= SPMM_FIXED_ITEMS * nwarps;
+            int next_item = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
             while (ok) {
-                const int i0 = warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET);
+                const int i0 = fixed ? next_item : warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET);
+                next_item += nwarps;
                 if (i0 >= a.nitems) break;
                 if (!pulled) {
                     ok = wait_counter(c, C_PULLS_DONE, n_pull, W_PULLS);
@@ -1063,8 +1069,12 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
             gate.br = br;
             if (is_puller && ok) gate.pull_all(lane);
             const int SPMM_ITEMS_PER_TICKET = per_ticket(a.nitems, nwarps, SPMM_ITEMS_PER_TICKET_MAX);
+            // few items, which are then short ones: dealt out in advance, without a counter to queue up on
+            const bool fixed = a.nitems <= SPMM_FIXED_ITEMS * nwarps;
+            int next_item = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
             while (ok) {
-                const int i0 = warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET);
+                const int i0 = fixed ? next_item : warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET);
+                next_item += nwarps;
                 if (i0 >= a.nitems) break;
                 const int i1 = i0 + SPMM_ITEMS_PER_TICKET < a.nitems ? i0 + SPMM_ITEMS_PER_TICKET : a.nitems;
                 ok = gate.ensure(i1, lane);
@@ -1096,8 +1106,8 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
         const vec* Sv = reinterpret_cast<const vec*>(a.slots) + (parity ? a.parity_off_v : 0);
         vec* Yv = reinterpret_cast<vec*>(a.Y);
         const long long lds_v = a.lds / VN, ldy_v = a.ldy / VN;
-        while (ok && !ATOMIC) {  // atomic mode: the contributions are already in Y
-            const int t = warp_ticket(c.ctrl + C_TICKET_FIN, lane);
+        // (atomic mode: the contributions are already in Y)
+        for (int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); ok && !ATOMIC; t += nwarps) {
             if (t >= n_chunks) break;
             const int r0 = t * per;
             const int r1 = r0 + per < a.n_crows ? r0 + per : a.n_crows;

@@ -51,6 +51,13 @@ else:
     _raw_stream = _stream
 
 
+def device_stream(device: torch.device):
+    """Raw handle of the current stream of `device`."""
+    if device.index is None or _raw_stream is _stream:
+        return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
 LAUNCHES = 0  # kernels launched through this module (bench.py reports the count)
 
 

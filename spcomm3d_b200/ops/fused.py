@@ -23,6 +23,7 @@ from ..utils import native
 from . import cuda_ops
 
 MAX_RANKS = 64
+SMALL_PULL_BYTES = int(os.environ.get("SP3_FUSED_SMALL_BYTES", 4 << 20))
 PULL_BLOCKS = 148 * 2   # resident blocks that can be counted on
 MAX_WAVES = 32   # pull waves a kernel can track (csrc/kernels/fused_impl.cuh)
 F_KINDS = 3
@@ -186,6 +187,10 @@ class _FusedBase:
             cfg.split = -(-cfg.tile_rows // max(16, min(share, cfg.tile_rows)))
         else:
             cfg.pullers, cfg.stage_bytes, cfg.tile_rows, cfg.split = 0, 0, 64, 1
+        if self.bulk_auto and n_rows * self.row_bytes <= SMALL_PULL_BYTES:
+            # few rows: every warp loads its share at once, 4 KB per ticket (same tiles, same waves)
+            cfg.pullers, cfg.stage_bytes = 0, 0
+            cfg.split = -(-cfg.tile_rows // max(1, 4096 // self.row_bytes))
         self.tile_rows, self.split = int(cfg.tile_rows), int(cfg.split)
 
     def _tickets(self, tiles: np.ndarray) -> np.ndarray:
@@ -255,9 +260,9 @@ class _FusedBase:
         return {"pull": max(0, t[1] - t[0]) / 1e6, "main": (t[2] - t[0]) / 1e6, "total": (t[3] - t[0]) / 1e6}
 
     def _launch(self, fn, phases):
-        self.args.comm.phases = phases
-        self.args.comm.epoch = self.epoch
-        rc = fn(C.byref(self.args), torch.cuda.current_stream(self.device).cuda_stream)
+        comm = self.args.comm
+        comm.phases, comm.epoch = phases, self.epoch
+        rc = fn(C.byref(self.args), cuda_ops.device_stream(self.device))
         cuda_ops.LAUNCHES += 1
         if rc != 0:
             raise RuntimeError(f"fused kernel launch failed: CUDA error {rc}")
@@ -277,7 +282,9 @@ class FusedSDDMM(_FusedBase):
                  overlap: bool = True, direct_push: bool | None = None, stage_a: bool | None = None,
                  zreduce: str | None = None, bulk_pull: bool | None = None):
         super().__init__(op, heap, fabric, timeout_s)
+        self._kernel = self._fn("sddmm")
         self.bulk_pull = _bulk_default(bulk_pull)
+        self.bulk_auto = bulk_pull is None and "SP3_FUSED_BULK" not in os.environ
         if zreduce is None:
             zreduce = os.environ.get("SP3_FUSED_ZREDUCE", "push")
         if zreduce not in ("push", "multimem"):
@@ -456,7 +463,7 @@ class FusedSDDMM(_FusedBase):
     def launch(self, phases=PH_ALL, new_epoch=True):
         if new_epoch:
             self.epoch += 1
-        self._launch(self._fn("sddmm"), phases)
+        self._launch(self._kernel, phases)
 
     def run(self):
         self.launch()
@@ -487,6 +494,7 @@ class FusedSpMM(_FusedBase):
                  reduce: str | None = None, red_v4: bool | None = None, bulk_pull: bool | None = None,
                  overlap: bool = True):
         self.bulk_pull = _bulk_default(bulk_pull)
+        self.bulk_auto = bulk_pull is None and "SP3_FUSED_BULK" not in os.environ
         if reduce is None:
             reduce = os.environ.get("SP3_FUSED_SPMM_REDUCE", "slots")
         if reduce not in ("slots", "atomic"):
@@ -495,6 +503,7 @@ class FusedSpMM(_FusedBase):
         if red_v4 is None:
             red_v4 = os.environ.get("SP3_FUSED_RED_V4", "1") == "1"
         super().__init__(op, heap, fabric, timeout_s)
+        self._kernel = self._fn("spmm")
         p, h, k, rb = self.plan, self.heap, self.k_loc, self.row_bytes
         rp = p.row
         if self.atomic and "Y" not in h.sizes:
@@ -611,7 +620,7 @@ class FusedSpMM(_FusedBase):
             raise ValueError(f"the result needs a 16-byte aligned base, rows that are a multiple of 16 bytes apart "
                              f"and a leading dimension of at least {self.kpad} (use DistSpMM.Y_owned)")
         a.Y, a.ldy, a.beta = Y.data_ptr(), ldy, float(beta)
-        self._launch(self._fn("spmm"), phases)
+        self._launch(self._kernel, phases)
 
     def run(self, Y: torch.Tensor, beta: float = 0.0):
         self.launch(Y, beta)
