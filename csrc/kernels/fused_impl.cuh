@@ -121,7 +121,7 @@ __device__ __forceinline__ int warp_ticket(int* ctr, int lane, int n = 1) {
 // the kernel, when other warps already idle) are short: about 1/32 of a warp's share, at most MAX.
 constexpr int SDDMM_WINDOWS_PER_TICKET_MAX = 8;
 constexpr int SPMM_ITEMS_PER_TICKET_MAX = 4;
-constexpr int SPMM_FIXED_ITEMS = 8;   // (items per ticket are 1 up to 64 items per warp)
+constexpr int SPMM_FIXED_ITEMS = 1;   // (items per ticket are 1 up to 64 items per warp)
 
 
 __device__ __forceinline__ bool aborted(const FusedComm& c) {

@@ -413,7 +413,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
                                                const char* __restrict__ X, unsigned ldx_bytes, int nvec, bool aligned,
                                                const Emit& emit, const SpmmLong& lg, int* ends, int lane) {
     constexpr unsigned FULL = 0xffffffffu;
-    constexpr int SLOTS = 32 / G;
+    constexpr int SLOTS = 32 / G;            // G need not divide 32: the lanes of slot SLOTS have no share
     const int slot = lane / G, gl = lane % G;
     unsigned off[R];
     bool on[R];
@@ -440,7 +440,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     // positions count from the 16-byte boundary at or before the first nonzero
     const int lead = (int)(p0 & 3), stop = lead + n;
     const int share = ((stop + 4 * SLOTS - 1) / (4 * SLOTS)) * 4;
-    const int begin = slot * share, end = begin + share < stop ? begin + share : stop;
+    const int begin = slot < SLOTS ? slot * share : stop, end = begin + share < stop ? begin + share : stop;
     int row_end_lane = stop;                 // lane l: end of row l of the item
     if (lane < nr) row_end_lane = lead + (int)(__ldg(rowptr + item.x + lane + 1) - p0);
     const int* cp = colidx + (p0 - lead);
@@ -557,13 +557,26 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     }
     // piece of a long row: add up the groups, leave the sum in the carry; the last piece to arrive adds the carries
     // in order
-    auto add_groups = [&]() {
+    auto add_groups = [&]() {                // slot 0 gets the sum of all slots
+        if constexpr ((G & (G - 1)) == 0) {
 #pragma unroll
-        for (int m = G; m < 32; m <<= 1)
+            for (int m = G; m < 32; m <<= 1)
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+#pragma unroll
+                    for (int h = 0; h < Row<T, NB>::N; ++h)
+                        acc[q].x[h] = e_add(acc[q].x[h], __shfl_xor_sync(FULL, acc[q].x[h], m));
+        } else {
 #pragma unroll
             for (int q = 0; q < R; ++q)
 #pragma unroll
-                for (int h = 0; h < Row<T, NB>::N; ++h) acc[q].x[h] = e_add(acc[q].x[h], __shfl_xor_sync(FULL, acc[q].x[h], m));
+                for (int h = 0; h < Row<T, NB>::N; ++h) {
+                    auto sum = acc[q].x[h];
+#pragma unroll
+                    for (int g = 1; g < SLOTS; ++g) sum = e_add(sum, __shfl_sync(FULL, acc[q].x[h], gl + g * G));
+                    acc[q].x[h] = sum;
+                }
+        }
     };
     add_groups();
     const int lr = item.w & ((1 << SPMM_PIECE_SHIFT) - 1);
@@ -586,7 +599,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     clear(acc);
     carry += first_piece * ldc_bytes + off[0];
 #pragma unroll 4
-    for (int j = slot; j < np; j += SLOTS) {
+    for (int j = slot < SLOTS ? slot : np; j < np; j += SLOTS) {
         Row<T, NB> x[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) {
@@ -664,7 +677,9 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
 //   SpMM   as many lanes as the row has vectors: an accumulator costs R vectors of registers, and nothing is
 //          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).  Where that leaves a quarter
 //          of the lanes idle, three vectors per lane (k = 96, R-MAT scale 17: 67 us as 8 x 3, 100 as 32 x 1;
-//          Erdos-Renyi 1 M rows: 1.81 against 1.96 ms; k = 192: 110 us as 16 x 3, 140 as 32 x 2).  Rows of 25 to 32
+//          Erdos-Renyi 1 M rows: 1.81 against 1.96 ms; k = 192: 110 us as 16 x 3, 140 as 32 x 2), and groups of 5, 6
+//          or 10 lanes, which share a warp one group more than 8 or 16 do (k = 40: 41 us as 10 x 1, 51 as 16 x 1;
+//          k = 20: 32 against 35 us; groups of 2 and 3 gained nothing over 4).  Rows of 25 to 32
 //          vectors that come out of the L2 (`cached`) go as 16 x 2, half the instructions per row (k = 128, scale
 //          17: 86 against 101 us); out of device memory the occupancy counts for more (scale 20: 0.74 against
 //          0.69 ms).
@@ -673,6 +688,8 @@ inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false)
     const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
     while (g < top && g < nvec) g <<= 1;
     if (spmm) {
+        if (nvec == 5 || nvec == 6) g = nvec;
+        if (nvec == 9 || nvec == 10) g = 10;
         if (nvec > 16 && nvec <= 24) g = 8;
         if (nvec > 24 && nvec <= 32 && cached) g = 16;
         if (nvec > 32 && nvec <= 48) g = 16;
@@ -700,6 +717,8 @@ constexpr long long CACHED_BYTES = 64ll << 20;
 #define SP3_SPMM_SHAPES(MACRO)                                                                            \
     switch (G * 16 + R) {                                                                                 \
         case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
+        case 5 * 16 + 1: MACRO(5, 1); break;   case 6 * 16 + 1: MACRO(6, 1); break;                       \
+        case 10 * 16 + 1: MACRO(10, 1); break;                                                            \
         case 16 * 16 + 1: MACRO(16, 1); break; case 32 * 16 + 1: MACRO(32, 1); break;                     \
         case 8 * 16 + 3: MACRO(8, 3); break;   case 16 * 16 + 2: MACRO(16, 2); break;                     \
         case 16 * 16 + 3: MACRO(16, 3); break; case 32 * 16 + 2: MACRO(32, 2); break;                     \

@@ -140,8 +140,8 @@ class _Dist3DOp:
 
     def _single_rank(self) -> bool:
         """One rank, one GPU, the default kernels: a run is a single launch, which can be bound to its tensors."""
-        return (not local.opt_in_kernels(self.kernel) and self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
-                and self._panels is None and self.plan.nnz > 0)
+        return (self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
+                and self._panels is None and self.plan.nnz > 0 and not local.opt_in_kernels(self.kernel))
 
     def _finish(self):
         if not self.timer.enabled:

@@ -34,8 +34,6 @@ def _row_major(t: torch.Tensor):
 
 def opt_in_kernels(kernel: str) -> bool:
     """Whether an opt-in kernel (the TMA gather twins) takes the place of the default one on a GPU."""
-    if not torch.cuda.is_available():
-        return False
     from . import cuda_ops
     return cuda_ops.USE_TMA if kernel == "sddmm" else cuda_ops.USE_SPMM_TMA
 
