@@ -352,10 +352,18 @@ struct SpmmLong {
                              // then handed out dynamically
 };
 
+// Previous values of a block of result rows on their way into the L2 (each row end waits for its own, one by one).
+__device__ __forceinline__ void prefetch_rows(const char* p, long long bytes, int lane) {
+    for (long long o = lane * 128; o < bytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
+}
+
 template <typename T, int NB> struct EmitLocal {
     char* Y;
     long long ldy_bytes;
     T beta;
+    __device__ __forceinline__ void expect(int row, int n, int nvec, int lane) const {
+        if (beta != (T)0) prefetch_rows(Y + row * ldy_bytes, (n - 1) * ldy_bytes + nvec * NB, lane);
+    }
     // writes vector v of row `row`
     __device__ __forceinline__ void operator()(int row, int v, Row<T, NB> acc) const {
         char* y = Y + row * ldy_bytes + (long long)v * NB;
@@ -374,6 +382,9 @@ template <typename T> struct EmitPacked {
     long long ldy;
     int k;
     T beta;
+    __device__ __forceinline__ void expect(int row, int n, int, int lane) const {
+        if (beta != (T)0) prefetch_rows(reinterpret_cast<const char*>(Y + row * ldy), ((n - 1) * ldy + k) * (long long)sizeof(T), lane);
+    }
     __device__ __forceinline__ void operator()(int row, int v, const Row<T, 16>& acc) const {
         constexpr int N = 16 / (int)sizeof(T);
         T x[N];
