@@ -32,6 +32,33 @@ sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const in
                                                       arows, B, ldb_bytes, nvec, aligned, store, threadIdx.x & 31);
 }
 
+// out[i] = sval[i] * dots[where[i]], four values per thread: dot products computed chunk by chunk of columns, back into
+// row order.  A row's values of one chunk lie together, so the reads use whole sectors; writing them from the SDDMM
+// itself left partial sectors in device memory and cost more than this pass (Erdos-Renyi 1 M rows, 33.5 M nonzeros,
+// k = 64: about 250 us).
+template <typename T>
+__global__ void __launch_bounds__(256)
+scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* __restrict__ sval, const T* dots, T* out,
+                    bool aligned) {
+    after_previous_kernel();
+    const int n = (int)nnz, i = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
+    if (i >= n) return;
+    const Quad<int> w = quad_load(where, i, n, aligned);
+    const Quad<T> s = quad_load(sval, i, n, aligned);
+    __align__(16) T v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __ldcg(dots + w.v[j]) * s.v[j];
+    if (aligned && i + 4 <= n) {
+        using V = typename Vec<T>::type;
+#pragma unroll
+        for (int j = 0; j < 4; j += Vec<T>::N) *reinterpret_cast<V*>(out + i + j) = *reinterpret_cast<const V*>(v + j);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (i + j < n) out[i + j] = v[j];
+}
+
 // Rows of more than 256 vectors: one warp per nonzero, scalar loads.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -432,6 +459,10 @@ struct SddmmCall {
     long long ldb;
     void* out;
     int k, f64;
+    // null, or: ri and ci are sorted by chunk of columns, the dot products go to `dots`, and the value of nonzero i (row
+    // order) is sv[i] * dots[where[i]]
+    const int* where;
+    void* dots;
 };
 struct SpmmCall {
     int nrows, nitems;
@@ -457,13 +488,18 @@ SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *spmm_bytes = (int)sizeof(SpmmCall);
     return 0;
 }
+template <typename T> static int sddmm_call(const SddmmCall& c, cudaStream_t st) {
+    T* out = (T*)(c.where ? c.dots : c.out);
+    const int rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,
+                                   (const T*)c.B, c.ldb, c.k, out, st);
+    if (rc != 0 || !c.where || c.nnz == 0) return rc;
+    const bool aligned = ((uintptr_t)c.where | (uintptr_t)c.sv | (uintptr_t)c.out) % 16 == 0;
+    return launch_early(scale_picked_kernel<T>, (unsigned)((c.nnz + 1023) / 1024), 0, st, c.nnz, c.where,
+                        (const T*)c.sv, (const T*)c.dots, (T*)c.out, aligned);
+}
 SP3_API int sp3_cuda_sddmm_call(const void* record, void* stream) {
     const SddmmCall& c = *static_cast<const SddmmCall*>(record);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (c.f64) return launch_sddmm<double>(c.nnz, c.ri, c.ci, (const double*)c.sv, (const double*)c.A, c.lda,
-                                           (const double*)c.B, c.ldb, c.k, (double*)c.out, st);
-    return launch_sddmm<float>(c.nnz, c.ri, c.ci, (const float*)c.sv, (const float*)c.A, c.lda, (const float*)c.B,
-                               c.ldb, c.k, (float*)c.out, st);
+    return c.f64 ? sddmm_call<double>(c, (cudaStream_t)stream) : sddmm_call<float>(c, (cudaStream_t)stream);
 }
 SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     const SpmmCall& c = *static_cast<const SpmmCall*>(record);

@@ -239,13 +239,21 @@ class DistSDDMM(_Dist3DOp):
         self.owned_off, self.owned_len = p.owned_nnz_slice()
         self._bound = None
         self._single = self._single_rank()
+        self._chunks = None
+        if self._single:   # the nonzeros once more, chunk by chunk of columns, where B outgrows the L2 and that pays
+            from ..ops import cuda_ops
+            row_bytes = self._B_full.stride(0) * self._B_full.element_size()
+            if 48 <= row_bytes <= 256 * 16:   # (narrower rows take other vectors, wider ones the scalar kernel)
+                self._chunks = cuda_ops.column_chunks(self.rowidx, self.colidx, p.col.n_local, row_bytes)
+            self._chunks_of = (self.rowidx, self.colidx)
 
     def _bind(self):
         t = (self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, self.partial)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
-            b = self._bound = cuda_ops.bind_sddmm(*t)
+            chunks = self._chunks if all(x is y for x, y in zip(t, self._chunks_of)) else None
+            b = self._bound = cuda_ops.bind_sddmm(*t, chunks)
             self._slice = self.partial[self.owned_off:self.owned_off + self.owned_len]
         return b
 
@@ -283,6 +291,8 @@ class DistSDDMM(_Dist3DOp):
             with t.span("comp"):
                 if self._panels is not None:
                     self._panels.run(self.A_loc, self.B_loc, self.partial)
+                elif self._chunks is not None:
+                    self._bind().launch()
                 else:
                     local.sddmm(self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, out=self.partial)
             with t.span("comm2"):

@@ -168,3 +168,55 @@ def test_step_from_host_operands(dtype, gen, k):
     step.host = {"A": step.host["A"] * 2, "B": step.host["B"] * 2}      # operands of the user's own
     twice = step.run_e2e()
     assert twice[1] == 2 * sums[1] and twice[0] == 4 * sums[0]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k, n", [(12, 1), (13, 5), (33, 259), (64, 3001), (128, 130), (200, 2048), (512, 77)])
+def test_sddmm_column_chunks(dtype, k, n, monkeypatch):
+    """Columns chunk by chunk: the values stay in row order and are those of the row-sorted lists, bit for bit (a dot
+    product is computed by the same lanes in either order), through the operator too."""
+    from spcomm3d_b200.models.dist_ops import DistSDDMM
+    from spcomm3d_b200.ops import cuda_ops, local
+    from spcomm3d_b200.parallel.mesh import Mesh3D
+    from spcomm3d_b200.parallel.plan import build_my_plan
+    from spcomm3d_b200.utils.sparse import CooMatrix
+    rng = np.random.default_rng(n)
+    keys = np.sort(rng.choice(60 * 64, n, replace=False))
+    m = CooMatrix(60, 64, (keys // 64).astype(np.int32), (keys % 64).astype(np.int32), rng.random(n))
+    _, plan = build_my_plan(m, Mesh3D(1, 1, 1), 0, seed=1)
+    chosen = []
+
+    def chunks(r, c, n_cols, row_bytes, _f=cuda_ops.column_chunks):
+        chosen.append(_f(r, c, n_cols, row_bytes, force=5))
+        return chosen[-1]
+    monkeypatch.setattr(cuda_ops, "column_chunks", chunks)
+    op = DistSDDMM(plan, None, k, dtype, "cuda")
+    assert chosen and op._chunks is chosen[0]
+    for t, stream in ((op.A_owned, 1), (op.B_owned, 2)):
+        t.copy_(torch.randn(t.shape, generator=torch.Generator().manual_seed(stream), dtype=torch.float64))
+    ref = torch.empty_like(op.partial)
+    local.sddmm(op.rowidx, op.colidx, op.vals, op._A_full, op._B_full, ref)
+    op.partial.fill_(float("nan"))
+    assert torch.equal(op.run_async(), ref)
+    op.partial.fill_(float("nan"))
+    assert torch.equal(op.run(), ref)
+
+
+def test_column_chunks_rule(monkeypatch):
+    """Chunks where every column is read equally often from a B larger than the limit, none where hub columns or the
+    size of B leave nothing to gain."""
+    from spcomm3d_b200.ops import cuda_ops
+    monkeypatch.setattr(cuda_ops, "CHUNK_BYTES", 1 << 18)
+    monkeypatch.setattr(cuda_ops, "CHUNK_MIN_NNZ", 1)
+    rng = np.random.default_rng(0)
+    rows = torch.arange(4096, dtype=torch.int32).repeat_interleave(64).cuda()
+
+    def lists(cols):
+        return rows, torch.from_numpy(np.sort(cols, 1).astype(np.int32)).reshape(-1).cuda()
+    even = lists(rng.integers(0, 4096, (4096, 64)))
+    r, c, where = cuda_ops.column_chunks(*even, 4096, 256)
+    assert torch.equal(r[where.long()], even[0]) and torch.equal(c[where.long()], even[1])
+    assert bool((torch.diff(c // 1024) >= 0).all()) and torch.unique(where).numel() == where.numel()
+    assert cuda_ops.column_chunks(*even, 4096, 48) is None      # fits
+    hubs = lists(np.where(rng.random((4096, 64)) < 0.8, rng.integers(0, 512, (4096, 64)), rng.integers(0, 4096, (4096, 64))))
+    assert cuda_ops.column_chunks(*hubs, 4096, 256) is None
