@@ -20,10 +20,10 @@ namespace sp3 {
 // SDDMM: out[i] = sval[i] * <A[rowidx[i]], B[colidx[i]]>; persistent grid,
 // warps stride over windows of nonzeros (see sddmm_windows).
 // ---------------------------------------------------------------------------
-template <typename T, int NB, int G, int R, bool EXACT, typename Store>
+template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R))
 sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
-                 const RowsByStride arows, const char* __restrict__ B, unsigned ldb_bytes, int nvec, bool aligned,
+                 const Rows arows, const char* __restrict__ B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
     after_previous_kernel();
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -285,11 +285,13 @@ template <typename T> int vector_bytes(unsigned long long bytes, unsigned long l
     return nb;
 }
 
-template <typename T, int NB, typename Store>
+template <typename T, int NB, typename Rows = RowsByStride, typename Store>
 int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, long long lda_bytes, const char* B,
                     long long ldb_bytes, int nvec, const Store& store, cudaStream_t st) {
     const bool aligned = ((uintptr_t)ri | (uintptr_t)ci) % 16 == 0;
-    const RowsByStride arows{A, (unsigned)lda_bytes};
+    Rows arows;
+    arows.base = A;
+    arows.ld_bytes = (unsigned)lda_bytes;
     int G, R;
     pick_shape(nvec, &G, &R, false);
     const bool exact = NB == 16 && nvec == G * R;
@@ -297,8 +299,8 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
     {                                                                                                         \
         static ResidentCache caches[2];                                                                       \
         ResidentCache& cache = caches[exact];                                                                 \
-        auto kernel = exact ? sddmm_vec_kernel<T, NB, GG, RR, NB == 16, Store>                                \
-                            : sddmm_vec_kernel<T, NB, GG, RR, false, Store>;                                  \
+        auto kernel = exact ? sddmm_vec_kernel<T, NB, GG, RR, NB == 16, Rows, Store>                                \
+                            : sddmm_vec_kernel<T, NB, GG, RR, false, Rows, Store>;                                  \
         const unsigned all = resident_blocks(kernel, cache, 0);                                               \
         const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
@@ -312,7 +314,7 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
 
 template <typename T>
 int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const T* A, long long lda, const T* B,
-                 long long ldb, int k, T* out, cudaStream_t st, const int* orig = nullptr) {
+                 long long ldb, int k, T* out, cudaStream_t st, const int* orig = nullptr, bool passing = false) {
     if (nnz == 0) return 0;
     const long long lda_b = lda * (long long)sizeof(T), ldb_b = ldb * (long long)sizeof(T);
     const unsigned long long bytes = (unsigned long long)k * sizeof(T);
@@ -330,6 +332,7 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
         if (nb != 16) return -1;
         return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, StoreScattered<T>{out, sv, orig}, st);
     }
+    if (nb == 16 && passing) return launch_sddmm_nb<T, 16, RowsPassing>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
     if (nb == 16) return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
     if (nb == 8) return launch_sddmm_nb<T, 8>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
     if constexpr (sizeof(T) == 4) return launch_sddmm_nb<T, 4>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
@@ -491,7 +494,7 @@ SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
 template <typename T> static int sddmm_call(const SddmmCall& c, cudaStream_t st) {
     T* out = (T*)(c.where ? c.dots : c.out);
     const int rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,
-                                   (const T*)c.B, c.ldb, c.k, out, st);
+                                   (const T*)c.B, c.ldb, c.k, out, st, nullptr, c.where != nullptr);
     if (rc != 0 || !c.where || c.nnz == 0) return rc;
     const bool aligned = ((uintptr_t)c.where | (uintptr_t)c.sv | (uintptr_t)c.out) % 16 == 0;
     return launch_early(scale_picked_kernel<T>, (unsigned)((c.nnz + 1023) / 1024), 0, st, c.nnz, c.where,

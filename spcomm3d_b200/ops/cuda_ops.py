@@ -367,10 +367,11 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
 
     Counted in dense rows that come from device memory: now every nonzero outside the most frequent columns that the
     L2 holds, with chunks one row of A per change of (row, chunk), every used column once, and four values per nonzero
-    for the pass that restores the row order.  The line lies at 1.5 times fewer.  Erdos-Renyi 1 M rows, 32 a row (3
-    times fewer): k = 64 1121 -> 936 us, k = 128 2519 -> 1945; 500 thousand rows, 12 a row, k = 128 (1.55): 422 -> 381;
-    1 M x 2 M, 12 a row, k = 64 (1.06): 499 -> 617; R-MAT scale 20, k = 128 (hub columns): 559 -> 669.  Chunks of 64 MB
-    are level with 96 at 32 a row, 128 and 48 MB slower.  Fewer reads per row of B than four leave little to save."""
+    for the pass that restores the row order.  The line lies at 1.25 times fewer.  Erdos-Renyi 1 M rows, 32 a row (3
+    times fewer): k = 64 1098 -> 900 us, k = 128 2473 -> 1782; uniform 500 thousand rows, 12 a row, k = 128 (1.4): 413
+    -> 342; 1 M x 2 M, 12 a row, k = 64 (1.05): 489 -> 576; R-MAT scale 20, k = 128 (hub columns): 564 -> 673.  Chunks
+    of 64 MB are level with 96 at 32 a row, 128 and 48 MB slower.  Fewer reads per row of B than four leave little to
+    save."""
     nnz = rowidx.shape[0]
     n = force or -(-n_cols * row_bytes // CHUNK_BYTES)
     if not force and (n < 2 or n > 32 or nnz < CHUNK_MIN_NNZ or nnz < 4 * n_cols):
@@ -381,7 +382,7 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
         top = torch.topk(count, min(n_cols, CHUNK_BYTES // row_bytes), sorted=False)[0]
         changes = int(((rowidx[1:] != rowidx[:-1]) | (chunk[1:] != chunk[:-1])).sum()) + 1   # columns ascend in a row
         now, then = nnz - int(top.sum()), changes + int((count > 0).sum()) + nnz * 16 // row_bytes
-        if 2 * now < 3 * then:
+        if 4 * now < 5 * then:
             return None
     index = torch.sort(chunk.to(torch.uint8), stable=True)[1]
     where = torch.empty_like(colidx)
