@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
             const long long u1 = u0 + UNITS_PER_TICKET < n_units ? u0 + UNITS_PER_TICKET : n_units;
             ok = gate.ensure(u1, lane);
             if (!ok) break;
-            sddmm_windows<real, 16, G, R, sddmm_unroll(R), false, false>(
+            sddmm_windows<real, 16, G, R, sddmm_unroll(R), false>(
                 u0, 1, u1, per_unit, a.nnz, a.rowidx, a.colidx, arows, reinterpret_cast<const char*>(Bv),
                 (unsigned)ldb_v * 16u, a.nvec, aligned, store, lane);
             if (self_push) {
@@ -1031,11 +1031,11 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
                     const EmitOwnedOrAdd add{reinterpret_cast<vec*>(a.Y), a.ldy / VN, (real)a.beta, a.n_owned_y, a.y_dst,
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
                                                                               ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
                                                                               ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
                 }
             }
@@ -1083,11 +1083,11 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
                     const EmitOwnedOrAdd add{reinterpret_cast<vec*>(a.Y), a.ldy / VN, (real)a.beta, a.n_owned_y, a.y_dst,
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
                                                                               ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
-                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false, false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
+                        spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
                                                                               ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
                 }
             }

@@ -23,12 +23,12 @@ namespace sp3 {
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R))
 sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
-                 const Rows arows, const char* __restrict__ B, unsigned ldb_bytes, int nvec, bool aligned,
+                 const Rows arows, const char* B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
     after_previous_kernel();
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    sddmm_windows<T, NB, G, R, sddmm_unroll(R), EXACT, true>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
+    sddmm_windows<T, NB, G, R, sddmm_unroll(R), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
                                                       arows, B, ldb_bytes, nvec, aligned, store, threadIdx.x & 31);
 }
 
@@ -38,7 +38,7 @@ sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const in
 // k = 64: about 250 us).
 template <typename T>
 __global__ void __launch_bounds__(256)
-scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* __restrict__ sval, const T* dots, T* out,
+scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* sval, const T* dots, T* out,
                     bool aligned) {
     after_previous_kernel();
     const int n = (int)nnz, i = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
@@ -87,7 +87,7 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
 __global__ void __launch_bounds__(256, spmm_min_blocks(G, R))
 spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
-                  const int* __restrict__ colidx, const T* __restrict__ val, const char* __restrict__ X,
+                  const int* __restrict__ colidx, const T* val, const char* X,
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
     after_previous_kernel();
     __shared__ int row_ends[256 / 32][SPMM_ENDS];
@@ -101,7 +101,7 @@ spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const l
         // (items of fewer rows wait for the previous values less often than the requests cost: Erdos-Renyi, 24 nonzeros
         // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
         if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
-        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT, true>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
+        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
                                                                  aligned, emit, lg, ends, lane);
     };
     if (lg.ticket && nitems > nwarps) {
@@ -215,7 +215,7 @@ __global__ void fill_rows_kernel(const long long* __restrict__ gid, long long nr
 // checksum: fixed-shape two-stage sum in fp64 (bitwise reproducible).
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) sum_stage1(const T* __restrict__ x, long long n, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) sum_stage1(const T* x, long long n, double* part) {
     after_previous_kernel();
     __shared__ double sh[256];
     double acc = 0;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) sum_stage1(const T* __restrict__ x, long 
     for (int s = 128; s > 0; s >>= 1) { if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s]; __syncthreads(); }
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
-__global__ void __launch_bounds__(256) sum_stage2(const double* __restrict__ part, int n, double* __restrict__ out) {
+__global__ void __launch_bounds__(256) sum_stage2(const double* part, int n, double* out) {
     after_previous_kernel();
     __shared__ double sh[256];
     double acc = 0;

@@ -44,23 +44,25 @@ template <> struct Row<float, 4> { using E = float; static constexpr int N = 1; 
 template <> struct Row<double, 16> { using E = double; static constexpr int N = 2; E x[2]; };
 template <> struct Row<double, 8> { using E = double; static constexpr int N = 1; E x[1]; };
 
-// NC = true: the non-coherent read-only path (ld.global.nc), for operands that no thread writes while the
-// kernel runs (the local kernels).  NC = false: an ordinary load.  The fused kernels use it for every dense
-// row, because rows of the pulled part of a block are written by other warps of the same launch; ordinary
-// loads are ordered after the acquire that tells a warp the rows are there, the read-only path is not.
-template <bool NC, typename T, int NB> __device__ __forceinline__ void row_load(Row<T, NB>& v, const char* p) {
+// Dense rows and values are read by ordinary loads, never through the read-only path (`ld.global.nc`, `__ldg`, or a
+// `const __restrict__` kernel parameter, from which the compiler infers it): that path is defined only for memory that
+// nobody writes while the kernel runs.  A kernel launched early runs while the kernel before it writes what may be its
+// values or rows (see after_previous_kernel), and in the fused kernels other warps of the launch write the pulled rows.
+// Ordinary loads are ordered behind the wait, or the acquire, that says the data is there.  Index arrays and work items
+// are fixed when an operator is built and keep the read-only path.
+template <typename T, int NB> __device__ __forceinline__ void row_load(Row<T, NB>& v, const char* p) {
     using E = typename Row<T, NB>::E;
     if constexpr (NB == 16 && sizeof(T) == 4) {
         const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
-        const ulonglong2 t = NC ? __ldg(q) : *q;
+        const ulonglong2 t = *q;
         v.x[0] = t.x; v.x[1] = t.y;
     } else if constexpr (NB == 16) {
         const double2* q = reinterpret_cast<const double2*>(p);
-        const double2 t = NC ? __ldg(q) : *q;
+        const double2 t = *q;
         v.x[0] = t.x; v.x[1] = t.y;
     } else {
         const E* q = reinterpret_cast<const E*>(p);
-        v.x[0] = NC ? __ldg(q) : *q;
+        v.x[0] = *q;
     }
 }
 template <typename T, int NB> __device__ __forceinline__ void row_store(char* p, const Row<T, NB>& v) {
@@ -118,26 +120,28 @@ __device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> 
     }
 }
 
-// Four consecutive values base[i .. i+3] of a read-only array, i a multiple of 4 counted from a 16-byte
-// boundary when `aligned`; positions at or past `end` repeat the last value before it.
+// Four consecutive values base[i .. i+3] of a list, i a multiple of 4 counted from a 16-byte boundary when `aligned`;
+// positions at or past `end` repeat the last value before it.  Lists of int are index lists (read-only path).
 template <typename I> struct Quad { I v[4]; };
 __device__ __forceinline__ Quad<int> quad_load_vec(const int* p) {
     const int4 t = __ldg(reinterpret_cast<const int4*>(p));
     return {{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ Quad<float> quad_load_vec(const float* p) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 t = *reinterpret_cast<const float4*>(p);
     return {{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ Quad<double> quad_load_vec(const double* p) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+    const double2 a = *reinterpret_cast<const double2*>(p), b = *(reinterpret_cast<const double2*>(p) + 1);
     return {{a.x, a.y, b.x, b.y}};
 }
+__device__ __forceinline__ int list_load(const int* p) { return __ldg(p); }
+template <typename T> __device__ __forceinline__ T list_load(const T* p) { return *p; }
 template <typename I> __device__ __forceinline__ Quad<I> quad_load(const I* base, int i, int end, bool aligned) {
     if (aligned && i + 4 <= end) return quad_load_vec(base + i);
     Quad<I> q;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q.v[j] = __ldg(base + (i + j < end ? i + j : end - 1));
+    for (int j = 0; j < 4; ++j) q.v[j] = list_load(base + (i + j < end ? i + j : end - 1));
     return q;
 }
 
@@ -167,14 +171,14 @@ __device__ __forceinline__ u64 evict_first_policy() {
 }
 template <typename T> __device__ __forceinline__ void row_load_passing(Row<T, 16>& v, const char* p, u64 policy) {
     u64 a, b;
-    asm("ld.global.nc.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(a), "=l"(b) : "l"(p), "l"(policy));
+    asm volatile("ld.global.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;" : "=l"(a), "=l"(b) : "l"(p), "l"(policy));
     if constexpr (sizeof(T) == 4) { v.x[0] = a; v.x[1] = b; }
     else { v.x[0] = __longlong_as_double((long long)a); v.x[1] = __longlong_as_double((long long)b); }
 }
 __device__ __forceinline__ Quad<int> quad_load_passing(const int* base, int i, int end, bool aligned, u64 policy) {
     if (!aligned || i + 4 > end) return quad_load(base, i, end, false);
     Quad<int> q;
-    asm("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;"
+    asm volatile("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;"
         : "=r"(q.v[0]), "=r"(q.v[1]), "=r"(q.v[2]), "=r"(q.v[3]) : "l"(base + i), "l"(policy));
     return q;
 }
@@ -198,14 +202,14 @@ struct RowsByPeerRef {
 template <typename T> struct StoreLocal {
     T* out;
     const T* sval;    // null: no scaling
-    __device__ __forceinline__ T scale(long long i) const { return sval ? __ldg(sval + i) : (T)1; }
+    __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
     __device__ __forceinline__ void put(long long i, T v) const { out[i] = v; }
 };
 template <typename T> struct StoreScattered {
     T* out;
     const T* sval;
     const int* orig;  // result position of nonzero i
-    __device__ __forceinline__ T scale(long long i) const { return sval ? __ldg(sval + i) : (T)1; }
+    __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
     __device__ __forceinline__ void put(long long i, T v) const { out[__ldg(orig + i)] = v; }
 };
 
@@ -253,10 +257,10 @@ __host__ __device__ inline int window_nnz(long long nnz, long long nwarps, int g
     return (int)(w < quantum ? quantum : (w > WINDOW_MAX ? WINDOW_MAX : w));
 }
 
-template <typename T, int NB, int G, int R, int U, bool EXACT, bool NC, typename ARows, typename Store>
+template <typename T, int NB, int G, int R, int U, bool EXACT, typename ARows, typename Store>
 __device__ __forceinline__ void sddmm_windows(long long first, long long step, long long end, int wn, long long nnz,
                                               const int* __restrict__ rowidx, const int* __restrict__ colidx,
-                                              const ARows& arows, const char* __restrict__ B, unsigned ldb_bytes,
+                                              const ARows& arows, const char* B, unsigned ldb_bytes,
                                               int nvec, bool aligned, const Store& store, int lane) {
     static_assert(G >= 4, "a group reduces four values");
     constexpr unsigned FULL = 0xffffffffu;
@@ -287,7 +291,7 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
     };
     auto fetch = [&](Row<T, NB> (&a)[R], const char* p) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) row_load<NC>(a[q], p + (off[q] - off[0]));
+        for (int q = 0; q < R; ++q) row_load(a[q], p + (off[q] - off[0]));
     };
     auto fetch_a = [&](Row<T, NB> (&a)[R], const char* p) {
         if constexpr (PASSING) {
@@ -408,7 +412,7 @@ template <typename T, int NB> struct EmitLocal {
         char* y = Y + row * ldy_bytes + (long long)v * NB;
         if (beta != (T)0) {
             Row<T, NB> old;
-            row_load<false>(old, y);
+            row_load(old, y);
             row_fma(acc, beta, old);
         }
         row_store(y, acc);
@@ -457,10 +461,10 @@ template <typename T> struct EmitPacked {
 // longest one: R-MAT scale 20, k = 32, 0.44 ms against 0.26 ms.)  Row ends are kept in shared memory (`ends`,
 // SPMM_ENDS ints per warp), indices and values come as quads that all lanes of a group read, requested one
 // quad ahead; U x R dense vectors are in flight per lane.  No atomics on values: bitwise reproducible.
-template <typename T, int NB, int G, int R, int U, bool EXACT, bool NC, typename Emit>
+template <typename T, int NB, int G, int R, int U, bool EXACT, typename Emit>
 __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* __restrict__ rowptr, long long nnz,
-                                               const int* __restrict__ colidx, const T* __restrict__ val,
-                                               const char* __restrict__ X, unsigned ldx_bytes, int nvec, bool aligned,
+                                               const int* __restrict__ colidx, const T* val,
+                                               const char* X, unsigned ldx_bytes, int nvec, bool aligned,
                                                const Emit& emit, const SpmmLong& lg, int* ends, int lane) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;            // G need not divide 32: the lanes of slot SLOTS have no share
@@ -546,7 +550,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
                 // (R-MAT scale 20, k = 128).
                 const char* row = X + (u64)(unsigned)c[h + u] * ldx_bytes;
 #pragma unroll
-                for (int q = 0; q < R; ++q) row_load<NC>(x[u][q], row + (off[q] - off[0]));
+                for (int q = 0; q < R; ++q) row_load(x[u][q], row + (off[q] - off[0]));
             }
             // the next quad is requested behind the rows of this one: loads come back in order, and the indices may
             // have to come from device memory (requested ahead of the rows: 0.84 ms instead of 0.66 ms at R-MAT
@@ -675,7 +679,8 @@ inline int env_int(const char* name, int dflt) {
 }
 
 // Launch that may begin while the previous kernel of the stream drains (programmatic dependent launch): the kernel
-// has to call `after_previous_kernel` before it touches memory.
+// has to call `after_previous_kernel` before it touches memory, and to read what an earlier kernel of this library may
+// have written by ordinary loads (see row_load): it is resident while that kernel still writes.
 template <typename... P, typename... A>
 inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute attr = {};
@@ -693,7 +698,7 @@ inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cuda
 __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    __threadfence();   // nothing of an earlier kernel's lines may be left in the L1
+    __threadfence();
 }
 
 constexpr int MAX_DEVICES = 64;

@@ -1,0 +1,112 @@
+"""Operators of one rank: what a program sees of them between the calls (its operands, their chain from kernel to
+kernel, the limits of what is accepted).
+
+References are fp64 sums of the same, already rounded inputs; the bounds are those of `test_kernel_edges.py`: a sum of
+n products in precision u is off by at most gamma(n) = n u / (1 - n u) times the sum of the products' magnitudes."""
+import numpy as np
+import pytest
+import torch
+
+U = {torch.float32: 2.0 ** -24, torch.float64: 2.0 ** -53}
+
+
+def _gamma(n, dtype):
+    return n * U[dtype] / (1 - n * U[dtype])
+
+
+def _plan(spec, seed=3):
+    from spcomm3d_b200.parallel.mesh import Mesh3D
+    from spcomm3d_b200.parallel.plan import build_my_plan
+    from spcomm3d_b200.utils import generate
+    m = generate.from_spec(spec, seed=seed)
+    return build_my_plan(m, Mesh3D(1, 1, 1), 0, seed=seed)[1]
+
+
+def _randn(t, seed):
+    g = torch.Generator().manual_seed(seed)
+    return torch.randn(t.shape, generator=g, dtype=torch.float64).to(t.dtype)
+
+
+def _lists(plan):
+    rowptr = torch.from_numpy(plan.rowptr)
+    return (torch.repeat_interleave(torch.arange(rowptr.shape[0] - 1), rowptr.diff()),
+            torch.from_numpy(plan.colidx).long(), rowptr.diff())
+
+
+def _scores(plan, A, B, vals):
+    """(values of S o (A B^T), the same of magnitudes) in fp64."""
+    r, c, _ = _lists(plan)
+    a, b, s = A.double()[r], B.double()[c], vals.double()
+    return (a * b).sum(1) * s, (a * b).abs().sum(1) * s.abs()
+
+
+def _product(plan, vals, X):
+    r, c, _ = _lists(plan)
+    return torch.zeros(plan.rowptr.shape[0] - 1, X.shape[1], dtype=torch.float64).index_add_(
+        0, r, vals.double()[:, None] * X.double()[c])
+
+
+def _check_layer(layer, plan, k, dtype, A, B, X, vals, scores, y):
+    """Scores and result of an attention chain; the SpMM adds products of scores that are off by gamma(k + 2)."""
+    c, cmag = _scores(plan, A, B, vals)
+    assert bool(((scores.cpu().double() - c).abs() <= _gamma(k + 2, dtype) * cmag).all())
+    deg = _lists(plan)[2]
+    bound = torch.from_numpy(_gamma(k + 5.0 + deg.numpy(), dtype))[:, None] * _product(plan, cmag, X.abs())
+    assert bool(((y.cpu().double() - _product(plan, c, X)).abs() <= bound).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("timers", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gen,k", [("uniform:4096:4096:16", 32), ("zipf:16384:131072:1.8:4096", 64), ("rmat:12:16", 33)])
+def test_gat_layer_one_rank(gen, k, dtype, timers):
+    """The SpMM reads the scores that the SDDMM before it has just written, pass after pass on new operands, without a
+    wait of the host in between."""
+    from spcomm3d_b200.models.layer import GatLayer
+    plan = _plan(gen)
+    layer = GatLayer(plan, None, k, dtype, "cuda")
+    layer.sddmm.timer.enabled = layer.spmm.timer.enabled = timers
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    ops = [[_randn(t, 10 * i + j) for j, t in enumerate((layer.sddmm.A_owned, layer.sddmm.B_owned, layer.spmm.X_owned))]
+           for i in range(4)]
+    on_gpu = [[t.cuda() for t in o] for o in ops]
+    out = []
+    for A, B, X in on_gpu:
+        layer.sddmm.A_owned.copy_(A), layer.sddmm.B_owned.copy_(B), layer.spmm.X_owned.copy_(X)
+        y = layer.run()
+        out.append((layer.spmm.vals.clone(), y.clone()))
+    for (A, B, X), (scores, y) in zip(ops, out):
+        _check_layer(layer, plan, k, dtype, A, B, X, vals, scores, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gen,k", [("uniform:4096:4096:16", 32), ("er:20000:20000:9", 128), ("rmat:14:8", 16)])
+def test_rows_written_by_the_kernel_before(gen, k, dtype):
+    """Y = S (S X), and an SDDMM on the result: every kernel reads rows that the kernel before it has just written."""
+    from spcomm3d_b200.ops import cuda_ops
+    plan = _plan(gen)
+    rowptr, ri, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.rowidx, plan.colidx))
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    n = max(plan.row.n_local, plan.col.n_local)
+    bufs = [torch.zeros(n, k, dtype=dtype, device="cuda") for _ in range(3)]
+    sched, v = cuda_ops.SpmmSchedule(rowptr), vals.cuda()
+    nr = plan.row.n_local
+    first = cuda_ops.bind_spmm(rowptr, ci, v, bufs[0], bufs[1][:nr], sched)
+    second = cuda_ops.bind_spmm(rowptr, ci, v, bufs[1], bufs[2][:nr], sched)
+    out = torch.zeros(plan.nnz, dtype=dtype, device="cuda")
+    dots = cuda_ops.bind_sddmm(ri, ci, v, bufs[1], bufs[2], out)
+    got = []
+    for i in range(3):
+        X = _randn(bufs[0], i)
+        bufs[0].copy_(X.cuda())
+        first.launch(0.0), second.launch(0.0), dots.launch()
+        got.append((X, *(t.clone() for t in (bufs[1], bufs[2], out))))
+    deg = _lists(plan)[2].numpy()
+    for X, y1, y2, c in got:
+        y1, y2, c = y1.cpu(), y2.cpu(), c.cpu()
+        for x, y in ((X, y1), (y1, y2)):   # each kernel against what it was given
+            bound = torch.from_numpy(_gamma(3.0 + deg, dtype))[:, None] * _product(plan, vals.abs(), x.abs())
+            assert bool(((y[:nr].double() - _product(plan, vals, x)).abs() <= bound).all())
+        ref, mag = _scores(plan, y1, y2, vals)
+        assert bool(((c.double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
