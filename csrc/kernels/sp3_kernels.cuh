@@ -430,6 +430,7 @@ template <typename T> struct EmitPacked {
     }
     __device__ __forceinline__ void operator()(int row, int v, const Row<T, 16>& acc) const {
         constexpr int N = 16 / (int)sizeof(T);
+        if (v * N >= k) return;   // X may be wider by whole vectors: nothing of this one belongs to the row
         T x[N];
         if constexpr (sizeof(T) == 4) {
             const float2 a = unpack2(acc.x[0]), b = unpack2(acc.x[1]);

@@ -110,3 +110,27 @@ def test_rows_written_by_the_kernel_before(gen, k, dtype):
             assert bool(((y[:nr].double() - _product(plan, vals, x)).abs() <= bound).all())
         ref, mag = _scores(plan, y1, y2, vals)
         assert bool(((c.double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+@pytest.mark.parametrize("k,wide", [(1, 4), (3, 4), (5, 8), (10, 16), (33, 36), (33, 64), (50, 52), (66, 68), (97, 100),
+                                    (130, 132), (200, 256), (255, 256), (4, 64)])
+def test_spmm_of_wider_rows(k, wide, beta, dtype):
+    """X with more columns than the result, by the padding to whole vectors and by whole vectors: the result takes the
+    first ones, nothing beyond a row is touched, rows end where the allocation ends."""
+    from spcomm3d_b200.ops import cuda_ops, local
+    plan = _plan("zipf:300:400:1.6:200")
+    rowptr, ri, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.rowidx, plan.colidx))
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    nr, deg = plan.row.n_local, _lists(plan)[2].numpy()
+    X, Y0 = _randn(torch.empty(plan.col.n_local, wide, dtype=dtype), 1), _randn(torch.empty(nr, k, dtype=dtype), 2)
+    sched = cuda_ops.SpmmSchedule(rowptr, long_row=64)
+    Y = (Y0 if beta else torch.full_like(Y0, float("nan"))).cuda()
+    local.spmm(rowptr, ri, ci, vals.cuda(), X.cuda(), Y, beta, sched)
+    ref, mag = _product(plan, vals, X[:, :k]), _product(plan, vals.abs(), X[:, :k].abs())
+    if beta:
+        ref, mag = ref + beta * Y0.double(), mag + beta * Y0.double().abs()
+    bound = torch.from_numpy(_gamma(3.0 + deg, dtype))[:, None] * mag
+    assert bool(((Y.cpu().double() - ref).abs() <= bound).all())
