@@ -152,12 +152,7 @@ __device__ __forceinline__ bool wait_flag(const FusedComm& c, int kind, int src,
     }
 }
 
-__device__ __forceinline__ bool wait_all(const FusedComm& c, int kind, const int* list, int n, int site) {
-    bool ok = true;
-    for (int i = 0; i < n; ++i) ok = wait_flag(c, kind, list[i], site) && ok;
-    return ok;
-}
-// The same for a whole block: thread i waits for flag i, the barrier passes the acquire on.  Every thread calls it.
+// Waits of a whole block: thread i waits for flag i, the barrier passes the acquire on.  Every thread calls it.
 __device__ __forceinline__ bool block_wait_all(const FusedComm& c, int kind, const int* list, int n, int site) {
     bool ok = true;
     for (int i = threadIdx.x; i < n; i += blockDim.x) ok = wait_flag(c, kind, list[i], site) && ok;
@@ -182,11 +177,11 @@ __device__ __forceinline__ bool poll_counter(const FusedComm& c, int which, int 
         }
     }
 }
-// The same for a warp: one lane polls (all lanes call it).
+// Bounded wait of a warp: one lane polls (all lanes call it).
 __device__ __forceinline__ bool wait_counter(const FusedComm& c, int which, int want, int site) {
     int ok = 0;
     if ((threadIdx.x & 31) == 0) ok = poll_counter(c, which, want, site);
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    return from_lane0(ok) != 0;
 }
 
 __device__ __forceinline__ void start_phase(const FusedComm& c) {
@@ -446,7 +441,7 @@ struct PullGate {
             flush(lane);   // never wait while a tile of this warp is unpublished
             int now = 0;
             if (lane == 0) now = await_wave(w, want);
-            waves_ready = __shfl_sync(0xffffffffu, now, 0);
+            waves_ready = from_lane0(now);
             if (waves_ready <= w) return false;
         }
         return true;
@@ -495,7 +490,7 @@ __device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane) {
     __syncwarp();
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_MAIN_DONE, 1);
-    old = __shfl_sync(0xffffffffu, old, 0);
+    old = from_lane0(old);
     if (old == (int)gridDim.x - 1) {
         __threadfence_system();
         for (int i = lane; i < c.n_read; i += 32) signal(c, F_DONE, c.read_from[i]);
@@ -512,7 +507,7 @@ __device__ __forceinline__ void finish_epilogue(const FusedComm& c, int lane) {
     if (threadIdx.x >= 32) return;
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_FIN_DONE, 1);
-    old = __shfl_sync(0xffffffffu, old, 0);
+    old = from_lane0(old);
     if (old == (int)gridDim.x - 1) {
         for (int i = lane; i < c.n_readers; i += 32) wait_flag(c, F_DONE, c.readers[i], W_DONE);
         __syncwarp();
@@ -973,7 +968,7 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
         __syncwarp();
         int old = 0;
         if (lane == 0) old = atomicAdd(c.ctrl + C_START_DONE, 1);
-        old = __shfl_sync(0xffffffffu, old, 0);
+        old = from_lane0(old);
         if (old == nwarps - 1) {
             __threadfence_system();
             for (int i = lane; i < c.n_readers; i += 32) signal(c, F_READY, c.readers[i]);

@@ -70,6 +70,12 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+// The value that lane 0 holds, for every lane, with what lane 0 has seen: a shuffle alone orders no memory, the
+// barrier makes an acquire, or a count, of lane 0 hold for the loads that the other lanes do next.
+__device__ __forceinline__ int from_lane0(int v) {
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, v, 0);
+}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));

@@ -646,7 +646,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     __syncwarp();
     int old = 0;
     if (lane == 0) old = atomicAdd(lg.counters + lr, 1);
-    old = __shfl_sync(FULL, old, 0);
+    old = from_lane0(old);
     if (old != np - 1) return;
     __threadfence();
     // group g adds every SLOTS-th carry, then the groups are added up (more loads in flight here would take registers
