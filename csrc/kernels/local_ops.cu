@@ -318,7 +318,9 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
     if (nnz == 0) return 0;
     const long long lda_b = lda * (long long)sizeof(T), ldb_b = ldb * (long long)sizeof(T);
     const unsigned long long bytes = (unsigned long long)k * sizeof(T);
-    const int nb = vector_bytes<T>(bytes, lda_b | ldb_b | (uintptr_t)A | (uintptr_t)B);
+    const unsigned long long bits = lda_b | ldb_b | (uintptr_t)A | (uintptr_t)B;
+    // the scatter form exists for 16-byte vectors only, and takes them for rows of one or two as well
+    const int nb = orig && (bytes | bits) % 16 == 0 ? 16 : vector_bytes<T>(bytes, bits);
     const unsigned long long nvec = bytes / nb;
     if (nvec > 256 || nvec == 0 || lda_b >= 1ll << 32 || ldb_b >= 1ll << 32) {
         if (orig) return -1;  // the scatter form exists for the vector kernel only

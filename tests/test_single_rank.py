@@ -134,3 +134,45 @@ def test_spmm_of_wider_rows(k, wide, beta, dtype):
         ref, mag = ref + beta * Y0.double(), mag + beta * Y0.double().abs()
     bound = torch.from_numpy(_gamma(3.0 + deg, dtype))[:, None] * mag
     assert bool(((Y.cpu().double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [8, 16, 24])
+def test_dense_panels_of_narrow_rows(k):
+    """The remainder beside the panels has rows of as few as two vectors.  The tensor cores ignore the low 13 of an
+    operand's 23 mantissa bits: a factor is cut by less than 2^-10 of itself, a product by less than 2^-9."""
+    from spcomm3d_b200.ops.panel import PanelSDDMM
+    rng = np.random.default_rng(k)
+    rr, cc = np.nonzero(rng.random((256, 96)) < 0.3)
+    keys = np.unique(np.concatenate([rr * 400 + cc, rng.integers(0, 500 * 400, 3000)]))
+    rows, cols = (keys // 400).astype(np.int32), (keys % 400).astype(np.int32)
+    vals = rng.random(keys.size).astype(np.float32)
+    op = PanelSDDMM(rows, cols, vals, 500, 400)
+    assert op.npanels > 0 and op.n_rest > 0
+    A, B = _randn(torch.empty(500, k), 1), _randn(torch.empty(400, k), 2)
+    got = op.run(A.cuda(), B.cuda()).cpu().double()
+    a, b, s = A.double()[rows], B.double()[cols], torch.from_numpy(vals).double()
+    ref, mag = (a * b).sum(1) * s, (a * b).abs().sum(1) * s
+    assert bool(((got - ref).abs() <= (2.0 ** -9 + _gamma(k + 2, torch.float32)) * mag).all())
+    rest = op.r_pos.cpu().long()
+    assert bool(((got - ref).abs() <= _gamma(k + 2, torch.float32) * mag)[rest].all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [4, 8, 12, 64])
+def test_sddmm_scattered_narrow_rows(k):
+    from spcomm3d_b200.utils import native
+    rng = np.random.default_rng(k)
+    n = 301
+    rows, cols = torch.from_numpy(np.sort(rng.integers(0, 40, n)).astype(np.int32)), torch.from_numpy(rng.integers(0, 50, n).astype(np.int32))
+    pos, s = torch.from_numpy(rng.permutation(n).astype(np.int32)), torch.from_numpy(rng.random(n).astype(np.float32))
+    A, B = _randn(torch.empty(40, k), 1), _randn(torch.empty(50, k), 2)
+    out = torch.full((n,), float("nan"), device="cuda")
+    t = [x.cuda() for x in (rows, cols, s, A, B, pos)]
+    p = native.ptr
+    rc = native.cuda().sp3_cuda_sddmm_orig_f32(n, p(t[0]), p(t[1]), p(t[2]), p(t[3]), k, p(t[4]), k, k, p(out), p(t[5]),
+                                               torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    prod = A.double()[rows.long()] * B.double()[cols.long()]
+    ref, mag = prod.sum(1) * s.double(), prod.abs().sum(1) * s.double()
+    assert bool(((out.cpu().double()[pos.long()] - ref).abs() <= _gamma(k + 2, torch.float32) * mag).all())
