@@ -90,7 +90,9 @@ class _Dist3DOp:
         if variant == "fused" and self.device.type != "cuda":
             raise ValueError("the fused variant runs on GPUs only")
         self.rowptr = torch.from_numpy(plan.rowptr).to(self.device)
-        self.vals = torch.from_numpy(plan.vals).to(device=self.device, dtype=dtype)
+        # values of its own: they may be written to (a chain puts its scores there), the plan's and those of other
+        # operators stay as they are
+        self.vals = torch.from_numpy(plan.vals).to(device=self.device, dtype=dtype, copy=True)
         rowidx, colidx = plan.rowidx, plan.colidx
         self._row_group = groups.row if groups else None
         self._col_group = groups.col if groups else None
