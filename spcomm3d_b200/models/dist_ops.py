@@ -386,8 +386,9 @@ class DistSpMM(_Dist3DOp):
             order = np.argsort(self.rowidx.cpu().numpy(), kind="stable")
             ri = self.rowidx.cpu().numpy()[order]
             self._d_rowidx = torch.from_numpy(ri).to(self.device)
-            self._d_colidx = self.colidx[torch.from_numpy(order).to(self.device)]
-            self._d_vals = self.vals[torch.from_numpy(order).to(self.device)]
+            self._d_order = torch.from_numpy(order).to(self.device)
+            self._d_colidx = self.colidx[self._d_order]
+            self._d_vals = self.vals[self._d_order]
             rp = np.zeros(self._Yslab.shape[0] + 1, np.int64)
             np.cumsum(np.bincount(ri, minlength=self._Yslab.shape[0]), out=rp[1:])
             self._d_rowptr = torch.from_numpy(rp).to(self.device)
@@ -426,11 +427,13 @@ class DistSpMM(_Dist3DOp):
         return [(self.X_loc, self.plan.col)]
 
     def values_changed(self):
-        """Tell the op that `vals` (the values of S, CSR order) was written to: the fused kernel keeps a
-        re-ordered copy.  The library variants read `vals` directly."""
+        """Tell the op that `vals` (the values of S, CSR order) was written to: the fused kernels and the dense
+        variant keep a re-ordered copy.  The sparse variants read `vals` directly."""
         f = getattr(self, "_fused", None)
         if f is not None:
             f.refresh_values()
+        if self.variant == "dense":
+            torch.index_select(self.vals, 0, self._d_order, out=self._d_vals)
 
     def run(self, beta: float = 0.0) -> torch.Tensor:
         """One distributed SpMM: Y_owned = beta*Y_owned + (S X)[owned rows]."""

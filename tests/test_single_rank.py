@@ -178,14 +178,15 @@ def test_sddmm_scattered_narrow_rows(k):
     assert bool(((out.cpu().double()[pos.long()] - ref).abs() <= _gamma(k + 2, torch.float32) * mag).all())
 
 
+@pytest.mark.parametrize("variant", ["sparseNRB", "sparse", "dense"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-def test_gat_layer_twice_on_the_host(dtype):
+def test_gat_layer_twice_on_the_host(dtype, variant):
     """The scores go into the values of the SpMM and nowhere else: a second run on the same operands is the first, and
     the plan keeps its values."""
     from spcomm3d_b200.models.layer import GatLayer
     plan = _plan("uniform:40:50:4")
     before = plan.vals.copy()
-    layer = GatLayer(plan, None, 8, dtype, "cpu")
+    layer = GatLayer(plan, None, 8, dtype, "cpu", variant)
     A, B, X = (_randn(t, i) for i, t in enumerate((layer.sddmm.A_owned, layer.sddmm.B_owned, layer.spmm.X_owned)))
     layer.sddmm.A_owned.copy_(A), layer.sddmm.B_owned.copy_(B), layer.spmm.X_owned.copy_(X)
     for _ in range(2):
