@@ -59,6 +59,46 @@ scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* sval,
         if (i + j < n) out[i + j] = v[j];
 }
 
+// Rows of k values, `ld` apart wherever they start, to rows of `nvec` whole 16-byte vectors, the rest zero: what the
+// SDDMM and the SpMM read in place of operands whose rows are no whole number of vectors (see `pack_rule` in
+// ops/cuda_ops.py for when that pays).  Bound by the copy; four vectors per thread, one block per 1024.
+struct PackRows {
+    const void* src;     // null: nothing to pack
+    long long ld;        // elements
+    void* dst;
+    long long rows;
+    int k, nvec;
+};
+constexpr int PACK_PER_BLOCK = 1024;
+inline unsigned pack_blocks(const PackRows& p) {
+    return p.src ? (unsigned)((p.rows * p.nvec + PACK_PER_BLOCK - 1) / PACK_PER_BLOCK) : 0;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) pack_rows_kernel(const PackRows first, const PackRows second, unsigned blocks_first) {
+    after_previous_kernel();
+    using V = typename Vec<T>::type;
+    constexpr int N = Vec<T>::N;
+    const bool one = blockIdx.x < blocks_first;
+    const PackRows p = one ? first : second;
+    const long long base = (long long)(one ? blockIdx.x : blockIdx.x - blocks_first) * PACK_PER_BLOCK;
+    const long long row0 = base / p.nvec, total = p.rows * p.nvec;
+    const unsigned lead = (unsigned)(base - row0 * p.nvec);
+    __align__(16) T x[4][N];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const unsigned i = u * 256 + threadIdx.x, at = lead + i, row = at / (unsigned)p.nvec;
+        const int j0 = (int)(at - row * (unsigned)p.nvec) * N;
+        const T* s = static_cast<const T*>(p.src) + (row0 + row) * p.ld + j0;
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[u][j] = base + i < total && j0 + j < p.k ? s[j] : (T)0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const long long i = base + u * 256 + threadIdx.x;
+        if (i < total) static_cast<V*>(p.dst)[i] = *reinterpret_cast<const V*>(x[u]);
+    }
+}
+
 // Rows of more than 256 vectors: one warp per nonzero, scalar loads.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -410,6 +450,12 @@ int launch_rows(int mode, long long n, const long long* idx, const T* src, long 
     return (int)cudaGetLastError();
 }
 
+// Packs one or two operands; nothing to do without sources.
+template <typename T> int launch_pack(const PackRows& first, const PackRows& second, cudaStream_t st) {
+    const unsigned a = pack_blocks(first), b = pack_blocks(second);
+    return a + b ? launch_early(pack_rows_kernel<T>, a + b, 0, st, first, second, a) : 0;
+}
+
 template <typename T> int launch_sum(const void* x, long long n, double* part, double* out, cudaStream_t st) {
     const int rc = launch_early(sum_stage1<T>, 1024, 0, st, (const T*)x, n, part);
     return rc ? rc : launch_early(sum_stage2, 1, 0, st, (const double*)part, 1024, out);
@@ -468,6 +514,7 @@ struct SddmmCall {
     // order) is sv[i] * dots[where[i]]
     const int* where;
     void* dots;
+    PackRows pack_a, pack_b;   // A and B are filled from here first
 };
 struct SpmmCall {
     int nrows, nitems;
@@ -487,6 +534,7 @@ struct SpmmCall {
     int k, f64, piece_len;
     int k_out;              // columns of Y (k of X counts the padding of its rows)
     int x_rows;             // rows of X
+    PackRows pack_x;        // X is filled from here first
 };
 SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *sddmm_bytes = (int)sizeof(SddmmCall);
@@ -495,7 +543,9 @@ SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
 }
 template <typename T> static int sddmm_call(const SddmmCall& c, cudaStream_t st) {
     T* out = (T*)(c.where ? c.dots : c.out);
-    const int rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,
+    int rc = launch_pack<T>(c.pack_a, c.pack_b, st);
+    if (rc != 0) return rc;
+    rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,
                                    (const T*)c.B, c.ldb, c.k, out, st, nullptr, c.where != nullptr);
     if (rc != 0 || !c.where || c.nnz == 0) return rc;
     const bool aligned = ((uintptr_t)c.where | (uintptr_t)c.sv | (uintptr_t)c.out) % 16 == 0;
@@ -510,6 +560,8 @@ SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     const SpmmCall& c = *static_cast<const SpmmCall*>(record);
     cudaStream_t st = (cudaStream_t)stream;
     const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.piece_len, c.ticket};
+    const int rc = c.f64 ? launch_pack<double>(c.pack_x, PackRows{}, st) : launch_pack<float>(c.pack_x, PackRows{}, st);
+    if (rc != 0) return rc;
     if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
                                           (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows);
     return launch_spmm<float>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const float*)c.val,
@@ -553,7 +605,7 @@ SP3_API int sp3_cuda_step_call(const void* record, void* stream) {
         SP3_TRY(cudaEventRecord((cudaEvent_t)c.ev_a[i], copy));
     }
     SpmmCall spmm = c.spmm;
-    spmm.X = c.dev_b;   // the same rows; X itself is filled while the last of A is on its way
+    (spmm.pack_x.src ? spmm.pack_x.src : spmm.X) = c.dev_b;   // the same rows; X itself is filled while A is on its way
     SP3_TRY(sp3_cuda_spmm_call(&spmm, stream));
     SP3_TRY(f64 ? launch_sum<double>(c.spmm.Y, c.y_values, c.part, c.sums + 1, st)
                 : launch_sum<float>(c.spmm.Y, c.y_values, c.part, c.sums + 1, st));

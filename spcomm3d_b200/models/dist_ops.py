@@ -111,16 +111,7 @@ class _Dist3DOp:
 
     # ---- helpers ---------------------------------------------------------
     def _alloc_local(self, side):
-        """A local dense block as (padded storage, block).  On a single GPU nothing is exchanged, so the rows of an
-        operand can lie a whole number of 16-byte vectors apart whatever k is; the padding columns are zero and stay
-        zero, and the kernels read full vectors across them.  Elsewhere the block is contiguous (the collectives
-        move whole rows)."""
-        ld = self.k_loc
-        if self.mesh.size == 1 and self.device.type == "cuda" and self.variant in ("sparse", "sparseNRB"):
-            per = 16 // torch.empty((), dtype=self.dtype).element_size()
-            ld = (ld + per - 1) // per * per
-        full = torch.zeros(side.n_local, ld, dtype=self.dtype, device=self.device)
-        return full, full[:, :self.k_loc]
+        return torch.zeros(side.n_local, self.k_loc, dtype=self.dtype, device=self.device)
 
     def _exchange(self, side, group):
         mode = "buffered" if self.variant == "sparse" else "nrb"
@@ -217,7 +208,7 @@ class DistSDDMM(_Dist3DOp):
                 "heap", "fabric", "timeout_s", "overlap", "direct_push", "stage_a", "zreduce", "bulk_pull")})
             self.A_loc, self.B_loc = self._fused.A_loc, self._fused.B_loc
         else:
-            (self._A_full, self.A_loc), (self._B_full, self.B_loc) = self._alloc_local(p.row), self._alloc_local(p.col)
+            self.A_loc, self.B_loc = self._alloc_local(p.row), self._alloc_local(p.col)
         self.A_owned, self.B_owned = self.A_loc[:p.row.n_owned], self.B_loc[:p.col.n_owned]
         self.partial = torch.zeros(p.nnz, dtype=dtype, device=self.device)
         self.exAB = None
@@ -244,13 +235,18 @@ class DistSDDMM(_Dist3DOp):
         self._chunks = None
         if self._single:   # the nonzeros once more, chunk by chunk of columns, where B outgrows the L2 and that pays
             from ..ops import cuda_ops
-            row_bytes = self._B_full.stride(0) * self._B_full.element_size()
+            row_bytes = self.k_loc * self.B_loc.element_size()
             if 48 <= row_bytes <= 256 * 16:   # (narrower rows take other vectors, wider ones the scalar kernel)
                 self._chunks = cuda_ops.column_chunks(self.rowidx, self.colidx, p.col.n_local, row_bytes)
             self._chunks_of = (self.rowidx, self.colidx)
+            self._bind()
+
+    # the operands as the local kernels are given them
+    _A_full = property(lambda self: self.A_loc)
+    _B_full = property(lambda self: self.B_loc)
 
     def _bind(self):
-        t = (self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, self.partial)
+        t = (self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
@@ -293,10 +289,10 @@ class DistSDDMM(_Dist3DOp):
             with t.span("comp"):
                 if self._panels is not None:
                     self._panels.run(self.A_loc, self.B_loc, self.partial)
-                elif self._chunks is not None:
+                elif self._single:
                     self._bind().launch()
                 else:
-                    local.sddmm(self.rowidx, self.colidx, self.vals, self._A_full, self._B_full, out=self.partial)
+                    local.sddmm(self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, out=self.partial)
             with t.span("comm2"):
                 c = self.fiber(self.partial)
         if self.mesh.Z == 1:
@@ -360,8 +356,7 @@ class DistSpMM(_Dist3DOp):
                                                        "overlap")})
             self.X_loc, self.Y_loc = self._fused.X_loc, self._fused.Y_loc
         else:
-            self._X_full, self.X_loc = self._alloc_local(p.col)
-            self.Y_loc = torch.zeros(p.row.n_local, self.k_loc, dtype=dtype, device=self.device)
+            self.X_loc, self.Y_loc = self._alloc_local(p.col), self._alloc_local(p.row)
         self.X_owned = self.X_loc[:p.col.n_owned]
         # sparse variants: the result is the owned head of the local Y block (no copy); fused and dense write
         # into a buffer of their own
@@ -409,9 +404,11 @@ class DistSpMM(_Dist3DOp):
 
         self._bound = None
         self._single = self._single_rank()
+        if self._single:
+            self._bind()
 
     def _bind(self):
-        t = (self.rowptr, self.colidx, self.vals, self._X_full, self.Y_loc)
+        t = (self.rowptr, self.colidx, self.vals, self.X_loc, self.Y_loc)
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
@@ -466,9 +463,10 @@ class DistSpMM(_Dist3DOp):
             with t.span("comp"):
                 if self._panels is not None:
                     self._panels.run(self.X_loc, self.Y_loc, b)
+                elif self._single:
+                    self._bind().launch(b)
                 else:
-                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self._X_full, self.Y_loc, b,
-                               self.sched)
+                    local.spmm(self.rowptr, self.rowidx, self.colidx, self.vals, self.X_loc, self.Y_loc, b, self.sched)
             with t.span("comm2"):
                 self.exY.reduce(self.Y_loc)  # adds the peers' partial rows into the owned head = Y_owned
                 if prev is not None:

@@ -55,40 +55,53 @@ class SddmmSpmmStep:
     # ---- end to end: operands start in pinned host memory -----------------
     def make_host_operands(self):
         sd = self.sddmm
-        pin = self.device.type == "cuda"
-        # whole storages travel (rows of an operand may be padded, see `_alloc_local`): one contiguous copy each
-        self._dev_full = {"A": self._owned_storage(sd.A_owned), "B": self._owned_storage(sd.B_owned)}
-        self._host_full = {n: t.cpu() for n, t in self._dev_full.items()}
-        if pin:
-            self._host_full = {n: t.pin_memory() for n, t in self._host_full.items()}
-        self.host = {n: t[:, :sd.k_loc] for n, t in self._host_full.items()}
-        self._host_views = dict(self.host)
+        self._dev_made = {"A": sd.A_owned, "B": sd.B_owned}
+        # padded rows (fused variant) travel with their padding: one contiguous copy each
+        full = {n: self._whole_rows(t).cpu() for n, t in self._dev_made.items()}
+        if self.device.type == "cuda":
+            full = {n: t.pin_memory() for n, t in full.items()}
+        self.host = {n: t[:, :sd.k_loc] for n, t in full.items()}
+        self._host_made = dict(self.host)
         self._native_step = None
         self._sums = torch.zeros(2, dtype=torch.float64, device=self.device)
         return self.host
 
     @staticmethod
-    def _owned_storage(t):
-        """The rows of `t` with their padding columns (contiguous)."""
-        return t.as_strided((t.shape[0], t.stride(0)), (t.stride(0), 1)) if t.shape[0] > 1 else t.contiguous()
+    def _whole_rows(t):
+        """The rows of `t` with what lies between one and the next."""
+        return t.as_strided((t.shape[0], t.stride(0)), (t.stride(0), 1)) if t.shape[0] > 1 else t
+
+    def _upload(self, name, dst):
+        src = self.host[name]
+        if src is self._host_made[name] and dst is self._dev_made[name]:
+            src, dst = self._whole_rows(src), self._whole_rows(dst)
+        dst.copy_(src, non_blocking=True)
 
     @property
     def h2d_bytes(self):
-        h = self._host_full
-        return int(h["A"].numel() * h["A"].element_size() + h["B"].numel() * h["B"].element_size())
+        made = [t if t is not self._host_made[n] else self._whole_rows(t) for n, t in self.host.items()]
+        return int(sum(t.numel() * t.element_size() for t in made))
 
     @property
     def d2h_bytes(self):
         return 16
 
     def _bound_step(self):
-        """The step of a single GPU as one native call (bound again when an operator had a tensor replaced)."""
+        """The step of a single GPU as one native call (bound again when an operator had a tensor replaced), or None
+        where that call would not be this step: several ranks, operands of the user's own on the host, or operands on
+        the device that are not those that the copies go to."""
+        sd, sp, h = self.sddmm, self.spmm, self.host
+        if not (sd._single and sp._single) or any(h[n] is not t for n, t in self._host_made.items()):
+            return None
+        for loc, owned, like in ((sd.A_loc, sd.A_owned, h["A"]), (sd.B_loc, sd.B_owned, h["B"]),
+                                 (sp.X_loc, sp.X_owned, h["B"]), (sp.Y_loc, sp.Y_owned, sp.Y_owned)):
+            if (loc.data_ptr() != owned.data_ptr() or not loc.shape == owned.shape == like.shape
+                    or loc.dtype != like.dtype or not (loc.is_contiguous() and owned.is_contiguous())):
+                return None
         from ..ops import cuda_ops
-        sd, sp, h, d = self.sddmm, self.spmm, self._host_full, self._dev_full
         bs, bp = sd._bind(), sp._bind()
         if self._native_step is None or self._native_step[0] is not bs or self._native_step[1] is not bp:
-            x = self._owned_storage(sp.X_owned)
-            self._native_step = (bs, bp, cuda_ops.HostStep(bs, bp, h["A"], h["B"], d["A"], d["B"], x, sp.Y_owned,
+            self._native_step = (bs, bp, cuda_ops.HostStep(bs, bp, h["A"], h["B"], sd.A_loc, sd.B_loc, sp.X_loc, sp.Y_loc,
                                                            self.plan.rowptr, self.device))
         return self._native_step[2]
 
@@ -97,30 +110,29 @@ class SddmmSpmmStep:
         SpMM is B: one device-to-device copy), runs SDDMM and SpMM (the SpMM
         overlaps the copy of A) and reads back the checksums of this rank's
         results (two fp64 scalars)."""
-        sd, sp, h, d = self.sddmm, self.spmm, self._host_full, self._dev_full
-        if any(self.host[n] is not v for n, v in self._host_views.items()):   # other operands put in their place
-            h, d = self.host, {"A": sd.A_owned, "B": sd.B_owned}
-        elif sd._single and sp._single:
-            return self._bound_step().run()
+        sd, sp = self.sddmm, self.spmm
+        native_step = self._bound_step()
+        if native_step is not None:
+            return native_step.run()
         if self.device.type == "cuda":
             # B first; while A follows on a copy stream the SpMM (which needs only X = B) already runs
             main = torch.cuda.current_stream(self.device)
             if getattr(self, "_copy_stream", None) is None:
                 self._copy_stream = torch.cuda.Stream(self.device)
                 self._ev_b, self._ev_a = torch.cuda.Event(), torch.cuda.Event()
-            d["B"].copy_(h["B"], non_blocking=True)
+            self._upload("B", sd.B_owned)
             self._ev_b.record(main)
             self._copy_stream.wait_event(self._ev_b)   # also orders this copy of A after the previous step's SDDMM
             with torch.cuda.stream(self._copy_stream):
-                d["A"].copy_(h["A"], non_blocking=True)
+                self._upload("A", sd.A_owned)
                 self._ev_a.record(self._copy_stream)
             sp.X_owned.copy_(sd.B_owned)
             y = sp.run_async()
             main.wait_event(self._ev_a)
             c = sd.run_async()
         else:
-            d["A"].copy_(h["A"])
-            d["B"].copy_(h["B"])
+            self._upload("A", sd.A_owned)
+            self._upload("B", sd.B_owned)
             sp.X_owned.copy_(sd.B_owned)
             c = sd.run_async()
             y = sp.run_async()
@@ -214,6 +226,8 @@ class GatLayer:
         if Z == 1 and self.sddmm.variant in ("sparse", "sparseNRB"):
             # one layer holds all of k: the SDDMM writes its scores where the SpMM reads its values
             self.sddmm.partial = self.spmm.vals
+            if self.sddmm._single:
+                self.sddmm._bind()
         # the SpMM wants its values in CSR order; a fused SDDMM stores them in its own order
         order = self.sddmm.value_order
         self._pos = None if order is None else torch.from_numpy(np.ascontiguousarray(order)).to(dev)

@@ -292,10 +292,16 @@ def spmm(rowptr, rowidx, colidx, vals, X, Y, beta, sched: SpmmSchedule | None):
 
 
 # ---- bound calls -------------------------------------------------------------
+class _PackRows(C.Structure):
+    _fields_ = [("src", C.c_void_p), ("ld", C.c_longlong), ("dst", C.c_void_p), ("rows", C.c_longlong), ("k", C.c_int),
+                ("nvec", C.c_int)]
+
+
 class _SddmmCall(C.Structure):
     _fields_ = [("nnz", C.c_longlong), ("ri", C.c_void_p), ("ci", C.c_void_p), ("sv", C.c_void_p), ("A", C.c_void_p),
                 ("lda", C.c_longlong), ("B", C.c_void_p), ("ldb", C.c_longlong), ("out", C.c_void_p), ("k", C.c_int),
-                ("f64", C.c_int), ("where", C.c_void_p), ("dots", C.c_void_p)]
+                ("f64", C.c_int), ("where", C.c_void_p), ("dots", C.c_void_p), ("pack_a", _PackRows),
+                ("pack_b", _PackRows)]
 
 
 class _SpmmCall(C.Structure):
@@ -304,7 +310,7 @@ class _SpmmCall(C.Structure):
                 ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
                 ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
                 ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int), ("k_out", C.c_int),
-                ("x_rows", C.c_int)]
+                ("x_rows", C.c_int), ("pack_x", _PackRows)]
 
 
 _checked_calls = False
@@ -315,7 +321,7 @@ class _BoundCall:
     time (the plain calls above convert every pointer each time, 15-25 us).  `bound_to` says whether the tensors
     are still the ones given; an operator that had its tensors replaced binds again."""
 
-    def __init__(self, name, record, tensors, keep=()):
+    def __init__(self, name, record, tensors, keep=(), launches=1):
         global _checked_calls
         lib = native.cuda()
         if not _checked_calls:
@@ -324,7 +330,7 @@ class _BoundCall:
             if (a.value, b.value) != (C.sizeof(_SddmmCall), C.sizeof(_SpmmCall)):
                 raise RuntimeError("call record layout differs between Python and the kernel library")
             _checked_calls = True
-        self._name, self._record, self._tensors, self._keep = name, record, tensors, keep
+        self._name, self._record, self._tensors, self._keep, self._launches = name, record, tensors, keep, launches
         self._addr = C.addressof(record)
         self._fn = getattr(lib, f"sp3_cuda_{name}_call")
         self._ptrs = [t.data_ptr() for t in tensors]
@@ -339,21 +345,63 @@ class _BoundCall:
         global LAUNCHES
         if beta is not None:
             self._record.beta = beta
-        LAUNCHES += 1
+        LAUNCHES += self._launches
         rc = self._fn(self._addr, _raw_stream())
         if rc != 0:
             raise RuntimeError(f"{self._name}: CUDA launch error {rc}")
 
 
-def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None):
+def has_room(nbytes, device):
+    """Whether an operator may take `nbytes` for good to run faster: at most a quarter of what the device has left."""
+    free = torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+    return 4 * nbytes <= free
+
+
+PACK_MIN_WORK = 20_000_000   # nonzeros x vectors saved per nonzero
+
+
+def pack_rule(kernel, nnz, rows, k, es, device):
+    """Whether a run first copies its operands (`rows` rows of `k` values of `es` bytes in all) to rows of whole 16-byte
+    vectors.  Operands are what the user sees, contiguous; rows that are no multiple of 16 bytes are otherwise read 8 or
+    4 bytes at a time.
+
+    The kernel gains with every narrow vector it does not read (0.3 to 0.6 ps each), the copy costs two passes over the
+    rows (0.3 ps a byte): the line lies at 0.7 vectors saved per byte copied.  Measured (copied / as they are):
+      R-MAT scale 20, SpMM      k = 33 358 / 571 us (1.7 per byte), k = 50 462 / 529 (0.9), k = 126 876 / 850 (0.9)
+      R-MAT scale 20, SDDMM     k = 33 374 / 432 (1.4), k = 50 474 / 438 (0.4), k = 99 830 / 1161 (1.4)
+      R-MAT scale 17, SpMM, beta k = 33 62 / 85; scale 18, 8 a row, k = 34 73 / 61 (0.45)
+      Erdos-Renyi 300 thousand rows, 24 a row, SDDMM, k = 70 268 / 327 (0.73), k = 50 193 / 186 (0.72)
+    Small products do not pay for the launch (scale 14, k = 50: SDDMM 17 / 11, SpMM 17 / 14), nor do narrow rows, where
+    the SpMM gains nothing from wide vectors (scale 20, k = 10: 216 / 176)."""
+    row_bytes = k * es
+    if row_bytes % 16 == 0 or row_bytes > 256 * 16 or row_bytes < (128 if kernel == "spmm" else 16):
+        return False
+    saved = row_bytes // (8 if row_bytes % 8 == 0 else 4) - -(-row_bytes // 16)
+    return nnz * saved >= max(PACK_MIN_WORK, 7 * row_bytes * rows // 10) and has_room(rows * (row_bytes + 16), device)
+
+
+def _packed(t):
+    """(copy of `t` with rows of whole 16-byte vectors, contents undefined; record that fills it)."""
+    n, k = t.shape
+    per = 16 // t.element_size()
+    nvec = -(-k // per)
+    full = torch.empty(n, nvec * per, dtype=t.dtype, device=t.device)
+    return full, _PackRows(native.ptr(t), _ld(t), native.ptr(full), n, k, nvec)
+
+
+def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None, pack=None):
     """`sddmm` bound to its tensors (all given); `chunks`: the lists of `column_chunks`, taken instead of the row-sorted
-    ones."""
+    ones; `pack`: whether the kernel reads packed copies of A and B, by `pack_rule` when not said."""
     p = native.ptr
     r, c, where = chunks or (rowidx, colidx, None)
     dots = torch.empty_like(out) if chunks else None
-    rec = _SddmmCall(rowidx.shape[0], p(r), p(c), p(svals), p(A), _ld(A), p(B), _ld(B), p(out), A.shape[1],
-                     int(A.dtype == torch.float64), p(where), p(dots))
-    return _BoundCall("sddmm", rec, (rowidx, colidx, svals, A, B, out), keep=(chunks, dots))
+    a, b, pa, pb = A, B, _PackRows(), _PackRows()
+    if pack_rule("sddmm", rowidx.shape[0], A.shape[0] + B.shape[0], A.shape[1], A.element_size(), A.device) if pack is None else pack:
+        (a, pa), (b, pb) = _packed(A), _packed(B)
+    rec = _SddmmCall(rowidx.shape[0], p(r), p(c), p(svals), p(a), _ld(a), p(b), _ld(b), p(out), a.shape[1],
+                     int(A.dtype == torch.float64), p(where), p(dots), pa, pb)
+    return _BoundCall("sddmm", rec, (rowidx, colidx, svals, A, B, out), keep=(chunks, dots, a, b),
+                      launches=1 + (a is not A))
 
 
 CHUNK_BYTES = 96 << 20     # rows of B that stay in the L2 (126 MB) next to what streams through it
@@ -390,15 +438,19 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
     return rowidx[index], colidx[index], where
 
 
-def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule):
-    """`spmm` bound to its tensors; `launch(beta)`.  X may be wider than Y, see `local.spmm`."""
+def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule, pack=None):
+    """`spmm` bound to its tensors; `launch(beta)`.  X may be wider than Y, see `local.spmm`; `pack` as in `bind_sddmm`."""
     p = native.ptr
-    carry, ldc = sched.carry_for(X.shape[1], X.dtype, X.device)
-    rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(X),
-                    _ld(X), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
-                    p(sched.ticket), 0.0, X.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1],
-                    X.shape[0])
-    return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry))
+    x, px = X, _PackRows()
+    if X.shape[1] == Y.shape[1] and (pack_rule("spmm", colidx.shape[0], X.shape[0], X.shape[1], X.element_size(), X.device)
+                                     if pack is None else pack):
+        x, px = _packed(X)
+    carry, ldc = sched.carry_for(x.shape[1], X.dtype, X.device)
+    rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(x),
+                    _ld(x), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
+                    p(sched.ticket), 0.0, x.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1],
+                    X.shape[0], px)
+    return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry, x), launches=1 + (x is not X))
 
 
 STEP_CHUNKS = 8
@@ -438,19 +490,18 @@ class HostStep:
         row_bytes = nbytes // max(1, nrows)
         ends = [int(rowptr[r]) // 4 * 4 for r in rows_end[:-1]] + [nnz]
         pad = [0] * (STEP_CHUNKS - n)
+        # the SDDMM follows the rows of A as they arrive: the row-sorted lists, rows as they are
         self._rec = _StepCall(
-            sddmm._record, spmm._record, p(host_a), p(host_b), p(dev_a), p(dev_b), p(dev_x), nbytes,
+            bind_sddmm(*sddmm._tensors, pack=False)._record, spmm._record, p(host_a), p(host_b), p(dev_a), p(dev_b), p(dev_x), nbytes,
             host_b.numel() * host_b.element_size(), Y.numel(), n, 0,
             (C.c_longlong * STEP_CHUNKS)(*([r * row_bytes for r in rows_end] + pad)),
             (C.c_longlong * STEP_CHUNKS)(*(ends + pad)), p(self._part), p(self._sums), p(self._out),
             self._copy.cuda_stream, self._events[0].cuda_event,
             (C.c_void_p * STEP_CHUNKS)(*([e.cuda_event for e in self._events[1:]] + pad)))
         self._rec.spmm.beta = 0.0
-        # the SDDMM follows the rows of A as they arrive: always the row-sorted lists
-        self._rec.sddmm.ri, self._rec.sddmm.ci, self._rec.sddmm.where = p(sddmm._tensors[0]), p(sddmm._tensors[1]), None
         self._addr, self._fn = C.addressof(self._rec), lib.sp3_cuda_step_call
         self._keep = (sddmm, spmm, host_a, host_b, dev_a, dev_b, dev_x, Y)
-        self._launches = 5 + n
+        self._launches = 4 + n + spmm._launches
         self._device = device
 
     def run(self):

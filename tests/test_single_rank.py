@@ -193,3 +193,98 @@ def test_gat_layer_twice_on_the_host(dtype, variant):
         y = layer.run()
         _check_layer(layer, plan, 8, dtype, A, B, X, torch.from_numpy(before).to(dtype), layer.spmm.vals, y)
     assert np.array_equal(plan.vals, before)
+
+
+def _bind_case(plan, k, dtype, ld, shift, seed=1):
+    """Operands as strided views that begin `shift` values behind a boundary, on the GPU, and their values."""
+    def make(rows, seed):
+        vals = _randn(torch.empty(rows, k, dtype=dtype), seed)
+        buf = torch.full((rows * ld + shift,), float("nan"), dtype=dtype, device="cuda")
+        view = buf[shift:].view(rows, ld)[:, :k]
+        view.copy_(vals)
+        return vals, view
+    return make(plan.row.n_local, seed), make(plan.col.n_local, seed + 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("spec", ["uniform:1:1:1", "uniform:37:5:2", "zipf:900:1200:1.6:300"])
+@pytest.mark.parametrize("k,extra,shift", [(1, 0, 0), (3, 0, 0), (5, 2, 1), (33, 0, 0), (50, 0, 1), (63, 1, 0),
+                                           (130, 0, 0), (259, 0, 3), (1023, 0, 0)])
+def test_packed_operands(spec, k, extra, shift, dtype):
+    """Kernels on packed copies: rows of every remainder, one row, views with anything (here NaN) between the rows."""
+    from spcomm3d_b200.ops import cuda_ops
+    if k * dtype.itemsize > 4096:
+        pytest.skip("wider than the packed form")
+    plan = _plan(spec)
+    (A, Ad), (B, Bd) = _bind_case(plan, k, dtype, k + extra, shift)
+    rowptr, ri, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.rowidx, plan.colidx))
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    v, out = vals.cuda(), torch.full((plan.nnz,), float("nan"), dtype=dtype, device="cuda")
+    cuda_ops.bind_sddmm(ri, ci, v, Ad, Bd, out, pack=True).launch()
+    ref, mag = _scores(plan, A, B, vals)
+    assert bool(((out.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+    deg = _lists(plan)[2].numpy()
+    Y0 = _randn(torch.empty(plan.row.n_local, k, dtype=dtype), 5)
+    Y = Y0.cuda()
+    cuda_ops.bind_spmm(rowptr, ci, v, Bd, Y, cuda_ops.SpmmSchedule(rowptr), pack=True).launch(-0.5)
+    bound = torch.from_numpy(_gamma(deg + 3.0, dtype))[:, None] * (_product(plan, vals.abs(), B.abs()) + 0.5 * Y0.double().abs())
+    assert bool(((Y.cpu().double() - (_product(plan, vals, B) - 0.5 * Y0.double())).abs() <= bound).all())
+
+
+def test_pack_rule(monkeypatch):
+    from spcomm3d_b200.ops import cuda_ops
+    monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: True)
+    n, rows = 16_000_000, 1 << 20
+    assert cuda_ops.pack_rule("spmm", n, rows, 33, 4, None) and cuda_ops.pack_rule("sddmm", n, 2 * rows, 33, 4, None)
+    for k in (32, 64, 256, 2):        # whole vectors; too narrow
+        assert not cuda_ops.pack_rule("spmm", n, rows, k, 4, None)
+    assert not cuda_ops.pack_rule("spmm", n // 16, rows, 33, 4, None)      # a nonzero per row
+    assert not cuda_ops.pack_rule("spmm", 100_000, 1000, 33, 4, None)      # small
+    assert not cuda_ops.pack_rule("sddmm", n, rows, 1025, 4, None)         # wider than the vector kernels
+    monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: False)
+    assert not cuda_ops.pack_rule("spmm", n, rows, 33, 4, None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("packs", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [1, 3, 33, 50, 64])
+def test_operands_are_the_users(k, dtype, packs, monkeypatch):
+    """Operands are contiguous whatever the width, and an operand that the user puts in the place of one is the one
+    that counts, with its own stride, in every kind of run."""
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    from spcomm3d_b200.ops import cuda_ops
+    if packs:
+        monkeypatch.setattr(cuda_ops, "pack_rule", lambda kernel, nnz, rows, k, es, device: k * es % 16 != 0)
+    plan = _plan("rmat:10:8")
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    step = SddmmSpmmStep(plan, None, k, dtype, "cuda", seed=2)
+    step.fill_device_operands()
+    sd, sp = step.sddmm, step.spmm
+    for t in (sd.A_owned, sd.B_owned, sp.X_owned, sp.Y_owned, sd.A_loc, sp.X_loc):
+        assert t.is_contiguous() and t.view(-1).numel() == t.shape[0] * k
+    deg = _lists(plan)[2].numpy()
+
+    def check(c, y, A, B, X):
+        A, B, X = A.cpu(), B.cpu(), X.cpu()
+        ref, mag = _scores(plan, A, B, vals)
+        assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+        bound = torch.from_numpy(_gamma(deg + 3.0, dtype))[:, None] * _product(plan, vals.abs(), X.abs())
+        assert bool(((y.cpu().double() - _product(plan, vals, X)).abs() <= bound).all())
+    check(*step.run_device(), sd.A_owned, sd.B_owned, sp.X_owned)
+    step.make_host_operands()
+    assert step.h2d_bytes == (plan.row.n_owned + plan.col.n_owned) * k * dtype.itemsize
+    step.run_e2e()
+    check(sd.partial, sp.Y_owned, step.host["A"], step.host["B"], step.host["B"])
+    (_, A), (_, B) = _bind_case(plan, k, dtype, k + 3, 1, seed=7)
+    X = _randn(sp.X_loc, 9).cuda()
+    sd.A_loc, sd.B_loc, sp.X_loc = A, B, X
+    check(*step.run_device(), A, B, X)
+    check(sd.run(), sp.run(), A, B, X)
+    step.run_e2e()                       # the copies go to the owned rows, which are not what the kernels read now
+    check(sd.partial, sp.Y_owned, A, B, X)
+    assert torch.equal(sd.A_owned.cpu(), step.host["A"]) and torch.equal(sp.X_owned.cpu(), step.host["B"])
+    sd.A_loc, sd.B_loc, sp.X_loc = sd.A_owned, sd.B_owned, sp.X_owned
+    step.run_e2e()
+    check(sd.partial, sp.Y_owned, step.host["A"], step.host["B"], step.host["B"])
