@@ -543,6 +543,7 @@ SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
 }
 template <typename T> static int sddmm_call(const SddmmCall& c, cudaStream_t st) {
     T* out = (T*)(c.where ? c.dots : c.out);
+    if (c.where && c.nnz > 0x7fffffffll - 1024) return (int)cudaErrorInvalidValue;   // scale_picked_kernel counts in 32 bits
     int rc = launch_pack<T>(c.pack_a, c.pack_b, st);
     if (rc != 0) return rc;
     rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,

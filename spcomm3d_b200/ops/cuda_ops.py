@@ -406,6 +406,8 @@ def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None, pack=None):
 
 CHUNK_BYTES = 96 << 20     # rows of B that stay in the L2 (126 MB) next to what streams through it
 CHUNK_MIN_NNZ = 1 << 20
+CHUNK_MAX_NNZ = 2 ** 31 - 1025   # positions are 32-bit numbers, rounded up to a block of 1024
+CHUNK_LIST_BYTES = 20      # per nonzero, for good: the two lists, the position and the dot product (up to 8)
 
 
 def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
@@ -422,8 +424,9 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
     save."""
     nnz = rowidx.shape[0]
     n = force or -(-n_cols * row_bytes // CHUNK_BYTES)
-    if not force and (n < 2 or n > 32 or nnz < CHUNK_MIN_NNZ or nnz < 4 * n_cols):
-        return None
+    if nnz > CHUNK_MAX_NNZ or not force and (n < 2 or n > 32 or nnz < CHUNK_MIN_NNZ or nnz < 4 * n_cols
+                                             or not has_room(CHUNK_LIST_BYTES * nnz, colidx.device)):
+        return None   # (sorting takes another 25 bytes per nonzero for a moment, which the quarter leaves)
     chunk = torch.div(colidx, -(-n_cols // n), rounding_mode="floor")
     if not force:
         count = torch.bincount(colidx, minlength=n_cols)

@@ -288,3 +288,20 @@ def test_operands_are_the_users(k, dtype, packs, monkeypatch):
     sd.A_loc, sd.B_loc, sp.X_loc = sd.A_owned, sd.B_owned, sp.X_owned
     step.run_e2e()
     check(sd.partial, sp.Y_owned, step.host["A"], step.host["B"], step.host["B"])
+
+
+def test_column_chunks_limits(monkeypatch):
+    """Blocks that the chunked lists cannot number, or that leave no room for them, keep the row-sorted ones."""
+    from spcomm3d_b200.ops import cuda_ops
+    huge = torch.empty(2 ** 31 - 1000, dtype=torch.int32, device="meta")
+    monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: True, raising=False)
+    assert cuda_ops.column_chunks(huge, huge, 1 << 22, 512) is None
+    monkeypatch.setattr(cuda_ops, "CHUNK_BYTES", 1 << 18)
+    monkeypatch.setattr(cuda_ops, "CHUNK_MIN_NNZ", 1)
+    rows = torch.arange(4096, dtype=torch.int32).repeat_interleave(64)
+    cols = torch.randint(0, 4096, (4096, 64), generator=torch.Generator().manual_seed(0)).sort(1)[0].int().reshape(-1)
+    asked = []
+    monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: bool(asked.append(nbytes)))
+    assert cuda_ops.column_chunks(rows, cols, 4096, 256) is None and asked == [20 * rows.numel()]
+    monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: True)
+    assert cuda_ops.column_chunks(rows, cols, 4096, 256) is not None
