@@ -341,10 +341,11 @@ class _BoundCall:
                 return False
         return True
 
-    def launch(self, beta=None):
+    def launch(self, *beta):
+        """One run; the SpMM is given its beta, a number."""
         global LAUNCHES
-        if beta is not None:
-            self._record.beta = beta
+        if beta:
+            (self._record.beta,) = beta
         LAUNCHES += self._launches
         rc = self._fn(self._addr, _raw_stream())
         if rc != 0:

@@ -305,3 +305,18 @@ def test_column_chunks_limits(monkeypatch):
     assert cuda_ops.column_chunks(rows, cols, 4096, 256) is None and asked == [20 * rows.numel()]
     monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: True)
     assert cuda_ops.column_chunks(rows, cols, 4096, 256) is not None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("beta", [None, "x", 1j])
+def test_beta_has_to_be_a_number(beta):
+    from spcomm3d_b200.models.dist_ops import DistSpMM
+    op = DistSpMM(_plan("uniform:30:40:3"), None, 8, torch.float32, "cuda")
+    op.X_owned.fill_(1.0), op.Y_owned.fill_(2.0)
+    op.timer.enabled = False
+    op.run(3.0)
+    y = op.Y_owned.clone()
+    for run in (op.run, op.run_async):
+        with pytest.raises(TypeError):
+            run(beta)
+    assert torch.equal(op.Y_owned, y)
