@@ -717,11 +717,17 @@ SP3_API int sp3_cuda_spmm_f32_noalloc(int nrows, int nitems, const void* items, 
                                       void* stream) {
     if (nrows < 0 || nitems < 0 || nlong < 0 || total_pieces < 0 || k <= 0) return SP3_NOALLOC_E_ARG;
     // layout of the scratch: [counters: SP3_NOALLOC_MAX_SPLIT_ROWS x int32][carry: total_pieces x ldc floats]
-    const long long ldc = ((long long)k + 3) / 4 * 4;  // keep carry rows 16-byte aligned
+    long long ldc = ((long long)k + 3) / 4 * 4;  // keep carry rows 16-byte aligned
     const size_t counters_bytes = (size_t)SP3_NOALLOC_MAX_SPLIT_ROWS * sizeof(int);
     const size_t carry_bytes = (size_t)total_pieces * (size_t)ldc * sizeof(float);
-    if (nlong > SP3_NOALLOC_MAX_SPLIT_ROWS || counters_bytes + carry_bytes > (size_t)SP3_NOALLOC_SCRATCH_BYTES)
-        return SP3_NOALLOC_E_TOO_LARGE;
+    if (nlong > SP3_NOALLOC_MAX_SPLIT_ROWS) return SP3_NOALLOC_E_TOO_LARGE;
+    if (counters_bytes + carry_bytes > (size_t)SP3_NOALLOC_SCRATCH_BYTES) {
+        // The short pieces of small matrices are up to sixteen times as many as the regular ones: what would have
+        // fitted with those is computed in parts of columns.
+        if (piece_len >= SP3_NOALLOC_REGULAR_PIECE) return SP3_NOALLOC_E_TOO_LARGE;
+        ldc = (long long)((SP3_NOALLOC_SCRATCH_BYTES - counters_bytes) / sizeof(float) / (size_t)total_pieces / 4 * 4);
+        if (ldc < 4) return SP3_NOALLOC_E_TOO_LARGE;
+    }
     int dev = -1;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return (int)err;
@@ -741,6 +747,12 @@ SP3_API int sp3_cuda_spmm_f32_noalloc(int nrows, int nitems, const void* items, 
         if (err != cudaSuccess) return (int)err;
     }
     sp3::SpmmLong lg{first_piece, npieces, (int*)base, (void*)(base + counters_bytes), ldc, piece_len, nullptr};
-    return sp3::launch_spmm<float>(nrows, nitems, (const int4*)items, rowptr, colidx, val, X, ldx, k, beta, Y, ldy,
-                                   lg, st);
+    // (a part leaves the counters at zero for the next)
+    for (int j = 0; j < k; j += (int)ldc) {
+        const int n = k - j < ldc ? k - j : (int)ldc;
+        const int rc = sp3::launch_spmm<float>(nrows, nitems, (const int4*)items, rowptr, colidx, val, X + j, ldx, n, beta,
+                                               Y + j, ldy, lg, st);
+        if (rc != 0) return rc;
+    }
+    return 0;
 }

@@ -25,7 +25,10 @@
  *         <= SP3_NOALLOC_SCRATCH_BYTES;
  * anything larger is refused with SP3_NOALLOC_E_TOO_LARGE and nothing is
  * launched.  (With k = 128 that is room for about 16,000 pieces of 512
- * nonzeros, i.e. 8 million nonzeros in split rows.)
+ * nonzeros, i.e. 8 million nonzeros in split rows.)  The scheduler cuts the
+ * rows of small matrices (below 454,656 nonzeros) into shorter and so into more
+ * pieces; with a piece_len below SP3_NOALLOC_REGULAR_PIECE a call that does not
+ * fit runs as several launches, each on as many columns as fit (at least 4).
  *
  * First call.  The first call on each device looks up the device address of
  * the array (cudaGetSymbolAddress) with that device current.  Make that first
@@ -44,10 +47,11 @@
  * int32, val), its work items (int32[nitems][4]) with the split-row tables
  * first_piece/npieces (int32[nlong]) as built by the framework's scheduler,
  * X [*, k] with leading dimension ldx, Y [nrows, k] with leading dimension
- * ldy, Y = beta*Y + A X.  All pointers are device pointers.  k, ldx and ldy
- * must be multiples of 4 and X, Y 16-byte aligned for the vector kernel;
- * otherwise the scalar kernel runs (it needs no scratch).
- * total_pieces = sum of npieces, piece_len = nonzeros per piece.
+ * ldy, Y = beta*Y + A X.  All pointers are device pointers.  Rows are read 16
+ * bytes at a time where k, ldx and ldy are multiples of 4 and X, Y 16-byte
+ * aligned, otherwise 8 or 4 bytes at a time; rows of more than 256 such vectors
+ * go to a scalar kernel (it needs no scratch).
+ * total_pieces = sum of npieces, piece_len = nonzeros of the largest piece.
  *
  * Returns 0, a negative SP3_NOALLOC_E_* code, or a positive cudaError_t.
  */
@@ -56,6 +60,7 @@
 
 #define SP3_NOALLOC_SCRATCH_BYTES (8 * 1024 * 1024)
 #define SP3_NOALLOC_MAX_SPLIT_ROWS 16384
+#define SP3_NOALLOC_REGULAR_PIECE 512
 #define SP3_NOALLOC_E_ARG (-4)
 #define SP3_NOALLOC_E_TOO_LARGE (-5)
 

@@ -320,3 +320,30 @@ def test_beta_has_to_be_a_number(beta):
         with pytest.raises(TypeError):
             run(beta)
     assert torch.equal(op.Y_owned, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [64, 1024, 1030])
+def test_noalloc_with_short_pieces(k):
+    """Rows of 40 nonzeros, cut into pieces of 32: too many for the fixed scratch at full width, where not one row
+    would be cut into regular pieces."""
+    import ctypes as C
+    from spcomm3d_b200.ops import cuda_ops
+    from spcomm3d_b200.utils import native
+    plan = _plan("uniform:2700:3000:40")
+    rowptr, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.colidx))
+    vals = torch.from_numpy(plan.vals).float()
+    sched = cuda_ops.SpmmSchedule(rowptr)
+    assert sched.total_pieces == 2 * 2700 and sched.nlong == 2700
+    X, Y0, v = _randn(torch.empty(plan.col.n_local, k), 1), _randn(torch.empty(2700, k), 2), vals.cuda()
+    Xd, Y, p = X.cuda(), Y0.cuda(), native.ptr
+    fn = native.cuda().sp3_cuda_spmm_f32_noalloc
+    fn.restype = C.c_int
+    fn.argtypes = [C.c_int, C.c_int] + [C.c_void_p] * 5 + [C.c_longlong, C.c_int, C.c_float, C.c_void_p, C.c_longlong,
+                                                           C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
+    rc = fn(2700, sched.items.shape[0], p(sched.items), p(rowptr), p(ci), p(v), p(Xd), k, k, 0.5, p(Y), k, p(sched.first),
+            p(sched.npieces), sched.nlong, sched.total_pieces, sched.piece_len, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    bound = torch.from_numpy(_gamma(_lists(plan)[2].numpy() + 3.0, torch.float32))[:, None] * (
+        _product(plan, vals.abs(), X.abs()) + 0.5 * Y0.double().abs())
+    assert bool(((Y.cpu().double() - (_product(plan, vals, X) + 0.5 * Y0.double())).abs() <= bound).all())
