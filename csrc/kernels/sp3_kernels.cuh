@@ -453,7 +453,8 @@ template <typename T> struct EmitPacked {
 };
 
 // One item, one warp (see build_spmm_items in ops/cuda_ops.py):
-//   rows item   (first row, end row, first nonzero, -1 - nonzeros): at most SPMM_ITEM_ROWS whole rows
+//   rows item   (first row, end row, first nonzero, -1 - nonzeros): at most SPMM_ITEM_ROWS whole rows; a first
+//               nonzero that 32 bits do not hold is -1 and read from the row pointer
 //   piece item  (row, first nonzero, end nonzero, long-row slot | piece number << SPMM_PIECE_SHIFT)
 //
 // The nonzeros of an item are dealt to the lane groups in equal shares of whole quads, wherever the rows end: a
@@ -490,7 +491,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     };
     const bool is_rows = item.w < 0;
     const int nr = is_rows ? item.y - item.x : 0;
-    const long long p0 = is_rows ? item.z : item.y;
+    const long long p0 = !is_rows ? item.y : (item.z >= 0 ? item.z : __ldg(rowptr + item.x));
     const int n = is_rows ? -1 - item.w : item.z - item.y;
     // positions count from the 16-byte boundary at or before the first nonzero
     const int lead = (int)(p0 & 3), stop = lead + n;

@@ -114,7 +114,7 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
     """Work items of the SpMM kernel from a CSR row pointer (host, vectorised).
 
     Returns (items int32[n,4], first_piece int32[nlong], npieces int32[nlong]).
-    rows item  = (row_begin, row_end, first nonzero, -1 - number of nonzeros)
+    rows item  = (row_begin, row_end, first nonzero (-1: from 2^31, see the row pointer), -1 - number of nonzeros)
     piece item = (row, nnz_begin, nnz_end, long_row_slot | piece_number_in_row << PIECE_SHIFT)
     """
     nrows = rowptr.shape[0] - 1
@@ -132,7 +132,8 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
     ends = np.append(starts[1:], nrows)
     short = ~is_long[starts]
     first_nnz = rowptr[starts[short]]
-    rows_items = np.stack([starts[short], ends[short], first_nnz, first_nnz - rowptr[ends[short]] - 1], axis=1)
+    rows_items = np.stack([starts[short], ends[short], np.where(first_nnz < 2 ** 31, first_nnz, -1),
+                           first_nnz - rowptr[ends[short]] - 1], axis=1)
     long_rows = np.flatnonzero(is_long)
     npieces = (deg[long_rows] + long_row - 1) // long_row
     first = np.concatenate([[0], np.cumsum(npieces)[:-1]]) if long_rows.size else np.zeros(0, np.int64)

@@ -347,3 +347,30 @@ def test_noalloc_with_short_pieces(k):
     bound = torch.from_numpy(_gamma(_lists(plan)[2].numpy() + 3.0, torch.float32))[:, None] * (
         _product(plan, vals.abs(), X.abs()) + 0.5 * Y0.double().abs())
     assert bool(((Y.cpu().double() - (_product(plan, vals, X) + 0.5 * Y0.double())).abs() <= bound).all())
+
+
+def test_items_beyond_2_31_nonzeros():
+    """Rows items are numbered by row: a block may hold more nonzeros than 32 bits count, as long as none of its split
+    rows lies beyond."""
+    from spcomm3d_b200.ops import cuda_ops
+    rowptr = np.array([0, 2 ** 30, 2 ** 31 - 8, 2 ** 31, 2 ** 31 + 5, 2 ** 31 + 5, 2 ** 31 + 9])
+    items, first, npieces = cuda_ops.build_spmm_items(rowptr, long_row=2 ** 31 - 1, item_nnz=1)
+    assert npieces.size == 0 and items[:, 2].tolist() == [0, 2 ** 30, 2 ** 31 - 8, -1, -1]
+    assert items[-2:, :2].tolist() == [[3, 4], [4, 6]] and items[-2:, 3].tolist() == [-6, -5]
+    with pytest.raises(ValueError):
+        cuda_ops.build_spmm_items(np.array([0, 2 ** 31, 2 ** 31 + 700]), long_row=512)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [8, 33, 64])
+def test_items_without_first_nonzero(k):
+    from spcomm3d_b200.ops import cuda_ops, local
+    plan = _plan("zipf:900:1200:1.6:300")
+    rowptr, ri, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.rowidx, plan.colidx))
+    v, X = torch.from_numpy(plan.vals).float().cuda(), _randn(torch.empty(plan.col.n_local, k), 1).cuda()
+    sched, out = cuda_ops.SpmmSchedule(rowptr), []
+    for _ in range(2):
+        out.append(torch.zeros(plan.row.n_local, k, device="cuda"))
+        local.spmm(rowptr, ri, ci, v, X, out[-1], 0.0, sched)
+        sched.items[sched.items[:, 3] < 0, 2] = -1
+    assert torch.equal(*out)
