@@ -237,7 +237,8 @@ class SpmmSchedule:
         else:   # (items, first_piece, npieces) built elsewhere, e.g. by build_spmm_wave_items
             items, first, npieces = arrays
         dev = rowptr.device
-        self.piece_len = kw.get("long_row") or item_sizes(int(rp[-1]) if arrays is None else int(rowptr[-1]))[0]
+        pieces = items[items[:, 3] >= 0]
+        self.piece_len = int((pieces[:, 2] - pieces[:, 1]).max(initial=0))   # nonzeros of the largest piece
         self.items = torch.from_numpy(items).to(dev).contiguous()
         self.first = torch.from_numpy(first).to(dev)
         self.npieces = torch.from_numpy(npieces).to(dev)

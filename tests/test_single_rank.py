@@ -374,3 +374,17 @@ def test_items_without_first_nonzero(k):
         local.spmm(rowptr, ri, ci, v, X, out[-1], 0.0, sched)
         sched.items[sched.items[:, 3] < 0, 2] = -1
     assert torch.equal(*out)
+
+
+def test_piece_len_is_that_of_the_largest_piece():
+    from spcomm3d_b200.ops import cuda_ops
+    deg = np.array([3, 100, 0, 33, 64, 5])
+    rowptr = np.concatenate([[0], np.cumsum(deg)])
+    t = torch.from_numpy(rowptr)
+    assert cuda_ops.SpmmSchedule(t).piece_len == 32
+    assert cuda_ops.SpmmSchedule(t, long_row=64).piece_len == 64
+    assert cuda_ops.SpmmSchedule(t, long_row=100).piece_len == 0      # nothing is cut
+    cls = (np.arange(deg.sum()) % 3 == 0).astype(np.int32)
+    _, items, first, npieces, _ = cuda_ops.build_spmm_wave_items(rowptr, cls, 2, long_row=80)
+    piece_len = cuda_ops.SpmmSchedule(t, arrays=(items, first, npieces)).piece_len
+    assert piece_len == max(int((cls[3:103] == c).sum()) for c in (0, 1))   # row 1, cut at the class boundary
