@@ -17,7 +17,7 @@ _F = {torch.float32: "f32", torch.float64: "f64"}
 
 # SpMM schedule parameters: rows with more than LONG_ROW nonzeros are cut into
 # pieces of LONG_ROW; other rows are grouped into items of about ITEM_NNZ
-# nonzeros and at most ITEM_ROWS rows (SPMM_ITEM_ROWS of csrc/kernels/sp3_kernels.cuh).
+# nonzeros and at most ITEM_ROWS rows (SPMM_ITEM_ROWS of csrc/kernels/sp3_kernels.cuh; SP3_ITEM_ROWS asks for fewer).
 LONG_ROW, ITEM_NNZ, ITEM_ROWS = 512, 128, 32
 _TARGET_ITEMS = 148 * 32   # warps that a B200 runs at once
 
@@ -122,7 +122,7 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
     nnz = int(rowptr[-1])
     long_row = _long_row(nnz, deg) if long_row is None else long_row
     item_nnz = item_sizes(nnz)[1] if item_nnz is None else item_nnz
-    item_rows = ITEM_ROWS if item_rows is None else min(item_rows, ITEM_ROWS)
+    item_rows = min(ITEM_ROWS, int(os.environ.get("SP3_ITEM_ROWS", ITEM_ROWS)) if item_rows is None else item_rows)
     is_long = deg > long_row
     key = rowptr[:-1] // item_nnz
     bnd = np.ones(nrows, bool)

@@ -388,3 +388,15 @@ def test_piece_len_is_that_of_the_largest_piece():
     _, items, first, npieces, _ = cuda_ops.build_spmm_wave_items(rowptr, cls, 2, long_row=80)
     piece_len = cuda_ops.SpmmSchedule(t, arrays=(items, first, npieces)).piece_len
     assert piece_len == max(int((cls[3:103] == c).sum()) for c in (0, 1))   # row 1, cut at the class boundary
+
+
+def test_item_rows_variable(monkeypatch):
+    from spcomm3d_b200.ops import cuda_ops
+    rowptr = np.arange(101)
+
+    def most_rows():
+        items = cuda_ops.build_spmm_items(rowptr, item_nnz=1000)[0]
+        return int((items[:, 1] - items[:, 0]).max())
+    for value, want in ((None, 32), ("5", 5), ("64", 32)):
+        monkeypatch.delenv("SP3_ITEM_ROWS", raising=False) if value is None else monkeypatch.setenv("SP3_ITEM_ROWS", value)
+        assert most_rows() == want
