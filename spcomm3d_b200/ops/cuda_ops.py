@@ -185,16 +185,16 @@ def build_spmm_wave_items(rowptr: np.ndarray, cls: np.ndarray, n_classes: int, l
         slot_of = np.repeat(np.arange(lrows.size, dtype=np.int32), ldeg)
         idx = np.arange(int(ldeg.sum()), dtype=np.int64)
         idx += np.repeat(rowptr[lrows] - lstart, ldeg)         # nonzeros of the long rows, ascending
-        key = slot_of * np.int32(256)                          # < 2^28: the slot count is checked below
-        key += cls[idx]
-        order = np.argsort(key, kind="stable")
-        src = idx[order]
-        perm[idx] = src
-        key = key[order]                                       # slot_of is already grouped by row
-        c_sorted = key & np.int32(255)
+        # nonzeros of every (row, class), laid out row by row and class by class in their old order
+        lcls = cls[idx].astype(np.uint8)
+        count = np.bincount(slot_of * np.int64(n_classes) + lcls, minlength=lrows.size * n_classes)
+        begin = np.cumsum(count) - count
+        by_class = count.reshape(-1, n_classes).T.ravel()      # the same groups, class by class
+        shift = begin.reshape(-1, n_classes).T.ravel() - (np.cumsum(by_class) - by_class)
+        perm[idx[np.arange(idx.size) + np.repeat(shift, by_class)]] = idx[np.argsort(lcls, kind="stable")]
         # runs of equal (row, class), cut every long_row nonzeros
-        run_start = np.flatnonzero(np.concatenate([[True], key[1:] != key[:-1]]))
-        run_len = np.diff(np.append(run_start, key.size))
+        runs = np.flatnonzero(count)
+        run_start, run_len, run_cls = begin[runs], count[runs], runs % n_classes
         nchunk = (run_len + long_row - 1) // long_row
         chunk_run = np.repeat(np.arange(run_start.size), nchunk)
         chunk_j = np.arange(int(nchunk.sum())) - np.repeat(np.cumsum(nchunk) - nchunk, nchunk)
@@ -207,7 +207,7 @@ def build_spmm_wave_items(rowptr: np.ndarray, cls: np.ndarray, n_classes: int, l
         if int(npieces.max()) >= 1 << (31 - PIECE_SHIFT):
             raise ValueError("too many pieces per row for the item encoding")
         pieces = np.stack([lrows[p_slot], idx[b_rel], idx[b_rel] + (e_rel - b_rel), p_slot + (p_num << PIECE_SHIFT)], axis=1)
-        pcls = c_sorted[b_rel].astype(np.int64)
+        pcls = run_cls[chunk_run]
     # class of a rows item: the largest class among its nonzeros
     rcls = np.zeros(rows_items.shape[0], np.int64)
     if rows_items.shape[0] and nnz:
