@@ -64,6 +64,7 @@ class SddmmSpmmStep:
         self._host_made = dict(self.host)
         self._native_step = None
         self._sums = torch.zeros(2, dtype=torch.float64, device=self.device)
+        self._bound_step()   # the pinned buffer, the stream and the events of the one-call form are made here
         return self.host
 
     @staticmethod

@@ -400,3 +400,16 @@ def test_item_rows_variable(monkeypatch):
     for value, want in ((None, 32), ("5", 5), ("64", 32)):
         monkeypatch.delenv("SP3_ITEM_ROWS", raising=False) if value is None else monkeypatch.setenv("SP3_ITEM_ROWS", value)
         assert most_rows() == want
+
+
+@pytest.mark.gpu
+def test_first_step_from_host_operands_builds_nothing(monkeypatch):
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    from spcomm3d_b200.ops import cuda_ops
+    step = SddmmSpmmStep(_plan("uniform:200:300:6"), None, 33, torch.float32, "cuda", seed=2)
+    step.fill_device_operands()
+    step.make_host_operands()
+    for name in ("HostStep", "bind_sddmm", "bind_spmm"):
+        monkeypatch.setattr(cuda_ops, name, None)
+    first, second = step.run_e2e(), step.run_e2e()
+    assert first == second
