@@ -404,7 +404,7 @@ def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None, pack=None):
     rec = _SddmmCall(rowidx.shape[0], p(r), p(c), p(svals), p(a), _ld(a), p(b), _ld(b), p(out), a.shape[1],
                      int(A.dtype == torch.float64), p(where), p(dots), pa, pb)
     return _BoundCall("sddmm", rec, (rowidx, colidx, svals, A, B, out), keep=(chunks, dots, a, b),
-                      launches=1 + (a is not A))
+                      launches=1 + (a is not A) + (chunks is not None))
 
 
 CHUNK_BYTES = 96 << 20     # rows of B that stay in the L2 (126 MB) next to what streams through it
@@ -507,7 +507,8 @@ class HostStep:
         self._rec.spmm.beta = 0.0
         self._addr, self._fn = C.addressof(self._rec), lib.sp3_cuda_step_call
         self._keep = (sddmm, spmm, host_a, host_b, dev_a, dev_b, dev_x, Y)
-        self._launches = 4 + n + spmm._launches
+        parts = sum(b > a for a, b in zip([0] + ends, ends))   # (a part without nonzeros launches nothing)
+        self._launches = parts + spmm._launches + 4            # two checksums of two kernels
         self._device = device
 
     def run(self):

@@ -413,3 +413,35 @@ def test_first_step_from_host_operands_builds_nothing(monkeypatch):
         monkeypatch.setattr(cuda_ops, name, None)
     first, second = step.run_e2e(), step.run_e2e()
     assert first == second
+
+
+@pytest.mark.gpu
+def test_launches_are_counted(monkeypatch):
+    """`cuda_ops.LAUNCHES` is the number of kernels: packing, the pass behind the column chunks, the parts of a step."""
+    from spcomm3d_b200.models.dist_ops import DistSDDMM
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    from spcomm3d_b200.ops import cuda_ops
+    plan = _plan("rmat:10:8")
+
+    def kernels(run):
+        run()
+        torch.cuda.synchronize()
+        before = cuda_ops.LAUNCHES
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            run()
+            torch.cuda.synchronize()
+        seen = sum(e.count for e in prof.key_averages() if "sp3::" in e.key)
+        return cuda_ops.LAUNCHES - before, seen
+    for packs in (False, True):
+        monkeypatch.setattr(cuda_ops, "pack_rule", lambda *a: packs, raising=False)
+        step = SddmmSpmmStep(plan, None, 33, torch.float32, "cuda", seed=2)
+        step.make_host_operands()
+        counted, seen = kernels(step.run_device)
+        assert counted == 2 + 2 * packs and seen in (0, counted)      # (0: no kernel activities on this machine)
+        counted, seen = kernels(step.run_e2e)
+        assert counted == 6 + packs and seen in (0, counted)
+        with monkeypatch.context() as mp:
+            mp.setattr(cuda_ops, "column_chunks", lambda *a, _f=cuda_ops.column_chunks: _f(*a, force=3))
+            op = DistSDDMM(plan, None, 33, torch.float32, "cuda")
+        counted, seen = kernels(op.run_async)
+        assert counted == 2 + packs and seen in (0, counted)
