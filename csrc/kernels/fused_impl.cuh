@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
             gate.side[1] = {nullptr, nullptr, 0};
             gate.order = a.pull_order;
             gate.limit = wave_limit;
-        gate.known = &block_waves;
+            gate.known = &block_waves;
             gate.ld_v = ldx_v;
             gate.nvec = a.nvec; gate.pc = a.pull; gate.n_pull = n_pull; gate.tiles1 = 0;
             gate.tpw = a.n_waves > 0 ? a.tiles_per_wave : (n_pull > 0 ? n_pull : 1);
@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
             gate.bulk = bulk;
             gate.pulls_left = n_pull > 0 && (!bulk || is_puller);
             gate.waves_ready = 0;
-        gate.pending = -1;
+            gate.pending = -1;
             gate.br = br;
             if (is_puller && ok) gate.pull_all(lane);
             const int SPMM_ITEMS_PER_TICKET = per_ticket(a.nitems, nwarps, SPMM_ITEMS_PER_TICKET_MAX);

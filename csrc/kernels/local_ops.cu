@@ -482,20 +482,21 @@ SP3_API int sp3_cuda_sddmm_f64(long long nnz, const int* ri, const int* ci, cons
 }
 
 // items may be null (then the unscheduled one-warp-per-row kernel runs).
-// Long-row arguments may be null/0 when the schedule has no long rows.
+// Long-row arguments may be null/0 when the schedule has no long rows; piece_len is not needed.  ticket: null or two
+// ints {next item, blocks done}, zero at the first launch and left at zero by every launch.
 SP3_API int sp3_cuda_spmm_f32(int nrows, int nitems, const void* items, const long long* rowptr, const int* ci,
                               const float* val, const float* X, long long ldx, int k, float beta, float* Y,
                               long long ldy, const int* first_piece, const int* npieces, int* counters,
-                              void* carry, long long ldc, int piece_len, int* ticket, void* stream) {
-    SpmmLong lg{first_piece, npieces, counters, carry, ldc, piece_len, ticket};
+                              void* carry, long long ldc, int, int* ticket, void* stream) {
+    SpmmLong lg{first_piece, npieces, counters, carry, ldc, ticket};
     return launch_spmm<float>(nrows, nitems, (const int4*)items, rowptr, ci, val, X, ldx, k, beta, Y, ldy, lg,
                               (cudaStream_t)stream);
 }
 SP3_API int sp3_cuda_spmm_f64(int nrows, int nitems, const void* items, const long long* rowptr, const int* ci,
                               const double* val, const double* X, long long ldx, int k, double beta, double* Y,
                               long long ldy, const int* first_piece, const int* npieces, int* counters,
-                              void* carry, long long ldc, int piece_len, int* ticket, void* stream) {
-    SpmmLong lg{first_piece, npieces, counters, carry, ldc, piece_len, ticket};
+                              void* carry, long long ldc, int, int* ticket, void* stream) {
+    SpmmLong lg{first_piece, npieces, counters, carry, ldc, ticket};
     return launch_spmm<double>(nrows, nitems, (const int4*)items, rowptr, ci, val, X, ldx, k, beta, Y, ldy, lg,
                                (cudaStream_t)stream);
 }
@@ -531,7 +532,7 @@ struct SpmmCall {
     long long ldc;
     int* ticket;
     double beta;
-    int k, f64, piece_len;
+    int k, f64;
     int k_out;              // columns of Y (k of X counts the padding of its rows)
     int x_rows;             // rows of X
     PackRows pack_x;        // X is filled from here first
@@ -560,7 +561,7 @@ SP3_API int sp3_cuda_sddmm_call(const void* record, void* stream) {
 SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     const SpmmCall& c = *static_cast<const SpmmCall*>(record);
     cudaStream_t st = (cudaStream_t)stream;
-    const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.piece_len, c.ticket};
+    const SpmmLong lg{c.first_piece, c.npieces, c.counters, c.carry, c.ldc, c.ticket};
     const int rc = c.f64 ? launch_pack<double>(c.pack_x, PackRows{}, st) : launch_pack<float>(c.pack_x, PackRows{}, st);
     if (rc != 0) return rc;
     if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
@@ -746,7 +747,7 @@ SP3_API int sp3_cuda_spmm_f32_noalloc(int nrows, int nitems, const void* items, 
         err = cudaMemsetAsync(base, 0, (size_t)nlong * sizeof(int), st);
         if (err != cudaSuccess) return (int)err;
     }
-    sp3::SpmmLong lg{first_piece, npieces, (int*)base, (void*)(base + counters_bytes), ldc, piece_len, nullptr};
+    sp3::SpmmLong lg{first_piece, npieces, (int*)base, (void*)(base + counters_bytes), ldc, nullptr};
     // (a part leaves the counters at zero for the next)
     for (int j = 0; j < k; j += (int)ldc) {
         const int n = k - j < ldc ? k - j : (int)ldc;

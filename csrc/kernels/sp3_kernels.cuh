@@ -390,7 +390,6 @@ struct SpmmLong {
     int* counters;           // [nlong] zero at launch; reset by the finishing warp
     void* carry;             // [total pieces, ldc] scratch
     long long ldc;           // elements per carry row
-    int piece_len;           // largest number of nonzeros of a piece
     int* ticket;             // optional work counters {next item, blocks done}, zero between launches: items are
                              // then handed out dynamically
 };

@@ -311,7 +311,7 @@ class _SpmmCall(C.Structure):
                 ("ci", C.c_void_p), ("val", C.c_void_p), ("X", C.c_void_p), ("ldx", C.c_longlong), ("Y", C.c_void_p),
                 ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
                 ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
-                ("k", C.c_int), ("f64", C.c_int), ("piece_len", C.c_int), ("k_out", C.c_int),
+                ("k", C.c_int), ("f64", C.c_int), ("k_out", C.c_int),
                 ("x_rows", C.c_int), ("pack_x", _PackRows)]
 
 
@@ -454,8 +454,8 @@ def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule, pack=None):
     carry, ldc = sched.carry_for(x.shape[1], X.dtype, X.device)
     rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(x),
                     _ld(x), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
-                    p(sched.ticket), 0.0, x.shape[1], int(X.dtype == torch.float64), sched.piece_len, Y.shape[1],
-                    X.shape[0], px)
+                    p(sched.ticket), 0.0, x.shape[1], int(X.dtype == torch.float64), Y.shape[1], X.shape[0],
+                    px)
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry, x), launches=1 + (x is not X))
 
 

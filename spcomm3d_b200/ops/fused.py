@@ -59,7 +59,7 @@ class _SddmmArgs(C.Structure):
 
 class _SpmmLong(C.Structure):
     _fields_ = [("first_piece", P), ("npieces", P), ("counters", P), ("carry", P), ("ldc", C.c_longlong),
-                ("piece_len", C.c_int), ("ticket", P)]
+                ("ticket", P)]
 
 
 class _SpmmArgs(C.Structure):
@@ -592,7 +592,6 @@ class FusedSpMM(_FusedBase):
         a.lg.counters = self.sched.counters.data_ptr()
         a.lg.carry = carry.data_ptr() if carry is not None else None
         a.lg.ldc = ldc if carry is not None else kp
-        a.lg.piece_len = self.sched.piece_len
         a.n_owned_y = rp.n_owned
         a.n_crows, a.crows = int(crows.size), self.crows.data_ptr()
         a.y_dst = self.y_dst.data_ptr()
