@@ -66,6 +66,7 @@ def _library_path_on_fiber_only_mesh(variant: str, plan, kw: dict) -> bool:
 
 class _Dist3DOp:
     kernel = "?"
+    _bound = None
 
     def __init__(self, plan: RankPlan, groups: MeshGroups | None, k: int, dtype=torch.float32,
                  device="cpu", variant: str = "sparseNRB", emulated: bool = False, check_plan: bool = True):
@@ -135,6 +136,10 @@ class _Dist3DOp:
         """One rank, one GPU, the default kernels: a run is a single launch, which can be bound to its tensors."""
         return (self.variant in ("sparse", "sparseNRB") and self.mesh.size == 1 and self.device.type == "cuda"
                 and self._panels is None and self.plan.nnz > 0 and not local.opt_in_kernels(self.kernel))
+
+    def __getstate__(self):
+        """Copies and pickles carry no bound call (raw addresses of this operator's tensors): they bind their own."""
+        return {**self.__dict__, "_bound": None}
 
     def _finish(self):
         if not self.timer.enabled:
@@ -230,7 +235,6 @@ class DistSDDMM(_Dist3DOp):
             self._panels = PanelSDDMM(p.rowidx, p.colidx, p.vals, p.row.n_local, p.col.n_local, self.device,
                                       **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
         self.owned_off, self.owned_len = p.owned_nnz_slice()
-        self._bound = None
         self._single = self._single_rank()
         self._chunks = None
         if self._single:   # the nonzeros once more, chunk by chunk of columns, where B outgrows the L2 and that pays
@@ -402,7 +406,6 @@ class DistSpMM(_Dist3DOp):
             self._panels = PanelSpMM(p.rowidx, p.colidx, p.vals, p.row.n_local, p.col.n_local, self.device,
                                      **{k_: v for k_, v in kw.items() if k_ in ("min_col_nnz", "min_panel_nnz")})
 
-        self._bound = None
         self._single = self._single_rank()
         if self._single:
             self._bind()

@@ -31,6 +31,10 @@ class SddmmSpmmStep:
         self.sddmm = DistSDDMM(plan, groups, k, dtype, device, variant, **kw)
         self.spmm = DistSpMM(plan, groups, k, dtype, device, variant, **kw)
         self.host = None
+        self._native_step = None
+
+    def __getstate__(self):
+        return {**self.__dict__, "_native_step": None}   # bound to this step's tensors, like the operators' calls
 
     def fill_device_operands(self):
         """A, B (and X = B) generated on the device from the seed."""

@@ -445,3 +445,73 @@ def test_launches_are_counted(monkeypatch):
             op = DistSDDMM(plan, None, 33, torch.float32, "cuda")
         counted, seen = kernels(op.run_async)
         assert counted == 2 + packs and seen in (0, counted)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ran", [False, True])
+@pytest.mark.parametrize("k", [32, 33])
+def test_copies_and_pickles_of_operators(k, ran):
+    """A copy works on tensors of its own, whether or not the original has run before.  (A pickle does not keep which
+    tensors are views of which, so of its operands the whole blocks are set.)"""
+    import copy
+    import pickle
+    from spcomm3d_b200.models.layer import GatLayer, SddmmSpmmStep
+    plan = _plan("rmat:10:8")
+    vals = torch.from_numpy(plan.vals).float()
+    step, layer = (cls(plan, None, k, torch.float32, "cuda") for cls in (SddmmSpmmStep, GatLayer))
+    layer.sddmm.timer.enabled = layer.spmm.timer.enabled = False
+    step.make_host_operands()
+    if ran:
+        step.run_device(), step.run_e2e(), layer.run()
+    A, B, X = (_randn(t, i) for i, t in enumerate((layer.sddmm.A_owned, layer.sddmm.B_owned, layer.spmm.X_owned)))
+    deg = _lists(plan)[2].numpy()
+    for make in (copy.deepcopy, lambda o: pickle.loads(pickle.dumps(o))):
+        s, g = make(step), make(layer)
+        for op in (s.sddmm, s.spmm, g.sddmm, g.spmm):
+            for name, t in (("A_loc", A), ("B_loc", B), ("X_loc", X)):
+                if hasattr(op, name):
+                    getattr(op, name).copy_(t)
+        mine = step.sddmm.partial, step.spmm.Y_owned, layer.spmm.vals, layer.spmm.Y_owned
+        before = [t.clone() for t in mine]
+        s.run_device(), g.run()
+        c, y = s.sddmm.partial, s.spmm.Y_loc
+        ref, mag = _scores(plan, A, B, vals)
+        assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, torch.float32) * mag).all())
+        bound = torch.from_numpy(_gamma(deg + 3.0, torch.float32))[:, None] * _product(plan, vals, X.abs())
+        assert bool(((y.cpu().double() - _product(plan, vals, X)).abs() <= bound).all())
+        _check_layer(g, plan, k, torch.float32, A, B, X, vals, g.spmm.vals, g.spmm.Y_loc)
+        s.run_e2e()
+        assert all(torch.equal(a, b) for a, b in zip(before, mine))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("packs", [False, True])
+def test_operators_under_capture(packs, monkeypatch):
+    """Runs recorded in a CUDA graph: replays on new operands are runs on new operands."""
+    from spcomm3d_b200.models.layer import GatLayer, SddmmSpmmStep
+    from spcomm3d_b200.ops import cuda_ops
+    if packs:
+        monkeypatch.setattr(cuda_ops, "pack_rule", lambda *a: True, raising=False)
+    plan, k = _plan("zipf:900:1200:1.6:300"), 33
+    chunks = cuda_ops.column_chunks
+    monkeypatch.setattr(cuda_ops, "column_chunks", lambda *a: chunks(*a, force=3))
+    step, layer = (cls(plan, None, k, torch.float32, "cuda") for cls in (SddmmSpmmStep, GatLayer))
+    layer.sddmm.timer.enabled = layer.spmm.timer.enabled = False
+
+    def run():
+        return [*step.run_device(), step.spmm.run_async(0.5), layer.run(), layer.spmm.vals]
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    run()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        out = run()
+    for i in range(3):
+        for op in (step.sddmm, step.spmm, layer.sddmm, layer.spmm):
+            for name in ("A_owned", "B_owned", "X_owned"):
+                if hasattr(op, name):
+                    getattr(op, name).copy_(_randn(getattr(op, name), 10 * i))
+        want = [t.clone() for t in run()]
+        for t in out:
+            t.zero_()
+        graph.replay(), graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(want, out))
