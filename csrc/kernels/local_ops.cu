@@ -36,10 +36,10 @@ sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const in
 // row order.  A row's values of one chunk lie together, so the reads use whole sectors; writing them from the SDDMM
 // itself left partial sectors in device memory and cost more than this pass (Erdos-Renyi 1 M rows, 33.5 M nonzeros,
 // k = 64: about 250 us).
-template <typename T>
+template <typename T, bool TWICE>
 __global__ void __launch_bounds__(256)
 scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* sval, const T* dots, T* out,
-                    bool aligned) {
+                    T* also, bool aligned) {
     after_previous_kernel();
     const int n = (int)nnz, i = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= n) return;
@@ -51,12 +51,18 @@ scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* sval,
     if (aligned && i + 4 <= n) {
         using V = typename Vec<T>::type;
 #pragma unroll
-        for (int j = 0; j < 4; j += Vec<T>::N) *reinterpret_cast<V*>(out + i + j) = *reinterpret_cast<const V*>(v + j);
+        for (int j = 0; j < 4; j += Vec<T>::N) {
+            *reinterpret_cast<V*>(out + i + j) = *reinterpret_cast<const V*>(v + j);
+            if (TWICE) *reinterpret_cast<V*>(also + i + j) = *reinterpret_cast<const V*>(v + j);
+        }
         return;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        if (i + j < n) out[i + j] = v[j];
+        if (i + j < n) {
+            out[i + j] = v[j];
+            if (TWICE) also[i + j] = v[j];
+        }
 }
 
 // Rows of k values, `ld` apart wherever they start, to rows of `nvec` whole 16-byte vectors, the rest zero: what the
@@ -354,7 +360,8 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
 
 template <typename T>
 int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const T* A, long long lda, const T* B,
-                 long long ldb, int k, T* out, cudaStream_t st, const int* orig = nullptr, bool passing = false) {
+                 long long ldb, int k, T* out, cudaStream_t st, const int* orig = nullptr, bool passing = false,
+                 T* also = nullptr) {
     if (nnz == 0) return 0;
     const long long lda_b = lda * (long long)sizeof(T), ldb_b = ldb * (long long)sizeof(T);
     const unsigned long long bytes = (unsigned long long)k * sizeof(T);
@@ -366,10 +373,19 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
         if (orig) return -1;  // the scatter form exists for the vector kernel only
         long long warps = nnz < (1ll << 22) ? nnz : (1ll << 22);
         sddmm_scalar_kernel<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(nnz, ri, ci, sv, A, lda, B, ldb, k, out);
-        return (int)cudaGetLastError();
+        const int rc = (int)cudaGetLastError();
+        return rc || !also ? rc : (int)cudaMemcpyAsync(also, out, nnz * sizeof(T), cudaMemcpyDeviceToDevice, st);
     }
     const StoreLocal<T> store{out, sv};
     const char *a = reinterpret_cast<const char*>(A), *b = reinterpret_cast<const char*>(B);
+    if (also) {
+        StoreTwice<T> twice;
+        twice.out = out; twice.sval = sv; twice.also = also;
+        if (nb == 16) return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
+        if (nb == 8) return launch_sddmm_nb<T, 8>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
+        if constexpr (sizeof(T) == 4) return launch_sddmm_nb<T, 4>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
+        return -1;
+    }
     if (orig) {
         if (nb != 16) return -1;
         return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, StoreScattered<T>{out, sv, orig}, st);
@@ -516,6 +532,7 @@ struct SddmmCall {
     const int* where;
     void* dots;
     PackRows pack_a, pack_b;   // A and B are filled from here first
+    void* also;                // null, or a second place for the values (scores that are values of the next kernel)
 };
 struct SpmmCall {
     int nrows, nitems;
@@ -548,11 +565,13 @@ template <typename T> static int sddmm_call(const SddmmCall& c, cudaStream_t st)
     int rc = launch_pack<T>(c.pack_a, c.pack_b, st);
     if (rc != 0) return rc;
     rc = launch_sddmm<T>(c.nnz, c.ri, c.ci, c.where ? nullptr : (const T*)c.sv, (const T*)c.A, c.lda,
-                                   (const T*)c.B, c.ldb, c.k, out, st, nullptr, c.where != nullptr);
+                                   (const T*)c.B, c.ldb, c.k, out, st, nullptr, c.where != nullptr,
+                         c.where ? nullptr : (T*)c.also);
     if (rc != 0 || !c.where || c.nnz == 0) return rc;
-    const bool aligned = ((uintptr_t)c.where | (uintptr_t)c.sv | (uintptr_t)c.out) % 16 == 0;
-    return launch_early(scale_picked_kernel<T>, (unsigned)((c.nnz + 1023) / 1024), 0, st, c.nnz, c.where,
-                        (const T*)c.sv, (const T*)c.dots, (T*)c.out, aligned);
+    const bool aligned = ((uintptr_t)c.where | (uintptr_t)c.sv | (uintptr_t)c.out | (uintptr_t)c.also) % 16 == 0;
+    return launch_early(c.also ? scale_picked_kernel<T, true> : scale_picked_kernel<T, false>,
+                        (unsigned)((c.nnz + 1023) / 1024), 0, st, c.nnz, c.where, (const T*)c.sv, (const T*)c.dots,
+                        (T*)c.out, (T*)c.also, aligned);
 }
 SP3_API int sp3_cuda_sddmm_call(const void* record, void* stream) {
     const SddmmCall& c = *static_cast<const SddmmCall*>(record);

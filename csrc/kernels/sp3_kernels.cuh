@@ -205,6 +205,10 @@ template <typename T> struct StoreLocal {
     __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
     __device__ __forceinline__ void put(long long i, T v) const { out[i] = v; }
 };
+template <typename T> struct StoreTwice : StoreLocal<T> {
+    T* also;          // a second place for the values (a form of its own: the choice in the kernel cost 1 %)
+    __device__ __forceinline__ void put(long long i, T v) const { this->out[i] = v; also[i] = v; }
+};
 template <typename T> struct StoreScattered {
     T* out;
     const T* sval;

@@ -249,13 +249,17 @@ class DistSDDMM(_Dist3DOp):
     _A_full = property(lambda self: self.A_loc)
     _B_full = property(lambda self: self.B_loc)
 
-    def _bind(self):
-        t = (self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial)
-        b = self._bound
+    def _bind(self, bound=None, also=()):
+        """The call that writes the values to `partial`; with `also`, the tensor of a chain, to that too (`bound`: the
+        caller's call of that kind, bound again when a tensor was replaced)."""
+        t = (self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial, *also)
+        b = bound if also else self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
             chunks = self._chunks if all(x is y for x, y in zip(t, self._chunks_of)) else None
-            b = self._bound = cuda_ops.bind_sddmm(*t, chunks)
+            b = cuda_ops.bind_sddmm(*t, chunks=chunks)
+            if not also:
+                self._bound = b
             self._slice = self.partial[self.owned_off:self.owned_off + self.owned_len]
         return b
 

@@ -228,22 +228,37 @@ class GatLayer:
         dev = torch.device(device)
         self._mine = torch.zeros(self.width, dtype=dtype, device=dev)
         self._all = torch.zeros(Z, self.width, dtype=dtype, device=dev)
-        if Z == 1 and self.sddmm.variant in ("sparse", "sparseNRB"):
-            # one layer holds all of k: the SDDMM writes its scores where the SpMM reads its values
-            self.sddmm.partial = self.spmm.vals
-            if self.sddmm._single:
-                self.sddmm._bind()
+        self._scores = None
+        if self._direct():
+            self._bind_scores()
+            self.sddmm._bound = None   # (its own call is bound when it runs alone: the scratch is not needed twice)
         # the SpMM wants its values in CSR order; a fused SDDMM stores them in its own order
         order = self.sddmm.value_order
         self._pos = None if order is None else torch.from_numpy(np.ascontiguousarray(order)).to(dev)
 
+    def __getstate__(self):
+        return {**self.__dict__, "_scores": None}   # bound to this layer's tensors, like the operators' calls
+
+    def _direct(self):
+        """Whether the kernel of the SDDMM itself can put the scores where the SpMM reads its values, next to the result
+        of the SDDMM (which stays what it is when the SpMM's values change)."""
+        c, v = self.sddmm.partial, self.spmm.vals
+        return (self.sddmm._single and v is not c and v.dtype == c.dtype and v.shape == c.shape and v.is_contiguous()
+                and v.device == c.device)
+
+    def _bind_scores(self):
+        self._scores = self.sddmm._bind(self._scores, (self.spmm.vals,))
+        return self._scores
+
     def run(self):
+        if not self.sddmm.timer.enabled and self._direct():
+            self._bind_scores().launch()
+            return self.spmm.run()
         c = self.sddmm.run()
         Z = self.plan.mesh.Z
         if Z == 1:
             if self._pos is None:
-                if c.data_ptr() != self.spmm.vals.data_ptr():
-                    self.spmm.vals.copy_(c)
+                self.spmm.vals.copy_(c)
             else:
                 self.spmm.vals.index_copy_(0, self._pos, c)
         else:

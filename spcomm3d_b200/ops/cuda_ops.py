@@ -303,7 +303,7 @@ class _SddmmCall(C.Structure):
     _fields_ = [("nnz", C.c_longlong), ("ri", C.c_void_p), ("ci", C.c_void_p), ("sv", C.c_void_p), ("A", C.c_void_p),
                 ("lda", C.c_longlong), ("B", C.c_void_p), ("ldb", C.c_longlong), ("out", C.c_void_p), ("k", C.c_int),
                 ("f64", C.c_int), ("where", C.c_void_p), ("dots", C.c_void_p), ("pack_a", _PackRows),
-                ("pack_b", _PackRows)]
+                ("pack_b", _PackRows), ("also", C.c_void_p)]
 
 
 class _SpmmCall(C.Structure):
@@ -392,9 +392,9 @@ def _packed(t):
     return full, _PackRows(native.ptr(t), _ld(t), native.ptr(full), n, k, nvec)
 
 
-def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None, pack=None):
+def bind_sddmm(rowidx, colidx, svals, A, B, out, also=None, chunks=None, pack=None):
     """`sddmm` bound to its tensors (all given); `chunks`: the lists of `column_chunks`, taken instead of the row-sorted
-    ones; `pack`: whether the kernel reads packed copies of A and B, by `pack_rule` when not said."""
+    ones; `also`: a second place for the values; `pack`: whether the kernel reads packed copies of A and B, by `pack_rule` when not said."""
     p = native.ptr
     r, c, where = chunks or (rowidx, colidx, None)
     dots = torch.empty_like(out) if chunks else None
@@ -402,8 +402,9 @@ def bind_sddmm(rowidx, colidx, svals, A, B, out, chunks=None, pack=None):
     if pack_rule("sddmm", rowidx.shape[0], A.shape[0] + B.shape[0], A.shape[1], A.element_size(), A.device) if pack is None else pack:
         (a, pa), (b, pb) = _packed(A), _packed(B)
     rec = _SddmmCall(rowidx.shape[0], p(r), p(c), p(svals), p(a), _ld(a), p(b), _ld(b), p(out), a.shape[1],
-                     int(A.dtype == torch.float64), p(where), p(dots), pa, pb)
-    return _BoundCall("sddmm", rec, (rowidx, colidx, svals, A, B, out), keep=(chunks, dots, a, b),
+                     int(A.dtype == torch.float64), p(where), p(dots), pa, pb, p(also))
+    tensors = (rowidx, colidx, svals, A, B, out) + (() if also is None else (also,))
+    return _BoundCall("sddmm", rec, tensors, keep=(chunks, dots, a, b),
                       launches=1 + (a is not A) + (chunks is not None))
 
 

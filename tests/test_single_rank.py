@@ -515,3 +515,35 @@ def test_operators_under_capture(packs, monkeypatch):
             t.zero_()
         graph.replay(), graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(want, out))
+
+
+@pytest.mark.parametrize("k", [1, 18, 20, 33, 1025])    # every vector width, the scalar kernel
+@pytest.mark.parametrize("chunked", [False, True])
+@pytest.mark.parametrize("timers", [False, True])
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_scores_and_values_of_a_layer_are_two_things(device, timers, chunked, k, monkeypatch):
+    """The operators of a layer can be run alone: the SDDMM leaves the values of the SpMM as they are, scores that were
+    computed stay when those values change, and a run of the layer sets both."""
+    from spcomm3d_b200.models.layer import GatLayer
+    from spcomm3d_b200.ops import cuda_ops
+    if chunked:
+        chunks = cuda_ops.column_chunks
+        monkeypatch.setattr(cuda_ops, "column_chunks", lambda *a: chunks(*a, force=3))
+    plan = _plan("zipf:301:400:1.6:200")
+    vals = torch.from_numpy(plan.vals).float()
+    layer = GatLayer(plan, None, k, torch.float32, device)
+    layer.sddmm.timer.enabled = layer.spmm.timer.enabled = timers
+    A, B, X = (_randn(t, i) for i, t in enumerate((layer.sddmm.A_owned, layer.sddmm.B_owned, layer.spmm.X_owned)))
+    layer.sddmm.A_owned.copy_(A), layer.sddmm.B_owned.copy_(B), layer.spmm.X_owned.copy_(X)
+    for _ in range(2):
+        c = layer.sddmm.run()
+        scores = c.clone()
+        assert torch.equal(layer.spmm.vals.cpu(), vals)
+        layer.spmm.vals.copy_(torch.exp(c))
+        assert torch.equal(c, scores)
+        layer.sddmm.partial.fill_(float("nan"))
+        _check_layer(layer, plan, k, torch.float32, A, B, X, vals, layer.spmm.vals, layer.run())
+        assert torch.equal(layer.spmm.vals, layer.sddmm.partial) and torch.equal(layer.spmm.vals, scores)
+        layer.spmm.vals.copy_(vals)
+    layer.spmm.vals = torch.zeros_like(layer.spmm.vals)      # values of the user's own
+    _check_layer(layer, plan, k, torch.float32, A, B, X, vals, layer.spmm.vals, layer.run())
