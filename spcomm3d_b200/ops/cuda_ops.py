@@ -379,8 +379,12 @@ def pack_rule(kernel, nnz, rows, k, es, device):
     row_bytes = k * es
     if row_bytes % 16 == 0 or row_bytes > 256 * 16 or row_bytes < (128 if kernel == "spmm" else 16):
         return False
-    saved = row_bytes // (8 if row_bytes % 8 == 0 else 4) - -(-row_bytes // 16)
-    return nnz * saved >= max(PACK_MIN_WORK, 7 * row_bytes * rows // 10) and has_room(rows * (row_bytes + 16), device)
+    narrow = row_bytes // (8 if row_bytes % 8 == 0 else 4)
+    saved = narrow - -(-row_bytes // 16)
+    pays = nnz * saved >= max(PACK_MIN_WORK, 7 * row_bytes * rows // 10)
+    # past 256 narrow vectors the SpMM is left with a kernel that cuts no rows (R-MAT scale 12, k = 259: 378 us, packed
+    # 16; 4000 nonzeros of even rows: 6.5 and 10)
+    return (pays or kernel == "spmm" and narrow > 256) and has_room(rows * (row_bytes + 16), device)
 
 
 def _packed(t):

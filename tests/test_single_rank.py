@@ -242,6 +242,8 @@ def test_pack_rule(monkeypatch):
     assert not cuda_ops.pack_rule("spmm", n // 16, rows, 33, 4, None)      # a nonzero per row
     assert not cuda_ops.pack_rule("spmm", 100_000, 1000, 33, 4, None)      # small
     assert not cuda_ops.pack_rule("sddmm", n, rows, 1025, 4, None)         # wider than the vector kernels
+    # more narrow vectors than the SpMM on work items takes: packed, or row by row one value at a time
+    assert cuda_ops.pack_rule("spmm", 1000, 1000, 301, 4, None) and not cuda_ops.pack_rule("spmm", 1000, 1000, 302, 4, None)
     monkeypatch.setattr(cuda_ops, "has_room", lambda nbytes, device: False)
     assert not cuda_ops.pack_rule("spmm", n, rows, 33, 4, None)
 
