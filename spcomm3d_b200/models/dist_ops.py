@@ -257,6 +257,8 @@ class DistSDDMM(_Dist3DOp):
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
             chunks = self._chunks if all(x is y for x, y in zip(t, self._chunks_of)) else None
+            if b is not None:
+                b.retire()
             b = cuda_ops.bind_sddmm(*t, chunks=chunks)
             if not also:
                 self._bound = b
@@ -419,6 +421,8 @@ class DistSpMM(_Dist3DOp):
         b = self._bound
         if b is None or not b.bound_to(*t):
             from ..ops import cuda_ops
+            if b is not None:
+                b.retire()
             b = self._bound = cuda_ops.bind_spmm(*t, self.sched)
         return b
 

@@ -343,6 +343,14 @@ class _BoundCall:
                 return False
         return True
 
+    def retire(self):
+        """Before this call makes way for another: its scratch may still be in use by a run on
+        the current stream, which need not be the one it was allocated on."""
+        if not torch.cuda.is_current_stream_capturing():
+            for t in self._keep:
+                if isinstance(t, torch.Tensor):
+                    t.record_stream(torch.cuda.current_stream(t.device))
+
     def launch(self, *beta):
         """One run; the SpMM is given its beta, a number."""
         global LAUNCHES

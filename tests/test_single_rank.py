@@ -549,3 +549,34 @@ def test_scores_and_values_of_a_layer_are_two_things(device, timers, chunked, k,
         layer.spmm.vals.copy_(vals)
     layer.spmm.vals = torch.zeros_like(layer.spmm.vals)      # values of the user's own
     _check_layer(layer, plan, k, torch.float32, A, B, X, vals, layer.spmm.vals, layer.run())
+
+
+@pytest.mark.gpu
+def test_scratch_of_a_call_that_makes_way(monkeypatch):
+    """Packed operands of a run on another stream are not handed out again before that run is done: an operand is
+    replaced behind a run that has not begun yet, and memory of the size of its scratch is asked for and written."""
+    from spcomm3d_b200.models.dist_ops import DistSpMM
+    from spcomm3d_b200.ops import cuda_ops
+    monkeypatch.setattr(cuda_ops, "pack_rule", lambda *a: True)
+    plan, k = _plan("er:20000:20000:9"), 33
+    op = DistSpMM(plan, None, k, torch.float32, "cuda")
+    X = _randn(op.X_loc, 1)
+    op.X_loc.copy_(X)
+    want = op.run_async().clone()
+    side, other = torch.cuda.Stream(), _randn(op.X_loc, 2).cuda()
+    scratch = op._bound._keep[-1]
+    shape, at = scratch.shape, scratch.data_ptr()
+    del scratch
+    torch.cuda.synchronize()
+    op.Y_owned.zero_()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)      # cycles: about a tenth of a second
+        op.run_async()
+        y = op.Y_owned.clone()
+        op.X_loc = other
+        op.run_async()
+    taken = [torch.full(shape, float("nan"), device="cuda") for _ in range(3)]
+    assert all(t.data_ptr() != at for t in taken)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
