@@ -267,7 +267,10 @@ class DistSDDMM(_Dist3DOp):
 
     def _run_bound(self) -> torch.Tensor:
         """The run of a single rank without phase timers: one launch."""
-        self._bind().launch()
+        b = self._bound
+        if b is None or not b.bound_to(self.rowidx, self.colidx, self.vals, self.A_loc, self.B_loc, self.partial):
+            b = self._bind()
+        b.launch()
         return self._slice
 
     def _local_buffers(self):

@@ -355,7 +355,7 @@ class _BoundCall:
         """One run; the SpMM is given its beta, a number."""
         global LAUNCHES
         if beta:
-            (self._record.beta,) = beta
+            self._record.beta = beta[0]
         LAUNCHES += self._launches
         rc = self._fn(self._addr, _raw_stream())
         if rc != 0:
@@ -433,11 +433,12 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
 
     Counted in dense rows that come from device memory: now every nonzero outside the most frequent columns that the
     L2 holds, with chunks one row of A per change of (row, chunk), every used column once, and four values per nonzero
-    for the pass that restores the row order.  The line lies at 1.25 times fewer.  Erdos-Renyi 1 M rows, 32 a row (3
-    times fewer): k = 64 1098 -> 900 us, k = 128 2473 -> 1782; uniform 500 thousand rows, 12 a row, k = 128 (1.4): 413
-    -> 342; 1 M x 2 M, 12 a row, k = 64 (1.05): 489 -> 576; R-MAT scale 20, k = 128 (hub columns): 564 -> 673.  Chunks
-    of 64 MB are level with 96 at 32 a row, 128 and 48 MB slower.  Fewer reads per row of B than four leave little to
-    save."""
+    for the pass that restores the row order.  The line lies at 1.25 times fewer.  Measured back to back on
+    the same operands (new operands in every run cost about 10 % more): Erdos-Renyi 1 M rows, 32 a row (3 times fewer)
+    k = 64 1118 -> 882 us, k = 128 2481 -> 1912; uniform 500 thousand rows, k = 128, 20 a row 638 -> 503, 12 a row (1.4)
+    413 -> 342; 1 M x 2 M, 12 a row, k = 64 (1.05): 489 -> 576; R-MAT scale 20, k = 128 (hub columns): 564 -> 673.
+    Chunks of 48 / 64 / 96 / 128 MB: 868 / 821 / 882 / 1048, 2031 / 1804 / 1912 / 2112 and 627 / 508 / 503 / 560 in the
+    first three of these.  Fewer reads per row of B than four leave little to save."""
     nnz = rowidx.shape[0]
     n = force or -(-n_cols * row_bytes // CHUNK_BYTES)
     if nnz > CHUNK_MAX_NNZ or not force and (n < 2 or n > 32 or nnz < CHUNK_MIN_NNZ or nnz < 4 * n_cols
