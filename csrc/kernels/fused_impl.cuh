@@ -634,8 +634,116 @@ __device__ __forceinline__ long long slice_off(int z, unsigned zbase, unsigned z
     return (long long)z * zbase + ((unsigned)z < zrem ? z : (int)zrem);
 }
 
+// The loop of sddmm_windows as it fits next to the state of three phases: indices in registers, handed round by shuffle,
+// a quad's rows requested when it is its turn, every value stored by itself.  The pipelined loop spilled 740 bytes of
+// registers a thread in here (eight ranks, 512 thousand nonzeros, k / Z = 64: MAIN 48 us, this one 37).
+template <typename T, int NB, int G, int R, int U, bool EXACT, typename ARows, typename Store>
+__device__ __forceinline__ void sddmm_units(long long first, long long step, long long end, int wn, long long nnz,
+                                              const int* __restrict__ rowidx, const int* __restrict__ colidx,
+                                              const ARows& arows, const char* B, unsigned ldb_bytes,
+                                              int nvec, bool aligned, const Store& store, int lane) {
+    static_assert(G >= 4, "a group reduces four values");
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int SLOTS = 32 / G;
+    const int slot = lane / G, gl = lane % G;
+    unsigned off[R];
+    bool on[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and do not count
+        const int v = gl + q * G;
+        on[q] = EXACT || v < nvec;
+        off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
+    }
+    auto length = [&](long long w) { return (int)(nnz - w * wn < wn ? nnz - w * wn : (long long)wn); };
+    auto load = [&](long long w, Quad<int>& c, Quad<int>& r) {
+        const int n = length(w), i = 4 * lane < n ? 4 * lane : (n - 1) & ~3;
+        c = quad_load(colidx + w * wn, i, n, aligned);
+        r = quad_load(rowidx + w * wn, i, n, aligned);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r.v[j] = arows.ref(r.v[j]);
+    };
+    auto fetch = [&](Row<T, NB> (&a)[R], const char* p) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) row_load(a[q], p + (off[q] - off[0]));
+    };
+    if (first >= end) return;
+    B += off[0];
+    const int mine = gl / (G / 4);              // which of the four results ends up in this lane
+    const bool writer = gl % (G / 4) == 0;
+    Quad<int> c4, r4;
+    load(first, c4, r4);
+    int cur = -1;
+    Row<T, NB> a[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) row_zero(a[q]);
+    for (long long w = first; w < end; w += step) {
+        Quad<int> cn = c4, rn = r4;
+        if (w + step < end) load(w + step, cn, rn);
+        const int n = length(w);
+        const long long w0 = w * wn;
+        const int nq = (((n + 3) >> 2) + SLOTS - 1) / SLOTS;   // quads per group
+        // lanes whose quad is not all one row (a list sorted by row class by class may leave and re-enter a row)
+        const unsigned mixed = __ballot_sync(FULL, r4.v[0] != r4.v[3] || r4.v[1] != r4.v[3] || r4.v[2] != r4.v[3]);
+        for (int i = 0; i < nq; ++i) {
+            const int src = slot * nq + i;                     // lane that holds this group's quad
+            int c[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u] = __shfl_sync(FULL, c4.v[u], src);
+            const int last = __shfl_sync(FULL, r4.v[3], src);
+            Row<T, NB> b[U][R];
+#pragma unroll
+            for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[u] * ldb_bytes);
+            const int pos = 4 * src + mine;
+            const bool st = writer && pos < n;
+            const T s = store.scale(w0 + (pos < n ? pos : n - 1));
+            T d[4];
+            if (__all_sync(FULL, last == cur && !(mixed >> src & 1))) {
+#pragma unroll
+                for (int h = 0; h < 4; h += U) {
+                    if (h > 0)
+#pragma unroll
+                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
+                }
+            } else {
+                int r[4];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) r[u] = __shfl_sync(FULL, r4.v[u], src);
+                r[3] = last;
+                Row<T, NB> a2[R];
+                const bool staged = last != cur;
+                fetch(a2, arows.resolve(last) + off[0]);   // (unconditional: a load under a condition costs more)
+#pragma unroll
+                for (int h = 0; h < 4; h += U) {
+                    if (h > 0)
+#pragma unroll
+                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (r[h + u] != cur) {
+                            cur = r[h + u];
+                            if (staged && cur == last) {
+#pragma unroll
+                                for (int q = 0; q < R; ++q) a[q] = a2[q];
+                            } else {
+                                fetch(a, arows.resolve(cur) + off[0]);
+                            }
+                        }
+                        d[h + u] = row_dot<EXACT>(a, b[u], on);
+                    }
+                }
+            }
+            const T total = group_sum4<T, G>(d, gl);
+            if (st) store.put(w0 + pos, total * s);
+        }
+        c4 = cn;
+        r4 = rn;
+    }
+}
+
 template <int G, int R>
-__global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(const FusedSddmmArgs a) {
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, true)) fused_sddmm_kernel(const FusedSddmmArgs a) {
     after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
@@ -712,7 +820,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R)) fused_sddmm_kernel(c
             const long long u1 = u0 + UNITS_PER_TICKET < n_units ? u0 + UNITS_PER_TICKET : n_units;
             ok = gate.ensure(u1, lane);
             if (!ok) break;
-            sddmm_windows<real, 16, G, R, sddmm_unroll(R), false>(
+            sddmm_units<real, 16, G, R, sddmm_unroll(R, true), false>(
                 u0, 1, u1, per_unit, a.nnz, a.rowidx, a.colidx, arows, reinterpret_cast<const char*>(Bv),
                 (unsigned)ldb_v * 16u, a.nvec, aligned, store, lane);
             if (self_push) {
@@ -930,7 +1038,7 @@ struct EmitOwnedOrAdd {
 // no wave state: its inner loop keeps all 64 registers of a thread, which is worth 10-15 % on blocks that pull
 // nothing or little (meshes 1 x Y x Z).
 template <int G, int R, bool ATOMIC, bool GATED>
-__global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(const FusedSpmmArgs a) {
+__global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(const FusedSpmmArgs a) {
     after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
@@ -940,8 +1048,8 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
     __shared__ long long wave_limit[MAX_WAVES + 1];
     __shared__ BlockWaves block_waves;
     if (threadIdx.x == 0) block_waves = {0, 0};
-    __shared__ int row_ends[256 / 32][SPMM_ENDS];
-    int* ends = row_ends[threadIdx.x >> 5];
+    __shared__ ItemSmem<real, 16, G, R> scratch[256 / 32];
+    ItemSmem<real, 16, G, R>& sm = scratch[threadIdx.x >> 5];
     const bool bulk = a.pull.pullers > 0;
     BulkRing br = bulk_ring_init(dyn_smem, a.pull, threadIdx.x >> 5, lane);
     __syncthreads();
@@ -1027,11 +1135,11 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
                         spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
-                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
+                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, sm, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
                         spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
-                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
+                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, sm, lane);
                 }
             }
         } else {
@@ -1079,11 +1187,11 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(G, R)) fused_spmm_kernel(
                                              a.crow_flag, a.red_v4};
                     for (int it = i0; it < i1; ++it)
                         spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
-                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, ends, lane);
+                                                                              ldx_bytes, a.nvec, aligned, add, a.lg, sm, lane);
                 } else {
                     for (int it = i0; it < i1; ++it)
                         spmm_warp_item<real, 16, G, R, spmm_unroll(R), false>(__ldg(a.items + it), a.rowptr, nnz, a.colidx, a.val, Xb,
-                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, ends, lane);
+                                                                              ldx_bytes, a.nvec, aligned, emit, a.lg, sm, lane);
                 }
             }
             if (ok) gate.pull_all(lane);  // no item left but tiles remain (tiny blocks)

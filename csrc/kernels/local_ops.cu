@@ -21,15 +21,17 @@ namespace sp3 {
 // warps stride over windows of nonzeros (see sddmm_windows).
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
-__global__ void __launch_bounds__(256, sddmm_min_blocks(R))
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
 sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
                  const Rows arows, const char* B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
-    after_previous_kernel();
+    let_next_kernel_start();
+    __shared__ __align__(16) WindowLists<T> lists[256 / 32];
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    sddmm_windows<T, NB, G, R, sddmm_unroll(R), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
-                                                      arows, B, ldb_bytes, nvec, aligned, store, threadIdx.x & 31);
+    sddmm_windows<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
+                                                      arows, B, ldb_bytes, nvec, aligned, store, lists[threadIdx.x >> 5],
+                                                      threadIdx.x & 31, true);
 }
 
 // out[i] = sval[i] * dots[where[i]], four values per thread: dot products computed chunk by chunk of columns, back into
@@ -131,13 +133,13 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // every row exactly once.
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
-__global__ void __launch_bounds__(256, spmm_min_blocks(G, R))
+__global__ void __launch_bounds__(256, spmm_min_blocks(R))
 spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
                   const int* __restrict__ colidx, const T* val, const char* X,
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
-    after_previous_kernel();
-    __shared__ int row_ends[256 / 32][SPMM_ENDS];
-    int* ends = row_ends[threadIdx.x >> 5];
+    let_next_kernel_start();
+    __shared__ ItemSmem<T, NB, G, R> scratch[256 / 32];
+    ItemSmem<T, NB, G, R>& sm = scratch[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warp0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
@@ -148,7 +150,7 @@ spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const l
         // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
         if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
         spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
-                                                                 aligned, emit, lg, ends, lane);
+                                                                 aligned, emit, lg, sm, lane, it == warp0);
     };
     if (lg.ticket && nitems > nwarps) {
         // dynamic hand-out: items differ too much in cost (cached or not, hub or not) for a fixed assignment to balance
@@ -376,11 +378,13 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
         const int rc = (int)cudaGetLastError();
         return rc || !also ? rc : (int)cudaMemcpyAsync(also, out, nnz * sizeof(T), cudaMemcpyDeviceToDevice, st);
     }
-    const StoreLocal<T> store{out, sv};
+    const bool vectors = ((uintptr_t)out | (uintptr_t)sv | (uintptr_t)also) % 16 == 0;
+    const StoreLocal<T> store{out, sv, vectors};
     const char *a = reinterpret_cast<const char*>(A), *b = reinterpret_cast<const char*>(B);
     if (also) {
         StoreTwice<T> twice;
-        twice.out = out; twice.sval = sv; twice.also = also;
+        static_cast<StoreLocal<T>&>(twice) = store;
+        twice.also = also;
         if (nb == 16) return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
         if (nb == 8) return launch_sddmm_nb<T, 8>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
         if constexpr (sizeof(T) == 4) return launch_sddmm_nb<T, 4>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, twice, st);
@@ -388,7 +392,10 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
     }
     if (orig) {
         if (nb != 16) return -1;
-        return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, StoreScattered<T>{out, sv, orig}, st);
+        StoreScattered<T> scattered;
+        static_cast<StoreLocal<T>&>(scattered) = store;
+        scattered.orig = orig;
+        return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, scattered, st);
     }
     if (nb == 16 && passing) return launch_sddmm_nb<T, 16, RowsPassing>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
     if (nb == 16) return launch_sddmm_nb<T, 16>(nnz, ri, ci, a, lda_b, b, ldb_b, (int)nvec, store, st);
@@ -397,6 +404,7 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
     return -1;
 }
 
+constexpr int SMS = 148;
 template <typename T, int NB, typename Emit>
 int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
                    const char* X, long long ldx_bytes, int nvec, bool cached, const Emit& emit, const SpmmLong& lg,
@@ -405,6 +413,12 @@ int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* ro
     constexpr bool VECTORS = std::is_same<Emit, EmitLocal<T, NB>>::value;
     int G, R;
     pick_shape(nvec, &G, &R, true, cached);
+    // Items that the shape of one vector per lane, with more warps, runs in one round and this one does not: 16384 rows
+    // of 16 nonzeros (4096 items) 8.8 us as 16 x 1 and 11.0 as 8 x 2, 12.4 as 32 x 1 and 13.5 as 8 x 4.
+    if (R > 1 && nvec <= 32 && nitems > SMS * 8 * spmm_min_blocks(R) && nitems <= SMS * 8 * spmm_min_blocks(1)) {
+        G = nvec <= 16 ? 16 : 32;
+        R = 1;
+    }
     const bool exact = VECTORS && NB == 16 && nvec == G * R;
     const long long needed = ((long long)nitems + 7) / 8;
 #define SP3_SPMM(GG, RR)                                                                                      \

@@ -20,6 +20,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 namespace sp3 {
 
@@ -47,7 +48,7 @@ template <> struct Row<double, 8> { using E = double; static constexpr int N = 1
 // Dense rows and values are read by ordinary loads, never through the read-only path (`ld.global.nc`, `__ldg`, or a
 // `const __restrict__` kernel parameter, from which the compiler infers it): that path is defined only for memory that
 // nobody writes while the kernel runs.  A kernel launched early runs while the kernel before it writes what may be its
-// values or rows (see after_previous_kernel), and in the fused kernels other warps of the launch write the pulled rows.
+// values or rows (see wait_for_previous_kernel), and in the fused kernels other warps of the launch write the pulled rows.
 // Ordinary loads are ordered behind the wait, or the acquire, that says the data is there.  Index arrays and work items
 // are fixed when an operator is built and keep the read-only path.
 template <typename T, int NB> __device__ __forceinline__ void row_load(Row<T, NB>& v, const char* p) {
@@ -122,7 +123,7 @@ __device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> 
 
 // Four consecutive values base[i .. i+3] of a list, i a multiple of 4 counted from a 16-byte boundary when `aligned`;
 // positions at or past `end` repeat the last value before it.  Lists of int are index lists (read-only path).
-template <typename I> struct Quad { I v[4]; };
+template <typename I> struct __align__(16) Quad { I v[4]; };
 __device__ __forceinline__ Quad<int> quad_load_vec(const int* p) {
     const int4 t = __ldg(reinterpret_cast<const int4*>(p));
     return {{t.x, t.y, t.z, t.w}};
@@ -143,6 +144,19 @@ template <typename I> __device__ __forceinline__ Quad<I> quad_load(const I* base
 #pragma unroll
     for (int j = 0; j < 4; ++j) q.v[j] = list_load(base + (i + j < end ? i + j : end - 1));
     return q;
+}
+
+// A kernel that is launched early (see launch_early): the next kernel of the stream may start, and the one before has
+// written what it writes.  Index lists and work items, fixed when an operator is built and written by no kernel that
+// lets the next one start, may be read before the wait.
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __threadfence();
+}
+__device__ __forceinline__ void after_previous_kernel() {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
 }
 
 // ---- row access policies ---------------------------------------------------
@@ -175,13 +189,6 @@ template <typename T> __device__ __forceinline__ void row_load_passing(Row<T, 16
     if constexpr (sizeof(T) == 4) { v.x[0] = a; v.x[1] = b; }
     else { v.x[0] = __longlong_as_double((long long)a); v.x[1] = __longlong_as_double((long long)b); }
 }
-__device__ __forceinline__ Quad<int> quad_load_passing(const int* base, int i, int end, bool aligned, u64 policy) {
-    if (!aligned || i + 4 > end) return quad_load(base, i, end, false);
-    Quad<int> q;
-    asm volatile("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;"
-        : "=r"(q.v[0]), "=r"(q.v[1]), "=r"(q.v[2]), "=r"(q.v[3]) : "l"(base + i), "l"(policy));
-    return q;
-}
 // Rows that live in the owners' heaps: reference = owner rank (6 bits) and row
 // number inside the owner's block (25 bits); `bases` (shared memory) holds the
 // block address of every rank as mapped into this process.
@@ -198,23 +205,52 @@ struct RowsByPeerRef {
     }
 };
 
-// Where values go: `scale(i)` is read together with the dense rows, `put(i, v)` stores dot * scale.
+// Where values go: `put4(i, n, dots)` stores min(n, 4) values from nonzero i on (i a multiple of 4), dot products times
+// values.  Quads are written as vectors where the places of all quads are 16-byte aligned (`vectors`).
+template <typename T> __device__ __forceinline__ void quad_store(T* p, const Quad<T>& q, int n, bool vectors) {
+    if (vectors && n >= 4) {
+        using V = typename Vec<T>::type;
+#pragma unroll
+        for (int j = 0; j < 4; j += Vec<T>::N) *reinterpret_cast<V*>(p + j) = *reinterpret_cast<const V*>(q.v + j);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < n) p[j] = q.v[j];
+}
 template <typename T> struct StoreLocal {
     T* out;
     const T* sval;    // null: no scaling
-    __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
-    __device__ __forceinline__ void put(long long i, T v) const { out[i] = v; }
+    bool vectors;
+    __device__ __forceinline__ Quad<T> scaled(long long i, int n, const T* dots) const {
+        Quad<T> q = quad_load(dots, 0, 4, true);
+        if (sval) {
+            const Quad<T> s = quad_load(sval + i, 0, n, vectors);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) q.v[j] *= s.v[j];
+        }
+        return q;
+    }
+    __device__ __forceinline__ void put4(long long i, int n, const T* dots) const {
+        quad_store(out + i, scaled(i, n, dots), n, vectors);
+    }
 };
 template <typename T> struct StoreTwice : StoreLocal<T> {
     T* also;          // a second place for the values (a form of its own: the choice in the kernel cost 1 %)
-    __device__ __forceinline__ void put(long long i, T v) const { this->out[i] = v; also[i] = v; }
+    __device__ __forceinline__ void put4(long long i, int n, const T* dots) const {
+        const Quad<T> q = this->scaled(i, n, dots);
+        quad_store(this->out + i, q, n, this->vectors);
+        quad_store(also + i, q, n, this->vectors);
+    }
 };
-template <typename T> struct StoreScattered {
-    T* out;
-    const T* sval;
+template <typename T> struct StoreScattered : StoreLocal<T> {
     const int* orig;  // result position of nonzero i
-    __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
-    __device__ __forceinline__ void put(long long i, T v) const { out[__ldg(orig + i)] = v; }
+    __device__ __forceinline__ void put4(long long i, int n, const T* dots) const {
+        const Quad<T> q = this->scaled(i, n, dots);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < n) this->out[__ldg(orig + i + j)] = q.v[j];
+    }
 };
 
 // Sums four values per lane over a group of G lanes (4 <= G) with a halving butterfly: log2(G) + 1 shuffles
@@ -242,16 +278,21 @@ template <typename T, int G> __device__ __forceinline__ T group_sum4(T (&v)[4], 
 
 // ---------------------------------------------------------------------------
 // SDDMM over windows first, first + step, ... < end of `wn` consecutive nonzeros each (wn a multiple of 4, at
-// most 128), one warp per window.  Lane l holds the indices of nonzeros 4l .. 4l+3 (one 16-byte load per array,
-// requested a whole window ahead); every group of G lanes works through an equal share of these quads: four
-// column indices by shuffle, four dense B rows in flight, four dot products reduced together, the A row kept in
-// registers until the row changes (the list is sorted by row).
+// most 128), one warp per window.  The indices of a window lie in shared memory, copied there asynchronously while the
+// window before it is computed; the groups of G lanes take its quads of nonzeros in turn: four
+// dense B rows in flight, four dot products reduced together, the A row kept in registers until the row changes (the
+// list is sorted by row).
 //
-// Bound by the row gathers out of L2 and by the issue of what surrounds them, so the split keeps the lanes per
-// row few (each shuffle then serves 32/G nonzeros) and fetches the A row of a quad's last nonzero together with
-// its B rows.
+// Bound by the row gathers out of the L2 and by what a warp does while it has none in flight.  So the rows of the next
+// quad (and the A row it ends in, if that is another one) are requested as soon as the products of this one are summed
+// per lane, and travel while the lanes are added up and the results stored; and the lanes per row are few, so that an
+// instruction of the reduction serves 32 / G nonzeros.
 // ---------------------------------------------------------------------------
 constexpr int WINDOW_MAX = 128;
+template <typename T> struct WindowLists {   // shared memory of a warp
+    int4 cols[2][WINDOW_MAX / 4], rows[2][WINDOW_MAX / 4];
+    T dots[WINDOW_MAX];
+};
 
 // Nonzeros per window: 128, less when that would leave warps without work.
 __host__ __device__ inline int window_nnz(long long nnz, long long nwarps, int groups_per_warp) {
@@ -261,11 +302,18 @@ __host__ __device__ inline int window_nnz(long long nnz, long long nwarps, int g
     return (int)(w < quantum ? quantum : (w > WINDOW_MAX ? WINDOW_MAX : w));
 }
 
+template <bool PASSING> __device__ __forceinline__ void copy_quad_async(int4* dst, const int* src, u64 policy) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (PASSING) asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "l"(policy) : "memory");
+    else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename ARows, typename Store>
 __device__ __forceinline__ void sddmm_windows(long long first, long long step, long long end, int wn, long long nnz,
                                               const int* __restrict__ rowidx, const int* __restrict__ colidx,
                                               const ARows& arows, const char* B, unsigned ldb_bytes,
-                                              int nvec, bool aligned, const Store& store, int lane) {
+                                              int nvec, bool aligned, const Store& store, WindowLists<T>& lists, int lane,
+                                              bool early = false) {
     static_assert(G >= 4, "a group reduces four values");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;
@@ -281,17 +329,18 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
     constexpr bool PASSING = passes_by<ARows>::value;
     const u64 policy = PASSING ? evict_first_policy() : 0;
     auto length = [&](long long w) { return (int)(nnz - w * wn < wn ? nnz - w * wn : (long long)wn); };
-    auto load = [&](long long w, Quad<int>& c, Quad<int>& r) {
+    // copies the indices of window w to buffer k, a quad per lane (behind the last quad: that quad again)
+    auto stage = [&](long long w, int k) {
         const int n = length(w), i = 4 * lane < n ? 4 * lane : (n - 1) & ~3;
-        if constexpr (PASSING) {
-            c = quad_load_passing(colidx + w * wn, i, n, aligned, policy);
-            r = quad_load_passing(rowidx + w * wn, i, n, aligned, policy);
+        const int *c = colidx + w * wn, *r = rowidx + w * wn;
+        if (aligned && i + 4 <= n) {
+            copy_quad_async<PASSING>(&lists.cols[k][lane], c + i, policy);
+            copy_quad_async<PASSING>(&lists.rows[k][lane], r + i, policy);
         } else {
-            c = quad_load(colidx + w * wn, i, n, aligned);
-            r = quad_load(rowidx + w * wn, i, n, aligned);
+            const Quad<int> cq = quad_load(c, i, n, false), rq = quad_load(r, i, n, false);
+            lists.cols[k][lane] = make_int4(cq.v[0], cq.v[1], cq.v[2], cq.v[3]);
+            lists.rows[k][lane] = make_int4(rq.v[0], rq.v[1], rq.v[2], rq.v[3]);
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r.v[j] = arows.ref(r.v[j]);
     };
     auto fetch = [&](Row<T, NB> (&a)[R], const char* p) {
 #pragma unroll
@@ -307,77 +356,103 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
     };
     if (first >= end) return;
     B += off[0];
-    const int mine = gl / (G / 4);              // which of the four results ends up in this lane
-    const bool writer = gl % (G / 4) == 0;
-    Quad<int> c4, r4;
-    load(first, c4, r4);
-    int cur = -1;
-    Row<T, NB> a[R];
+    const bool writer = gl % (G / 4) == 0;      // (lane gl ends up with value gl / (G / 4) of its group's quad)
+    long long w = first;
+    int k = 1, tag = 0;
+    int src = 0, quads = 0;                     // quad of this group, quads of the window (rounded up for all groups)
+    auto enter = [&]() {                        // window w, whose indices are on their way to the other buffer
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        k ^= 1;
+        const int4 r = lists.rows[k][lane];
+        // the row in which the lane's quad ends, negative: the quad is not all of that row (a list sorted by row class
+        // by class may also leave and re-enter a row)
+        tag = r.x == r.w && r.y == r.w && r.z == r.w ? r.w : r.w | (1 << 31);
+        __syncwarp();
+        if (w + step < end) stage(w + step, k ^ 1);
+        src = slot;
+        quads = (((length(w) + 3) >> 2) + SLOTS - 1) / SLOTS * SLOTS;
+    };
+    int cur = -1, next = -1;                    // row in `a`; tag of the quad in flight
+    Row<T, NB> a[R], a2[R], b[U][R];
 #pragma unroll
-    for (int q = 0; q < R; ++q) row_zero(a[q]);
-    for (long long w = first; w < end; w += step) {
-        Quad<int> cn = c4, rn = r4;
-        if (w + step < end) load(w + step, cn, rn);
-        const int n = length(w);
-        const long long w0 = w * wn;
-        const int nq = (((n + 3) >> 2) + SLOTS - 1) / SLOTS;   // quads per group
-        // lanes whose quad is not all one row (a list sorted by row class by class may leave and re-enter a row)
-        const unsigned mixed = __ballot_sync(FULL, r4.v[0] != r4.v[3] || r4.v[1] != r4.v[3] || r4.v[2] != r4.v[3]);
-        for (int i = 0; i < nq; ++i) {
-            const int src = slot * nq + i;                     // lane that holds this group's quad
-            int c[4];
+    for (int q = 0; q < R; ++q) { row_zero(a[q]); row_zero(a2[q]); }
+    auto request = [&]() {                      // the rows of B of quad src, the row of A it ends in if that is another one
+        const int4 c = lists.cols[k][src];
+        const int cs[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-            for (int u = 0; u < 4; ++u) c[u] = __shfl_sync(FULL, c4.v[u], src);
-            const int last = __shfl_sync(FULL, r4.v[3], src);
-            Row<T, NB> b[U][R];
+        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)cs[u] * ldb_bytes);
+        next = __shfl_sync(FULL, tag, src);
+        if (__any_sync(FULL, next != cur)) fetch_a(a2, arows.resolve(next & 0x7fffffff) + off[0]);
+    };
+    stage(first, 0);
+    if (early) wait_for_previous_kernel();      // (the lists come while the kernel before ends)
+    enter();
+    request();
+    for (bool more = true; more;) {
+        auto second = [&](int h) {              // the rows of the second half, where only half a quad is in flight
+            if (h > 0) {
+                const int4 c = lists.cols[k][src];
+                const int cs[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-            for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[u] * ldb_bytes);
-            const int pos = 4 * src + mine;
-            const bool st = writer && pos < n;
-            const T s = store.scale(w0 + (pos < n ? pos : n - 1));
-            T d[4];
-            if (__all_sync(FULL, last == cur && !(mixed >> src & 1))) {
+                for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)cs[(h + u) & 3] * ldb_bytes);
+            }
+        };
+        T d[4];
+        if (__all_sync(FULL, next >= 0)) {      // every group: four nonzeros of one row
+            if (next != cur) {
+                cur = next;
 #pragma unroll
-                for (int h = 0; h < 4; h += U) {
-                    if (h > 0)
+                for (int q = 0; q < R; ++q) a[q] = a2[q];
+            }
 #pragma unroll
-                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
+            for (int h = 0; h < 4; h += U) {
+                second(h);
 #pragma unroll
-                    for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
-                }
-            } else {
-                int r[4];
+                for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
+            }
+        } else {
+            // where a row ends in a quad, both of its rows are here as a rule: both products, and the one that counts
+            const int4 rq = lists.rows[k][src];
+            const int r[4] = {rq.x, rq.y, rq.z, rq.w};
+            const bool here = (r[0] == cur || r[0] == r[3]) && (r[1] == cur || r[1] == r[3]) && (r[2] == cur || r[2] == r[3]);
+            const bool both = __all_sync(FULL, here);
 #pragma unroll
-                for (int u = 0; u < 3; ++u) r[u] = __shfl_sync(FULL, r4.v[u], src);
-                r[3] = last;
-                Row<T, NB> a2[R];
-                const bool staged = last != cur;
-                fetch_a(a2, arows.resolve(last) + off[0]);   // (unconditional: a load under a condition costs more)
+            for (int h = 0; h < 4; h += U) {
+                second(h);
 #pragma unroll
-                for (int h = 0; h < 4; h += U) {
-                    if (h > 0)
-#pragma unroll
-                        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)c[h + u] * ldb_bytes);
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        if (r[h + u] != cur) {
-                            cur = r[h + u];
-                            if (staged && cur == last) {
-#pragma unroll
-                                for (int q = 0; q < R; ++q) a[q] = a2[q];
-                            } else {
-                                fetch_a(a, arows.resolve(cur) + off[0]);
-                            }
-                        }
-                        d[h + u] = row_dot<EXACT>(a, b[u], on);
+                for (int u = 0; u < U; ++u) {
+                    if (!both && r[h + u] != cur && r[h + u] != r[3]) {
+                        cur = r[h + u];
+                        fetch_a(a, arows.resolve(cur) + off[0]);
                     }
+                    const T d1 = row_dot<EXACT>(a, b[u], on), d2 = row_dot<EXACT>(a2, b[u], on);
+                    d[h + u] = r[h + u] == r[3] ? d2 : d1;
                 }
             }
-            const T total = group_sum4<T, G>(d, gl);
-            if (st) store.put(w0 + pos, total * s);
+            cur = r[3];
+#pragma unroll
+            for (int q = 0; q < R; ++q) a[q] = a2[q];
         }
-        c4 = cn;
-        r4 = rn;
+        // the next quad travels while this one is reduced and stored (behind the last one: that one again)
+        T* const place = lists.dots + 4 * src + gl / (G / 4);
+        const bool last = src + SLOTS >= quads;
+        if (!last) {
+            src += SLOTS;
+        } else {
+            w += step;
+            more = w < end;
+            if (more) enter();
+        }
+        request();
+        const T total = group_sum4<T, G>(d, gl);
+        if (writer) *place = total;
+        if (last) {                             // the values of the window, four per lane
+            __syncwarp();
+            const long long at = (w - step) * wn;
+            const int j = 4 * lane, n = (int)(nnz - at < wn ? nnz - at : (long long)wn);
+            if (j < n) store.put4(at + j, n - j, lists.dots + j);
+            __syncwarp();
+        }
     }
 }
 
@@ -386,7 +461,6 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
 // ---------------------------------------------------------------------------
 constexpr int SPMM_PIECE_SHIFT = 20;   // at most 2^20 split rows, 2^11 pieces per row
 constexpr int SPMM_ITEM_ROWS = 32;     // most rows of a rows item: a lane holds the end of one row
-constexpr int SPMM_ENDS = SPMM_ITEM_ROWS + 1;   // ints of shared memory per warp for the row ends
 
 struct SpmmLong {
     const int* first_piece;  // [nlong] first carry slot of each long row
@@ -455,6 +529,17 @@ template <typename T> struct EmitPacked {
     }
 };
 
+// Shared memory of a warp that works on items: the rows of the item that hold nonzeros, as (end, row number), behind
+// them a sentinel, and from the back the numbers of the empty rows; and for every lane the part of a row that began in
+// an earlier group (see below).
+template <int R, int N, typename E, bool HEADS> struct ItemScratch {
+    int2 rows[SPMM_ITEM_ROWS + 2];
+    int4 item;
+    E heads[HEADS ? R * N * 32 : 1];
+};
+template <typename T, int NB, int G, int R>
+using ItemSmem = ItemScratch<R, Row<T, NB>::N, typename Row<T, NB>::E, (32 / G > 1)>;
+
 // One item, one warp (see build_spmm_items in ops/cuda_ops.py):
 //   rows item   (first row, end row, first nonzero, -1 - nonzeros): at most SPMM_ITEM_ROWS whole rows; a first
 //               nonzero that 32 bits do not hold is -1 and read from the row pointer
@@ -463,16 +548,25 @@ template <typename T> struct EmitPacked {
 // The nonzeros of an item are dealt to the lane groups in equal shares of whole quads, wherever the rows end: a
 // group emits the rows that lie inside its share, and the sums of rows that go on in the next group travel along
 // the groups by shuffle, in order, at the end.  (Dealing whole rows to the groups left most lanes idle behind the
-// longest one: R-MAT scale 20, k = 32, 0.44 ms against 0.26 ms.)  Row ends are kept in shared memory (`ends`,
-// SPMM_ENDS ints per warp), indices and values come as quads that all lanes of a group read, requested one
-// quad ahead; U x R dense vectors are in flight per lane.  No atomics on values: bitwise reproducible.
+// longest one: R-MAT scale 20, k = 32, 0.44 ms against 0.26 ms.)  Indices and values come as quads that all lanes of
+// a group read, requested one quad ahead; U x R dense vectors are in flight per lane.  No atomics on values: bitwise
+// reproducible.
+//
+// Bound by the latency of the row gathers: a warp that adds up, or ends a row, has none in flight, and a quad waits for
+// the slowest of its rows.  So what lies between two quads is kept short -- one comparison tells whether a quad ends a
+// row, the rows that hold nonzeros are listed once per item, empty rows are written apart from them -- and what is not
+// needed in every quad (where rows end, the part of a group's first row) stays in shared memory, which makes room for
+// 40 warps per SM instead of 32 where a lane holds one vector per row.
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename Emit>
 __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* __restrict__ rowptr, long long nnz,
                                                const int* __restrict__ colidx, const T* val,
                                                const char* X, unsigned ldx_bytes, int nvec, bool aligned,
-                                               const Emit& emit, const SpmmLong& lg, int* ends, int lane) {
+                                               const Emit& emit, const SpmmLong& lg, ItemSmem<T, NB, G, R>& sm, int lane,
+                                               bool early = false) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;            // G need not divide 32: the lanes of slot SLOTS have no share
+    constexpr int N = Row<T, NB>::N;
+    constexpr int NO_END = 0x7fffffff;
     const int slot = lane / G, gl = lane % G;
     unsigned off[R];
     bool on[R];
@@ -492,130 +586,162 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
         for (int q = 0; q < R; ++q)
             if ((q < R - 1 && R <= 4) || on[q]) emit(row, gl + q * G, v[q]);
     };
-    const bool is_rows = item.w < 0;
-    const int nr = is_rows ? item.y - item.x : 0;
-    const long long p0 = !is_rows ? item.y : (item.z >= 0 ? item.z : __ldg(rowptr + item.x));
-    const int n = is_rows ? -1 - item.w : item.z - item.y;
+    const bool is_piece = item.w >= 0, is_rows = !is_piece && item.y - item.x > 1;   // else: one whole row
+    const int nr = item.y - item.x;
+    const long long p0 = is_piece ? item.y : (item.z >= 0 ? item.z : __ldg(rowptr + item.x));
+    const int n = is_piece ? item.z - item.y : -1 - item.w;
     // positions count from the 16-byte boundary at or before the first nonzero
     const int lead = (int)(p0 & 3), stop = lead + n;
     const int share = ((stop + 4 * SLOTS - 1) / (4 * SLOTS)) * 4;
     const int begin = slot < SLOTS ? slot * share : stop, end = begin + share < stop ? begin + share : stop;
-    int row_end_lane = stop;                 // lane l: end of row l of the item
-    if (lane < nr) row_end_lane = lead + (int)(__ldg(rowptr + item.x + lane + 1) - p0);
     const int* cp = colidx + (p0 - lead);
     const T* vp = val + (p0 - lead);
-    const int avail = (int)(nnz - (p0 - lead) < 0x7fffffff ? nnz - (p0 - lead) : 0x7fffffff);
-    Quad<int> c4;
-    Quad<T> v4;
-    if (begin < end) {
-        c4 = quad_load(cp, begin, avail, aligned);
-        v4 = quad_load(vp, begin, avail, aligned);
-    }
-    int r = 0;                               // row of the item this group is in
+    const int avail = (int)(nnz - (p0 - lead) < NO_END ? nnz - (p0 - lead) : NO_END);
+    int row_end_lane = stop;                 // lane l: end of row l of the item
+    if (is_rows && lane < nr) row_end_lane = lead + (int)(__ldg(rowptr + item.x + lane + 1) - p0);
+    if (early) wait_for_previous_kernel();   // the first item of a warp: its lists came while the kernel before ended
+    Row<T, NB> acc[R];
+    clear(acc);
+    int r = 0;                               // row (of those that hold nonzeros) this group is in
+    bool open = false;                       // it began in an earlier group
     if (is_rows) {
-        ends[lane] = row_end_lane;
+        int row_begin_lane = __shfl_up_sync(FULL, row_end_lane, 1);
+        if (lane == 0) row_begin_lane = lead;
+        const bool mine = lane < nr, full = mine && row_end_lane > row_begin_lane;
+        const unsigned filled = __ballot_sync(FULL, full), below = (1u << lane) - 1;
+        const int n_full = __popc(filled), n_empty = nr - n_full;
+        if (full) sm.rows[__popc(filled & below)] = make_int2(row_end_lane, item.x + lane);
+        else if (mine) sm.rows[SPMM_ITEM_ROWS + 1 - __popc(~filled & below)].y = item.x + lane;
+        if (lane == 0) sm.rows[n_full].x = NO_END;
 #pragma unroll
         for (int g = 1; g < SLOTS; ++g) {
-            const unsigned done = __ballot_sync(FULL, lane < nr && row_end_lane <= g * share);
+            const unsigned done = __ballot_sync(FULL, full && row_end_lane <= g * share);
             if (slot == g) r = __popc(done);
         }
         __syncwarp();
+        for (int e = slot; e < n_empty; e += SLOTS)   // (slot SLOTS: every row is written by a group before it)
+            if (slot < SLOTS) flush(sm.rows[SPMM_ITEM_ROWS + 1 - e].y, acc);
+        open = slot > 0 && begin < end && (r == 0 ? lead : sm.rows[r - 1].x) < begin;
+    } else {
+        if (lane == 0) {
+            sm.rows[0].x = NO_END;
+            sm.item = item;
+        }
+        __syncwarp();
     }
-    int row_end = r < nr ? ends[r] : stop;
-    const bool open = is_rows && slot > 0 && begin < end && (r == 0 ? lead : ends[r - 1]) < begin;   // began in an earlier group
     bool in_head = open;
-    Row<T, NB> acc[R], first[R];             // first: this group's part of a row that began in an earlier group
-    clear(acc);
-    if (SLOTS > 1) clear(first);
+    // quads that end at or before `plain` lie inside the item and end no row
+    int plain = 0;
+    auto look = [&]() {
+        const int row_end = sm.rows[r].x;
+        plain = row_end <= end ? row_end - 1 : end;
+    };
+    if (begin >= lead) look();
     auto close = [&]() {                     // the current row ends here
         if (SLOTS > 1 && in_head) {
 #pragma unroll
-            for (int q = 0; q < R; ++q) first[q] = acc[q];
+            for (int q = 0; q < R; ++q)
+#pragma unroll
+                for (int h = 0; h < N; ++h) sm.heads[(q * N + h) * 32 + lane] = acc[q].x[h];
             in_head = false;
         } else {
-            flush(item.x + r, acc);
+            flush(sm.rows[r].y, acc);
         }
         clear(acc);
         ++r;
-        row_end = ends[r];
     };
-    for (int i = begin; i < end; i += 4) {
-        int c[4];
-        T v[4];
+    // VEC: every quad of the item lies inside the lists, and is a vector of them
+    auto walk = [&](auto vec) {
+        constexpr bool VEC = decltype(vec)::value;
+        auto columns = [&](int i) {
+            if constexpr (VEC) return quad_load_vec(cp + i);
+            else return quad_load(cp, i, avail, false);
+        };
+        const int tail = (end - 1) & ~3;     // last quad of this group
+        Quad<int> c4 = columns(begin);
+        for (int i = begin; i < end; i += 4) {
+            Quad<T> v4;
+            const bool fast = i + 4 <= plain;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { c[u] = c4.v[u]; v[u] = v4.v[u]; }
-        const bool whole = i >= lead && i + 4 <= end;      // no position of this quad lies outside the item
-#pragma unroll
-        for (int h = 0; h < 4; h += U) {
-            Row<T, NB> x[U][R];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                // Positions outside the item are read too (their columns are those of the neighbouring items) and
-                // left out below: with the loads under a condition the kernel took 0.71 ms instead of 0.65 ms
-                // (R-MAT scale 20, k = 128).
-                const char* row = X + (u64)(unsigned)c[h + u] * ldx_bytes;
-#pragma unroll
-                for (int q = 0; q < R; ++q) row_load(x[u][q], row + (off[q] - off[0]));
-            }
-            // the next quad is requested behind the rows of this one: loads come back in order, and the indices may
-            // have to come from device memory (requested ahead of the rows: 0.84 ms instead of 0.66 ms at R-MAT
-            // scale 20, k = 128)
-            if (h == 0 && i + 4 < end) {
-                c4 = quad_load(cp, i + 4, avail, aligned);
-                v4 = quad_load(vp, i + 4, avail, aligned);
-            }
-            if (whole && i + h + U <= row_end) {
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int q = 0; q < R; ++q) row_fma(acc[q], v[h + u], x[u][q]);
-            } else {
+            for (int h = 0; h < 4; h += U) {
+                Row<T, NB> x[U][R];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const int p = i + h + u;
-                    if (p >= lead && p < end) {
-                        while (p >= row_end) close();
+                    // Positions outside the item are read too (their columns are those of the neighbouring items) and
+                    // left out below: with the loads under a condition the kernel took 0.71 ms instead of 0.65 ms
+                    // (R-MAT scale 20, k = 128).
+                    const char* row = X + (u64)(unsigned)c4.v[h + u] * ldx_bytes;
 #pragma unroll
-                        for (int q = 0; q < R; ++q) row_fma(acc[q], v[h + u], x[u][q]);
+                    for (int q = 0; q < R; ++q) row_load(x[u][q], row + (off[q] - off[0]));
+                }
+                // the values, and the indices of the next quad, are requested behind the rows of this one: loads come
+                // back in order, and the lists may have to come from device memory (requested ahead of the rows: 0.84
+                // ms instead of 0.66 ms at R-MAT scale 20, k = 128)
+                if (h == 0) {
+                    if constexpr (VEC) v4 = quad_load_vec(vp + i);
+                    else v4 = quad_load(vp, i, avail, false);
+                }
+                if (h + U == 4) c4 = columns(i < tail ? i + 4 : tail);
+                if (fast) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int q = 0; q < R; ++q) row_fma(acc[q], v4.v[h + u], x[u][q]);
+                } else {
+                    int row_end = sm.rows[r].x;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int p = i + h + u;
+                        if (p >= lead && p < end) {
+#pragma unroll
+                            for (int q = 0; q < R; ++q) row_fma(acc[q], v4.v[h + u], x[u][q]);
+                            if (p + 1 == row_end) {
+                                close();
+                                row_end = sm.rows[r].x;
+                            }
+                        }
                     }
+                    if (h + U == 4) look();
                 }
             }
         }
+    };
+    if (begin < end) {
+        if (aligned && ((stop + 3) & ~3) <= avail) walk(std::true_type{});
+        else walk(std::false_type{});
     }
     if (is_rows) {
-        // rows that end with this share, and the empty rows after them
-        if (begin < end || (slot == 0 && n == 0))
-            while (r < nr && ends[r] <= end) close();
-        if (SLOTS > 1) {
-            // A row that goes on: its sum so far (acc) moves to the next group.  in_head still set: the whole share
-            // lies inside one row that began earlier and goes on.
-            if (__any_sync(FULL, open)) {
-                Row<T, NB> carry[R];
-                clear(carry);
+        // A row that goes on: its sum so far (acc) moves to the next group.  in_head still set: the whole share
+        // lies inside one row that began earlier and goes on.
+        if (SLOTS > 1 && __any_sync(FULL, open)) {
+            Row<T, NB> carry[R];
+            clear(carry);
 #pragma unroll
-                for (int g = 1; g < SLOTS; ++g)
+            for (int g = 1; g < SLOTS; ++g)
 #pragma unroll
-                    for (int q = 0; q < R; ++q)
+                for (int q = 0; q < R; ++q)
 #pragma unroll
-                        for (int h = 0; h < Row<T, NB>::N; ++h) {
-                            const auto sum = in_head ? e_add(carry[q].x[h], acc[q].x[h]) : acc[q].x[h];
-                            const auto up = __shfl_up_sync(FULL, sum, G);
-                            if (slot == g) carry[q].x[h] = up;
-                        }
-                if (open && !in_head) {
+                    for (int h = 0; h < N; ++h) {
+                        const auto sum = in_head ? e_add(carry[q].x[h], acc[q].x[h]) : acc[q].x[h];
+                        const auto up = __shfl_up_sync(FULL, sum, G);
+                        if (slot == g) carry[q].x[h] = up;
+                    }
+            if (open && !in_head) {
 #pragma unroll
-                    for (int q = 0; q < R; ++q) row_add(carry[q], first[q]);
-                    int h = 0;           // the row in which this share begins
-                    while (ends[h] <= begin) ++h;
-                    flush(item.x + h, carry);
-                }
+                for (int q = 0; q < R; ++q)
+#pragma unroll
+                    for (int h = 0; h < N; ++h) carry[q].x[h] = e_add(carry[q].x[h], sm.heads[(q * N + h) * 32 + lane]);
+                int h = 0;           // the row in which this share begins
+                while (sm.rows[h].x <= begin) ++h;
+                flush(sm.rows[h].y, carry);
             }
         }
         __syncwarp();
         return;
     }
-    // piece of a long row: add up the groups, leave the sum in the carry; the last piece to arrive adds the carries
-    // in order
+    __syncwarp();
+    // one row: add up the groups; a piece of a long row leaves the sum in the carry, and the last piece to arrive adds
+    // the carries in order
     auto add_groups = [&]() {                // slot 0 gets the sum of all slots
         if constexpr ((G & (G - 1)) == 0) {
 #pragma unroll
@@ -638,14 +764,20 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
         }
     };
     add_groups();
-    const int lr = item.w & ((1 << SPMM_PIECE_SHIFT) - 1);
+    const int row = sm.item.x, code = sm.item.w;
+    if (code < 0) {
+        if (slot == 0) flush(row, acc);
+        __syncwarp();
+        return;
+    }
+    const int lr = code & ((1 << SPMM_PIECE_SHIFT) - 1);
     const int first_piece = __ldg(lg.first_piece + lr), np = __ldg(lg.npieces + lr);
     char* carry = static_cast<char*>(lg.carry);
     const long long ldc_bytes = lg.ldc * (long long)sizeof(T);
     if (slot == 0)
 #pragma unroll
         for (int q = 0; q < R; ++q)
-            if (on[q]) row_store(carry + (first_piece + (item.w >> SPMM_PIECE_SHIFT)) * ldc_bytes + (gl + q * G) * NB, acc[q]);
+            if (on[q]) row_store(carry + (first_piece + (code >> SPMM_PIECE_SHIFT)) * ldc_bytes + (gl + q * G) * NB, acc[q]);
     __threadfence();
     __syncwarp();
     int old = 0;
@@ -667,7 +799,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
         }
     }
     add_groups();
-    if (slot == 0) flush(item.x, acc);
+    if (slot == 0) flush(row, acc);
     if (lane == 0) lg.counters[lr] = 0;
 }
 
@@ -684,8 +816,9 @@ inline int env_int(const char* name, int dflt) {
 }
 
 // Launch that may begin while the previous kernel of the stream drains (programmatic dependent launch): the kernel
-// has to call `after_previous_kernel` before it touches memory, and to read what an earlier kernel of this library may
-// have written by ordinary loads (see row_load): it is resident while that kernel still writes.
+// has to wait (`wait_for_previous_kernel`) before it touches memory other than index lists and work items, and to read
+// what an earlier kernel of this library may have written by ordinary loads (see row_load): it is resident while that
+// kernel still writes.
 template <typename... P, typename... A>
 inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute attr = {};
@@ -699,11 +832,6 @@ inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cuda
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     return (int)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-__device__ __forceinline__ void after_previous_kernel() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    __threadfence();
 }
 
 constexpr int MAX_DEVICES = 64;
@@ -730,19 +858,19 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
 }
 
 // Lanes per row (G) and vectors per lane (R) for a row of `nvec` vectors, at most 256.
-//   SDDMM  few lanes with several vectors each: every index shuffle and every step of the reduction then serves
-//          32 / G nonzeros (R-MAT scale 20, fp32: k = 64 0.35 ms as 8 x 2, 0.38 as 16 x 1; k = 128 0.60 ms as
-//          8 x 4, 0.71 as 32 x 1).  9 to 12 vectors go as 4 x 3 (R-MAT scale 17, k = 40: 39 us, 47 as 8 x 2, where a
-//          third of the lanes idles); 13 to 16 do not fit 4 x 4 as well (k = 64, scale 20: 0.375 ms).
-//   SpMM   as many lanes as the row has vectors: an accumulator costs R vectors of registers, and nothing is
-//          reduced across lanes inside a row (k = 64: 0.40 ms as 16 x 1, 0.41 as 8 x 2).  Where that leaves a quarter
-//          of the lanes idle, three vectors per lane (k = 96, R-MAT scale 17: 67 us as 8 x 3, 100 as 32 x 1;
-//          Erdos-Renyi 1 M rows: 1.81 against 1.96 ms; k = 192: 110 us as 16 x 3, 140 as 32 x 2), and groups of 5, 6
-//          or 10 lanes, which share a warp one group more than 8 or 16 do (k = 40: 41 us as 10 x 1, 51 as 16 x 1;
-//          k = 20: 32 against 35 us; groups of 2 and 3 gained nothing over 4).  Rows of 25 to 32
-//          vectors that come out of the L2 (`cached`) go as 16 x 2, half the instructions per row (k = 128, scale
-//          17: 86 against 101 us); out of device memory the occupancy counts for more (scale 20: 0.74 against
-//          0.69 ms).
+//   SDDMM  few lanes with several vectors each: every step of the reduction then serves 32 / G nonzeros (R-MAT scale
+//          20, fp32: k = 64 278 us as 8 x 2, 394 as 16 x 1; k = 128 490 us as 8 x 4, 568 as 16 x 2, 707 as 32 x 1).  9 to
+//          12 vectors go as 4 x 3 (R-MAT scale 17, k = 40: 39 us, 47 as 8 x 2, where a third of the lanes idles); 13 to
+//          16 do not fit 4 x 4 as well (k = 64, scale 20: 0.375 ms).
+//   SpMM   several vectors per lane from 11 vectors on: what all lanes of a group read and compute for a nonzero (its
+//          index, its value, its address) then serves that many more bytes.  R-MAT scale 20: k = 64 331 us as 8 x 2, 350
+//          as 16 x 1; k = 128 569 as 16 x 2, 571 as 8 x 4, 606 as 32 x 1; scale 17: 43 against 48 us, 72 (8 x 4), 76
+//          (16 x 2) and 88.  25 to 32 vectors go as 8 x 4 where X comes out of the L2 (`cached`), and as 16 x 2, which
+//          keeps half as many warps more, where it does not (scale 22: 2640 against 2692 us).  49 to 64: 16 x 4 (Zipf
+//          rows, k = 256: 885 us, 909 as 32 x 2).  17 to 24 go as 8 x 3 (k = 96, scale 17: 67 us, 100 as 32 x 1), 33 to
+//          48 as 16 x 3 (k = 192: 110 us, 140 as 32 x 2), and groups of 5, 6 and 10 lanes share a warp one group more than
+//          8 or 16 do (k = 40: 41 us as 10 x 1, 51 as 16 x 1; k = 20: 32 against 35 us; groups of 2 and 3 gained nothing
+//          over 4).
 inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false) {
     int g = 4;
     const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
@@ -750,9 +878,9 @@ inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false)
     if (spmm) {
         if (nvec == 5 || nvec == 6) g = nvec;
         if (nvec == 9 || nvec == 10) g = 10;
-        if (nvec > 16 && nvec <= 24) g = 8;
-        if (nvec > 24 && nvec <= 32 && cached) g = 16;
-        if (nvec > 32 && nvec <= 48) g = 16;
+        if (nvec > 10 && nvec <= 24) g = 8;
+        if (nvec > 24 && nvec <= 32) g = cached ? 8 : 16;
+        if (nvec > 32 && nvec <= 64) g = 16;
     } else if (nvec > 8 && nvec <= 12) {
         g = 4;
     }
@@ -778,18 +906,19 @@ constexpr long long CACHED_BYTES = 64ll << 20;
     switch (G * 16 + R) {                                                                                 \
         case 4 * 16 + 1: MACRO(4, 1); break;   case 8 * 16 + 1: MACRO(8, 1); break;                       \
         case 5 * 16 + 1: MACRO(5, 1); break;   case 6 * 16 + 1: MACRO(6, 1); break;                       \
-        case 10 * 16 + 1: MACRO(10, 1); break;                                                            \
+        case 10 * 16 + 1: MACRO(10, 1); break; case 8 * 16 + 2: MACRO(8, 2); break;                       \
         case 16 * 16 + 1: MACRO(16, 1); break; case 32 * 16 + 1: MACRO(32, 1); break;                     \
         case 8 * 16 + 3: MACRO(8, 3); break;   case 16 * 16 + 2: MACRO(16, 2); break;                     \
-        case 16 * 16 + 3: MACRO(16, 3); break; case 32 * 16 + 2: MACRO(32, 2); break;                     \
-        case 32 * 16 + 3: MACRO(32, 3); break; case 32 * 16 + 4: MACRO(32, 4); break;                     \
-        default: MACRO(32, 8); break;                                                                     \
+        case 8 * 16 + 4: MACRO(8, 4); break;   case 16 * 16 + 3: MACRO(16, 3); break;                     \
+        case 16 * 16 + 4: MACRO(16, 4); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \
+        case 32 * 16 + 4: MACRO(32, 4); break; default: MACRO(32, 8); break;                              \
     }
 // Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
-// half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.
-__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 3 ? 4 : (R == 4 ? 2 : 1); }
-__host__ __device__ constexpr int sddmm_unroll(int R) { return R <= 4 ? 4 : 2; }
-__host__ __device__ constexpr int sddmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : (R <= 4 ? 2 : 1)); }
-__host__ __device__ constexpr int spmm_min_blocks(int G, int R) { return R == 1 ? 4 : (R == 2 && G == 32 ? 3 : 2); }
+// half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.  More blocks
+// than these spill registers in the inner loops.
+__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? 4 : 1; }
+__host__ __device__ constexpr int sddmm_unroll(int R, bool f32) { return R <= (f32 ? 4 : 3) ? 4 : 2; }
+__host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32) { return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 ? 2 : 1)); }
+__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : 2); }
 
 }  // namespace sp3

@@ -26,13 +26,15 @@ def item_sizes(nnz: int):
     """(long_row, item_nnz) of a block of `nnz` nonzeros: LONG_ROW and ITEM_NNZ once there is enough work for every
     warp, smaller powers of two (down to 16 nonzeros) below that, because the time of a small SpMM is that of its
     longest item: each group of four nonzeros costs one trip to memory.  SP3_LONG_ROW / SP3_ITEM_NNZ override."""
-    item = ITEM_NNZ
+    # twice as many where that still leaves every warp five of them (R-MAT scale 20, k = 64: 322 us instead of 331;
+    # Erdos-Renyi, 7.2 M nonzeros, k = 32: 95 instead of 100; Zipf rows, 5.7 M, k = 128: 465 instead of 456)
+    item = ITEM_NNZ if nnz < 2 * ITEM_NNZ * _TARGET_ITEMS * 5 else 2 * ITEM_NNZ
     while item > 16 and nnz < item * _TARGET_ITEMS * 3 // 4:
         item //= 2
     # a piece costs a partial row and a fence beyond its nonzeros: four items long where that has to be cheap, two
     # where the longest chain decides (Zipf rows, 357 thousand nonzeros, k = 64: 16.5 us with pieces of 128, 20.2
     # with 256, 20.1 with 64)
-    long_row = LONG_ROW if item == ITEM_NNZ else 2 * item
+    long_row = LONG_ROW if item >= ITEM_NNZ else 2 * item
     return int(os.environ.get("SP3_LONG_ROW", long_row)), int(os.environ.get("SP3_ITEM_NNZ", item))
 
 
