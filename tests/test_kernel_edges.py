@@ -220,3 +220,18 @@ def test_column_chunks_rule(monkeypatch):
     assert cuda_ops.column_chunks(*even, 4096, 48) is None      # fits
     hubs = lists(np.where(rng.random((4096, 64)) < 0.8, rng.integers(0, 512, (4096, 64)), rng.integers(0, 4096, (4096, 64))))
     assert cuda_ops.column_chunks(*hubs, 4096, 256) is None
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [32, 44, 64, 100, 128, 200, 256, 400])   # every number of vectors per lane
+def test_rows_shorter_than_quads(dtype, k):
+    """Rows of one nonzero and more: quads of one to four rows (SDDMM), several row ends in a quad, in every quad of a
+    group and at its last position, and one long row alone (SpMM)."""
+    for run in ([1], [2], [3], [4], [5], [1, 3], [2, 1, 1], [1, 2, 7, 40], [4, 4, 1, 300]):
+        deg = (run * 40)[:40]
+        rows = np.repeat(np.arange(40), deg)
+        _check_sddmm(rows, np.random.default_rng(len(rows)).integers(0, 50, len(rows)), k, dtype)
+        _check_spmm(deg, k, dtype, 0.0)
+        _check_spmm(deg, k, dtype, 0.5, shift=1)
+    _check_spmm([130], k, dtype, 0.5)
+    _check_spmm([0, 511, 0, 512], k, dtype, 0.0)
