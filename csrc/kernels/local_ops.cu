@@ -22,16 +22,16 @@ namespace sp3 {
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
-sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const int* __restrict__ colidx,
+sddmm_vec_kernel(long long nnz, int wn, const int* rowidx, const int* colidx,
                  const Rows arows, const char* B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
-    let_next_kernel_start();
+    after_previous_kernel();
     __shared__ __align__(16) WindowLists<T> lists[256 / 32];
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     sddmm_windows<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
                                                       arows, B, ldb_bytes, nvec, aligned, store, lists[threadIdx.x >> 5],
-                                                      threadIdx.x & 31, true);
+                                                      threadIdx.x & 31);
 }
 
 // out[i] = sval[i] * dots[where[i]], four values per thread: dot products computed chunk by chunk of columns, back into
@@ -40,7 +40,7 @@ sddmm_vec_kernel(long long nnz, int wn, const int* __restrict__ rowidx, const in
 // k = 64: about 250 us).
 template <typename T, bool TWICE>
 __global__ void __launch_bounds__(256)
-scale_picked_kernel(long long nnz, const int* __restrict__ where, const T* sval, const T* dots, T* out,
+scale_picked_kernel(long long nnz, const int* where, const T* sval, const T* dots, T* out,
                     T* also, bool aligned) {
     after_previous_kernel();
     const int n = (int)nnz, i = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
@@ -134,23 +134,23 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
 __global__ void __launch_bounds__(256, spmm_min_blocks(R))
-spmm_items_kernel(int nitems, const int4* __restrict__ items, int nrows, const long long* __restrict__ rowptr,
-                  const int* __restrict__ colidx, const T* val, const char* X,
+spmm_items_kernel(int nitems, const int4* items, int nrows, const long long* rowptr,
+                  const int* colidx, const T* val, const char* X,
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
-    let_next_kernel_start();
+    after_previous_kernel();
     __shared__ ItemSmem<T, NB, G, R> scratch[256 / 32];
     ItemSmem<T, NB, G, R>& sm = scratch[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int warp0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-    const long long nnz = __ldg(rowptr + nrows);
+    const long long nnz = rowptr[nrows];
     auto run = [&](int it) {
-        const int4 item = __ldg(items + it);
+        const int4 item = items[it];
         // (items of fewer rows wait for the previous values less often than the requests cost: Erdos-Renyi, 24 nonzeros
         // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
         if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
         spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
-                                                                 aligned, emit, lg, sm, lane, it == warp0);
+                                                                 aligned, emit, lg, sm, lane);
     };
     if (lg.ticket && nitems > nwarps) {
         // dynamic hand-out: items differ too much in cost (cached or not, hub or not) for a fixed assignment to balance

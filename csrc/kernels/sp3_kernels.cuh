@@ -45,12 +45,12 @@ template <> struct Row<float, 4> { using E = float; static constexpr int N = 1; 
 template <> struct Row<double, 16> { using E = double; static constexpr int N = 2; E x[2]; };
 template <> struct Row<double, 8> { using E = double; static constexpr int N = 1; E x[1]; };
 
-// Dense rows and values are read by ordinary loads, never through the read-only path (`ld.global.nc`, `__ldg`, or a
-// `const __restrict__` kernel parameter, from which the compiler infers it): that path is defined only for memory that
-// nobody writes while the kernel runs.  A kernel launched early runs while the kernel before it writes what may be its
-// values or rows (see wait_for_previous_kernel), and in the fused kernels other warps of the launch write the pulled rows.
-// Ordinary loads are ordered behind the wait, or the acquire, that says the data is there.  Index arrays and work items
-// are fixed when an operator is built and keep the read-only path.
+// Dense rows, values, index lists and work items are read by ordinary loads, never through the read-only path
+// (`ld.global.nc`, `__ldg`, or a `const __restrict__` kernel parameter, from which the compiler infers it): that path is
+// defined only for memory that nobody writes while the kernel runs.  A kernel launched early runs while the kernel before
+// it writes what may be its values, rows or lists (see after_previous_kernel), and in the fused kernels other warps of
+// the launch write the pulled rows.  Ordinary loads are ordered behind the wait, or the acquire, that says the data is
+// there.  (Lists through the read-only path took the same time: 192 products of 10 to 600 thousand nonzeros within 0.2 %.)
 template <typename T, int NB> __device__ __forceinline__ void row_load(Row<T, NB>& v, const char* p) {
     using E = typename Row<T, NB>::E;
     if constexpr (NB == 16 && sizeof(T) == 4) {
@@ -122,10 +122,10 @@ __device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> 
 }
 
 // Four consecutive values base[i .. i+3] of a list, i a multiple of 4 counted from a 16-byte boundary when `aligned`;
-// positions at or past `end` repeat the last value before it.  Lists of int are index lists (read-only path).
+// positions at or past `end` repeat the last value before it.
 template <typename I> struct __align__(16) Quad { I v[4]; };
 __device__ __forceinline__ Quad<int> quad_load_vec(const int* p) {
-    const int4 t = __ldg(reinterpret_cast<const int4*>(p));
+    const int4 t = *reinterpret_cast<const int4*>(p);
     return {{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ Quad<float> quad_load_vec(const float* p) {
@@ -136,27 +136,22 @@ __device__ __forceinline__ Quad<double> quad_load_vec(const double* p) {
     const double2 a = *reinterpret_cast<const double2*>(p), b = *(reinterpret_cast<const double2*>(p) + 1);
     return {{a.x, a.y, b.x, b.y}};
 }
-__device__ __forceinline__ int list_load(const int* p) { return __ldg(p); }
-template <typename T> __device__ __forceinline__ T list_load(const T* p) { return *p; }
 template <typename I> __device__ __forceinline__ Quad<I> quad_load(const I* base, int i, int end, bool aligned) {
     if (aligned && i + 4 <= end) return quad_load_vec(base + i);
     Quad<I> q;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q.v[j] = list_load(base + (i + j < end ? i + j : end - 1));
+    for (int j = 0; j < 4; ++j) q.v[j] = base[i + j < end ? i + j : end - 1];
     return q;
 }
 
-// A kernel that is launched early (see launch_early): the next kernel of the stream may start, and the one before has
-// written what it writes.  Index lists and work items, fixed when an operator is built and written by no kernel that
-// lets the next one start, may be read before the wait.
-__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous_kernel() {
+// First in a kernel that is launched early (see launch_early): the next kernel of the stream may start, and the one
+// before has written what it writes.  No memory is read ahead of the wait, index lists and work items included: callers
+// hand over any tensors, and what the kernel before writes is visible behind the wait only, whether that kernel signals
+// early or just ends.
+__device__ __forceinline__ void after_previous_kernel() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __threadfence();
-}
-__device__ __forceinline__ void after_previous_kernel() {
-    let_next_kernel_start();
-    wait_for_previous_kernel();
 }
 
 // ---- row access policies ---------------------------------------------------
@@ -249,7 +244,7 @@ template <typename T> struct StoreScattered : StoreLocal<T> {
         const Quad<T> q = this->scaled(i, n, dots);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (j < n) this->out[__ldg(orig + i + j)] = q.v[j];
+            if (j < n) this->out[orig[i + j]] = q.v[j];
     }
 };
 
@@ -310,10 +305,9 @@ template <bool PASSING> __device__ __forceinline__ void copy_quad_async(int4* ds
 
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename ARows, typename Store>
 __device__ __forceinline__ void sddmm_windows(long long first, long long step, long long end, int wn, long long nnz,
-                                              const int* __restrict__ rowidx, const int* __restrict__ colidx,
+                                              const int* rowidx, const int* colidx,
                                               const ARows& arows, const char* B, unsigned ldb_bytes,
-                                              int nvec, bool aligned, const Store& store, WindowLists<T>& lists, int lane,
-                                              bool early = false) {
+                                              int nvec, bool aligned, const Store& store, WindowLists<T>& lists, int lane) {
     static_assert(G >= 4, "a group reduces four values");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;
@@ -385,7 +379,6 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
         if (__any_sync(FULL, next != cur)) fetch_a(a2, arows.resolve(next & 0x7fffffff) + off[0]);
     };
     stage(first, 0);
-    if (early) wait_for_previous_kernel();      // (the lists come while the kernel before ends)
     enter();
     request();
     for (bool more = true; more;) {
@@ -558,11 +551,10 @@ using ItemSmem = ItemScratch<R, Row<T, NB>::N, typename Row<T, NB>::E, (32 / G >
 // needed in every quad (where rows end, the part of a group's first row) stays in shared memory, which makes room for
 // 40 warps per SM instead of 32 where a lane holds one vector per row.
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename Emit>
-__device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* __restrict__ rowptr, long long nnz,
-                                               const int* __restrict__ colidx, const T* val,
+__device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* rowptr, long long nnz,
+                                               const int* colidx, const T* val,
                                                const char* X, unsigned ldx_bytes, int nvec, bool aligned,
-                                               const Emit& emit, const SpmmLong& lg, ItemSmem<T, NB, G, R>& sm, int lane,
-                                               bool early = false) {
+                                               const Emit& emit, const SpmmLong& lg, ItemSmem<T, NB, G, R>& sm, int lane) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;            // G need not divide 32: the lanes of slot SLOTS have no share
     constexpr int N = Row<T, NB>::N;
@@ -588,7 +580,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     };
     const bool is_piece = item.w >= 0, is_rows = !is_piece && item.y - item.x > 1;   // else: one whole row
     const int nr = item.y - item.x;
-    const long long p0 = is_piece ? item.y : (item.z >= 0 ? item.z : __ldg(rowptr + item.x));
+    const long long p0 = is_piece ? item.y : (item.z >= 0 ? item.z : rowptr[item.x]);
     const int n = is_piece ? item.z - item.y : -1 - item.w;
     // positions count from the 16-byte boundary at or before the first nonzero
     const int lead = (int)(p0 & 3), stop = lead + n;
@@ -598,8 +590,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     const T* vp = val + (p0 - lead);
     const int avail = (int)(nnz - (p0 - lead) < NO_END ? nnz - (p0 - lead) : NO_END);
     int row_end_lane = stop;                 // lane l: end of row l of the item
-    if (is_rows && lane < nr) row_end_lane = lead + (int)(__ldg(rowptr + item.x + lane + 1) - p0);
-    if (early) wait_for_previous_kernel();   // the first item of a warp: its lists came while the kernel before ended
+    if (is_rows && lane < nr) row_end_lane = lead + (int)(rowptr[item.x + lane + 1] - p0);
     Row<T, NB> acc[R];
     clear(acc);
     int r = 0;                               // row (of those that hold nonzeros) this group is in
@@ -771,7 +762,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
         return;
     }
     const int lr = code & ((1 << SPMM_PIECE_SHIFT) - 1);
-    const int first_piece = __ldg(lg.first_piece + lr), np = __ldg(lg.npieces + lr);
+    const int first_piece = lg.first_piece[lr], np = lg.npieces[lr];
     char* carry = static_cast<char*>(lg.carry);
     const long long ldc_bytes = lg.ldc * (long long)sizeof(T);
     if (slot == 0)
@@ -816,9 +807,8 @@ inline int env_int(const char* name, int dflt) {
 }
 
 // Launch that may begin while the previous kernel of the stream drains (programmatic dependent launch): the kernel
-// has to wait (`wait_for_previous_kernel`) before it touches memory other than index lists and work items, and to read
-// what an earlier kernel of this library may have written by ordinary loads (see row_load): it is resident while that
-// kernel still writes.
+// has to call `after_previous_kernel` before it touches memory, and to read what an earlier kernel of this library may
+// have written by ordinary loads (see row_load): it is resident while that kernel still writes.
 template <typename... P, typename... A>
 inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute attr = {};

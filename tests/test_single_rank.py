@@ -113,6 +113,53 @@ def test_rows_written_by_the_kernel_before(gen, k, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("early", [False, True])    # whether the kernel that writes the lists lets the next one start
+@pytest.mark.parametrize("gen,k", [("uniform:4096:4096:16", 32), ("er:20000:20000:9", 128), ("rmat:14:8", 16)])
+def test_lists_written_by_the_kernel_before(gen, k, early):
+    """Column indices written by the kernel directly in front of the one that reads them, new ones in every launch."""
+    from spcomm3d_b200.ops import cuda_ops
+    plan = _plan(gen)
+    rowptr, ri, ci = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (plan.rowptr, plan.rowidx, plan.colidx))
+    vals = torch.from_numpy(plan.vals).float()
+    A, X = _randn(torch.empty(plan.row.n_local, k), 1), _randn(torch.empty(plan.col.n_local, k), 2)
+    sched, v, Ad, Xd = cuda_ops.SpmmSchedule(rowptr), vals.cuda(), A.cuda(), X.cuda()
+    turned = [(ci.long() + i * 7).remainder(plan.col.n_local).int() for i in range(4)]
+    buf = torch.zeros(plan.nnz, device="cuda")
+    cols = buf.view(torch.int32)
+    one, every, zeros = torch.zeros(1, 4, device="cuda"), torch.arange(plan.nnz, dtype=torch.int32, device="cuda"), torch.zeros_like(ci)
+    one[0, 0] = 1.0
+    bits = [torch.zeros(plan.nnz, 4, device="cuda") for _ in turned]
+    for b, t in zip(bits, turned):
+        b[:, 0] = t.view(torch.float32)      # (indices as denormal numbers: times 1 they are what they were)
+    torch.cuda.synchronize()
+
+    def write(i):
+        if early:
+            cuda_ops.sddmm(every, zeros, None, bits[i], one, buf)
+        else:
+            torch.add(turned[i], 0, out=cols)
+    got = []
+    for i in range(4):
+        c, y = torch.empty(plan.nnz, device="cuda"), torch.empty(plan.row.n_local, k, device="cuda")
+        write(i)
+        cuda_ops.sddmm(ri, cols, v, Ad, Xd, c)
+        write((i + 1) % 4)
+        cuda_ops.spmm(rowptr, ri, cols, v, Xd, y, 0.0, sched)
+        got.append((c, y))
+    rows, deg = ri.cpu().long(), torch.from_numpy(np.diff(plan.rowptr)).double()
+    for i, (c, y) in enumerate(got):
+        prod = A.double()[rows] * X.double()[turned[i].cpu().long()]
+        ref, mag = prod.sum(1) * vals.double(), prod.abs().sum(1) * vals.double()
+        assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, torch.float32) * mag).all())
+        prod = X.double()[turned[(i + 1) % 4].cpu().long()] * vals.double()[:, None]
+        ref = torch.zeros(plan.row.n_local, k, dtype=torch.float64)
+        mag = ref.clone().index_add_(0, rows, prod.abs())
+        ref.index_add_(0, rows, prod)
+        bound = torch.from_numpy(_gamma(deg.numpy() + 3.0, torch.float32))[:, None] * mag
+        assert bool(((y.cpu().double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("beta", [0.0, 0.5])
 @pytest.mark.parametrize("k,wide", [(1, 4), (3, 4), (5, 8), (10, 16), (33, 36), (33, 64), (50, 52), (66, 68), (97, 100),
