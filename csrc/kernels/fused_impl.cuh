@@ -1280,11 +1280,8 @@ static int launch_resident(K kernel, ResidentCache& cache, const A& args, long l
         (args.pull.pullers > 0 && (args.pull.stage_bytes < 1024 || args.pull.stage_bytes % 16)))
         return (int)cudaErrorInvalidValue;
     const size_t smem = bulk_smem_bytes(args.pull);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
     const unsigned blocks = resident_blocks(kernel, cache, needed, 256, smem);
+    if (blocks == 0) return (int)cudaErrorInvalidConfiguration;   // the rings and the kernel's own arrays do not fit an SM
     // phases without MAIN wait for nothing that a warp of the same launch still has to do
     if (!(args.comm.phases & PH_MAIN)) return launch_early(kernel, blocks, smem, st, copy);
     return (int)cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(256), params, smem, st);

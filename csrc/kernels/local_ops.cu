@@ -350,6 +350,7 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
         auto kernel = exact ? sddmm_vec_kernel<T, NB, GG, RR, NB == 16, Rows, Store>                                \
                             : sddmm_vec_kernel<T, NB, GG, RR, false, Rows, Store>;                                  \
         const unsigned all = resident_blocks(kernel, cache, 0);                                               \
+        if (all == 0) return (int)cudaErrorInvalidConfiguration;                                              \
         const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
         launch_early(kernel, needed < all ? (unsigned)needed : all, 0, st, nnz, wn, ri, ci, arows, B,               \

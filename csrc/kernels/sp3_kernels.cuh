@@ -827,8 +827,9 @@ inline int launch_early(void (*kernel)(P...), unsigned blocks, size_t smem, cuda
 constexpr int MAX_DEVICES = 64;
 
 // Blocks of `threads` threads of a persistent launch of `kernel`: all that fit at once, at most `needed` (0: no
-// limit).  `cache` belongs to this kernel and keeps the answer for the dynamic shared memory asked for last: the
-// occupancy query costs more than a launch.
+// limit), none if not even one does.  `cache` belongs to this kernel and keeps the answer for the dynamic shared memory
+// asked for last: the occupancy query costs more than a launch.  Without the attribute a launch has 48 KB, static and
+// dynamic shared memory together; it is raised to what a block can have, the same value whoever sets it.
 struct ResidentCache { std::atomic<unsigned long long> last[MAX_DEVICES] = {}; };   // smem << 32 | blocks
 template <typename K>
 unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int threads = 256, size_t smem = 0) {
@@ -838,9 +839,16 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
     if (v == 0 || v >> 32 != smem) {
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-        const int b = sms * (per_sm > 0 ? per_sm : 1);
-        v = (unsigned long long)smem << 32 | (unsigned)(b > 0 ? b : 1);
+        if (smem > 0) {
+            int most = 0;
+            cudaFuncAttributes own = {};
+            cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            if (cudaFuncGetAttributes(&own, kernel) != cudaSuccess ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)own.sharedSizeBytes) != cudaSuccess)
+                return 0;
+        }
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1 || sms < 1) return 0;
+        v = (unsigned long long)smem << 32 | (unsigned)(sms * per_sm);
         if (dev < MAX_DEVICES) cache.last[dev].store(v, std::memory_order_relaxed);
     }
     const long long b = (long long)(v & 0xffffffffu);

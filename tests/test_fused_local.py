@@ -270,6 +270,64 @@ def test_atomic_spmm_start_and_main_in_one_launch():
             assert err <= 2e-5 * max(1.0, ref.abs().max()) * 8, (epoch, op.plan.rank, float(err))
 
 
+# (one puller with stages of 12 KB: the ring and the arrays of the SpMM are 55 KB together; three with 4 KB; and 64 KB
+# stages, 210 KB, at most one block per SM)
+@pytest.mark.parametrize("pullers,stage", [(1, 12288), (1, 16352), (3, 4096), (1, 65536)])
+@pytest.mark.parametrize("k", [96, 128, 256])
+def test_rings_beyond_48_kb(k, pullers, stage, monkeypatch):
+    """Rings that fit the SM but not, next to the arrays of the kernel, the 48 KB of a launch that asks for nothing."""
+    from spcomm3d_b200.models.dist_ops import DistSDDMM, DistSpMM
+    from spcomm3d_b200.ops import oracle
+    from spcomm3d_b200.ops.fused import FusedSDDMM, FusedSpMM, run_lockstep
+    from spcomm3d_b200.parallel.symm import LocalFabric
+    from spcomm3d_b200.utils.sparse import CooMatrix
+    monkeypatch.setenv("SP3_FUSED_PULLERS", str(pullers))
+    monkeypatch.setenv("SP3_FUSED_STAGE_BYTES", str(stage))
+    mesh, m, plans, A, B = _setup("2x1x1", "uniform:600:500:7", k)
+    for cls, F in ((DistSDDMM, FusedSDDMM), (DistSpMM, FusedSpMM)):
+        fabric = LocalFabric(mesh.size)
+        heaps = fabric.heaps([F.region_sizes(p, k) for p in plans.values()])
+        ops = [cls(p, None, k, torch.float32, "cuda", "fused", heap=h, timeout_s=2.0, bulk_pull=True) for p, h in zip(plans.values(), heaps)]
+        for op in ops:
+            if cls is DistSDDMM:
+                op.fill_owned(op.A_owned, op.plan.row.owned_gids, seed=5, stream=1)
+            op.fill_owned(op.B_owned if cls is DistSDDMM else op.X_owned, op.plan.col.owned_gids, seed=5, stream=2)
+            op.poison_unowned()
+        run_lockstep([op._fused for op in ops], [(op.Y_owned, 0.0) for op in ops] if cls is DistSpMM else None)
+        for op in ops:
+            op._fused.check()
+            p = op.plan
+            if cls is DistSDDMM:
+                pos = op.owned_positions()
+                mine = CooMatrix(m.nrows, m.ncols, p.global_rows()[pos], p.global_cols()[pos], p.vals[pos])
+                ref, got = oracle.sddmm_ref(mine, A, B), op._fused.out[:op._fused.out_len].cpu().double()
+                off, ln = p.owned_nnz_slice()
+                got = got[off:off + ln]
+            else:
+                ref, got = oracle.spmm_ref(m, B)[p.row.owned_gids], op.Y_owned.cpu().double()
+            assert got.shape == ref.shape and (got - ref).abs().max() <= 2e-5 * max(1.0, float(ref.abs().max())) * k ** 0.5
+
+
+def test_ring_that_does_not_fit_is_refused(monkeypatch):
+    """A launch that the device cannot hold is an error of the launch, and the next one runs."""
+    from spcomm3d_b200.models.dist_ops import DistSpMM
+    from spcomm3d_b200.ops.fused import FusedSpMM, run_lockstep
+    from spcomm3d_b200.parallel.symm import LocalFabric
+    mesh, m, plans, A, B = _setup("2x1x1", "uniform:600:500:7", 128)
+    for stage, fits in ((80 << 10, False), (8 << 10, True)):
+        monkeypatch.setenv("SP3_FUSED_STAGE_BYTES", str(stage))
+        heaps = LocalFabric(mesh.size).heaps([FusedSpMM.region_sizes(p, 128) for p in plans.values()])
+        ops = [DistSpMM(p, None, 128, torch.float32, "cuda", "fused", heap=h, timeout_s=2.0, bulk_pull=True) for p, h in zip(plans.values(), heaps)]
+        args = [op._fused for op in ops], [(op.Y_owned, 0.0) for op in ops]
+        if fits:
+            run_lockstep(*args)
+            for op in ops:
+                op._fused.check()
+        else:
+            with pytest.raises(RuntimeError):
+                run_lockstep(*args)
+
+
 def test_wait_runs_out_without_hanging():
     """A flag that nobody sets: the kernel gives up after its limit, records
     where, and the context stays usable."""
