@@ -1035,8 +1035,8 @@ struct EmitOwnedOrAdd {
 // Resident blocks per SM as in the local kernel: left to itself the compiler takes 128 registers for the wave
 // bookkeeping and halves the occupancy, which costs the gather-bound inner loop far more than the few spills do.
 // GATED: the items follow the pull waves (wave_items given).  The other form pulls everything first and carries
-// no wave state: its inner loop keeps all 64 registers of a thread, which is worth 10-15 % on blocks that pull
-// nothing or little (meshes 1 x Y x Z).
+// no wave state: its inner loop keeps all registers of a thread (64 where a lane holds one vector per row, 80 with
+// two), which is worth 10-15 % on blocks that pull nothing or little (meshes 1 x Y x Z).
 template <int G, int R, bool ATOMIC, bool GATED>
 __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(const FusedSpmmArgs a) {
     after_previous_kernel();
