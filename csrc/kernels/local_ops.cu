@@ -405,41 +405,76 @@ int launch_sddmm(long long nnz, const int* ri, const int* ci, const T* sv, const
     return -1;
 }
 
-constexpr int SMS = 148;
+template <typename T, int NB, int G, int R, bool EXACT, typename Emit> unsigned spmm_blocks(long long needed) {
+    static ResidentCache cache;
+    return resident_blocks(spmm_items_kernel<T, NB, G, R, EXACT, Emit>, cache, needed);
+}
+// the shapes of pick_shape and the one that only small products take
+#define SP3_SPMM_LOCAL_SHAPES(MACRO) if (G == 32 && R == 2) MACRO(32, 2); else SP3_SPMM_SHAPES(MACRO)
+// nnz: 0 where it is not known
 template <typename T, int NB, typename Emit>
-int launch_spmm_nb(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
+int launch_spmm_nb(int nrows, long long nnz, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
                    const char* X, long long ldx_bytes, int nvec, bool cached, const Emit& emit, const SpmmLong& lg,
                    cudaStream_t st) {
     const bool aligned = ((uintptr_t)ci | (uintptr_t)val) % 16 == 0;
     constexpr bool VECTORS = std::is_same<Emit, EmitLocal<T, NB>>::value;
     int G, R;
     pick_shape(nvec, &G, &R, true, cached);
-    // Items that the shape of one vector per lane, with more warps, runs in one round and this one does not: 16384 rows
-    // of 16 nonzeros (4096 items) 8.8 us as 16 x 1 and 11.0 as 8 x 2, 12.4 as 32 x 1 and 13.5 as 8 x 4.
-    if (R > 1 && nvec <= 32 && nitems > SMS * 8 * spmm_min_blocks(R) && nitems <= SMS * 8 * spmm_min_blocks(1)) {
-        G = nvec <= 16 ? 16 : 32;
-        R = 1;
+    // Warps that are resident at once in a shape, at most `needed` blocks of them.
+    auto blocks = [&](int G, int R, long long needed) {
+        unsigned b = 0;
+#define SP3_SPMM(GG, RR)                                                                                      \
+        b = VECTORS && NB == 16 && nvec == GG * RR ? spmm_blocks<T, NB, GG, RR, VECTORS && NB == 16, Emit>(needed) \
+                                                   : spmm_blocks<T, NB, GG, RR, false, Emit>(needed)
+        SP3_SPMM_LOCAL_SHAPES(SP3_SPMM)
+#undef SP3_SPMM
+        return b;
+    };
+    // Small products of matrices without split rows: a shape with half the vectors per lane, or a quarter, where that
+    // saves a second round or where row ends lie inside the shares of the groups (several rows per item: what a row leaves
+    // in one group has to reach the next).  Rows that are split have their pieces added up by the groups of one warp, which
+    // wants many groups (Zipf rows, 107 thousand nonzeros, k = 96: 9.9 us as 8 x 3, 14.5 as 32 x 1).  Items of one row
+    // unless it says otherwise, us:
+    //   k = 64   8 x 2, 16 x 1          2,500 items of 16: 2.9, 3.1; 4,375 of 16: 6.2, 3.3; 4,687 of 128: 14.3, 11.4;
+    //                                   1,250 of 2 rows of 8: 3.3, 2.8; 1,666 rows of 6: 3.9, 3.4
+    //   k = 96   8 x 3, 16 x 2, 32 x 1  1,250 of 32: 3.6, 4.6, 4.9; 2,500 of 16: 5.0, 3.5, 3.9; 4,375 of 16: 6.4, 6.9, 4.0;
+    //                                   4,687 of 64: 11.4, 12.9, 10.2; 4,687 of 128: 17.2, 21.0, 17.5 (rows of 4: 29.6, 35.5)
+    //                                   1,666 rows of 6: 4.3, 4.0, 4.1; 2,500 rows of 4: 3.1, 3.6, 4.0
+    //   k = 128  8 x 4, 16 x 2, 32 x 1  1,250 of 32: 4.0, 4.4, 4.9; 2,500 of 16: 5.3, 3.5, 3.9; 4,375 of 16: 6.7, 6.9, 4.1;
+    //                                   4,687 of 128: 20.6, 24.2, 19.4; 1,666 rows of 6: 4.7, 3.8, 3.9
+    //   k = 192  16 x 3, 32 x 2         2,500 of 16: 5.6, 4.4; 4,375 of 16: 7.4, 8.4; 1,666 rows of 6: 4.3, 4.5
+    //   k = 256  16 x 4, 32 x 2         2,500 of 16: 6.1, 4.8; 4,375 of 16: 8.0, 8.6; 1,666 rows of 6: 4.8, 4.5
+    if (R > 1 && nvec <= 64 && lg.carry == nullptr) {
+        auto fits = [&](int g, int r) { return nitems <= 8ll * blocks(g, r, 0); };
+        const int half_g = nvec <= 32 ? 16 : 32, half_r = nvec <= 16 ? 1 : 2;
+        const bool one_round = fits(G, R);
+        if (one_round ? (nvec <= 16 || (nvec > 24 && nvec <= 32)) && 2ll * nrows > 3ll * nitems : fits(half_g, half_r)) {
+            G = half_g;
+            R = half_r;
+        } else if (!one_round && nvec > 16 && nvec <= 32 && fits(32, 1) && (nvec > 24 || (nnz > 0 && nnz <= 64ll * nitems))) {
+            G = 32;
+            R = 1;
+        }
     }
     const bool exact = VECTORS && NB == 16 && nvec == G * R;
-    const long long needed = ((long long)nitems + 7) / 8;
+    const unsigned grid = blocks(G, R, ((long long)nitems + 7) / 8);
 #define SP3_SPMM(GG, RR)                                                                                      \
-    {                                                                                                         \
-        static ResidentCache caches[2];                                                                       \
-        ResidentCache& cache = caches[exact];                                                                 \
+    do {                                                                                                        \
         auto kernel = exact ? spmm_items_kernel<T, NB, GG, RR, VECTORS && NB == 16, Emit>                     \
                             : spmm_items_kernel<T, NB, GG, RR, false, Emit>;                                  \
-        launch_early(kernel, resident_blocks(kernel, cache, needed), 0, st, nitems, items, nrows, rowptr, ci, val, X, \
+        launch_early(kernel, grid, 0, st, nitems, items, nrows, rowptr, ci, val, X,                           \
                      (unsigned)ldx_bytes, nvec, aligned, emit, lg);                                           \
-    }
-    SP3_SPMM_SHAPES(SP3_SPMM)
+    } while (0)
+    SP3_SPMM_LOCAL_SHAPES(SP3_SPMM)
 #undef SP3_SPMM
+#undef SP3_SPMM_LOCAL_SHAPES
     return (int)cudaGetLastError();
 }
 
 template <typename T>
 int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
                 const T* X, long long ldx, int k, T beta, T* Y, long long ldy, SpmmLong lg, cudaStream_t st,
-                int k_out = 0, long long x_rows = 0) {
+                int k_out = 0, long long x_rows = 0, long long nnz = 0) {
     if (nrows == 0) return 0;
     const long long ldx_b = ldx * (long long)sizeof(T), ldy_b = ldy * (long long)sizeof(T);
     unsigned long long bits = ldx_b | (uintptr_t)X;
@@ -451,7 +486,7 @@ int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowpt
     const int nb = vector_bytes<T>(bytes, bits);
     const unsigned long long nvec = bytes / nb;
     if (padded && (bytes | bits) % 16 == 0 && items != nullptr && bytes <= 256 * 16 && ldx_b < 1ll << 32)
-        return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, reinterpret_cast<const char*>(X), ldx_b,
+        return launch_spmm_nb<T, 16>(nrows, nnz, nitems, items, rowptr, ci, val, reinterpret_cast<const char*>(X), ldx_b,
                                      (int)(bytes / 16), cached, EmitPacked<T>{Y, ldy, k_out, beta}, lg, st);
     if (padded) k = k_out;
     if (padded || items == nullptr || nvec > 256 || nvec == 0 || ldx_b >= 1ll << 32) {
@@ -460,9 +495,9 @@ int launch_spmm(int nrows, int nitems, const int4* items, const long long* rowpt
     }
     const char* x = reinterpret_cast<const char*>(X);
     char* y = reinterpret_cast<char*>(Y);
-    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 16>{y, ldy_b, beta}, lg, st);
-    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 8>{y, ldy_b, beta}, lg, st);
-    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 4>{y, ldy_b, beta}, lg, st);
+    if (nb == 16) return launch_spmm_nb<T, 16>(nrows, nnz, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 16>{y, ldy_b, beta}, lg, st);
+    if (nb == 8) return launch_spmm_nb<T, 8>(nrows, nnz, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 8>{y, ldy_b, beta}, lg, st);
+    if constexpr (sizeof(T) == 4) return launch_spmm_nb<T, 4>(nrows, nnz, nitems, items, rowptr, ci, val, x, ldx_b, (int)nvec, cached, EmitLocal<T, 4>{y, ldy_b, beta}, lg, st);
     return -1;
 }
 
@@ -568,6 +603,7 @@ struct SpmmCall {
     int k_out;              // columns of Y (k of X counts the padding of its rows)
     int x_rows;             // rows of X
     PackRows pack_x;        // X is filled from here first
+    long long nnz;
 };
 SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *sddmm_bytes = (int)sizeof(SddmmCall);
@@ -599,9 +635,9 @@ SP3_API int sp3_cuda_spmm_call(const void* record, void* stream) {
     const int rc = c.f64 ? launch_pack<double>(c.pack_x, PackRows{}, st) : launch_pack<float>(c.pack_x, PackRows{}, st);
     if (rc != 0) return rc;
     if (c.f64) return launch_spmm<double>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const double*)c.val,
-                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows);
+                                          (const double*)c.X, c.ldx, c.k, c.beta, (double*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows, c.nnz);
     return launch_spmm<float>(c.nrows, c.nitems, (const int4*)c.items, c.rowptr, c.ci, (const float*)c.val,
-                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows);
+                              (const float*)c.X, c.ldx, c.k, (float)c.beta, (float*)c.Y, c.ldy, lg, st, c.k_out, c.x_rows, c.nnz);
 }
 
 // One step of a single GPU whose dense operands A and B (X of the SpMM is B) start in pinned host memory: SDDMM, SpMM

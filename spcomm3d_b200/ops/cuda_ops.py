@@ -314,7 +314,7 @@ class _SpmmCall(C.Structure):
                 ("ldy", C.c_longlong), ("first_piece", C.c_void_p), ("npieces", C.c_void_p), ("counters", C.c_void_p),
                 ("carry", C.c_void_p), ("ldc", C.c_longlong), ("ticket", C.c_void_p), ("beta", C.c_double),
                 ("k", C.c_int), ("f64", C.c_int), ("k_out", C.c_int),
-                ("x_rows", C.c_int), ("pack_x", _PackRows)]
+                ("x_rows", C.c_int), ("pack_x", _PackRows), ("nnz", C.c_longlong)]
 
 
 _checked_calls = False
@@ -471,7 +471,7 @@ def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule, pack=None):
     rec = _SpmmCall(rowptr.shape[0] - 1, sched.items.shape[0], p(sched.items), p(rowptr), p(colidx), p(vals), p(x),
                     _ld(x), p(Y), _ld(Y), p(sched.first), p(sched.npieces), p(sched.counters), p(carry), ldc,
                     p(sched.ticket), 0.0, x.shape[1], int(X.dtype == torch.float64), Y.shape[1], X.shape[0],
-                    px)
+                    px, colidx.shape[0])
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry, x), launches=1 + (x is not X))
 
 

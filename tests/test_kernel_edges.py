@@ -78,7 +78,7 @@ def test_sddmm_row_changes(k, nnz):
     _check_sddmm(again, rng.integers(0, 50, nnz), k, torch.float32)
 
 
-def _check_spmm(deg, k, dtype, beta, shift=0, ld=None, ncols=60, seed=0):
+def _check_spmm(deg, k, dtype, beta, shift=0, ld=None, ncols=60, seed=0, bound_call=False, **items):
     from spcomm3d_b200.ops import cuda_ops, local
     g = torch.Generator().manual_seed(seed)
     deg = np.asarray(deg, np.int64)
@@ -97,14 +97,17 @@ def _check_spmm(deg, k, dtype, beta, shift=0, ld=None, ncols=60, seed=0):
     Xd = torch.empty(ncols, ld, dtype=dtype, device="cuda")[:, :k]
     Xd.copy_(X)
     args = (rowptr.cuda(), ri.cuda(), _on_gpu(ci, shift), _on_gpu(v, shift), Xd)
-    sched = cuda_ops.SpmmSchedule(args[0])
+    sched = cuda_ops.SpmmSchedule(args[0], **items)
     bound = torch.from_numpy(_gamma(deg + 3.0, dtype))[:, None] * mag
     got = []
     for _ in range(2):
         wide = torch.full((nrows, ld), 7.0, dtype=dtype, device="cuda")
         Yd = wide[:, :k]
         Yd.copy_(Y0) if beta else Yd.fill_(float("nan"))
-        local.spmm(*args, Yd, beta, sched)
+        if bound_call:
+            cuda_ops.bind_spmm(args[0], *args[2:], Yd, sched).launch(beta)
+        else:
+            local.spmm(*args, Yd, beta, sched)
         assert bool(((Yd.cpu().double() - ref).abs() <= bound).all())
         assert bool((wide[:, k:] == 7.0).all())
         got.append(Yd)
@@ -139,6 +142,28 @@ def test_spmm_many_items(k):
     deg = np.minimum(rng.zipf(1.9, 30_000), 3000)
     deg = np.concatenate([deg, np.full(8000, 90), [5000, 513, 512]])
     _check_spmm(deg, k, torch.float32, 0.5)
+
+
+# Items that one round of a shape with fewer vectors per lane takes, and ones of several rows: (bytes of a row) / 16 from
+# 11 to 64, both sides of 17, 25, 33 and 49.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("nvec", [11, 16, 17, 24, 25, 32, 33, 48, 49, 64])
+def test_spmm_one_round(dtype, nvec):
+    k = nvec * 16 // (4 if dtype == torch.float32 else 8)
+    rows = 4375 if nvec <= 32 else 2500
+    _check_spmm([16] * rows, k, dtype, 0.5 if nvec % 2 else 0.0, bound_call=True)
+    _check_spmm([4] * rows, k, dtype, 0.0, bound_call=True, item_nnz=4)
+    _check_spmm([16] * rows, k, dtype, 0.5)
+    _check_spmm([16] * 3000, k, dtype, 0.0)
+    _check_spmm([6, 7] * 900, k, dtype, 0.5, bound_call=True)
+    _check_spmm([16] * 4000 + [90], k, dtype, 0.0, bound_call=True)    # one split row
+
+
+@pytest.mark.parametrize("k", [8, 20, 64, 96, 128, 256])
+def test_spmm_longest_items(k):
+    """Items of 256 nonzeros, which matrices of more than six million take: one row, 32 short ones, and pieces of 512."""
+    _check_spmm([8] * 70 + [300, 1, 511] + [0] * 40 + [513, 1400] + [37] * 20, k, torch.float32, 0.5, item_nnz=256, long_row=512)
+    _check_spmm([256] * 9 + [255, 257, 1] * 3, k, torch.float64, 0.0, item_nnz=256, long_row=512)
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
