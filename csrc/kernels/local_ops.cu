@@ -18,7 +18,7 @@ namespace sp3 {
 
 // ---------------------------------------------------------------------------
 // SDDMM: out[i] = sval[i] * <A[rowidx[i]], B[colidx[i]]>; persistent grid,
-// warps stride over windows of nonzeros (see sddmm_windows).
+// warps stride over windows of nonzeros (see sddmm_windows), or take one each.
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
 __global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
@@ -32,6 +32,19 @@ sddmm_vec_kernel(long long nnz, int wn, const int* rowidx, const int* colidx,
     sddmm_windows<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
                                                       arows, B, ldb_bytes, nvec, aligned, store, lists[threadIdx.x >> 5],
                                                       threadIdx.x & 31);
+}
+
+// One window per warp (see sddmm_window).
+template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
+sddmm_once_kernel(long long nnz, int wn, const int* rowidx, const int* colidx, const Rows arows, const char* B,
+                  unsigned ldb_bytes, int nvec, bool aligned, const Store store) {
+    after_previous_kernel();
+    __shared__ int4 cols[256 / 32][WINDOW_MAX / 4], rows[256 / 32][WINDOW_MAX / 4];
+    const int warp = threadIdx.x >> 5;
+    sddmm_window<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>((long long)blockIdx.x * (256 / 32) + warp, wn, nnz, rowidx, colidx,
+                                                                      arows, B, ldb_bytes, nvec, aligned, store, cols[warp],
+                                                                      rows[warp], threadIdx.x & 31);
 }
 
 // out[i] = sval[i] * dots[where[i]], four values per thread: dot products computed chunk by chunk of columns, back into
@@ -353,6 +366,10 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
         if (all == 0) return (int)cudaErrorInvalidConfiguration;                                              \
         const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
+        if constexpr (!passes_by<Rows>::value)   /* (lists by chunk are of a million nonzeros and more) */    \
+            if (needed <= all)                                                                                \
+                kernel = exact ? sddmm_once_kernel<T, NB, GG, RR, NB == 16, Rows, Store>                      \
+                               : sddmm_once_kernel<T, NB, GG, RR, false, Rows, Store>;                        \
         launch_early(kernel, needed < all ? (unsigned)needed : all, 0, st, nnz, wn, ri, ci, arows, B,               \
                      (unsigned)ldb_bytes, nvec, aligned, store);                                              \
     }

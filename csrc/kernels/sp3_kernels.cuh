@@ -164,7 +164,6 @@ __device__ __forceinline__ void after_previous_kernel() {
 struct RowsByStride {
     const char* base;
     unsigned ld_bytes;
-    __device__ __forceinline__ int ref(int row) const { return row; }
     __device__ __forceinline__ const char* resolve(int r) const { return base + (u64)(unsigned)r * ld_bytes; }
 };
 // The same for lists sorted by chunk of columns: what is read once per chunk (A rows, indices) leaves the L2 first, so
@@ -201,7 +200,8 @@ struct RowsByPeerRef {
 };
 
 // Where values go: `put4(i, n, dots)` stores min(n, 4) values from nonzero i on (i a multiple of 4), dot products times
-// values.  Quads are written as vectors where the places of all quads are 16-byte aligned (`vectors`).
+// values.  Quads are written as vectors where the places of all quads are 16-byte aligned (`vectors`).  `scale(i)` is the
+// value of nonzero i, `put(i, v)` stores one that is scaled.
 template <typename T> __device__ __forceinline__ void quad_store(T* p, const Quad<T>& q, int n, bool vectors) {
     if (vectors && n >= 4) {
         using V = typename Vec<T>::type;
@@ -229,6 +229,8 @@ template <typename T> struct StoreLocal {
     __device__ __forceinline__ void put4(long long i, int n, const T* dots) const {
         quad_store(out + i, scaled(i, n, dots), n, vectors);
     }
+    __device__ __forceinline__ T scale(long long i) const { return sval ? sval[i] : (T)1; }
+    __device__ __forceinline__ void put(long long i, T v) const { out[i] = v; }
 };
 template <typename T> struct StoreTwice : StoreLocal<T> {
     T* also;          // a second place for the values (a form of its own: the choice in the kernel cost 1 %)
@@ -237,6 +239,7 @@ template <typename T> struct StoreTwice : StoreLocal<T> {
         quad_store(this->out + i, q, n, this->vectors);
         quad_store(also + i, q, n, this->vectors);
     }
+    __device__ __forceinline__ void put(long long i, T v) const { this->out[i] = v; also[i] = v; }
 };
 template <typename T> struct StoreScattered : StoreLocal<T> {
     const int* orig;  // result position of nonzero i
@@ -246,6 +249,7 @@ template <typename T> struct StoreScattered : StoreLocal<T> {
         for (int j = 0; j < 4; ++j)
             if (j < n) this->out[orig[i + j]] = q.v[j];
     }
+    __device__ __forceinline__ void put(long long i, T v) const { this->out[orig[i]] = v; }
 };
 
 // Sums four values per lane over a group of G lanes (4 <= G) with a halving butterfly: log2(G) + 1 shuffles
@@ -303,12 +307,63 @@ template <bool PASSING> __device__ __forceinline__ void copy_quad_async(int4* ds
     else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
+// A quad that ends in one row or has two or more, as the list of a window marks it: the row it ends in, negative where it
+// is not all of that row (a list sorted by row class by class may also leave and re-enter a row).
+__device__ __forceinline__ int quad_tag(const int4& r) {
+    return r.x == r.w && r.y == r.w && r.z == r.w ? r.w : r.w | (1 << 31);
+}
+// Products of the rows in `b` with row `cur` in `a` and the row the quad ends in, in `a2` unless that is `cur` and the
+// whole quad with it; afterwards the latter is `cur`.  `second(h)` brings the rows of the second half where only half a
+// quad is in flight, `rows()` the quad's row indices, `fetch_a(row)` a row to `a`.
+template <typename T, int NB, int R, int U, bool EXACT, typename Rows, typename Second, typename FetchA>
+__device__ __forceinline__ void quad_products(T (&d)[4], Row<T, NB> (&a)[R], Row<T, NB> (&a2)[R], Row<T, NB> (&b)[U][R],
+                                              const bool (&on)[R], int& cur, int next, Rows&& rows, Second&& second,
+                                              FetchA&& fetch_a) {
+    constexpr unsigned FULL = 0xffffffffu;
+    if (__all_sync(FULL, next >= 0)) {      // every group: four nonzeros of one row
+        if (next != cur) {
+            cur = next;
+#pragma unroll
+            for (int q = 0; q < R; ++q) a[q] = a2[q];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h += U) {
+            second(h);
+#pragma unroll
+            for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
+        }
+    } else {
+        // where a row ends in a quad, both of its rows are here as a rule: both products, and the one that counts
+        const int4 rq = rows();
+        const int r[4] = {rq.x, rq.y, rq.z, rq.w};
+        const bool here = (r[0] == cur || r[0] == r[3]) && (r[1] == cur || r[1] == r[3]) && (r[2] == cur || r[2] == r[3]);
+        const bool both = __all_sync(FULL, here);
+#pragma unroll
+        for (int h = 0; h < 4; h += U) {
+            second(h);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!both && r[h + u] != cur && r[h + u] != r[3]) {
+                    cur = r[h + u];
+                    fetch_a(cur);
+                }
+                const T d1 = row_dot<EXACT>(a, b[u], on), d2 = row_dot<EXACT>(a2, b[u], on);
+                d[h + u] = r[h + u] == r[3] ? d2 : d1;
+            }
+        }
+        cur = r[3];
+#pragma unroll
+        for (int q = 0; q < R; ++q) a[q] = a2[q];
+    }
+}
+
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename ARows, typename Store>
 __device__ __forceinline__ void sddmm_windows(long long first, long long step, long long end, int wn, long long nnz,
                                               const int* rowidx, const int* colidx,
                                               const ARows& arows, const char* B, unsigned ldb_bytes,
                                               int nvec, bool aligned, const Store& store, WindowLists<T>& lists, int lane) {
     static_assert(G >= 4, "a group reduces four values");
+    static_assert(std::is_base_of<RowsByStride, ARows>::value, "row indices are used as they are");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int SLOTS = 32 / G;
     const int slot = lane / G, gl = lane % G;
@@ -357,10 +412,7 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
     auto enter = [&]() {                        // window w, whose indices are on their way to the other buffer
         asm volatile("cp.async.wait_all;" ::: "memory");
         k ^= 1;
-        const int4 r = lists.rows[k][lane];
-        // the row in which the lane's quad ends, negative: the quad is not all of that row (a list sorted by row class
-        // by class may also leave and re-enter a row)
-        tag = r.x == r.w && r.y == r.w && r.z == r.w ? r.w : r.w | (1 << 31);
+        tag = quad_tag(lists.rows[k][lane]);
         __syncwarp();
         if (w + step < end) stage(w + step, k ^ 1);
         src = slot;
@@ -391,41 +443,8 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
             }
         };
         T d[4];
-        if (__all_sync(FULL, next >= 0)) {      // every group: four nonzeros of one row
-            if (next != cur) {
-                cur = next;
-#pragma unroll
-                for (int q = 0; q < R; ++q) a[q] = a2[q];
-            }
-#pragma unroll
-            for (int h = 0; h < 4; h += U) {
-                second(h);
-#pragma unroll
-                for (int u = 0; u < U; ++u) d[h + u] = row_dot<EXACT>(a, b[u], on);
-            }
-        } else {
-            // where a row ends in a quad, both of its rows are here as a rule: both products, and the one that counts
-            const int4 rq = lists.rows[k][src];
-            const int r[4] = {rq.x, rq.y, rq.z, rq.w};
-            const bool here = (r[0] == cur || r[0] == r[3]) && (r[1] == cur || r[1] == r[3]) && (r[2] == cur || r[2] == r[3]);
-            const bool both = __all_sync(FULL, here);
-#pragma unroll
-            for (int h = 0; h < 4; h += U) {
-                second(h);
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (!both && r[h + u] != cur && r[h + u] != r[3]) {
-                        cur = r[h + u];
-                        fetch_a(a, arows.resolve(cur) + off[0]);
-                    }
-                    const T d1 = row_dot<EXACT>(a, b[u], on), d2 = row_dot<EXACT>(a2, b[u], on);
-                    d[h + u] = r[h + u] == r[3] ? d2 : d1;
-                }
-            }
-            cur = r[3];
-#pragma unroll
-            for (int q = 0; q < R; ++q) a[q] = a2[q];
-        }
+        quad_products<T, NB, R, U, EXACT>(d, a, a2, b, on, cur, next, [&] { return lists.rows[k][src]; }, second,
+                                          [&](int row) { fetch_a(a, arows.resolve(row) + off[0]); });
         // the next quad travels while this one is reduced and stored (behind the last one: that one again)
         T* const place = lists.dots + 4 * src + gl / (G / 4);
         const bool last = src + SLOTS >= quads;
@@ -446,6 +465,93 @@ __device__ __forceinline__ void sddmm_windows(long long first, long long step, l
             if (j < n) store.put4(at + j, n - j, lists.dots + j);
             __syncwarp();
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same for matrices with no more windows than warps: window w, one per warp.  Nothing but the trips to memory one after
+// the other counts there, and there are three: the lists, the rows with the values, the store.  So the lists come by
+// ordinary loads and pass through shared memory without a second buffer, the values travel with the rows, every value is
+// stored when it is there, and nothing is requested behind the last quad.  5 to 400 thousand nonzeros, k = 16 to 256,
+// back to back: 27 % less time than sddmm_windows (10 thousand of 4 a row, k = 64: 2.5 against 3.7 us; 200 thousand of 6 a
+// row, k = 32: 3.9 against 5.5).  Two windows per warp and more are faster there (600 thousand nonzeros of 6 a row, k = 50:
+// 17.4 us, 18.8 with this).
+//
+// A group takes every SLOTS-th quad where rows are long, so that all groups are in the same row, and its share in one piece
+// where a quarter of the quads or more end a row (rows of 6: 5.2 against 4.7 us).
+// ---------------------------------------------------------------------------
+template <typename T, int NB, int G, int R, int U, bool EXACT, typename Store>
+__device__ __forceinline__ void sddmm_window(long long w, int wn, long long nnz, const int* rowidx, const int* colidx,
+                                             const RowsByStride& arows, const char* B, unsigned ldb_bytes, int nvec,
+                                             bool aligned, const Store& store, int4 (&cols)[WINDOW_MAX / 4],
+                                             int4 (&rows)[WINDOW_MAX / 4], int lane) {
+    static_assert(G >= 4, "a group reduces four values");
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int SLOTS = 32 / G;
+    const int slot = lane / G, gl = lane % G;
+    const long long w0 = w * wn;
+    if (w0 >= nnz) return;
+    const int n = (int)(nnz - w0 < wn ? nnz - w0 : (long long)wn);
+    unsigned off[R];
+    bool on[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and do not count
+        const int v = gl + q * G;
+        on[q] = EXACT || v < nvec;
+        off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
+    }
+    B += off[0];
+    auto fetch = [&](Row<T, NB> (&a)[R], const char* p) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) row_load(a[q], p + (off[q] - off[0]));
+    };
+    int tag;
+    {
+        const int i = 4 * lane < n ? 4 * lane : (n - 1) & ~3;   // (behind the last quad: that quad again)
+        const Quad<int> c = quad_load(colidx + w0, i, n, aligned), r = quad_load(rowidx + w0, i, n, aligned);
+        cols[lane] = make_int4(c.v[0], c.v[1], c.v[2], c.v[3]);
+        rows[lane] = make_int4(r.v[0], r.v[1], r.v[2], r.v[3]);
+        tag = quad_tag(rows[lane]);
+        __syncwarp();
+    }
+    const int quads = (n + 3) >> 2, each = (quads + SLOTS - 1) / SLOTS;
+    const bool apart = 4 * __popc(__ballot_sync(FULL, tag < 0 && lane < quads)) >= quads;
+    int src = apart ? slot * each : slot;       // quad of this group
+    const int inc = apart ? 1 : SLOTS;
+    const int mine = gl / (G / 4);              // which of the four results ends up in this lane
+    const bool writer = gl % (G / 4) == 0;
+    int cur = -1, next = -1;                    // row in `a`; tag of the quad in flight
+    T s_next = 1;
+    Row<T, NB> a[R], a2[R], b[U][R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) { row_zero(a[q]); row_zero(a2[q]); }
+    auto fetch_b = [&](int h) {                 // the rows of nonzeros h .. h + U - 1 of quad src
+        const int4 c = cols[src];
+        const int cs[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int u = 0; u < U; ++u) fetch(b[u], B + (u64)(unsigned)cs[(h + u) & 3] * ldb_bytes);
+    };
+    auto request = [&]() {                      // as in sddmm_windows, and the value that this lane will scale
+        fetch_b(0);
+        next = __shfl_sync(FULL, tag, src);
+        if (__any_sync(FULL, next != cur)) fetch(a2, arows.resolve(next & 0x7fffffff) + off[0]);
+        const int pos = 4 * src + mine;
+        s_next = store.scale(w0 + (pos < n ? pos : n - 1));
+    };
+    request();
+    for (int left = each - 1; left >= 0; --left) {
+        const int pos = 4 * src + mine;
+        const T s = s_next;
+        T d[4];
+        quad_products<T, NB, R, U, EXACT>(d, a, a2, b, on, cur, next, [&] { return rows[src]; },
+                                          [&](int h) { if (h > 0) fetch_b(h); },
+                                          [&](int row) { fetch(a, arows.resolve(row) + off[0]); });
+        if (left > 0) {
+            src += inc;
+            request();
+        }
+        const T total = group_sum4<T, G>(d, gl);
+        if (writer && pos < n) store.put(w0 + pos, total * s);
     }
 }
 

@@ -66,6 +66,49 @@ def test_sddmm_list_ends(k, nnz):
     _check_sddmm(np.sort(rng.integers(0, 40, nnz)), rng.integers(0, 50, nnz), k, torch.float32)
 
 
+def _check_sddmm_places(nnz, k, dtype, place, lists=0, twice=False, runs=(1, 2, 3, 5, 6, 90)):
+    """SDDMM whose values, results and second results start `place` elements behind a 16-byte boundary, the index lists
+    `lists` elements."""
+    from spcomm3d_b200.ops import cuda_ops
+    rng = np.random.default_rng(nnz)
+    deg = rng.choice(runs, nnz)
+    r = torch.from_numpy(np.repeat(np.arange(deg.size), deg)[:nnz] % 40).int()
+    c = torch.from_numpy(rng.integers(0, 50, nnz)).int()
+    g = torch.Generator().manual_seed(k)
+    A, B = _strided(40, k, k, dtype, g), _strided(50, k, k, dtype, g)
+    s = torch.rand(nnz, generator=g, dtype=torch.float64).to(dtype)
+    at = r.long() * 50 + c.long()
+    ref = (A.double() @ B.double().T).reshape(-1)[at] * s.double()
+    mag = (A.double().abs() @ B.double().abs().T).reshape(-1)[at] * s.double()
+    bufs = [torch.full((nnz + 8,), float("nan"), dtype=dtype, device="cuda") for _ in range(2)]
+    out, also = (b[place:place + nnz] for b in bufs)
+    cuda_ops.bind_sddmm(_on_gpu(r, lists), _on_gpu(c, lists), _on_gpu(s, place), A.cuda(), B.cuda(), out,
+                        also if twice else None, pack=False).launch()
+    for b in bufs[:1 + twice]:
+        got = b.cpu().double()
+        assert bool(((got[place:place + nnz] - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+        assert bool(got[:place].isnan().all()) and bool(got[place + nnz:].isnan().all())   # nothing else is written
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [4, 16, 20, 32, 44, 64, 100, 128, 200, 256, 400, 600])   # every lanes-per-row shape
+def test_sddmm_many_windows(dtype, k):
+    """More windows than warps (606,208 nonzeros where a lane holds one vector), the last one short, and the lists,
+    values and results at places that take no vectors."""
+    _check_sddmm_places(650_003, k, dtype, 0)
+    _check_sddmm_places(650_002, k, dtype, 1, lists=1, twice=True)
+    _check_sddmm_places(650_001, k, dtype, 0, runs=(1,))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [4, 33, 50, 64, 128])
+@pytest.mark.parametrize("nnz", [1, 5, 130, 4097, 100_001, 420_001])
+def test_sddmm_places(dtype, k, nnz):
+    """One window per warp, and two or three (420,001 where a lane holds several vectors)."""
+    for place, twice in ((0, True), (1, False), (2, True), (3, True)):
+        _check_sddmm_places(nnz, k, dtype, place, lists=place, twice=twice)
+
+
 @pytest.mark.parametrize("k", [32, 64, 128])
 @pytest.mark.parametrize("nnz", [200, 700_000])   # 700,000: full windows of 128 nonzeros
 def test_sddmm_row_changes(k, nnz):
