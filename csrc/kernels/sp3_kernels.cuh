@@ -1,13 +1,14 @@
 // Warp-level bodies of the SDDMM and SpMM kernels, shared by the local
 // kernels (local_ops.cu) and the fused compute+communication kernels
 // (fused_impl.cuh).  Where dense rows come from and where results go is a
-// template policy, so both families run the same inner loops:
+// template policy:
 //
-//   SDDMM   A rows:  RowsByStride (one local block) | RowsByPeerRef (rows that
-//                    stay in their owners' memory, local or peer)
+//   SDDMM   A rows:  RowsByStride (one local block) here, RowsByPeerRef (rows
+//                    that stay in their owners' memory, local or peer) in the
+//                    fused kernel, which has a loop of its own (sddmm_units)
 //           output:  StoreLocal | the fused kernel's slice-routing store
 //   SpMM    emit:    EmitLocal (Y = beta*Y + acc) | the fused kernel's
-//                    owned-or-push emit
+//                    owned-or-push emit; one loop for both families
 //
 // Layout of the math: a dense row is cut into vectors of NB bytes (16, 8 or 4:
 // the widest that the width and the alignment of the operands allow); a group
@@ -155,12 +156,10 @@ __device__ __forceinline__ void after_previous_kernel() {
 }
 
 // ---- row access policies ---------------------------------------------------
-// A policy turns the local row index of a nonzero into a 31-bit *reference*
-// (`ref`, evaluated by every lane for its own nonzeros when a window of indices
-// is read, so a table lookup is off the critical path) and a reference into
-// the address of the dense row (`resolve`, pure arithmetic).  The reference is
-// what the lane group passes round by shuffle and compares to detect a row
-// change.
+// `resolve` turns a 31-bit *reference* to a row into its address (pure arithmetic); references are what a loop compares
+// to detect a row change.  In one local block they are the row indices.  Rows at their owners have a table of them, which
+// `ref` reads, by every lane for its own nonzeros when a window of indices is read, so that the lookup is off the
+// critical path.
 struct RowsByStride {
     const char* base;
     unsigned ld_bytes;
@@ -654,8 +653,8 @@ using ItemSmem = ItemScratch<R, Row<T, NB>::N, typename Row<T, NB>::E, (32 / G >
 // Bound by the latency of the row gathers: a warp that adds up, or ends a row, has none in flight, and a quad waits for
 // the slowest of its rows.  So what lies between two quads is kept short -- one comparison tells whether a quad ends a
 // row, the rows that hold nonzeros are listed once per item, empty rows are written apart from them -- and what is not
-// needed in every quad (where rows end, the part of a group's first row) stays in shared memory, which makes room for
-// 40 warps per SM instead of 32 where a lane holds one vector per row.
+// needed in every quad (where rows end, the part of a group's first row) stays in shared memory, so that the loop spills
+// little or nothing within the registers of 32 (one vector per row and lane), 24 or 16 warps per SM.
 template <typename T, int NB, int G, int R, int U, bool EXACT, typename Emit>
 __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long* rowptr, long long nnz,
                                                const int* colidx, const T* val,

@@ -15,25 +15,26 @@ from ..utils import native
 
 _F = {torch.float32: "f32", torch.float64: "f64"}
 
-# SpMM schedule parameters: rows with more than LONG_ROW nonzeros are cut into
-# pieces of LONG_ROW; other rows are grouped into items of about ITEM_NNZ
-# nonzeros and at most ITEM_ROWS rows (SPMM_ITEM_ROWS of csrc/kernels/sp3_kernels.cuh; SP3_ITEM_ROWS asks for fewer).
+# SpMM schedule parameters of a block with enough work for every warp (`item_sizes` has the smaller and the largest
+# ones): rows with more than LONG_ROW nonzeros are cut into pieces of LONG_ROW; other rows are grouped into items of about
+# ITEM_NNZ nonzeros and at most ITEM_ROWS rows (SPMM_ITEM_ROWS of csrc/kernels/sp3_kernels.cuh; SP3_ITEM_ROWS asks for fewer).
 LONG_ROW, ITEM_NNZ, ITEM_ROWS = 512, 128, 32
 _TARGET_ITEMS = 148 * 32   # warps that a B200 runs at once
 
 
 def item_sizes(nnz: int):
     """(long_row, item_nnz) of a block of `nnz` nonzeros: LONG_ROW and ITEM_NNZ once there is enough work for every
-    warp, smaller powers of two (down to 16 nonzeros) below that, because the time of a small SpMM is that of its
-    longest item: each group of four nonzeros costs one trip to memory.  SP3_LONG_ROW / SP3_ITEM_NNZ override."""
+    warp, twice the items once there is for five of them per warp, and smaller powers of two (down to 16 nonzeros) below,
+    because the time of a small SpMM is that of its longest item: each group of four nonzeros costs one trip to memory.
+    SP3_LONG_ROW / SP3_ITEM_NNZ override."""
     # twice as many where that still leaves every warp five of them (R-MAT scale 20, k = 64: 322 us instead of 331;
     # Erdos-Renyi, 7.2 M nonzeros, k = 32: 95 instead of 100; Zipf rows, 5.7 M, k = 128: 465 instead of 456)
     item = ITEM_NNZ if nnz < 2 * ITEM_NNZ * _TARGET_ITEMS * 5 else 2 * ITEM_NNZ
     while item > 16 and nnz < item * _TARGET_ITEMS * 3 // 4:
         item //= 2
-    # a piece costs a partial row and a fence beyond its nonzeros: four items long where that has to be cheap, two
-    # where the longest chain decides (Zipf rows, 357 thousand nonzeros, k = 64: 16.5 us with pieces of 128, 20.2
-    # with 256, 20.1 with 64)
+    # a piece costs a partial row and a fence beyond its nonzeros: LONG_ROW, two or four items, where that has to be cheap,
+    # two items where the longest chain decides (Zipf rows, 357 thousand nonzeros, k = 64: 16.5 us with pieces of 128,
+    # 20.2 with 256, 20.1 with 64)
     long_row = LONG_ROW if item >= ITEM_NNZ else 2 * item
     return int(os.environ.get("SP3_LONG_ROW", long_row)), int(os.environ.get("SP3_ITEM_NNZ", item))
 
