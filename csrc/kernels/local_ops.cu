@@ -364,7 +364,7 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
                             : sddmm_vec_kernel<T, NB, GG, RR, false, Rows, Store>;                                  \
         const unsigned all = resident_blocks(kernel, cache, 0);                                               \
         if (all == 0) return (int)cudaErrorInvalidConfiguration;                                              \
-        const int wn = window_nnz(nnz, (long long)all * 8, 32 / GG);                                          \
+        const int wn = balanced_window_nnz(nnz, (long long)all * 8, 32 / GG);                                 \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
         if constexpr (!passes_by<Rows>::value)   /* (lists by chunk are of a million nonzeros and more) */    \
             if (needed <= all)                                                                                \

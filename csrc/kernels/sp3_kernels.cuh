@@ -300,6 +300,15 @@ __host__ __device__ inline int window_nnz(long long nnz, long long nwarps, int g
     return (int)(w < quantum ? quantum : (w > WINDOW_MAX ? WINDOW_MAX : w));
 }
 
+// The same, and equal rounds where the warps take up to four windows each: with windows of 128 the last round may find work
+// for a fifth of them (Zipf rows, 357 thousand nonzeros, fp64, k = 32: 2790 windows on 2368 warps 14.3 us, as two rounds
+// of 80 nonzeros 11.2; k = 128, fp32 23.5 and 18.7).  Four rounds and more are level or lose to the longer windows (R-MAT
+// scale 17, k = 192, seven rounds: 113 us with windows of 120, 104 with 128).
+inline int balanced_window_nnz(long long nnz, long long nwarps, int groups_per_warp) {
+    const long long rounds = (nnz - 1) / (nwarps * WINDOW_MAX) + 1;
+    return window_nnz(nnz, rounds <= 4 ? rounds * nwarps : nwarps, groups_per_warp);
+}
+
 template <bool PASSING> __device__ __forceinline__ void copy_quad_async(int4* dst, const int* src, u64 policy) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     if constexpr (PASSING) asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "l"(policy) : "memory");
