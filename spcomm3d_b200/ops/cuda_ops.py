@@ -27,8 +27,9 @@ def item_sizes(nnz: int):
     warp, twice the items once there is for five of them per warp, and smaller powers of two (down to 16 nonzeros) below,
     because the time of a small SpMM is that of its longest item: each group of four nonzeros costs one trip to memory.
     SP3_LONG_ROW / SP3_ITEM_NNZ override."""
-    # twice as many where that still leaves every warp five of them (R-MAT scale 20, k = 64: 322 us instead of 331;
-    # Erdos-Renyi, 7.2 M nonzeros, k = 32: 95 instead of 100; Zipf rows, 5.7 M, k = 128: 465 instead of 456)
+    # twice as many where that still leaves every warp five of them (k = 64, 128 -> 256 nonzeros an item, us: R-MAT 16.1 M
+    # nonzeros 331 -> 322, 5.8 M 110 -> 109, 4.2 M 86.3 -> 86.9; Zipf rows 6.8 M 208 -> 206, 4.1 M 125 -> 124; rows of 9,
+    # 5.4 M 183 -> 186; Erdos-Renyi 6.7 M 155 -> 142, 4.8 M 101 -> 94; k = 128: 0 to 3 % either way)
     item = ITEM_NNZ if nnz < 2 * ITEM_NNZ * _TARGET_ITEMS * 5 else 2 * ITEM_NNZ
     while item > 16 and nnz < item * _TARGET_ITEMS * 3 // 4:
         item //= 2
