@@ -356,9 +356,9 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
     int G, R;
     pick_shape(nvec, &G, &R, false);
     const bool exact = NB == 16 && nvec == G * R;
-    // One window per warp, but for three vectors of 4 bytes per lane (odd rows of 33 to 96 values) with windows of more than
-    // 16 nonzeros: Zipf rows, 107 thousand nonzeros, k = 47, 6.8 us with sddmm_windows, 7.4 with sddmm_window; R-MAT scale
-    // 14, k = 75, 16.4 and 19.2; with windows of 16 4.0 and 2.9 (R-MAT scale 11, k = 47).
+    // One window per warp, but for three narrow vectors of fp32 per lane (odd rows of 33 to 96 values, others of 66 to 190)
+    // with windows of more than 16 nonzeros: Zipf rows, 107 thousand nonzeros, k = 47, 6.8 us with sddmm_windows, 7.4 with sddmm_window; R-MAT scale
+    // 14, k = 75, 16.4 and 19.2, k = 90 13.3 and 15.5; with windows of 16 4.0 and 2.9 (R-MAT scale 11, k = 47).
 #define SP3_SDDMM(GG, RR)                                                                                     \
     {                                                                                                         \
         static ResidentCache caches[2];                                                                       \
@@ -370,7 +370,7 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
         const int wn = balanced_window_nnz(nnz, (long long)all * 8, 32 / GG);                                 \
         const long long needed = ((nnz + wn - 1) / wn + 7) / 8;                                               \
         if constexpr (!passes_by<Rows>::value)   /* (lists by chunk are of a million nonzeros and more) */    \
-            if (needed <= all && !(NB == 4 && RR == 3 && wn > 16))                                            \
+            if (needed <= all && !(NB < 16 && sizeof(T) == 4 && RR == 3 && wn > 16))                          \
                 kernel = exact ? sddmm_once_kernel<T, NB, GG, RR, NB == 16, Rows, Store>                      \
                                : sddmm_once_kernel<T, NB, GG, RR, false, Rows, Store>;                        \
         launch_early(kernel, needed < all ? (unsigned)needed : all, 0, st, nnz, wn, ri, ci, arows, B,               \
