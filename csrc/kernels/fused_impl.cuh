@@ -471,6 +471,40 @@ struct PullGate {
     }
 };
 
+// Receive lists that one round of loads covers (see `small_pull`): every warp copies the tickets that are dealt to it in
+// advance, each block counts once when all its copies are written, and goes on when all blocks have.  Every thread calls
+// it; every row is in the local block when it returns true.
+//
+// Bound by trips to memory one after the other (address, row, store, count), so nothing is drawn from a counter and nothing
+// is published ticket by ticket.  Eight ranks of R-MAT scale 16, k / Z = 64 (3.4 MB in 832 tickets per rank and SDDMM): the
+// last row is there 7 us after the start of MAIN, with tickets, four waves and one poll for each 14 to 17 us.
+__device__ __forceinline__ bool pull_fixed(const FusedComm& c, const PullConfig& pc, const PullSide& first,
+                                           const PullSide& second, long long ld_v, int nvec, int nwarps, int lane) {
+    const int n_first = pull_tickets(pc, first.n_rows), n_pull = n_first + pull_tickets(pc, second.n_rows);
+    if (n_pull == 0) return true;
+    for (int t = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); t < n_pull; t += nwarps) {
+        const PullSide& sd = t < n_first ? first : second;
+        int r0, r1;
+        pull_range(pc, t < n_first ? t : t - n_first, sd.n_rows, r0, r1);
+        if (r0 < r1) pull_rows(r0, r1, sd.src, sd.dst, ld_v, nvec, lane);
+    }
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();   // behind the barrier: for what the other warps of the block wrote, too
+        if (atomicAdd(c.ctrl + C_PULLS_DONE, 1) == (int)gridDim.x - 1) stamp(c, T_PULLED);
+        ok = poll_counter(c, C_PULLS_DONE, (int)gridDim.x, W_PULLS);
+    }
+    return __syncthreads_and(ok);
+}
+// Whether the rows to pull are so few that they are there before computing ahead of them would pay: vector loads (the
+// host's choice below 4 MB, see `_pull_config` in ops/fused.py) of at most that many bytes.  SDDMM and SpMM of all ranks on
+// one GPU, waves / everything first, us: 2x2x2, R-MAT scale 16, k = 128 (3.4 and 1.7 MB) 948 / 767.
+constexpr long long SMALL_PULL_BYTES = 4ll << 20;
+inline bool small_pull(const PullConfig& pc, long long n_rows, int nvec) {
+    return n_rows == 0 || (pc.pullers == 0 && n_rows * nvec * 16 <= SMALL_PULL_BYTES);
+}
+
 // The control words are zero between launches: the last warp to be done with a launch clears them (a memset before
 // every launch cost 1 us of stream time and a second launch).
 __device__ __forceinline__ void clear_ctrl(const FusedComm& c, int lane) {
@@ -742,8 +776,72 @@ __device__ __forceinline__ void sddmm_units(long long first, long long step, lon
     }
 }
 
+// Pushes the values [i0, i1) of `part`, which this warp wrote just now (still in the L2): the pieces that belong to other
+// fiber ranks travel as contiguous remote stores while other warps compute.
+__device__ __forceinline__ void push_values(const FusedSddmmArgs& a, int parity, long long i0, long long i1, int lane) {
+    __syncwarp();
+    for (int z = 0; z < a.Z; ++z) {
+        if (z == a.my_z) continue;
+        const long long s0 = slice_off(z, a.zbase, a.zrem);
+        const long long s1 = s0 + a.zbase + ((unsigned)z < a.zrem ? 1 : 0);
+        const long long j0 = i0 > s0 ? i0 : s0, j1 = i1 < s1 ? i1 : s1;
+        if (j0 >= j1) continue;
+        real* dst = a.zbuf[z] + ((long long)parity * a.Z + a.my_z) * a.zwidth - s0;
+        for (long long j = j0 + lane; j < j1; j += 128) {
+            real v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = (j + 32 * q < j1) ? __ldcg(a.part + j + 32 * q) : (real)0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) if (j + 32 * q < j1) __stcs(dst + j + 32 * q, v[q]);
+        }
+    }
+}
+
+// MAIN of a rank that pulls nothing or little: all rows first, then the loops of the local kernels, which have the
+// registers here that the wave bookkeeping takes in the other form.
 template <int G, int R>
-__global__ void __launch_bounds__(256, sddmm_min_blocks(R, true)) fused_sddmm_kernel(const FusedSddmmArgs a) {
+__device__ __forceinline__ bool sddmm_after_pulls(const FusedSddmmArgs& a, int nwarps, int parity, WindowLists<real>& lists,
+                                                  int lane) {
+    const FusedComm& c = a.comm;
+    constexpr int SLOTS = 32 / G;
+    const long long ldb_v = a.ldb / VN;
+    vec* const Bv = reinterpret_cast<vec*>(a.B_loc);
+    bool ok = pull_fixed(c, a.pull, {a.a_src, reinterpret_cast<float4*>(a.A_stage), a.n_recv_a},
+                         {a.b_src, reinterpret_cast<float4*>(Bv + (long long)a.n_owned_b * ldb_v), a.n_recv_b}, ldb_v, a.nvec,
+                         nwarps, lane);
+    if (!ok) return false;
+    const int wn = window_nnz(a.nnz, nwarps, SLOTS);
+    const long long n_windows = (a.nnz + wn - 1) / wn;
+    const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const bool aligned = ((unsigned long long)a.rowidx | (unsigned long long)a.colidx) % 16 == 0;
+    const bool push = a.Z > 1 && a.direct_push == 2;
+    real* const dst = a.Z == 1 ? a.out : a.part + (a.direct_push == 3 ? (long long)parity * a.part_stride : 0);
+    const StoreLocal<real> store{dst, a.sval, ((unsigned long long)dst | (unsigned long long)a.sval) % 16 == 0};
+    RowsByStride arows;
+    arows.base = reinterpret_cast<const char*>(a.a_bases[c.me]);
+    arows.ld_bytes = (unsigned)a.nvec * 16u;
+    const char* B = reinterpret_cast<const char*>(Bv);
+    if (n_windows <= nwarps) {
+        sddmm_window<real, 16, G, R, sddmm_unroll(R, IS_F32), false>(gwarp, wn, a.nnz, a.rowidx, a.colidx, arows, B,
+                                                                     (unsigned)ldb_v * 16u, a.nvec, aligned, store,
+                                                                     lists.cols[0], lists.rows[0], lane);
+        if (push && gwarp < n_windows) push_values(a, parity, gwarp * wn, (gwarp + 1) * wn < a.nnz ? (gwarp + 1) * wn : a.nnz, lane);
+        return true;
+    }
+    // every warp has its first ticket, the others are drawn
+    const int per = per_ticket(n_windows, nwarps, SDDMM_WINDOWS_PER_TICKET_MAX);
+    for (long long w0 = gwarp * per; w0 < n_windows; w0 = (long long)nwarps * per + warp_ticket(c.ctrl + C_TICKET_WORK, lane, per)) {
+        const long long w1 = w0 + per < n_windows ? w0 + per : n_windows;
+        sddmm_windows<real, 16, G, R, sddmm_unroll(R, IS_F32), false>(w0, 1, w1, wn, a.nnz, a.rowidx, a.colidx, arows, B,
+                                                                      (unsigned)ldb_v * 16u, a.nvec, aligned, store, lists, lane);
+        if (push) push_values(a, parity, w0 * wn, w1 * wn < a.nnz ? w1 * wn : a.nnz, lane);
+    }
+    return true;
+}
+
+// GATED: the work follows the pull waves.  The other form pulls everything first (`sddmm_after_pulls`).
+template <int G, int R, bool GATED>
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, GATED || IS_F32)) fused_sddmm_kernel(const FusedSddmmArgs a) {
     after_previous_kernel();
     const FusedComm& c = a.comm;
     const int lane = threadIdx.x & 31;
@@ -762,6 +860,10 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R, true)) fused_sddmm_ke
     if (c.phases & PH_MAIN) {
         if (!(c.phases & PH_START) && blockIdx.x == 0 && threadIdx.x == 0) stamp(c, T_START);
         bool ok = block_wait_all(c, F_READY, c.read_from, c.n_read, W_READY);
+        if constexpr (!GATED) {
+            __shared__ __align__(16) WindowLists<real> lists[256 / 32];
+            if (ok) sddmm_after_pulls<G, R>(a, nwarps, parity, lists[threadIdx.x >> 5], lane);
+        } else {
         constexpr int SLOTS = 32 / G;
         // pull tickets: tiles of needed A rows first (when A rows are staged), then tiles of needed B rows
         const int n_pull_a = pull_tickets(a.pull, a.n_recv_a);
@@ -823,27 +925,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R, true)) fused_sddmm_ke
             sddmm_units<real, 16, G, R, sddmm_unroll(R, true), false>(
                 u0, 1, u1, per_unit, a.nnz, a.rowidx, a.colidx, arows, reinterpret_cast<const char*>(Bv),
                 (unsigned)ldb_v * 16u, a.nvec, aligned, store, lane);
-            if (self_push) {
-                // the values [i0, i1) of `part` were written by this warp just now (still in L2): send the pieces
-                // that belong to other fiber ranks as contiguous remote stores while other warps compute
-                __syncwarp();
-                const long long i0 = u0 * per_unit, i1 = u1 * per_unit < a.nnz ? u1 * per_unit : a.nnz;
-                for (int z = 0; z < a.Z; ++z) {
-                    if (z == a.my_z) continue;
-                    const long long s0 = slice_off(z, a.zbase, a.zrem);
-                    const long long s1 = s0 + a.zbase + ((unsigned)z < a.zrem ? 1 : 0);
-                    const long long j0 = i0 > s0 ? i0 : s0, j1 = i1 < s1 ? i1 : s1;
-                    if (j0 >= j1) continue;
-                    real* dst = a.zbuf[z] + ((long long)parity * a.Z + a.my_z) * a.zwidth - s0;
-                    for (long long j = j0 + lane; j < j1; j += 128) {
-                        real v[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) v[q] = (j + 32 * q < j1) ? __ldcg(a.part + j + 32 * q) : (real)0;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) if (j + 32 * q < j1) __stcs(dst + j + 32 * q, v[q]);
-                    }
-                }
-            }
+            if (self_push) push_values(a, parity, u0 * per_unit, u1 * per_unit < a.nnz ? u1 * per_unit : a.nnz, lane);
         }
         if (ok) gate.pull_all(lane);  // no compute left but tiles remain (tiny blocks)
         if (a.Z > 1 && !direct && !self_push && !in_switch) {
@@ -872,6 +954,7 @@ __global__ void __launch_bounds__(256, sddmm_min_blocks(R, true)) fused_sddmm_ke
                     for (int u = 0; u < 4; ++u) if (j + 32 * u < j1) __stcs(dst + j + 32 * u, v[u]);
                 }
             }
+        }
         }
         main_epilogue(c, lane);
     }
@@ -1091,6 +1174,7 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
         // atomic mode, START and MAIN in one launch: my own START warps scale (or clear) the rows that receive
         // contributions with plain stores; nobody may add into them, me included, before all of them are done
         if (ATOMIC && (c.phases & PH_START)) ok = wait_counter(c, C_START_DONE, nwarps, W_READY) && ok;
+        if (ATOMIC) ok = __syncthreads_and(ok);   // (what follows may have block barriers)
         const int n_pull = pull_tickets(a.pull, a.n_recv_x);
         vec* Xv = reinterpret_cast<vec*>(a.X_loc);
         const long long ldx_v = a.ldx / VN;
@@ -1102,28 +1186,30 @@ __global__ void __launch_bounds__(256, spmm_min_blocks(R)) fused_spmm_kernel(con
                                    parity ? a.parity_off_v : 0};
         if constexpr (!GATED) {
             // pull everything (bulk mode: the puller warps; else all warps), then compute
-            bool pulled = n_pull == 0;
             float4* xdst = reinterpret_cast<float4*>(Xv + (long long)a.n_owned_x * ldx_v);
-            while (ok && (!bulk || (int)(threadIdx.x >> 5) < a.pull.pullers) && !aborted(c)) {
-                const int t = warp_ticket(c.ctrl + C_TICKET_MAIN, lane);
-                if (t >= n_pull) break;
-                int r0, r1;
-                pull_range(a.pull, t, a.n_recv_x, r0, r1);
-                if (r0 >= r1) {}
-                else if (bulk) { if (!bulk_pull_tile(br, c, r0, r1, a.x_src, xdst, a.nvec, lane, true, [] {})) break; }
-                else pull_rows(r0, r1, a.x_src, xdst, ldx_v, a.nvec, lane);
-                __threadfence();
-                __syncwarp();
-                if (lane == 0 && atomicAdd(c.ctrl + C_PULLS_DONE, 1) == n_pull - 1) stamp(c, T_PULLED);
+            bool pulled = true;
+            if (!bulk) {
+                if (ok) ok = pull_fixed(c, a.pull, {a.x_src, xdst, a.n_recv_x}, {nullptr, nullptr, 0}, ldx_v, a.nvec, nwarps, lane);
+            } else if (n_pull > 0) {
+                pulled = false;
+                while (ok && (int)(threadIdx.x >> 5) < a.pull.pullers && !aborted(c)) {
+                    const int t = warp_ticket(c.ctrl + C_TICKET_MAIN, lane);
+                    if (t >= n_pull) break;
+                    int r0, r1;
+                    pull_range(a.pull, t, a.n_recv_x, r0, r1);
+                    if (r0 < r1 && !bulk_pull_tile(br, c, r0, r1, a.x_src, xdst, a.nvec, lane, true, [] {})) break;
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0 && atomicAdd(c.ctrl + C_PULLS_DONE, 1) == n_pull - 1) stamp(c, T_PULLED);
+                }
             }
             const int SPMM_ITEMS_PER_TICKET = per_ticket(a.nitems, nwarps, SPMM_ITEMS_PER_TICKET_MAX);
-            // few items, which are then short ones: dealt out in advance, without a counter to queue up on
-            const bool fixed = a.nitems <= SPMM_FIXED_ITEMS * nwarps;
-            int next_item = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-            while (ok) {
-                const int i0 = fixed ? next_item : warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET);
-                next_item += nwarps;
-                if (i0 >= a.nitems) break;
+            // every warp has its first items, the others are drawn (with all of them drawn, thousands of warps queue up on
+            // the counter at the start)
+            const int gwarp = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+            for (long long i = (long long)gwarp * SPMM_ITEMS_PER_TICKET; ok && i < a.nitems;
+                 i = (long long)nwarps * SPMM_ITEMS_PER_TICKET + warp_ticket(c.ctrl + C_TICKET_WORK, lane, SPMM_ITEMS_PER_TICKET)) {
+                const int i0 = (int)i;
                 if (!pulled) {
                     ok = wait_counter(c, C_PULLS_DONE, n_pull, W_PULLS);
                     pulled = true;
@@ -1314,9 +1400,14 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_sddmm_, SP3_FUSED_SUFFIX)(const void* args, 
     const long long units = (a.nnz + 4 * (32 / G) - 1) / (4 * (32 / G));
     const long long pulls = (long long)pull_tickets(a.pull, a.n_recv_a) + pull_tickets(a.pull, a.n_recv_b);
     const long long needed = blocks_needed(a.comm.phases, units > pulls ? units : pulls, fin, 1);
-#define SP3_FSDDMM(GG, RR) { static ResidentCache cache; rc = launch_resident(fused_sddmm_kernel<GG, RR>, cache, a, needed, st); }
+    // A rows in one local block, values to one local array in their order: what the loops of the local kernels can do
+    const bool gated = !small_pull(a.pull, (long long)a.n_recv_a + a.n_recv_b, a.nvec) || a.a_refs || a.orig ||
+                       (a.Z > 1 && a.direct_push != 2 && a.direct_push != 3);
+#define SP3_FSDDMM_ONE(GG, RR, GA) { static ResidentCache cache; rc = launch_resident(fused_sddmm_kernel<GG, RR, GA>, cache, a, needed, st); }
+#define SP3_FSDDMM(GG, RR) if (gated) SP3_FSDDMM_ONE(GG, RR, true) else SP3_FSDDMM_ONE(GG, RR, false)
     SP3_SDDMM_SHAPES(SP3_FSDDMM)
 #undef SP3_FSDDMM
+#undef SP3_FSDDMM_ONE
     return rc ? rc : (int)cudaGetLastError();
 }
 
@@ -1327,7 +1418,7 @@ SP3_API int SP3_FUSED_CAT(sp3_fused_spmm_, SP3_FUSED_SUFFIX)(const void* args, v
     int G, R, rc = 0;
     const long long x_rows = (long long)a.n_owned_x + a.n_recv_x;
     pick_shape(a.nvec, &G, &R, true, x_rows * a.nvec * 16 <= CACHED_BYTES);
-    const bool gated = a.wave_items != nullptr && a.n_waves > 0 && a.n_recv_x > 0;
+    const bool gated = a.wave_items != nullptr && a.n_waves > 0 && !small_pull(a.pull, a.n_recv_x, a.nvec);
     const long long rows = ((long long)a.n_crows * a.nvec + 31) / 32;
     const long long pulls = pull_tickets(a.pull, a.n_recv_x);
     const long long needed = blocks_needed(a.comm.phases, a.nitems > pulls ? a.nitems : pulls, a.atomic ? 1 : rows,

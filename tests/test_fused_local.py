@@ -345,3 +345,57 @@ def test_wait_runs_out_without_hanging():
         op._fused.check()
     x = torch.ones(8, device="cuda")
     assert float(x.sum()) == 8.0  # context still healthy
+
+
+# Small receive lists (pulled first, then the loops of the local kernels) against bulk copies with waves: one row, one
+# nonzero per rank and less, one window per warp and several, fp64, no pulls at all, partial values pushed along Z.
+@pytest.mark.parametrize("meshstr,gen,k,f64", [("2x2x1", "uniform:3:5:2", 4, False), ("2x2x2", "uniform:600:500:7", 50, False),
+                                               ("1x2x2", "uniform:60000:4096:24", 16, False), ("2x1x1", "rmat:16:16", 12, False),
+                                               ("1x1x2", "uniform:30000:3000:40", 8, False), ("2x2x2", "rmat:12:8", 66, True)])
+def test_small_pulls_against_waves(meshstr, gen, k, f64):
+    from spcomm3d_b200.models.dist_ops import DistSDDMM, DistSpMM
+    from spcomm3d_b200.ops.fused import FusedSDDMM, FusedSpMM, run_lockstep
+    from spcomm3d_b200.parallel.mesh import split_k
+    from spcomm3d_b200.parallel.symm import LocalFabric
+    mesh, m, plans, _, _ = _setup(meshstr, gen, k)
+    dt = torch.float64 if f64 else torch.float32
+    kl = [split_k(k, mesh.Z, plans[r].coords[2])[1] for r in range(mesh.size)]
+    got = {}
+    for bulk in (None, True):
+        fabric = LocalFabric(mesh.size)
+        for cls, F in ((DistSDDMM, FusedSDDMM), (DistSpMM, FusedSpMM)):
+            heaps = fabric.heaps([F.region_sizes(plans[r], kl[r], dtype=dt) for r in range(mesh.size)])
+            ops = [cls(plans[r], None, k, dt, "cuda", "fused", heap=heaps[r], timeout_s=2.0, bulk_pull=bulk)
+                   for r in range(mesh.size)]
+            for epoch in range(2):   # (both halves of the double buffers)
+                for op in ops:
+                    op.poison_unowned()
+                    for i, t in enumerate((op.A_owned, op.B_owned) if cls is DistSDDMM else (op.X_owned,)):
+                        op.fill_owned(t, (op.plan.row if (cls is DistSDDMM and i == 0) else op.plan.col).owned_gids,
+                                      seed=9 + epoch, stream=1 + i)
+                run_lockstep([op._fused for op in ops], [(op.Y_owned, 0.0) for op in ops] if cls is DistSpMM else None)
+                for op in ops:
+                    op._fused.check()
+                    if cls is DistSpMM:
+                        got[bulk, cls, epoch, op.plan.rank] = op.Y_owned.clone()
+                    else:   # values of this rank by their position in the plan's order
+                        out = torch.zeros(op.plan.nnz, dtype=dt, device="cuda")
+                        vals = op._fused.out[:op._fused.out_len]
+                        off, ln = op.plan.owned_nnz_slice()
+                        out[torch.from_numpy(op.owned_positions()).cuda()] = vals[off:off + ln] if mesh.Z == 1 else vals
+                        got[bulk, cls, epoch, op.plan.rank] = out
+    # Z slices follow the storage order, which differs between the two forms: compare the sum over a fiber
+    eps = torch.finfo(dt).eps
+    for cls in (DistSDDMM, DistSpMM):
+        for epoch in range(2):
+            for x in range(mesh.X):
+                for y in range(mesh.Y):
+                    fiber = [mesh.rank_of(x, y, z) for z in range(mesh.Z)]
+                    if cls is DistSDDMM:
+                        pairs = [tuple(sum(got[b, cls, epoch, r] for r in fiber) for b in (None, True))]
+                    else:
+                        pairs = [tuple(got[b, cls, epoch, r] for b in (None, True)) for r in fiber]
+                    for a, b in pairs:
+                        assert a.shape == b.shape and torch.isfinite(a).all()
+                        if a.numel():   # sums of at most k, or a row's nonzeros, products in another order
+                            assert (a - b).abs().max() <= 64 * eps * max(1.0, float(b.abs().max()))
