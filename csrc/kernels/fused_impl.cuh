@@ -187,8 +187,9 @@ __device__ __forceinline__ bool wait_counter(const FusedComm& c, int which, int 
 __device__ __forceinline__ void start_phase(const FusedComm& c) {
     if (blockIdx.x == 0 && threadIdx.x == 0) stamp(c, T_START);
     if (blockIdx.x == 0 && threadIdx.x < c.n_readers) {
+        int* const ready = c.peer_pad[c.readers[threadIdx.x]] + F_READY * MAX_RANKS + c.me;
         __threadfence_system();
-        signal(c, F_READY, c.readers[threadIdx.x]);
+        st_relaxed_sys(ready, c.epoch);
     }
 }
 
@@ -499,7 +500,8 @@ __device__ __forceinline__ bool pull_fixed(const FusedComm& c, const PullConfig&
 }
 // Whether the rows to pull are so few that they are there before computing ahead of them would pay: vector loads (the
 // host's choice below 4 MB, see `_pull_config` in ops/fused.py) of at most that many bytes.  SDDMM and SpMM of all ranks on
-// one GPU, waves / everything first, us: 2x2x2, R-MAT scale 16, k = 128 (3.4 and 1.7 MB) 948 / 767.
+// one GPU, waves / everything first, us: 2x2x2, R-MAT scale 16, k = 128 (3.4 and 1.7 MB) 948 / 667, scale 14, k = 32 652 / 397;
+// 2x2x1, Erdos-Renyi 40 thousand rows, k = 32 424 / 252; 2x1x2, R-MAT scale 16, k = 64 509 / 371.
 constexpr long long SMALL_PULL_BYTES = 4ll << 20;
 inline bool small_pull(const PullConfig& pc, long long n_rows, int nvec) {
     return n_rows == 0 || (pc.pullers == 0 && n_rows * nvec * 16 <= SMALL_PULL_BYTES);
@@ -513,22 +515,31 @@ __device__ __forceinline__ void clear_ctrl(const FusedComm& c, int lane) {
 
 // Every thread calls this after its MAIN work; the last block to arrive publishes
 // DONE and PART for this rank.
+//
+// A chain of trips that the next phase waits for, so: the addresses of the flags are read while the block's other warps
+// still work, the blocks order their writes at device scope, and one fence at system scope stands before all flags.  (A
+// release is cumulative: what the blocks stored to other ranks is ordered before the last block's fence by their fences
+// and counts, and by that fence before the flags.)  Last value to last block: 11.5 us with a system fence per block and a
+// release, behind two loads, per flag (eight ranks of R-MAT scale 16 on one GPU), now 3 to 4.
 __device__ __forceinline__ void main_epilogue(const FusedComm& c, int lane) {
+    int *done = nullptr, *part = nullptr;
+    if (threadIdx.x < 32) {
+        if (lane < c.n_read) done = c.peer_pad[c.read_from[lane]] + F_DONE * MAX_RANKS + c.me;
+        if (lane < c.n_push) part = c.peer_pad[c.push_to[lane]] + F_PART * MAX_RANKS + c.me;
+    }
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    // remote stores (pushed partial results) must be visible system-wide before PART is signalled; a rank
-    // that pushed nothing only has to order its local writes.  One fence per block, behind the barrier: it covers
-    // what the other warps of the block wrote.
-    if (c.n_push > 0) __threadfence_system();
-    else __threadfence();
+    __threadfence();   // one per block, behind the barrier: it covers what the other warps of the block wrote
     __syncwarp();
     int old = 0;
     if (lane == 0) old = atomicAdd(c.ctrl + C_MAIN_DONE, 1);
     old = from_lane0(old);
     if (old == (int)gridDim.x - 1) {
         __threadfence_system();
-        for (int i = lane; i < c.n_read; i += 32) signal(c, F_DONE, c.read_from[i]);
-        for (int i = lane; i < c.n_push; i += 32) signal(c, F_PART, c.push_to[i]);
+        if (done) st_relaxed_sys(done, c.epoch);
+        if (part) st_relaxed_sys(part, c.epoch);
+        for (int i = lane + 32; i < c.n_read; i += 32) signal(c, F_DONE, c.read_from[i]);
+        for (int i = lane + 32; i < c.n_push; i += 32) signal(c, F_PART, c.push_to[i]);
         if (lane == 0) stamp(c, T_MAIN);
         if (!(c.phases & PH_FINISH)) clear_ctrl(c, lane);
     }
