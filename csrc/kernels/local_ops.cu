@@ -10,6 +10,7 @@
 // The inner loops are in sp3_kernels.cuh.  Both kernels are bound by the gathers
 // of dense rows from HBM/L2.
 #include "sp3_kernels.cuh"
+#include "sp3_calls.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -83,13 +84,6 @@ scale_picked_kernel(long long nnz, const int* where, const T* sval, const T* dot
 // Rows of k values, `ld` apart wherever they start, to rows of `nvec` whole 16-byte vectors, the rest zero: what the
 // SDDMM and the SpMM read in place of operands whose rows are no whole number of vectors (see `pack_rule` in
 // ops/cuda_ops.py for when that pays).  Bound by the copy; four vectors per thread, one block per 1024.
-struct PackRows {
-    const void* src;     // null: nothing to pack
-    long long ld;        // elements
-    void* dst;
-    long long rows;
-    int k, nvec;
-};
 constexpr int PACK_PER_BLOCK = 1024;
 inline unsigned pack_blocks(const PackRows& p) {
     return p.src ? (unsigned)((p.rows * p.nvec + PACK_PER_BLOCK - 1) / PACK_PER_BLOCK) : 0;
@@ -152,37 +146,8 @@ spmm_items_kernel(int nitems, const int4* items, int nrows, const long long* row
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {
     after_previous_kernel();
     __shared__ ItemSmem<T, NB, G, R> scratch[256 / 32];
-    ItemSmem<T, NB, G, R>& sm = scratch[threadIdx.x >> 5];
-    const int lane = threadIdx.x & 31;
-    const int warp0 = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-    const long long nnz = rowptr[nrows];
-    auto run = [&](int it) {
-        const int4 item = items[it];
-        // (items of fewer rows wait for the previous values less often than the requests cost: Erdos-Renyi, 24 nonzeros
-        // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
-        if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
-        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
-                                                                 aligned, emit, lg, sm, lane);
-    };
-    if (lg.ticket && nitems > nwarps) {
-        // dynamic hand-out: items differ too much in cost (cached or not, hub or not) for a fixed assignment to balance
-        // (a ticket drawn while the item before it runs binds work to a busy warp: R-MAT scale 17, k = 33, 51 us
-        // instead of 48)
-        for (int it = warp0; it < nitems;) {
-            run(it);
-            if (lane == 0) it = nwarps + atomicAdd(lg.ticket, 1);
-            it = __shfl_sync(0xffffffffu, it, 0);
-        }
-        // the last block to finish leaves the counters at zero for the next launch (no memset per launch)
-        __syncthreads();
-        if (threadIdx.x == 0 && atomicAdd(lg.ticket + 1, 1) == (int)gridDim.x - 1) {
-            lg.ticket[0] = 0;
-            lg.ticket[1] = 0;
-        }
-        return;
-    }
-    for (int it = warp0; it < nitems; it += nwarps) run(it);
+    spmm_items<T, NB, G, R, EXACT>(blockIdx.x, gridDim.x, nitems, items, nrows, rowptr, colidx, val, X, ldx_bytes, nvec, aligned,
+                                   emit, lg, scratch[threadIdx.x >> 5]);
 }
 
 // Rows of more than 256 vectors, or no work items: one warp per row, scalar loads.
@@ -586,45 +551,6 @@ SP3_API int sp3_cuda_spmm_f64(int nrows, int nitems, const void* items, const lo
     return launch_spmm<double>(nrows, nitems, (const int4*)items, rowptr, ci, val, X, ldx, k, beta, Y, ldy, lg,
                                (cudaStream_t)stream);
 }
-// The same two calls with their arguments in a record that the caller keeps between launches (field order:
-// ops/cuda_ops.py): converting some twenty arguments costs the Python front end more than a small kernel runs.
-struct SddmmCall {
-    long long nnz;
-    const int *ri, *ci;
-    const void *sv, *A;
-    long long lda;
-    const void* B;
-    long long ldb;
-    void* out;
-    int k, f64;
-    // null, or: ri and ci are sorted by chunk of columns, the dot products go to `dots`, and the value of nonzero i (row
-    // order) is sv[i] * dots[where[i]]
-    const int* where;
-    void* dots;
-    PackRows pack_a, pack_b;   // A and B are filled from here first
-    void* also;                // null, or a second place for the values (scores that are values of the next kernel)
-};
-struct SpmmCall {
-    int nrows, nitems;
-    const void* items;
-    const long long* rowptr;
-    const int* ci;
-    const void *val, *X;
-    long long ldx;
-    void* Y;
-    long long ldy;
-    const int *first_piece, *npieces;
-    int* counters;
-    void* carry;
-    long long ldc;
-    int* ticket;
-    double beta;
-    int k, f64;
-    int k_out;              // columns of Y (k of X counts the padding of its rows)
-    int x_rows;             // rows of X
-    PackRows pack_x;        // X is filled from here first
-    long long nnz;
-};
 SP3_API int sp3_cuda_call_sizes(int* sddmm_bytes, int* spmm_bytes) {
     *sddmm_bytes = (int)sizeof(SddmmCall);
     *spmm_bytes = (int)sizeof(SpmmCall);

@@ -908,6 +908,52 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     if (lane == 0) lg.counters[lr] = 0;
 }
 
+// Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
+// half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.  More blocks
+// than these spill registers in the inner loops.
+__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? 4 : 1; }
+__host__ __device__ constexpr int sddmm_unroll(int R, bool f32) { return R <= (f32 ? 4 : 3) ? 4 : 2; }
+__host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32) { return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 ? 2 : 1)); }
+__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : 2); }
+
+// All items of an SpMM, by block `block` of `nblocks` blocks of 256 threads that do so (every one of them calls it).
+template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
+__device__ __forceinline__ void spmm_items(unsigned block, unsigned nblocks, int nitems, const int4* items, int nrows,
+                                           const long long* rowptr, const int* colidx, const T* val, const char* X,
+                                           unsigned ldx_bytes, int nvec, bool aligned, const Emit& emit, const SpmmLong& lg,
+                                           ItemSmem<T, NB, G, R>& sm) {
+    const int lane = threadIdx.x & 31;
+    const int warp0 = (int)(((long long)block * blockDim.x + threadIdx.x) >> 5);
+    const int nwarps = (int)(((long long)nblocks * blockDim.x) >> 5);
+    const long long nnz = rowptr[nrows];
+    auto run = [&](int it) {
+        const int4 item = items[it];
+        // (items of fewer rows wait for the previous values less often than the requests cost: Erdos-Renyi, 24 nonzeros
+        // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
+        if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
+        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
+                                                                 aligned, emit, lg, sm, lane);
+    };
+    if (lg.ticket && nitems > nwarps) {
+        // dynamic hand-out: items differ too much in cost (cached or not, hub or not) for a fixed assignment to balance
+        // (a ticket drawn while the item before it runs binds work to a busy warp: R-MAT scale 17, k = 33, 51 us
+        // instead of 48)
+        for (int it = warp0; it < nitems;) {
+            run(it);
+            if (lane == 0) it = nwarps + atomicAdd(lg.ticket, 1);
+            it = __shfl_sync(0xffffffffu, it, 0);
+        }
+        // the last block to finish leaves the counters at zero for the next launch (no memset per launch)
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(lg.ticket + 1, 1) == (int)nblocks - 1) {
+            lg.ticket[0] = 0;
+            lg.ticket[1] = 0;
+        }
+        return;
+    }
+    for (int it = warp0; it < nitems; it += nwarps) run(it);
+}
+
 // Work items per ticket of a dynamically scheduled kernel: about 1/32 of a warp's share, at most max_per.
 __device__ __forceinline__ int per_ticket(long long n_work, int nwarps, int max_per) {
     const long long p = n_work / ((long long)nwarps * 32);
@@ -1025,12 +1071,4 @@ constexpr long long CACHED_BYTES = 64ll << 20;
         case 16 * 16 + 4: MACRO(16, 4); break; case 32 * 16 + 3: MACRO(32, 3); break;                     \
         case 32 * 16 + 4: MACRO(32, 4); break; default: MACRO(32, 8); break;                              \
     }
-// Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
-// half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.  More blocks
-// than these spill registers in the inner loops.
-__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? 4 : 1; }
-__host__ __device__ constexpr int sddmm_unroll(int R, bool f32) { return R <= (f32 ? 4 : 3) ? 4 : 2; }
-__host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32) { return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 ? 2 : 1)); }
-__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : 2); }
-
 }  // namespace sp3

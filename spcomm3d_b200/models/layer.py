@@ -23,7 +23,17 @@ from .dist_ops import DistSDDMM, DistSpMM
 STREAM_A, STREAM_B = 1, 2
 
 
+def _bind_pair(old, sddmm, spmm):
+    """Two bound calls as one, in place of `old`."""
+    from ..ops.cuda_ops import BoundPair
+    if old is not None:
+        old.retire()
+    return BoundPair(sddmm, spmm)
+
+
 class SddmmSpmmStep:
+    _pair = None   # the two bound calls as one
+
     def __init__(self, plan, groups, k, dtype=torch.float32, device="cuda", variant="sparseNRB", seed=0,
                  **kw):
         self.plan, self.k, self.seed = plan, k, seed
@@ -32,9 +42,11 @@ class SddmmSpmmStep:
         self.spmm = DistSpMM(plan, groups, k, dtype, device, variant, **kw)
         self.host = None
         self._native_step = None
+        if self.sddmm._single and self.spmm._single:
+            self._bind()
 
     def __getstate__(self):
-        return {**self.__dict__, "_native_step": None}   # bound to this step's tensors, like the operators' calls
+        return {**self.__dict__, "_native_step": None, "_pair": None}   # bound to this step's tensors, like the operators' calls
 
     def fill_device_operands(self):
         """A, B (and X = B) generated on the device from the seed."""
@@ -51,10 +63,20 @@ class SddmmSpmmStep:
             sd.fill_owned(sd.B_owned, p.col.owned_gids, seed=self.seed, stream=STREAM_B)
             sp.X_owned.copy_(sd.B_owned)
 
+    def _bind(self):
+        self._pair = _bind_pair(self._pair, self.sddmm._bind(), self.spmm._bind())
+        self._pair.c = self.sddmm._slice
+        return self._pair
+
     def run_device(self):
-        c = self.sddmm.run_async()
-        y = self.spmm.run_async()
-        return c, y
+        sd, sp, pair = self.sddmm, self.spmm, self._pair
+        if sd._single and sp._single:
+            if pair is None or not pair.bound_to(sd.rowidx, sd.colidx, sd.vals, sd.A_loc, sd.B_loc, sd.partial,
+                                                 sp.rowptr, sp.colidx, sp.vals, sp.X_loc, sp.Y_loc):
+                pair = self._bind()
+            pair.launch()
+            return pair.c, sp.Y_owned
+        return sd.run_async(), sp.run_async()
 
     # ---- end to end: operands start in pinned host memory -----------------
     def make_host_operands(self):
@@ -216,6 +238,8 @@ class SddmmSpmmStep:
 class GatLayer:
     """Y = (S o (A B^T)) X on the mesh; returns owned rows of Y."""
 
+    _pair = None   # the two bound calls as one
+
     def __init__(self, plan, groups, k, dtype=torch.float32, device="cpu", variant="sparseNRB", **kw):
         self.plan, self.groups = plan, groups
         self.sddmm = DistSDDMM(plan, groups, k, dtype, device, variant, **kw)
@@ -230,14 +254,16 @@ class GatLayer:
         self._all = torch.zeros(Z, self.width, dtype=dtype, device=dev)
         self._scores = None
         if self._direct():
-            self._bind_scores()
+            scores = self._bind_scores()
+            if self.spmm._single:
+                self._pair = _bind_pair(None, scores, self.spmm._bind())
             self.sddmm._bound = None   # (its own call is bound when it runs alone: the scratch is not needed twice)
         # the SpMM wants its values in CSR order; a fused SDDMM stores them in its own order
         order = self.sddmm.value_order
         self._pos = None if order is None else torch.from_numpy(np.ascontiguousarray(order)).to(dev)
 
     def __getstate__(self):
-        return {**self.__dict__, "_scores": None}   # bound to this layer's tensors, like the operators' calls
+        return {**self.__dict__, "_scores": None, "_pair": None}   # bound to this layer's tensors, like the operators' calls
 
     def _direct(self):
         """Whether the kernel of the SDDMM itself can put the scores where the SpMM reads its values, next to the result
@@ -251,10 +277,22 @@ class GatLayer:
         return self._scores
 
     def run(self):
-        if not self.sddmm.timer.enabled and self._direct():
-            self._bind_scores().launch()
-            return self.spmm.run()
-        c = self.sddmm.run()
+        sd, sp = self.sddmm, self.spmm
+        if not sd.timer.enabled and sd._single:
+            pair = self._pair if sp._single and not sp.timer.enabled else None
+            if pair is not None and pair.bound_to(sd.rowidx, sd.colidx, sd.vals, sd.A_loc, sd.B_loc, sd.partial, sp.vals,
+                                                  sp.rowptr, sp.colidx, sp.vals, sp.X_loc, sp.Y_loc):
+                pair.launch()
+                return sp.Y_owned
+            if self._direct():
+                scores = self._bind_scores()
+                if sp._single and not sp.timer.enabled:
+                    self._pair = _bind_pair(self._pair, scores, sp._bind())
+                    self._pair.launch()
+                    return sp.Y_owned
+                scores.launch()
+                return sp.run()
+        c = sd.run()
         Z = self.plan.mesh.Z
         if Z == 1:
             if self._pos is None:

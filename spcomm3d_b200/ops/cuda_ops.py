@@ -477,6 +477,49 @@ def bind_spmm(rowptr, colidx, vals, X, Y, sched: SpmmSchedule, pack=None):
     return _BoundCall("spmm", rec, (rowptr, colidx, vals, X, Y), keep=(sched, carry, x), launches=1 + (x is not X))
 
 
+def _span(t: torch.Tensor):
+    """First byte of a tensor and the one behind its last."""
+    p = t.data_ptr()
+    if t.is_contiguous():
+        return p, p + t.numel() * t.element_size()
+    return p, p + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
+
+
+class BoundPair:
+    """An SDDMM and the SpMM behind it, two bound calls, queued by one native call; small steps (neither call touches
+    what the other writes) are one launch (csrc/kernels/pair_ops.cu)."""
+
+    c = None   # what the caller returns for the SDDMM
+
+    def __init__(self, sddmm: _BoundCall, spmm: _BoundCall):
+        lib = native.cuda()
+        self.sddmm, self.spmm = sddmm, spmm
+        self._fn, self._record, self._addrs = lib.sp3_cuda_pair_call, spmm._record, (sddmm._addr, spmm._addr)
+        self._tensors, self._ptrs = sddmm._tensors + spmm._tensors, sddmm._ptrs + spmm._ptrs
+        # (rowidx, colidx, svals, A, B, out[, also]) and (rowptr, colidx, vals, X, Y)
+        y0, y1 = _span(spmm._tensors[4])
+        self._independent = int(all(a1 <= b0 or b1 <= a0 for a0, a1 in map(_span, sddmm._tensors[5:])
+                                    for b0, b1 in map(_span, spmm._tensors))
+                                and all(b <= y0 or y1 <= a for a, b in map(_span, sddmm._tensors[:5])))
+        one = lib.sp3_cuda_pair_fuses(*self._addrs, self._independent)
+        self._launches = 1 if one else sddmm._launches + spmm._launches
+
+    bound_to = _BoundCall.bound_to
+
+    def retire(self):
+        self.sddmm.retire()
+        self.spmm.retire()
+
+    def launch(self):
+        """One run, with beta 0."""
+        global LAUNCHES
+        self._record.beta = 0.0
+        LAUNCHES += self._launches
+        rc = self._fn(*self._addrs, self._independent, _raw_stream())
+        if rc != 0:
+            raise RuntimeError(f"sddmm and spmm: CUDA launch error {rc}")
+
+
 STEP_CHUNKS = 8
 STEP_CHUNK_BYTES = 4 << 20   # parts of A of this size: a fraction of the copy, many times the cost of a launch
 

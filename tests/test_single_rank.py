@@ -627,3 +627,36 @@ def test_scratch_of_a_call_that_makes_way(monkeypatch):
     assert all(t.data_ptr() != at for t in taken)
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+# One launch for both kernels: single rows, rows shorter and longer than an item, split rows, empty rows, every shape of the
+# pair (numbers of 16-byte vectors), a size that takes two launches; and operators that share tensors, which must not run
+# side by side.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gen", ["uniform:1:3:2", "uniform:700:500:3", "rmat:11:16", "zipf:900:4000:1.8:2000", "uniform:9000:9000:24"])
+@pytest.mark.parametrize("vectors", [1, 5, 6, 7, 9, 11, 15, 16, 20, 25, 32, 40, 64, 65])
+def test_step_in_one_launch(vectors, gen, dtype):
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    plan, k = _plan(gen), vectors * 16 // dtype.itemsize
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    step = SddmmSpmmStep(plan, None, k, dtype, "cuda", seed=2)
+    step.fill_device_operands()
+    sd, sp = step.sddmm, step.spmm
+    deg = _lists(plan)[2].numpy()
+    ref, mag = _scores(plan, sd.A_owned.cpu(), sd.B_owned.cpu(), vals)
+
+    def check(y, values):
+        bound = torch.from_numpy(_gamma(deg + 3.0, dtype))[:, None] * _product(plan, values.abs(), sp.X_owned.cpu().abs())
+        assert bool(((y.cpu().double() - _product(plan, values, sp.X_owned.cpu())).abs() <= bound).all())
+    for _ in range(2):                   # (the second time with what the first left in the counters)
+        sd.partial.fill_(float("nan")), sp.Y_owned.fill_(float("nan"))
+        c, y = step.run_device()
+        assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+        check(y, vals)
+    sp.vals = sd.partial                 # a chain now: the SpMM reads what the SDDMM writes
+    sd.partial.fill_(float("nan"))
+    c, y = step.run_device()
+    assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+    check(y, c.cpu())
+    assert step._pair._independent == 0
