@@ -104,14 +104,14 @@ template <typename T> unsigned pair_resident(const PairShape& s) {
 }
 
 // Whether the two calls can be one launch that pays; the shape, the blocks of the SpMM and the nonzeros per window of the
-// SDDMM if so.  It saves a launch on the host (2.2 us of 8.1) and a ramp on the device, and loses where the SpMM alone would
-// have all its items in flight at once and has not beside the SDDMM: with rows of more than 16 vectors by more than the host
-// gains.  One launch / two, us on the device:
-//   fp32, k = 16       1 k rows of 4 2.7 / 4.2; 10 k of 10 8.1 / 10.4; 16 k of 16 8.5 / 8.2; R-MAT scale 14 (233 k nonzeros) 9.0 / 11.2
-//   fp32, k = 64       1 k of 4 3.1 / 4.8; 4 k of 16 (one round alone) 8.1 / 6.5 (with the host 8.1 / 8.1); 10 k of 10 9.7 / 12.2; 16 k of 16 14.9 / 12.8;
-//                      Zipf rows, 176 k nonzeros 13.9 / 15.0; R-MAT scale 14 17.0 / 19.0
-//   fp32, k = 128      4 k of 16 9.8 / 7.8; 10 k of 10 13.7 / 16.7; Zipf 21.9 / 22.9; R-MAT 24.3 / 26.6
-//   fp64, k = 32, 128  4 k of 16 6.5 / 6.2 (with the host 6.8 / 8.2), 15.2 / 13.5; 10 k of 10 12.4 / 12.5, 19.3 / 21.3; Zipf 18.7 / 16.4, 48 / 41; R-MAT 20.3 / 20.4, 40.5 / 39.2
+// SDDMM if so.  It saves a launch on the host (2.2 us of 7.4) and a ramp on the device, and loses where the SpMM alone has
+// all its items in flight at once and has not beside the SDDMM, unless split rows make one long chain of it anyway.  One
+// launch / two, us with the host:
+//   fp32, k = 32    1 k rows of 4 5.5 / 7.4; 4 k of 16 5.4 / 7.2; 10 k of 10 (not in flight at once) 9.6 / 8.2;
+//                   Zipf rows, 176 k nonzeros 10.0 / 13.0; R-MAT scale 14 (228 k) 12.2 / 14.4
+//   fp32, k = 64    1 k of 4 5.5 / 7.1; 4 k of 16 (not at once) 8.7 / 7.3; Zipf 14.0 / 14.6; R-MAT 17.4 / 18.5
+//   fp32, k = 128   5 k of 4 5.6 / 7.6; R-MAT scale 11 7.2 / 10.8
+//   fp64, k = 32    1 k of 4 5.5 / 7.5; R-MAT scale 11 6.4 / 9.2; Zipf 176 k 19.0 / 15.9; R-MAT scale 14 20.7 / 19.7
 constexpr long long PAIR_MAX_NNZ = 1 << 18;   // with split rows (half as many without, and with fp64)
 template <typename T> bool pair_plan(const SddmmCall& d, const SpmmCall& p, PairShape* s, unsigned* spmm_blocks, int* wn) {
     const long long lda = d.lda * (long long)sizeof(T), ldb = d.ldb * (long long)sizeof(T), ldx = p.ldx * (long long)sizeof(T),
@@ -127,7 +127,7 @@ template <typename T> bool pair_plan(const SddmmCall& d, const SpmmCall& p, Pair
     if (all < 2) return false;
     const unsigned items = (unsigned)((p.nitems + 7) / 8), least = (unsigned)((d.nnz + 8 * WINDOW_MAX - 1) / (8 * WINDOW_MAX));
     const unsigned alone = all / pair_min_blocks(s->rs, s->rp, sizeof(T) == 4) * (bytes <= 32 * 16 ? 4 : 3);
-    if (items + least > all && items <= alone && bytes > 16 * 16) return false;
+    if (items + least > all && items <= alone && !p.carry) return false;
     unsigned half = all > least + all / 2 ? all - least : all / 2;
     *spmm_blocks = items < half ? items : half;
     *wn = window_nnz(d.nnz, (long long)(all - *spmm_blocks) * 8, 32 / s->gs);

@@ -158,6 +158,90 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
     return items.astype(np.int32), first.astype(np.int32), npieces.astype(np.int32)
 
 
+SMALL_NNZ = 1_100_000   # blocks up to here have their items made to fit the warps (`fit_spmm_items`)
+
+
+def spmm_warps(nvec: int, split: bool) -> int:
+    """Warps that run at once in an SpMM of rows of `nvec` vectors (see pick_shape and launch_spmm_nb: blocks per SM by
+    vectors per lane, for matrices without split rows those of the shape that has most)."""
+    blocks = (4 if nvec <= 10 else 3 if nvec <= 16 else 2) if split else (4 if nvec <= 32 else 3 if nvec <= 64 else 2)
+    return 148 * 8 * blocks
+
+
+def fit_spmm_items(rowptr: np.ndarray, nvec: int):
+    """Work items as `build_spmm_items` returns them, for a small block whose dense rows have `nvec` 16-byte vectors: as
+    many as there are warps, or twice or three times as many, and of equal weight.
+
+    A warp takes 3 to 4 us from one item to the first rows of the next, and a last round with work for few warps takes as
+    long as a full one; items cut where buckets of nonzeros and blocks of 32 rows end differ by a factor of four.  Weight:
+    1 for a nonzero, 1/32 of an item for a row, which also bounds the rows.  Rows of more than one item (64 nonzeros, 32 if
+    wide, at least) are cut into equal pieces.  One round as long as items stay below 140 nonzeros (220 where no row is split: their
+    cost varies less), us, fp32, buckets / these:
+      100 thousand nonzeros, k = 64, uniform rows of 4, 10, 24   8.5 / 4.9, 8.4 / 5.5, 3.9 / 3.9; Zipf rows 10.9 / 8.6
+      400 thousand, k = 32   rows of 10, 24 11.3 / 9.8, 10.3 / 6.2; Zipf rows 11.1 / 9.9; R-MAT scale 15 16.5 / 10.5
+      500 thousand, k = 256  Zipf rows, two rounds 70 / 57; R-MAT scale 15 41 / 32
+      1 million, k = 64, 128, Zipf rows, two and three rounds 32.9 / 28.6, 72 / 57; R-MAT scale 16 25.2 / 23.9, 38.9 / 36.9
+    From there on the buckets are level or faster (R-MAT scale 17, k = 64: 39.7, equal items 41 to 42)."""
+    nrows, nnz = rowptr.shape[0] - 1, int(rowptr[-1])
+    deg = np.diff(rowptr)
+    begin, rows = rowptr[:-1] * 32, np.arange(nrows)
+
+    def cut(w, long_row):
+        is_long = deg > long_row
+        key = (begin + rows * w) // (32 * w)
+        bnd = np.ones(nrows, bool)
+        bnd[1:] = (key[1:] != key[:-1]) | is_long[1:] | is_long[:-1]
+        return bnd, is_long, int(bnd.sum() - is_long.sum() + ((deg[is_long] + long_row - 1) // long_row).sum())
+
+    split = bool((deg > max(64, nnz // spmm_warps(nvec, False))).any())
+    warps = spmm_warps(nvec, split)
+    if nnz < 120_000 or not split:
+        buckets = build_spmm_items(rowptr)   # buckets of whole quads, where they fit the warps as they are
+        n = buckets[0].shape[0]
+        if n <= warps or not split and nrows > 0.9 * ITEM_ROWS * n:   # (as many rows as an item may have)
+            return buckets
+    rounds = -(-nnz // (warps * (140 if split else 220)))
+    while warps * rounds < 1.05 * nrows / 32:
+        rounds += 1
+    # the weight that makes `target` items: a first guess, corrected by what it makes beyond one per `w` nonzeros
+    target = warps * rounds
+    least = max(32 if nvec > 32 else 64, int(deg.max()) // 2000 + 1)   # (at most 2^11 - 1 pieces a row)
+    w, low, high = max(16, int(nnz / (target - nrows / 32))), 0, 0   # low: too many items, high: not too many
+    for _ in range(14):
+        long_row = max(least, w)
+        bnd, is_long, n = cut(w, long_row)
+        if n > target:
+            low, free = w, target - (n - nnz / w)
+            w = max(w + 1, min(4 * w, int(nnz / free) + 1 if free > 0 else 4 * w))
+        else:
+            high = w
+            if n > 0.96 * target or w <= max(16, low + 1):
+                break
+            w = max(16, w * 7 // 8)
+        if low and high:
+            w = (low + high + 1) // 2
+            if w == high:
+                break
+    if n > target and high:
+        long_row = max(least, high)
+        bnd, is_long, n = cut(high, long_row)
+    starts = np.flatnonzero(bnd)
+    ends = np.append(starts[1:], nrows)
+    short = ~is_long[starts]
+    first_nnz = rowptr[starts[short]]
+    rows_items = np.stack([starts[short], ends[short], first_nnz, first_nnz - rowptr[ends[short]] - 1], axis=1)
+    long_rows = np.flatnonzero(is_long)
+    npieces = (deg[long_rows] + long_row - 1) // long_row
+    first = np.cumsum(npieces) - npieces
+    slot = np.repeat(np.arange(long_rows.size), npieces)
+    j = np.arange(slot.size) - np.repeat(first, npieces)
+    size = (-(-deg[long_rows] // np.maximum(npieces, 1)) + 3)[slot] // 4 * 4
+    b = rowptr[long_rows[slot]] + j * size
+    e = np.minimum(b + size, rowptr[long_rows[slot] + 1])
+    items = np.concatenate([np.stack([long_rows[slot], np.minimum(b, e), e, slot + (j << PIECE_SHIFT)], axis=1), rows_items])
+    return items.astype(np.int32), first.astype(np.int32), npieces.astype(np.int32)
+
+
 def build_spmm_wave_items(rowptr: np.ndarray, cls: np.ndarray, n_classes: int, long_row: int | None = None,
                           item_nnz: int | None = None, item_rows: int | None = None):
     """Work items for an SpMM whose column-side rows arrive in waves.  `cls[q]` is the class of nonzero q
@@ -234,10 +318,15 @@ class SpmmSchedule:
     """Device-resident SpMM work items plus the scratch the long-row path
     needs: one carry row per piece and one counter per long row."""
 
-    def __init__(self, rowptr: torch.Tensor, k_max: int = 0, dtype=torch.float32, arrays=None, **kw):
+    def __init__(self, rowptr: torch.Tensor, k_max: int = 0, dtype=torch.float32, arrays=None, nvec: int = 0, **kw):
+        """`nvec`: 16-byte vectors of a dense row, where the items may be made for one width (see `fit_spmm_items`)."""
         if arrays is None:
             rp = rowptr.cpu().numpy()
-            items, first, npieces = build_spmm_items(rp, **kw)
+            if 0 < nvec <= 256 and 0 < rp[-1] <= SMALL_NNZ and not kw and not any(
+                    v in os.environ for v in ("SP3_LONG_ROW", "SP3_ITEM_NNZ", "SP3_ITEM_ROWS")):
+                items, first, npieces = fit_spmm_items(rp, nvec)
+            else:
+                items, first, npieces = build_spmm_items(rp, **kw)
         else:   # (items, first_piece, npieces) built elsewhere, e.g. by build_spmm_wave_items
             items, first, npieces = arrays
         dev = rowptr.device

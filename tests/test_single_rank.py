@@ -660,3 +660,55 @@ def test_step_in_one_launch(vectors, gen, dtype):
     assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
     check(y, c.cpu())
     assert step._pair._independent == 0
+
+
+def _degrees(kind):
+    rng = np.random.default_rng(4)
+    return {"one row": np.array([5]), "empty ends": np.array([0, 0, 7, 0]), "one long row": np.array([1_000_000]),
+            "rows of 4": np.full(150_000, 4), "rows of 10": np.full(60_000, 10), "zipf": np.minimum(rng.zipf(1.8, 30_000), 4096),
+            "mostly empty": np.where(rng.random(400_000) < 0.02, 50, 0), "around a piece": np.array([63, 64, 65, 129, 1, 0] * 2000),
+            "short": rng.integers(0, 3, 300_000)}[kind]
+
+
+@pytest.mark.parametrize("nvec", [1, 16, 32, 64, 256])
+@pytest.mark.parametrize("kind", ["one row", "empty ends", "one long row", "rows of 4", "rows of 10", "zipf", "mostly empty",
+                                  "around a piece", "short"])
+def test_fitted_items_cover_every_row_once(kind, nvec):
+    from spcomm3d_b200.ops.cuda_ops import ITEM_ROWS, PIECE_SHIFT, fit_spmm_items
+    deg = _degrees(kind)
+    rowptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    items, first, npieces = fit_spmm_items(rowptr, nvec)
+    rows, pieces = items[items[:, 3] < 0], items[items[:, 3] >= 0]
+    a, b = rows[:, 0], rows[:, 1]
+    assert np.all(b > a) and np.all(b - a <= ITEM_ROWS)
+    assert np.array_equal(rows[:, 2], rowptr[a]) and np.array_equal(-1 - rows[:, 3], rowptr[b] - rowptr[a])
+    covered = np.zeros(deg.size + 1, np.int64)
+    np.add.at(covered, a, 1), np.add.at(covered, b, -1)
+    covered = np.cumsum(covered)[:-1]
+    slot, number = pieces[:, 3] & ((1 << PIECE_SHIFT) - 1), pieces[:, 3] >> PIECE_SHIFT
+    for s in range(first.size):
+        mine = pieces[slot == s]
+        r = mine[0, 0]
+        covered[r] += 1
+        assert mine.shape[0] == npieces[s] and np.array_equal(number[slot == s], np.arange(npieces[s]))
+        assert mine[0, 1] == rowptr[r] and mine[-1, 2] == rowptr[r + 1] and np.array_equal(mine[1:, 1], mine[:-1, 2])
+    assert np.all(covered == 1)
+    assert np.array_equal(first, np.cumsum(npieces) - npieces)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+@pytest.mark.parametrize("vectors", [1, 8, 16, 32, 48, 64, 80])
+@pytest.mark.parametrize("gen", ["uniform:9000:9000:10", "zipf:6000:20000:1.8:3000", "rmat:14:8", "er:2000:3000:60"])
+def test_spmm_with_fitted_items(gen, vectors, beta):
+    from spcomm3d_b200.models.dist_ops import DistSpMM
+    plan, dtype = _plan(gen), torch.float32
+    op = DistSpMM(plan, None, 4 * vectors, dtype, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    op.X_owned.normal_(generator=g), op.Y_owned.normal_(generator=g)
+    deg, vals = _lists(plan)[2].numpy(), torch.from_numpy(plan.vals).to(dtype)
+    X, old = op.X_owned.cpu(), op.Y_owned.cpu()
+    y = op.run_async(beta).cpu().double()
+    ref = _product(plan, vals, X) + beta * old.double()
+    bound = torch.from_numpy(_gamma(deg + 4.0, dtype))[:, None] * (_product(plan, vals.abs(), X.abs()) + beta * old.double().abs())
+    assert bool(((y - ref).abs() <= bound).all())
