@@ -499,10 +499,12 @@ __device__ __forceinline__ bool pull_fixed(const FusedComm& c, const PullConfig&
     return __syncthreads_and(ok);
 }
 // Whether the rows to pull are so few that they are there before computing ahead of them would pay: vector loads (the
-// host's choice below 4 MB, see `_pull_config` in ops/fused.py) of at most that many bytes.  SDDMM and SpMM of all ranks on
-// one GPU, waves / everything first, us: 2x2x2, R-MAT scale 16, k = 128 (3.4 and 1.7 MB) 948 / 667, scale 14, k = 32 652 / 397;
-// 2x2x1, Erdos-Renyi 40 thousand rows, k = 32 424 / 252; 2x1x2, R-MAT scale 16, k = 64 509 / 371.
-constexpr long long SMALL_PULL_BYTES = 4ll << 20;
+// host's choice below the same line, see `_pull_config` in ops/fused.py) of at most that many bytes.  SDDMM and SpMM of all
+// ranks on one GPU, waves / everything first, us: 2x2x2, R-MAT scale 16, k = 128 (3.4 and 1.7 MB) 948 / 623, scale 14, k = 32
+// 652 / 389; 2x2x1, R-MAT scale 16, k = 128 (6.8 MB) 450 / 363; 2x2x1, Erdos-Renyi 60 thousand rows, k = 128 (15 and 7.6 MB)
+// 643 / 476; 2x1x2, uniform 50 thousand rows of 40, k = 256 (12.8 MB) 814 / 622.  Over NVLink the rows take longer (16 MB
+// 23 us at 700 GB/s, 10 here), which is less than the 18 to 30 us that the waves cost beside it.
+constexpr long long SMALL_PULL_BYTES = 16ll << 20;
 inline bool small_pull(const PullConfig& pc, long long n_rows, int nvec) {
     return n_rows == 0 || (pc.pullers == 0 && n_rows * nvec * 16 <= SMALL_PULL_BYTES);
 }

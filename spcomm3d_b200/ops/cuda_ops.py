@@ -168,7 +168,7 @@ def spmm_warps(nvec: int, split: bool) -> int:
     return 148 * 8 * blocks
 
 
-def fit_spmm_items(rowptr: np.ndarray, nvec: int):
+def fit_spmm_items(rowptr: np.ndarray, nvec: int, one_shape: bool = False):
     """Work items as `build_spmm_items` returns them, for a small block whose dense rows have `nvec` 16-byte vectors: as
     many as there are warps, or twice or three times as many, and of equal weight.
 
@@ -181,7 +181,8 @@ def fit_spmm_items(rowptr: np.ndarray, nvec: int):
       400 thousand, k = 32   rows of 10, 24 11.3 / 9.8, 10.3 / 6.2; Zipf rows 11.1 / 9.9; R-MAT scale 15 16.5 / 10.5
       500 thousand, k = 256  Zipf rows, two rounds 70 / 57; R-MAT scale 15 41 / 32
       1 million, k = 64, 128, Zipf rows, two and three rounds 32.9 / 28.6, 72 / 57; R-MAT scale 16 25.2 / 23.9, 38.9 / 36.9
-    From there on the buckets are level or faster (R-MAT scale 17, k = 64: 39.7, equal items 41 to 42)."""
+    From there on the buckets are level or faster (R-MAT scale 17, k = 64: 39.7, equal items 41 to 42).  `one_shape`: for a
+    kernel that takes the shape of split rows whatever the matrix."""
     nrows, nnz = rowptr.shape[0] - 1, int(rowptr[-1])
     deg = np.diff(rowptr)
     begin, rows = rowptr[:-1] * 32, np.arange(nrows)
@@ -194,7 +195,7 @@ def fit_spmm_items(rowptr: np.ndarray, nvec: int):
         return bnd, is_long, int(bnd.sum() - is_long.sum() + ((deg[is_long] + long_row - 1) // long_row).sum())
 
     split = bool((deg > max(64, nnz // spmm_warps(nvec, False))).any())
-    warps = spmm_warps(nvec, split)
+    warps = spmm_warps(nvec, split or one_shape)
     if nnz < 120_000 or not split:
         buckets = build_spmm_items(rowptr)   # buckets of whole quads, where they fit the warps as they are
         n = buckets[0].shape[0]

@@ -23,7 +23,7 @@ from ..utils import native
 from . import cuda_ops
 
 MAX_RANKS = 64
-SMALL_PULL_BYTES = int(os.environ.get("SP3_FUSED_SMALL_BYTES", 4 << 20))
+SMALL_PULL_BYTES = int(os.environ.get("SP3_FUSED_SMALL_BYTES", 16 << 20))   # (the same line in csrc/kernels/fused_impl.cuh)
 PULL_BLOCKS = 148 * 2   # resident blocks that can be counted on
 MAX_WAVES = 32   # pull waves a kernel can track (csrc/kernels/fused_impl.cuh)
 F_KINDS = 3
@@ -548,7 +548,9 @@ class FusedSpMM(_FusedBase):
         self._val_perm, a.n_waves, a.tiles_per_wave, a.wave_items, a.pull_order = None, 0, 0, None, None
         if os.environ.get("SP3_FUSED_SPMM_WAVES") == "0":   # tuning: no overlap, compute after the last pull
             overlap = False
-        if overlap and p.col.n_recv > 0 and p.nnz > 0:
+        # few rows to pull: all of them first (as the kernel decides, `small_pull` in csrc/kernels/fused_impl.cuh)
+        pulls_first = a.pull.pullers == 0 and p.col.n_recv * self.row_bytes <= SMALL_PULL_BYTES
+        if overlap and p.col.n_recv > 0 and p.nnz > 0 and not pulls_first:
             target = max(1, min(MAX_WAVES, int(os.environ.get("SP3_FUSED_SPMM_WAVES", "4"))))
             n_pull = -(-p.col.n_recv // self.tile_rows)
             tpw = -(-n_pull // target)
@@ -569,7 +571,8 @@ class FusedSpMM(_FusedBase):
             self._pull_order = self._dev_i32(self._tickets(pull_order))
             a.pull_order = self._pull_order.data_ptr()
         else:
-            self.sched = cuda_ops.SpmmSchedule(op.rowptr)
+            fit = pulls_first and 0 < p.nnz <= cuda_ops.SMALL_NNZ
+            self.sched = cuda_ops.SpmmSchedule(op.rowptr, arrays=cuda_ops.fit_spmm_items(p.rowptr, self.nvec, True) if fit else None)
             self._colidx, self._vals = op.colidx, op.vals
         carry, ldc = self.sched.carry_for(kp, self.dtype, self.device)
         self.slots = h.view("slots", self.dtype, (h.sizes["slots"] // self.es,))
