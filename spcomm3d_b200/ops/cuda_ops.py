@@ -514,7 +514,7 @@ def bind_sddmm(rowidx, colidx, svals, A, B, out, also=None, chunks=None, pack=No
                       launches=1 + (a is not A) + (chunks is not None))
 
 
-CHUNK_BYTES = 96 << 20     # rows of B that stay in the L2 (126 MB) next to what streams through it
+CHUNK_BYTES = 80 << 20     # rows of B that stay in the L2 (126 MB) next to what streams through it
 CHUNK_MIN_NNZ = 1 << 20
 CHUNK_MAX_NNZ = 2 ** 31 - 1025   # positions are 32-bit numbers, rounded up to a block of 1024
 CHUNK_LIST_BYTES = 20      # per nonzero, for good: the two lists, the position and the dot product (up to 8)
@@ -531,8 +531,8 @@ def column_chunks(rowidx, colidx, n_cols, row_bytes, force=0):
     the same operands (new operands in every run cost about 10 % more): Erdos-Renyi 1 M rows, 32 a row (3 times fewer)
     k = 64 1118 -> 882 us, k = 128 2481 -> 1912; uniform 500 thousand rows, k = 128, 20 a row 638 -> 503, 12 a row (1.4)
     413 -> 342; 1 M x 2 M, 12 a row, k = 64 (1.05): 489 -> 576; R-MAT scale 20, k = 128 (hub columns): 564 -> 673.
-    Chunks of 48 / 64 / 96 / 128 MB: 868 / 821 / 882 / 1048, 2031 / 1804 / 1912 / 2112 and 627 / 508 / 503 / 560 in the
-    first three of these.  Fewer reads per row of B than four leave little to save."""
+    Chunks of 48 / 64 / 80 / 96 MB: 807 / 781 / 782 / 801, 1637 / 1554 / 1555 / 1567 and 462 / 423 / 423 / 436 in the first
+    three of these (rows gathered evenly from 80 MB come at the rate of 32 MB, from 96 MB 8 % slower, from 128 MB 26 %).  Fewer reads per row of B than four leave little to save."""
     nnz = rowidx.shape[0]
     n = force or -(-n_cols * row_bytes // CHUNK_BYTES)
     if nnz > CHUNK_MAX_NNZ or not force and (n < 2 or n > 32 or nnz < CHUNK_MIN_NNZ or nnz < 4 * n_cols
