@@ -140,7 +140,7 @@ sddmm_scalar_kernel(long long nnz, const int* __restrict__ rowidx, const int* __
 // every row exactly once.
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
-__global__ void __launch_bounds__(256, spmm_min_blocks(R))
+__global__ void __launch_bounds__(256, spmm_min_blocks(R, NB))
 spmm_items_kernel(int nitems, const int4* items, int nrows, const long long* rowptr,
                   const int* colidx, const T* val, const char* X,
                   unsigned ldx_bytes, int nvec, bool aligned, const Emit emit, const SpmmLong lg) {

@@ -679,7 +679,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
 #pragma unroll
     for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and emit nothing
         const int v = gl + q * G;
-        on[q] = EXACT || v < nvec;
+        on[q] = EXACT || (q < R - 1 && R <= 4) || v < nvec;   // (pick_shape: only a lane's last vector can be past the row)
         off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
     }
     X += off[0];
@@ -908,13 +908,16 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     if (lane == 0) lg.counters[lr] = 0;
 }
 
-// Dense vectors a lane has in flight (U nonzeros x R vectors) and blocks of 256 threads an SM should hold: about
+// Dense vectors a lane has in flight (U nonzeros x R vectors of NB bytes) and blocks of 256 threads an SM should hold: about
 // half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.  More blocks
-// than these spill registers in the inner loops.
-__host__ __device__ constexpr int spmm_unroll(int R) { return R <= 4 ? 4 : 1; }
+// than these spill registers in the inner loops.  What counts in the SpMM is the bytes of a lane: three or four vectors of 4
+// bytes take the registers of one of 16, and in the blocks that three or four wide ones leave they have a quarter of the
+// bytes in flight (k = 75, R-MAT scale 14 22.5 us in two blocks, 16.9 in four; k = 101 18.9 and 16.1; R-MAT scale 16 5 %
+// less).  (The SDDMM gains nothing: level over 91 odd widths, 18 % either way.)
+__host__ __device__ constexpr int spmm_unroll(int R, int NB = 16) { return R * NB <= 64 ? 4 : 1; }
 __host__ __device__ constexpr int sddmm_unroll(int R, bool f32) { return R <= (f32 ? 4 : 3) ? 4 : 2; }
 __host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32) { return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 ? 2 : 1)); }
-__host__ __device__ constexpr int spmm_min_blocks(int R) { return R == 1 ? 4 : (R == 2 ? 3 : 2); }
+__host__ __device__ constexpr int spmm_min_blocks(int R, int NB = 16) { return R * NB <= 16 ? 4 : (R * NB <= 32 ? 3 : 2); }
 
 // All items of an SpMM, by block `block` of `nblocks` blocks of 256 threads that do so (every one of them calls it).
 template <typename T, int NB, int G, int R, bool EXACT, typename Emit>
@@ -931,7 +934,7 @@ __device__ __forceinline__ void spmm_items(unsigned block, unsigned nblocks, int
         // (items of fewer rows wait for the previous values less often than the requests cost: Erdos-Renyi, 24 nonzeros
         // a row, fp64, k = 64, 457 us with them, 448 without; R-MAT scale 20, k = 32, beta 0.5, 280 against 313)
         if (item.w < 0 && item.y - item.x >= 8) emit.expect(item.x, item.y - item.x, nvec, lane);
-        spmm_warp_item<T, NB, G, R, spmm_unroll(R), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
+        spmm_warp_item<T, NB, G, R, spmm_unroll(R, NB), EXACT>(item, rowptr, nnz, colidx, val, X, ldx_bytes, nvec,
                                                                  aligned, emit, lg, sm, lane);
     };
     if (lg.ticket && nitems > nwarps) {

@@ -406,7 +406,8 @@ class DistSpMM(_Dist3DOp):
             if variant == "dense":
                 self._d_sched = cuda_ops.SpmmSchedule(self._d_rowptr)
             else:
-                self.sched = cuda_ops.SpmmSchedule(self.rowptr, nvec=-(-self.k_loc * self.vals.element_size() // 16))
+                nvec, nb = cuda_ops.spmm_row_vectors(p.nnz, p.col.n_local, self.k_loc, self.vals.element_size(), self.device)
+                self.sched = cuda_ops.SpmmSchedule(self.rowptr, nvec=nvec, nb=nb)
         # opt-in: dense (128-row x 64-column) panels of S as TF32 products on the tensor cores
         self._panels = None
         if (kw.get("panels") and variant in ("sparse", "sparseNRB") and self.device.type == "cuda"

@@ -161,15 +161,21 @@ def build_spmm_items(rowptr: np.ndarray, long_row: int | None = None, item_nnz: 
 SMALL_NNZ = 1_100_000   # blocks up to here have their items made to fit the warps (`fit_spmm_items`)
 
 
-def spmm_warps(nvec: int, split: bool) -> int:
-    """Warps that run at once in an SpMM of rows of `nvec` vectors (see pick_shape and launch_spmm_nb: blocks per SM by
-    vectors per lane, for matrices without split rows those of the shape that has most)."""
-    blocks = (4 if nvec <= 10 else 3 if nvec <= 16 else 2) if split else (4 if nvec <= 32 else 3 if nvec <= 64 else 2)
-    return 148 * 8 * blocks
+def spmm_warps(nvec: int, split: bool, nb: int = 16) -> int:
+    """Warps that run at once in an SpMM of rows of `nvec` vectors of `nb` bytes (see pick_shape, spmm_min_blocks and
+    launch_spmm_nb: blocks per SM by the bytes of a lane, for matrices without split rows those of the shape that has most)."""
+    if split or nvec > 64:
+        g = (8 if 10 < nvec <= 32 else 16 if 32 < nvec <= 64 else
+             next((g for g in (4, 5, 6, 8, 10, 16) if g >= nvec), 32))
+        r = -(-nvec // g)
+        r = r if r <= 4 else 8
+    else:
+        r = 1 if nvec <= 32 else 2
+    return 148 * 8 * (4 if r * nb <= 16 else 3 if r * nb <= 32 else 2)
 
 
-def fit_spmm_items(rowptr: np.ndarray, nvec: int, one_shape: bool = False):
-    """Work items as `build_spmm_items` returns them, for a small block whose dense rows have `nvec` 16-byte vectors: as
+def fit_spmm_items(rowptr: np.ndarray, nvec: int, one_shape: bool = False, nb: int = 16):
+    """Work items as `build_spmm_items` returns them, for a small block whose dense rows have `nvec` vectors of `nb` bytes: as
     many as there are warps, or twice or three times as many, and of equal weight.
 
     A warp takes 3 to 4 us from one item to the first rows of the next, and a last round with work for few warps takes as
@@ -194,8 +200,8 @@ def fit_spmm_items(rowptr: np.ndarray, nvec: int, one_shape: bool = False):
         bnd[1:] = (key[1:] != key[:-1]) | is_long[1:] | is_long[:-1]
         return bnd, is_long, int(bnd.sum() - is_long.sum() + ((deg[is_long] + long_row - 1) // long_row).sum())
 
-    split = bool((deg > max(64, nnz // spmm_warps(nvec, False))).any())
-    warps = spmm_warps(nvec, split or one_shape)
+    split = bool((deg > max(64, nnz // spmm_warps(nvec, False, nb))).any())
+    warps = spmm_warps(nvec, split or one_shape, nb)
     if nnz < 120_000 or not split:
         buckets = build_spmm_items(rowptr)   # buckets of whole quads, where they fit the warps as they are
         n = buckets[0].shape[0]
@@ -206,7 +212,7 @@ def fit_spmm_items(rowptr: np.ndarray, nvec: int, one_shape: bool = False):
         rounds += 1
     # the weight that makes `target` items: a first guess, corrected by what it makes beyond one per `w` nonzeros
     target = warps * rounds
-    least = max(32 if nvec > 32 else 64, int(deg.max()) // 2000 + 1)   # (at most 2^11 - 1 pieces a row)
+    least = max(32 if nvec * nb > 512 else 64, int(deg.max()) // 2000 + 1)   # (at most 2^11 - 1 pieces a row)
     w, low, high = max(16, int(nnz / (target - nrows / 32))), 0, 0   # low: too many items, high: not too many
     for _ in range(14):
         long_row = max(least, w)
@@ -319,13 +325,14 @@ class SpmmSchedule:
     """Device-resident SpMM work items plus the scratch the long-row path
     needs: one carry row per piece and one counter per long row."""
 
-    def __init__(self, rowptr: torch.Tensor, k_max: int = 0, dtype=torch.float32, arrays=None, nvec: int = 0, **kw):
-        """`nvec`: 16-byte vectors of a dense row, where the items may be made for one width (see `fit_spmm_items`)."""
+    def __init__(self, rowptr: torch.Tensor, k_max: int = 0, dtype=torch.float32, arrays=None, nvec: int = 0, nb: int = 16,
+                 **kw):
+        """`nvec`, `nb`: vectors of a dense row and their bytes, where the items may be made for one width (`fit_spmm_items`)."""
         if arrays is None:
             rp = rowptr.cpu().numpy()
             if 0 < nvec <= 256 and 0 < rp[-1] <= SMALL_NNZ and not kw and not any(
                     v in os.environ for v in ("SP3_LONG_ROW", "SP3_ITEM_NNZ", "SP3_ITEM_ROWS")):
-                items, first, npieces = fit_spmm_items(rp, nvec)
+                items, first, npieces = fit_spmm_items(rp, nvec, nb=nb)
             else:
                 items, first, npieces = build_spmm_items(rp, **kw)
         else:   # (items, first_piece, npieces) built elsewhere, e.g. by build_spmm_wave_items
@@ -496,6 +503,17 @@ def _packed(t):
     nvec = -(-k // per)
     full = torch.empty(n, nvec * per, dtype=t.dtype, device=t.device)
     return full, _PackRows(native.ptr(t), _ld(t), native.ptr(full), n, k, nvec)
+
+
+def spmm_row_vectors(nnz, rows, k, es, device):
+    """(vectors, bytes of one) that the SpMM reads its rows of X in: as `vector_bytes` of csrc/kernels/local_ops.cu cuts
+    contiguous rows of k values of `es` bytes, whole 16-byte vectors where they are packed first."""
+    if pack_rule("spmm", nnz, rows, k, es, device):
+        return -(-k * es // 16), 16
+    nb = 16
+    while nb > es and (k * es % nb or k * es // nb <= 2):
+        nb //= 2
+    return k * es // nb, nb
 
 
 def bind_sddmm(rowidx, colidx, svals, A, B, out, also=None, chunks=None, pack=None):
