@@ -22,7 +22,7 @@ namespace sp3 {
 // warps stride over windows of nonzeros (see sddmm_windows), or take one each.
 // ---------------------------------------------------------------------------
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
-__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4, NB, G))
 sddmm_vec_kernel(long long nnz, int wn, const int* rowidx, const int* colidx,
                  const Rows arows, const char* B, unsigned ldb_bytes, int nvec, bool aligned,
                  const Store store) {
@@ -30,20 +30,20 @@ sddmm_vec_kernel(long long nnz, int wn, const int* rowidx, const int* colidx,
     __shared__ __align__(16) WindowLists<T> lists[256 / 32];
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    sddmm_windows<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
+    sddmm_windows<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4, NB), EXACT>(warp0, nwarps, (nnz + wn - 1) / wn, wn, nnz, rowidx, colidx,
                                                       arows, B, ldb_bytes, nvec, aligned, store, lists[threadIdx.x >> 5],
                                                       threadIdx.x & 31);
 }
 
 // One window per warp (see sddmm_window).
 template <typename T, int NB, int G, int R, bool EXACT, typename Rows, typename Store>
-__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4))
+__global__ void __launch_bounds__(256, sddmm_min_blocks(R, sizeof(T) == 4, NB, G))
 sddmm_once_kernel(long long nnz, int wn, const int* rowidx, const int* colidx, const Rows arows, const char* B,
                   unsigned ldb_bytes, int nvec, bool aligned, const Store store) {
     after_previous_kernel();
     __shared__ int4 cols[256 / 32][WINDOW_MAX / 4], rows[256 / 32][WINDOW_MAX / 4];
     const int warp = threadIdx.x >> 5;
-    sddmm_window<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4), EXACT>((long long)blockIdx.x * (256 / 32) + warp, wn, nnz, rowidx, colidx,
+    sddmm_window<T, NB, G, R, sddmm_unroll(R, sizeof(T) == 4, NB), EXACT>((long long)blockIdx.x * (256 / 32) + warp, wn, nnz, rowidx, colidx,
                                                                       arows, B, ldb_bytes, nvec, aligned, store, cols[warp],
                                                                       rows[warp], threadIdx.x & 31);
 }
@@ -319,7 +319,14 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
     arows.base = A;
     arows.ld_bytes = (unsigned)lda_bytes;
     int G, R;
-    pick_shape(nvec, &G, &R, false);
+    pick_shape(nvec, &G, &R, false, false, NB < 16);
+    // One value per vector: five per lane where that takes half the lanes of three, for two nonzeros an instruction instead of
+    // one (R-MAT scale 14, k = 75 16.5 -> 12.7 us, fp64 k = 75 22 -> 17; k = 33 1.12 times, Erdos-Renyi 100 thousand rows,
+    // fp64, k = 75 1.42); six with fp64 only (k = 85, fp32 5 % slower), eight never (k = 51, fp64 0.68 times).
+    if (NB == sizeof(T) && ((nvec > 32 && nvec <= 40) || (nvec > 64 && nvec <= (sizeof(T) == 8 ? 96 : 80)))) {
+        G = nvec <= 40 ? 8 : 16;
+        R = (nvec + G - 1) / G;
+    }
     const bool exact = NB == 16 && nvec == G * R;
     // One window per warp, but for three narrow vectors of fp32 per lane (odd rows of 33 to 96 values, others of 66 to 190)
     // with windows of more than 16 nonzeros: Zipf rows, 107 thousand nonzeros, k = 47, 6.8 us with sddmm_windows, 7.4 with sddmm_window; R-MAT scale
@@ -340,6 +347,17 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
                                : sddmm_once_kernel<T, NB, GG, RR, false, Rows, Store>;                        \
         launch_early(kernel, needed < all ? (unsigned)needed : all, 0, st, nnz, wn, ri, ci, arows, B,               \
                      (unsigned)ldb_bytes, nvec, aligned, store);                                              \
+    }
+    if constexpr (NB < 16) {
+        if (G == 32 && R == 5) { SP3_SDDMM(32, 5); return (int)cudaGetLastError(); }
+        if (G == 32 && R == 6) { SP3_SDDMM(32, 6); return (int)cudaGetLastError(); }
+    }
+    if constexpr (NB == sizeof(T)) {
+        if (G == 8 && R == 5) { SP3_SDDMM(8, 5); return (int)cudaGetLastError(); }
+        if (G == 16 && R == 5) { SP3_SDDMM(16, 5); return (int)cudaGetLastError(); }
+        if constexpr (sizeof(T) == 8) {
+            if (G == 16 && R == 6) { SP3_SDDMM(16, 6); return (int)cudaGetLastError(); }
+        }
     }
     SP3_SDDMM_SHAPES(SP3_SDDMM)
 #undef SP3_SDDMM
@@ -394,8 +412,14 @@ template <typename T, int NB, int G, int R, bool EXACT, typename Emit> unsigned 
     static ResidentCache cache;
     return resident_blocks(spmm_items_kernel<T, NB, G, R, EXACT, Emit>, cache, needed);
 }
-// the shapes of pick_shape and the one that only small products take
-#define SP3_SPMM_LOCAL_SHAPES(MACRO) if (G == 32 && R == 2) MACRO(32, 2); else SP3_SPMM_SHAPES(MACRO)
+// the shapes of pick_shape, those of narrow rows and the one that only small products take
+#define SP3_SPMM_LOCAL_SHAPES(MACRO)                                                                      \
+    if constexpr (NB < 16) {                                                                              \
+        if (G == 32 && R == 5) { MACRO(32, 5); }                                                          \
+        if (G == 32 && R == 6) { MACRO(32, 6); }                                                          \
+    }                                                                                                     \
+    if (G == 32 && R == 2) { MACRO(32, 2); }                                                              \
+    else if (R != 5 && R != 6) SP3_SPMM_SHAPES(MACRO)
 // nnz: 0 where it is not known
 template <typename T, int NB, typename Emit>
 int launch_spmm_nb(int nrows, long long nnz, int nitems, const int4* items, const long long* rowptr, const int* ci, const T* val,
@@ -404,7 +428,7 @@ int launch_spmm_nb(int nrows, long long nnz, int nitems, const int4* items, cons
     const bool aligned = ((uintptr_t)ci | (uintptr_t)val) % 16 == 0;
     constexpr bool VECTORS = std::is_same<Emit, EmitLocal<T, NB>>::value;
     int G, R;
-    pick_shape(nvec, &G, &R, true, cached);
+    pick_shape(nvec, &G, &R, true, cached, NB < 16);
     // Warps that are resident at once in a shape, at most `needed` blocks of them.
     auto blocks = [&](int G, int R, long long needed) {
         unsigned b = 0;

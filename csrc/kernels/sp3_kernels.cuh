@@ -111,7 +111,7 @@ __device__ __forceinline__ T row_dot(const Row<T, NB> (&a)[R], const Row<T, NB> 
     E s = 0;
 #pragma unroll
     for (int q = 0; q < R; ++q)
-        if (ALL || (q < R - 1 && R <= 4) || on[q])   // (pick_shape: only the last vector of a lane can be past the row)
+        if (ALL || (q < R - 1 && R < 8) || on[q])   // (pick_shape: only the last vector of a lane can be past the row, but for R = 8)
 #pragma unroll
             for (int h = 0; h < Row<T, NB>::N; ++h) s = e_fma(a[q].x[h], b[q].x[h], s);
     if constexpr (sizeof(E) == 8 && sizeof(T) == 4) {
@@ -679,7 +679,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
 #pragma unroll
     for (int q = 0; q < R; ++q) {   // lanes past the row's last vector read it too and emit nothing
         const int v = gl + q * G;
-        on[q] = EXACT || (q < R - 1 && R <= 4) || v < nvec;   // (pick_shape: only a lane's last vector can be past the row)
+        on[q] = EXACT || (q < R - 1 && R < 8) || v < nvec;   // (see row_dot)
         off[q] = (unsigned)(on[q] ? v : nvec - 1) * NB;
     }
     X += off[0];
@@ -690,7 +690,7 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
     auto flush = [&](int row, const Row<T, NB> (&v)[R]) {
 #pragma unroll
         for (int q = 0; q < R; ++q)
-            if ((q < R - 1 && R <= 4) || on[q]) emit(row, gl + q * G, v[q]);
+            if ((q < R - 1 && R < 8) || on[q]) emit(row, gl + q * G, v[q]);
     };
     const bool is_piece = item.w >= 0, is_rows = !is_piece && item.y - item.x > 1;   // else: one whole row
     const int nr = item.y - item.x;
@@ -913,10 +913,16 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
 // than these spill registers in the inner loops.  What counts in the SpMM is the bytes of a lane: three or four vectors of 4
 // bytes take the registers of one of 16, and in the blocks that three or four wide ones leave they have a quarter of the
 // bytes in flight (k = 75, R-MAT scale 14 22.5 us in two blocks, 16.9 in four; k = 101 18.9 and 16.1; R-MAT scale 16 5 %
-// less).  (The SDDMM gains nothing: level over 91 odd widths, 18 % either way.)
+// less).  In the SDDMM that pays for rows of 16 lanes and more (8-byte vectors, k = 90, 126, 178 7 to 11 %; rows of 8 lanes
+// level, 15 % either way) and for five vectors and more.
 __host__ __device__ constexpr int spmm_unroll(int R, int NB = 16) { return R * NB <= 64 ? 4 : 1; }
-__host__ __device__ constexpr int sddmm_unroll(int R, bool f32) { return R <= (f32 ? 4 : 3) ? 4 : 2; }
-__host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32) { return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 ? 2 : 1)); }
+__host__ __device__ constexpr int sddmm_unroll(int R, bool f32, int NB = 16) {
+    return R <= (f32 ? 4 : 3) || (NB < 16 && R * NB <= 48) ? 4 : 2;
+}
+__host__ __device__ constexpr int sddmm_min_blocks(int R, bool f32, int NB = 16, int G = 32) {
+    if (NB < 16 && R > 2 && R <= 4 && G >= 16 && f32) return R * NB <= 16 ? 4 : 3;
+    return R == 1 ? 4 : (R == 2 && f32 ? 3 : (R <= 4 || R * NB <= 48 ? 2 : 1));
+}
 __host__ __device__ constexpr int spmm_min_blocks(int R, int NB = 16) { return R * NB <= 16 ? 4 : (R * NB <= 32 ? 3 : 2); }
 
 // All items of an SpMM, by block `block` of `nblocks` blocks of 256 threads that do so (every one of them calls it).
@@ -1032,7 +1038,10 @@ unsigned resident_blocks(K kernel, ResidentCache& cache, long long needed, int t
 //          48 as 16 x 3 (k = 192: 110 us, 140 as 32 x 2), and groups of 5, 6 and 10 lanes share a warp one group more than
 //          8 or 16 do (k = 40: 41 us as 10 x 1, 51 as 16 x 1; k = 20: 32 against 35 us; groups of 2 and 3 gained nothing
 //          over 4).
-inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false) {
+//
+// 129 to 192 vectors narrower than 16 bytes (`narrow`) go as 32 x 5 and 32 x 6; wider rows take eight per lane, where up to
+// three read the last vector again.
+inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false, bool narrow = false) {
     int g = 4;
     const int top = spmm ? 32 : (nvec <= 32 ? 8 : (nvec <= 64 ? 16 : 32));
     while (g < top && g < nvec) g <<= 1;
@@ -1046,7 +1055,7 @@ inline void pick_shape(int nvec, int* G, int* R, bool spmm, bool cached = false)
         g = 4;
     }
     int r = (nvec + g - 1) / g;
-    r = r <= 4 ? r : 8;
+    r = r <= (narrow ? 6 : 4) ? r : 8;
     *G = g;
     *R = r;
 }

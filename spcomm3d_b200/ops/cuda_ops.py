@@ -168,7 +168,7 @@ def spmm_warps(nvec: int, split: bool, nb: int = 16) -> int:
         g = (8 if 10 < nvec <= 32 else 16 if 32 < nvec <= 64 else
              next((g for g in (4, 5, 6, 8, 10, 16) if g >= nvec), 32))
         r = -(-nvec // g)
-        r = r if r <= 4 else 8
+        r = r if r <= (4 if nb == 16 else 6) else 8
     else:
         r = 1 if nvec <= 32 else 2
     return 148 * 8 * (4 if r * nb <= 16 else 3 if r * nb <= 32 else 2)
@@ -477,23 +477,37 @@ def pack_rule(kernel, nnz, rows, k, es, device):
     vectors.  Operands are what the user sees, contiguous; rows that are no multiple of 16 bytes are otherwise read 8 or
     4 bytes at a time.
 
-    The kernel gains with every narrow vector it does not read (0.3 to 0.6 ps each), the copy costs two passes over the
-    rows (0.3 ps a byte): the line lies at 0.7 vectors saved per byte copied.  Measured (copied / as they are):
-      R-MAT scale 20, SpMM      k = 33 358 / 571 us (1.7 per byte), k = 50 462 / 529 (0.9), k = 126 876 / 850 (0.9)
-      R-MAT scale 20, SDDMM     k = 33 374 / 432 (1.4), k = 50 474 / 438 (0.4), k = 99 830 / 1161 (1.4)
-      R-MAT scale 17, SpMM, beta k = 33 62 / 85; scale 18, 8 a row, k = 34 73 / 61 (0.45)
-      Erdos-Renyi 300 thousand rows, 24 a row, SDDMM, k = 70 268 / 327 (0.73), k = 50 193 / 186 (0.72)
-    Small products do not pay for the launch (scale 14, k = 50: SDDMM 17 / 11, SpMM 17 / 14), nor do narrow rows, where
-    the SpMM gains nothing from wide vectors (scale 20, k = 10: 216 / 176)."""
-    row_bytes = k * es
-    if row_bytes % 16 == 0 or row_bytes > 256 * 16 or row_bytes < (128 if kernel == "spmm" else 16):
+    The copy is two passes over the rows, and the kernels lose little to narrow vectors, so that it pays only where every
+    row is read often (vectors saved per byte copied, as they are / copied, us):
+      4 bytes, SpMM from 6 on        uniform 200 thousand rows of 40 (7.4) k = 53 171 / 158, k = 127 393 / 330; Erdos-Renyi 100
+                                     thousand rows of 20 (3.7) k = 53 52 / 57, k = 101 79 / 99; R-MAT scale 17 (2.8) k = 75 78 / 82
+      4 bytes, SDDMM from 3 on       the first of these (3.7) k = 53 189 / 157, k = 101 373 / 332; the second (1.9) k = 75 67 / 77,
+                                     k = 127 102 / 94; R-MAT scale 17 (1.4) k = 51 57 / 67, k = 101 119 / 106
+      4 bytes, few and large         R-MAT scale 20, k = 33 SpMM 339 / 322, SDDMM 323 / 356; Erdos-Renyi 1 M rows 511 / 504, 566 / 511
+      8 bytes, 25 to 32 vectors      uniform 200 thousand rows of 40, k = 62 SpMM (2.4) 172 / 155, SDDMM (1.2) 184 / 150; R-MAT scale
+                                     18, k = 50 SpMM (0.9) 94 / 110, SDDMM (0.5) 106 / 114; others (k = 42, 90, 126) 5 to 15 % slower
+      fp64                           the first of these, SpMM k = 75 485 / 544, SDDMM k = 75 463 / 562 (k = 51 359 / 320)
+      193 to 256 vectors of 4 bytes, SpMM (lanes read the last one more than once), k = 201  R-MAT scale 14 23.5 / 28.6, 17 198 / 165
+    Past 256 narrow vectors the kernels left cut no rows (SpMM, R-MAT scale 12, k = 259: 378 us, packed 16; 4000 nonzeros of
+    even rows: 6.5 and 10) and a nonzero takes a warp (SDDMM: with 0.7 vectors saved per byte copied)."""
+    row_bytes, spmm = k * es, kernel == "spmm"
+    if row_bytes % 16 == 0 or row_bytes > 256 * 16:
         return False
     narrow = row_bytes // (8 if row_bytes % 8 == 0 else 4)
-    saved = narrow - -(-row_bytes // 16)
-    pays = nnz * saved >= max(PACK_MIN_WORK, 7 * row_bytes * rows // 10)
-    # past 256 narrow vectors the SpMM is left with a kernel that cuts no rows (R-MAT scale 12, k = 259: 378 us, packed
-    # 16; 4000 nonzeros of even rows: 6.5 and 10)
-    return (pays or kernel == "spmm" and narrow > 256) and has_room(rows * (row_bytes + 16), device)
+    saved = nnz * (narrow - -(-row_bytes // 16))
+    per_byte = saved / (row_bytes * rows)
+    if narrow > 256:
+        pays = spmm or saved >= PACK_MIN_WORK and per_byte >= 0.7
+    elif es == 8 or narrow <= 16:
+        pays = False
+    elif row_bytes % 8 == 0:
+        pays = 24 < narrow <= 32 and (saved >= 90_000_000 and per_byte >= 2.4 if spmm else saved >= PACK_MIN_WORK and per_byte >= 1.1)
+    elif narrow <= 128:
+        pays = saved >= 90_000_000 and per_byte >= 6 if spmm else saved >= 45_000_000 and per_byte >= 3
+        pays = pays or narrow <= 40 and saved >= 350_000_000 and per_byte >= (2.6 if spmm else 1.3)
+    else:
+        pays = spmm and narrow > 192 and saved >= 130_000_000 and per_byte >= 2
+    return bool(pays) and has_room(rows * (row_bytes + 16), device)
 
 
 def _packed(t):

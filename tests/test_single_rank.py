@@ -712,3 +712,25 @@ def test_spmm_with_fitted_items(gen, vectors, beta):
     ref = _product(plan, vals, X) + beta * old.double()
     bound = torch.from_numpy(_gamma(deg + 4.0, dtype))[:, None] * (_product(plan, vals.abs(), X.abs()) + beta * old.double().abs())
     assert bool(((y - ref).abs() <= bound).all())
+
+
+# Rows of an odd number of values at the edges of the shapes that narrow vectors take (five, six and eight per lane), one
+# window per warp and several, items of one round, split rows.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gen", ["uniform:300:200:7", "rmat:14:24", "zipf:3000:9000:1.8:2000"])
+@pytest.mark.parametrize("k", [33, 39, 41, 65, 79, 81, 95, 97, 129, 159, 161, 191, 193, 255, 258, 318])
+def test_odd_rows(k, gen, dtype):
+    from spcomm3d_b200.models.layer import SddmmSpmmStep
+    plan = _plan(gen)
+    vals = torch.from_numpy(plan.vals).to(dtype)
+    step = SddmmSpmmStep(plan, None, k, dtype, "cuda", seed=2)
+    step.fill_device_operands()
+    sd, sp = step.sddmm, step.spmm
+    sd.partial.fill_(float("nan")), sp.Y_owned.fill_(float("nan"))
+    c, y = step.run_device()
+    A, B = sd.A_owned.cpu(), sd.B_owned.cpu()
+    ref, mag = _scores(plan, A, B, vals)
+    assert bool(((c.cpu().double() - ref).abs() <= _gamma(k + 2, dtype) * mag).all())
+    bound = torch.from_numpy(_gamma(_lists(plan)[2].numpy() + 3.0, dtype))[:, None] * _product(plan, vals.abs(), B.abs())
+    assert bool(((y.cpu().double() - _product(plan, vals, B)).abs() <= bound).all())
