@@ -321,7 +321,7 @@ int launch_sddmm_nb(long long nnz, const int* ri, const int* ci, const char* A, 
     int G, R;
     pick_shape(nvec, &G, &R, false, false, NB < 16);
     // One value per vector: five per lane where that takes half the lanes of three, for two nonzeros an instruction instead of
-    // one (R-MAT scale 14, k = 75 16.5 -> 12.7 us, fp64 k = 75 22 -> 17; k = 33 1.12 times, Erdos-Renyi 100 thousand rows,
+    // one (R-MAT scale 14, k = 75 16.5 -> 12.6 us, fp64 k = 75 22 -> 17; k = 33 1.12 times, Erdos-Renyi 100 thousand rows,
     // fp64, k = 75 1.42); six with fp64 only (k = 85, fp32 5 % slower), eight never (k = 51, fp64 0.68 times).
     if (NB == sizeof(T) && ((nvec > 32 && nvec <= 40) || (nvec > 64 && nvec <= (sizeof(T) == 8 ? 96 : 80)))) {
         G = nvec <= 40 ? 8 : 16;

@@ -912,8 +912,8 @@ __device__ __forceinline__ void spmm_warp_item(const int4 item, const long long*
 // half of the registers belong to loads in flight; more would halve the warps, fewer leave the memory idle.  More blocks
 // than these spill registers in the inner loops.  What counts in the SpMM is the bytes of a lane: three or four vectors of 4
 // bytes take the registers of one of 16, and in the blocks that three or four wide ones leave they have a quarter of the
-// bytes in flight (k = 75, R-MAT scale 14 22.5 us in two blocks, 16.9 in four; k = 101 18.9 and 16.1; R-MAT scale 16 5 %
-// less).  In the SDDMM that pays for rows of 16 lanes and more (8-byte vectors, k = 90, 126, 178 7 to 11 %; rows of 8 lanes
+// bytes in flight (SpMM, R-MAT scale 14, items fitted to the warps of each: k = 75 22.5 us in two blocks, 13.3 in four;
+// k = 101 24.2 and 14.8; scale 16 5 % less).  In the SDDMM that pays for rows of 16 lanes and more (8-byte vectors, k = 90, 126, 178 7 to 11 %; rows of 8 lanes
 // level, 15 % either way) and for five vectors and more.
 __host__ __device__ constexpr int spmm_unroll(int R, int NB = 16) { return R * NB <= 64 ? 4 : 1; }
 __host__ __device__ constexpr int sddmm_unroll(int R, bool f32, int NB = 16) {
